@@ -964,7 +964,7 @@ int launch_tc(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_
   const long long items = SPLIT ? static_cast<long long>(n_blocks) * chunks : static_cast<long long>(n_blocks) * m_blocks;
   if (PAIR) {
     const unsigned pairs = static_cast<unsigned>(items < max_pairs ? items : max_pairs);
-    bw::launch_pdl_cluster2(kernel, dim3(2 * pairs), dim3(threads), smem, stream, map_x, map_w, y, y_is_f32, residual, m,
+    bw::launch_pdl_cluster(2, kernel, dim3(2 * pairs), dim3(threads), smem, stream, map_x, map_w, y, y_is_f32, residual, m,
                             n, k, error_word, partials, bn, GroupItems{nullptr, nullptr, 0});
     return bw::launch_status();
   }

@@ -1,5 +1,5 @@
-// Kernels that both precisions share: embedding gather into the 32-bit residual stream,
-// sampling from 32-bit logits, and the logits fingerprint.
+// Kernels that both precisions share: embedding gather into the 32-bit residual stream and the
+// logits fingerprint.
 #include <cstdarg>
 #include <cstdio>
 
@@ -126,118 +126,6 @@ __global__ void patch_tokens_kernel(int* __restrict__ tokens, const int* __restr
 BW_API int bw_patch_tokens(int* tokens, const int* rows, const int* src, const int* values, int count, cudaStream_t stream) {
   if (count <= 0) return 0;
   bw::launch_pdl(patch_tokens_kernel, dim3((count + 127) / 128), dim3(128), 0, stream, tokens, rows, src, values, count);
-  return bw::launch_status();
-}
-
-// ---------------------------------------------------------------------------------------
-// Sampling. One block per logits row.
-//   temperature <= 0: the first index of the maximum (src/engine.cpp:40-45).
-//   otherwise: w_i = exp((l_i - max) / T) in 32-bit, total and running sums in 64-bit in
-//   vocabulary order, the first i with cum > u * total, skipping w_i <= 0, else the last
-//   positive one (src/engine.cpp:50-80).  The 64-bit sums are formed per contiguous
-//   segment of the vocabulary (one per thread) and chained over the segments in order; the
-//   reference adds strictly one by one, which differs from this by 64-bit rounding only.
-constexpr int kSampleThreads = 512;
-
-__global__ void __launch_bounds__(kSampleThreads)
-sample_rows_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
-                   const double* __restrict__ uniform, int* __restrict__ out_token) {
-  bw::pdl_enter();
-  const int row = blockIdx.x;
-  const float* l = logits + static_cast<size_t>(row) * vocab;
-  const int tid = threadIdx.x;
-  __shared__ float s_val[kSampleThreads];
-  __shared__ int s_idx[kSampleThreads];
-  __shared__ double s_sum[kSampleThreads];
-  __shared__ double s_total;
-  __shared__ int s_pick;
-  __shared__ int s_last;
-
-  // maximum and its first index
-  float best = -INFINITY;
-  int best_i = -1;
-  for (int i = tid; i < vocab; i += kSampleThreads) {
-    const float v = l[i];
-    if (best_i < 0 || v > best) {  // indices come in increasing order: ">" keeps the first maximum
-      best = v;
-      best_i = i;
-    }
-  }
-  s_val[tid] = best;
-  s_idx[tid] = best_i;
-  __syncthreads();
-  for (int s = kSampleThreads / 2; s > 0; s >>= 1) {
-    if (tid < s) {
-      const float ov = s_val[tid + s];
-      const int oi = s_idx[tid + s];
-      const int mi = s_idx[tid];
-      if (oi >= 0 && (mi < 0 || ov > s_val[tid] || (ov == s_val[tid] && oi < mi))) {
-        s_val[tid] = ov;
-        s_idx[tid] = oi;
-      }
-    }
-    __syncthreads();
-  }
-  const float mx = s_val[0];
-  const int arg = s_idx[0];
-  __syncthreads();  // s_idx is reused below
-  const float temp = temperature[row];
-  if (!(temp > 0.0f)) {
-    if (tid == 0) out_token[row] = arg;
-    return;
-  }
-
-  // contiguous segment of this thread
-  const int seg = (vocab + kSampleThreads - 1) / kSampleThreads;
-  const int lo = min(vocab, tid * seg), hi = min(vocab, lo + seg);
-  double local = 0.0;
-  int last_pos = -1;
-  for (int i = lo; i < hi; ++i) {
-    const float w = bw::det_expf(__fdiv_rn(__fsub_rn(l[i], mx), temp));
-    if (w > 0.0f) last_pos = i;
-    local += static_cast<double>(w);
-  }
-  s_sum[tid] = local;
-  s_idx[tid] = last_pos;
-  if (tid == 0) s_pick = 0x7fffffff;
-  __syncthreads();
-  if (tid == 0) {  // exclusive prefix over segments, in order
-    double run = 0.0;
-    int lastp = 0;
-    for (int t = 0; t < kSampleThreads; ++t) {
-      const double v = s_sum[t];
-      s_sum[t] = run;
-      run += v;
-      if (s_idx[t] >= 0) lastp = s_idx[t];
-    }
-    s_last = lastp;
-    s_total = run;
-  }
-  __syncthreads();
-  const double total = s_total;
-  const double target = uniform[row] * total;
-  double cum = s_sum[tid];
-  for (int i = lo; i < hi; ++i) {
-    const float w = bw::det_expf(__fdiv_rn(__fsub_rn(l[i], mx), temp));
-    if (w <= 0.0f) continue;
-    cum += static_cast<double>(w);
-    if (cum > target) {
-      atomicMin(&s_pick, i);
-      break;
-    }
-  }
-  __syncthreads();
-  if (tid == 0) out_token[row] = (s_pick != 0x7fffffff) ? s_pick : s_last;
-}
-
-BW_API int bw_sample_rows(const float* logits, int rows, int vocab, const float* temperature,
-                          const double* uniform, int* out_token, cudaStream_t stream) {
-  if (rows <= 0) return 0;
-  if (vocab <= 0) {
-    bw::set_error("sample_rows: vocabulary size %d", vocab);
-    return -1;
-  }
-  bw::launch_pdl(sample_rows_kernel, dim3(rows), dim3(kSampleThreads), 0, stream, logits, vocab, temperature, uniform, out_token);
   return bw::launch_status();
 }
 

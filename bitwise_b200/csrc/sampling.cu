@@ -1,0 +1,309 @@
+// Sampling from 32-bit logits, for both precisions.
+#include "bw_common.cuh"
+
+// ---------------------------------------------------------------------------------------
+// Sampling. One block per logits row.
+//   temperature <= 0: the first index of the maximum (src/engine.cpp:40-45).
+//   otherwise: w_i = exp((l_i - max) / T) in 32-bit, total and running sums in 64-bit in
+//   vocabulary order, the first i with cum > u * total, skipping w_i <= 0, else the last
+//   positive one (src/engine.cpp:50-80).  The 64-bit sums are formed per contiguous
+//   segment of the vocabulary (one per thread) and chained over the segments in order; the
+//   reference adds strictly one by one, which differs from this by 64-bit rounding only.
+constexpr int kSampleThreads = 512;
+
+__global__ void __launch_bounds__(kSampleThreads)
+sample_rows_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
+                   const double* __restrict__ uniform, int* __restrict__ out_token) {
+  bw::pdl_enter();
+  const int row = blockIdx.x;
+  const float* l = logits + static_cast<size_t>(row) * vocab;
+  const int tid = threadIdx.x;
+  __shared__ float s_val[kSampleThreads];
+  __shared__ int s_idx[kSampleThreads];
+  __shared__ double s_sum[kSampleThreads];
+  __shared__ double s_total;
+  __shared__ int s_pick;
+  __shared__ int s_last;
+
+  // maximum and its first index
+  float best = -INFINITY;
+  int best_i = -1;
+  for (int i = tid; i < vocab; i += kSampleThreads) {
+    const float v = l[i];
+    if (best_i < 0 || v > best) {  // indices come in increasing order: ">" keeps the first maximum
+      best = v;
+      best_i = i;
+    }
+  }
+  s_val[tid] = best;
+  s_idx[tid] = best_i;
+  __syncthreads();
+  for (int s = kSampleThreads / 2; s > 0; s >>= 1) {
+    if (tid < s) {
+      const float ov = s_val[tid + s];
+      const int oi = s_idx[tid + s];
+      const int mi = s_idx[tid];
+      if (oi >= 0 && (mi < 0 || ov > s_val[tid] || (ov == s_val[tid] && oi < mi))) {
+        s_val[tid] = ov;
+        s_idx[tid] = oi;
+      }
+    }
+    __syncthreads();
+  }
+  const float mx = s_val[0];
+  const int arg = s_idx[0];
+  __syncthreads();  // s_idx is reused below
+  const float temp = temperature[row];
+  if (!(temp > 0.0f)) {
+    if (tid == 0) out_token[row] = arg;
+    return;
+  }
+
+  // contiguous segment of this thread
+  const int seg = (vocab + kSampleThreads - 1) / kSampleThreads;
+  const int lo = min(vocab, tid * seg), hi = min(vocab, lo + seg);
+  double local = 0.0;
+  int last_pos = -1;
+  for (int i = lo; i < hi; ++i) {
+    const float w = bw::det_expf(__fdiv_rn(__fsub_rn(l[i], mx), temp));
+    if (w > 0.0f) last_pos = i;
+    local += static_cast<double>(w);
+  }
+  s_sum[tid] = local;
+  s_idx[tid] = last_pos;
+  if (tid == 0) s_pick = 0x7fffffff;
+  __syncthreads();
+  if (tid == 0) {  // exclusive prefix over segments, in order
+    double run = 0.0;
+    int lastp = 0;
+    for (int t = 0; t < kSampleThreads; ++t) {
+      const double v = s_sum[t];
+      s_sum[t] = run;
+      run += v;
+      if (s_idx[t] >= 0) lastp = s_idx[t];
+    }
+    s_last = lastp;
+    s_total = run;
+  }
+  __syncthreads();
+  const double total = s_total;
+  const double target = uniform[row] * total;
+  double cum = s_sum[tid];
+  for (int i = lo; i < hi; ++i) {
+    const float w = bw::det_expf(__fdiv_rn(__fsub_rn(l[i], mx), temp));
+    if (w <= 0.0f) continue;
+    cum += static_cast<double>(w);
+    if (cum > target) {
+      atomicMin(&s_pick, i);
+      break;
+    }
+  }
+  __syncthreads();
+  if (tid == 0) out_token[row] = (s_pick != 0x7fffffff) ? s_pick : s_last;
+}
+
+// The same for larger vocabularies, a cluster of eight blocks per row. A row is a stream of logits with two short serial
+// parts (the 64-bit sums within a segment, and over the segments); one block per row spent its time on strided reads of
+// 1 KB segments by 512 threads and on computing every weight twice with few warps to hide it. Each block of the cluster
+// brings the logits of 64 of the 512 segments into shared memory with coalesced reads, forms the weights in place with all
+// its threads, and one thread per segment walks them there. Segments, weights and the order of every 64-bit sum are those
+// of the kernel above, so the tokens are the same. A segment's row in shared memory has an odd length: the 64 threads that
+// walk one each meet in no bank. Head and sampler together for 64 rows of 128,256 logits, half of them greedy: 550 us with
+// the kernel above, 279 us with this one (the product alone takes most of the rest).
+constexpr int kSampleBlocks = 8, kSampleBlockThreads = 256, kSegmentsPerBlock = kSampleThreads / kSampleBlocks;
+
+__device__ __forceinline__ void sample_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// the address of a shared-memory location in the block of the given rank, and reads through it
+__device__ __forceinline__ uint32_t sample_peer(const void* p, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ int sample_peer_int(const int* p, uint32_t rank) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(sample_peer(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float sample_peer_float(const float* p, uint32_t rank) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(sample_peer(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ double sample_peer_double(const double* p, uint32_t rank) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(sample_peer(p, rank)) : "memory");
+  return v;
+}
+// whether candidate (v, i) comes before (best, best_i): larger, or as large and earlier; index -1 is no candidate
+__device__ __forceinline__ bool sample_better(float v, int i, float best, int best_i) {
+  return i >= 0 && (best_i < 0 || v > best || (v == best && i < best_i));
+}
+
+__global__ void __launch_bounds__(kSampleBlockThreads)
+sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
+                           const double* __restrict__ uniform, int* __restrict__ out_token) {
+  extern __shared__ float seg_values[];  // [kSegmentsPerBlock][seg | 1]
+  constexpr int kWarps = kSampleBlockThreads / 32;
+  __shared__ float w_val[kWarps];
+  __shared__ int w_idx[kWarps];
+  __shared__ float b_val;                         // this block's maximum and its first index
+  __shared__ int b_idx;
+  __shared__ double b_sum[kSegmentsPerBlock];     // this block's segments: sum of weights, last positive index
+  __shared__ int b_last[kSegmentsPerBlock];
+  __shared__ double all_sum[kSampleThreads];      // every segment's: sum, then the sum of those before it
+  __shared__ double total;
+  __shared__ int b_pick;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = blockIdx.x % kSampleBlocks;  // the cluster is eight blocks along x
+  const int row = blockIdx.x / kSampleBlocks;
+  const int seg = (vocab + kSampleThreads - 1) / kSampleThreads, pitch = seg | 1;
+  const float* l = logits + static_cast<size_t>(row) * vocab;
+  const int seg0 = static_cast<int>(rank) * kSegmentsPerBlock;
+  if (tid == 0) b_pick = 0x7fffffff;
+  bw::pdl_enter();
+
+  // the logits of this block's segments, and their maximum
+  float best = -INFINITY;
+  int best_i = -1;
+  for (int s = warp; s < kSegmentsPerBlock; s += kWarps) {
+    const int lo = min(vocab, (seg0 + s) * seg), len = min(vocab, (seg0 + s) * seg + seg) - lo;
+    float* dst = seg_values + s * pitch;
+#pragma unroll 4
+    for (int j = lane; j < len; j += 32) {
+      const float v = l[lo + j];
+      dst[j] = v;
+      if (best_i < 0 || v > best) best = v, best_i = lo + j;  // a lane's indices come in increasing order
+    }
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, best, d);
+    const int oi = __shfl_xor_sync(0xffffffffu, best_i, d);
+    if (sample_better(ov, oi, best, best_i)) best = ov, best_i = oi;
+  }
+  if (lane == 0) w_val[warp] = best, w_idx[warp] = best_i;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < kWarps; ++w)
+      if (sample_better(w_val[w], w_idx[w], best, best_i)) best = w_val[w], best_i = w_idx[w];
+    b_val = best, b_idx = best_i;
+  }
+  sample_cluster_sync();
+  float mx = -INFINITY;
+  int arg = -1;
+#pragma unroll
+  for (int b = 0; b < kSampleBlocks; ++b) {
+    const float v = sample_peer_float(&b_val, b);
+    const int i = sample_peer_int(&b_idx, b);
+    if (sample_better(v, i, mx, arg)) mx = v, arg = i;
+  }
+  const float temp = temperature[row];
+  if (!(temp > 0.0f)) {  // the same for the whole cluster
+    if (rank == 0 && tid == 0) out_token[row] = arg;
+    sample_cluster_sync();  // no block leaves while another may still read its shared memory
+    return;
+  }
+
+  // the weights, in place, then one thread per segment adds its own in order
+  for (int s = warp; s < kSegmentsPerBlock; s += kWarps) {
+    const int lo = min(vocab, (seg0 + s) * seg), len = min(vocab, (seg0 + s) * seg + seg) - lo;
+    float* v = seg_values + s * pitch;
+    for (int j = lane; j < len; j += 32) v[j] = bw::det_expf(__fdiv_rn(__fsub_rn(v[j], mx), temp));
+  }
+  __syncthreads();
+  const int my_lo = tid < kSegmentsPerBlock ? min(vocab, (seg0 + tid) * seg) : 0;
+  const int my_len = tid < kSegmentsPerBlock ? min(vocab, (seg0 + tid) * seg + seg) - my_lo : 0;
+  const float* mine = seg_values + tid * pitch;
+  if (tid < kSegmentsPerBlock) {
+    double local = 0.0;
+    int last_pos = -1;
+#pragma unroll 8
+    for (int j = 0; j < my_len; ++j) {
+      const float w = mine[j];
+      if (w > 0.0f) last_pos = my_lo + j;
+      local += static_cast<double>(w);
+    }
+    b_sum[tid] = local;
+    b_last[tid] = last_pos;
+  }
+  sample_cluster_sync();
+  for (int t = tid; t < kSampleThreads; t += kSampleBlockThreads)
+    all_sum[t] = sample_peer_double(&b_sum[t % kSegmentsPerBlock], t / kSegmentsPerBlock);
+  __syncthreads();
+  if (tid == 0) {  // what lies before every segment, in order
+    double run = 0.0;
+    for (int t = 0; t < kSampleThreads; t += 16) {
+      double v[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) v[e] = all_sum[t + e];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        all_sum[t + e] = run;
+        run += v[e];
+      }
+    }
+    total = run;
+  }
+  __syncthreads();
+  if (tid < kSegmentsPerBlock) {
+    const double target = uniform[row] * total;
+    double cum = all_sum[seg0 + tid];
+    for (int j = 0; j < my_len; ++j) {
+      const float w = mine[j];
+      if (w <= 0.0f) continue;
+      cum += static_cast<double>(w);
+      if (cum > target) {
+        atomicMin(&b_pick, my_lo + j);
+        break;
+      }
+    }
+  }
+  sample_cluster_sync();
+  if (rank == 0 && tid == 0) {
+    int pick = 0x7fffffff;
+    for (int b = 0; b < kSampleBlocks; ++b) pick = min(pick, sample_peer_int(&b_pick, b));
+    if (pick == 0x7fffffff) {  // the uniform number lies at the end: the last positive weight, or index 0
+      pick = 0;
+      for (int t = 0; t < kSampleThreads; ++t) {
+        const int i = sample_peer_int(&b_last[t % kSegmentsPerBlock], t / kSegmentsPerBlock);
+        if (i >= 0) pick = i;
+      }
+    }
+    out_token[row] = pick;
+  }
+  sample_cluster_sync();
+}
+
+BW_API int bw_sample_rows(const float* logits, int rows, int vocab, const float* temperature,
+                          const double* uniform, int* out_token, cudaStream_t stream) {
+  if (rows <= 0) return 0;
+  if (vocab <= 0) {
+    bw::set_error("sample_rows: vocabulary size %d", vocab);
+    return -1;
+  }
+  // A cluster per row from kClusterVocab logits on, as far as the segments fit into shared memory.
+  constexpr int kClusterVocab = 4096, kMaxSmem = 200 * 1024, kMaxDevices = 64;
+  const int seg = (vocab + kSampleThreads - 1) / kSampleThreads;
+  const long long smem = 4ll * kSegmentsPerBlock * (seg | 1);
+  if (vocab >= kClusterVocab && smem <= kMaxSmem && rows <= 0x7fffffff / kSampleBlocks) {
+    static bool configured[kMaxDevices] = {false};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = 0;
+    if (!configured[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(sample_rows_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+      if (e != cudaSuccess) {
+        bw::set_error("sample_rows: cannot raise shared memory: %s", cudaGetErrorString(e));
+        return static_cast<int>(e);
+      }
+      configured[dev] = true;
+    }
+    bw::launch_pdl_cluster(kSampleBlocks, sample_rows_cluster_kernel, dim3(static_cast<unsigned>(rows) * kSampleBlocks),
+                           dim3(kSampleBlockThreads), static_cast<size_t>(smem), stream, logits, vocab, temperature, uniform, out_token);
+    return bw::launch_status();
+  }
+  bw::launch_pdl(sample_rows_kernel, dim3(rows), dim3(kSampleThreads), 0, stream, logits, vocab, temperature, uniform, out_token);
+  return bw::launch_status();
+}

@@ -221,6 +221,28 @@ def test_sample_rows_greedy_and_temperature():
     assert got[0] == 17
 
 
+@pytest.mark.parametrize("vocab", [4095, 4096, 4097, 6143, 32000, 128256])
+def test_sample_rows_over_the_vocabulary(vocab):
+    """Around the size where a row goes to a cluster of blocks, and vocabularies whose segments are of even and odd length or
+    do not fill the last ones: the plain sampler's token, for uniform numbers towards both ends too."""
+    rng = np.random.default_rng(vocab)
+    rows = 7
+    logits = rnd(rng, rows, vocab, scale=3.0)
+    logits[1, vocab - 1] = logits[1, vocab // 2] = 60.0  # tie across segments: the first maximum wins
+    logits[2, :] = -np.inf
+    logits[2, vocab - 2] = 1.0                           # one positive weight
+    logits[3, vocab // 3:] = -np.inf                     # no weight in the last segments
+    temps = np.array([0.0, 0.0, 0.7, 1.5, 0.9, 1.0, 0.02], dtype=np.float32)
+    us = np.array([0.3, 0.1, 0.5, 0.9999999, 0.0, 0.25, 0.77], dtype=np.float64)
+    out = torch.empty(rows, dtype=torch.int32, device=DEV)
+    _ops("bfloat16").sample_rows(t(logits), t(temps), torch.from_numpy(us).to(DEV), out)
+    got = out.cpu().numpy()
+    for r in range(rows):
+        want = P.argmax_row(logits[r]) if temps[r] <= 0 else P.sample_row(logits[r], temps[r], us[r], exp="det")
+        assert got[r] == want, f"row {r}: sampled {got[r]}, plain sampler says {want}"
+    assert got[1] == vocab // 2 and got[2] == vocab - 2
+
+
 def test_fingerprint_rows():
     rng = np.random.default_rng(7)
     for vocab in (256, 385):
