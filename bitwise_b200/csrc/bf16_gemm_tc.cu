@@ -26,6 +26,8 @@
 // memory and the block drains and returns instead of hanging; the host reports the flag.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "bw_common.cuh"
 
 namespace {
@@ -33,7 +35,8 @@ namespace {
 constexpr int BM = 128, BN = 128, BK = 64;  // BN: columns one epilogue thread carries; a wide tile has 2 BN
 constexpr int kChunk = 512;
 constexpr int kTilesPerChunk = kChunk / BK;
-constexpr int kSmemBudget = 200 * 1024;        // ring of stages (plus barriers) per block
+constexpr int kSmemBudget = 192 * 1024;        // ring of stages per block
+constexpr int kStoreBytes = 32 * 128;          // per epilogue warp: 32 rows x 128 bytes on their way to global memory
 
 // The x tile of a stage holds A_ROWS rows: 128 for large batches, fewer for small ones. The
 // tensor core always reads 128 rows; with a shorter tile the rows beyond it are whatever lies
@@ -85,6 +88,17 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // Bounded wait: false when the limit ran out (or another thread of the block already gave up).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* failed) {
   return bw::mbar_wait_bounded(bar, parity, failed);
+}
+
+// One lane of a whole, converged warp. The roles below that hand out copies and MMAs run with all lanes of their warp and
+// let one of them issue: the compiler then knows that the operands are the same for the warp and keeps them in uniform
+// registers, where a lone lane's loop moved every descriptor there instruction by instruction (50 to 100 cycles for each
+// MMA, as many as a 256 x 256 x 16 step of a pair takes). With the epilogues' totals out of local memory beside it,
+// gate/up of 2,048 rows x 4,096 x 28,672: 552 -> 411 us.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -232,18 +246,42 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[32]) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
-// 32-byte accesses: a thread of the epilogue owns a row, so a warp's store touches 32 rows;
-// whole 32-byte sectors keep the memory system from merging partial ones.
-__device__ __forceinline__ void st256(void* p, const uint32_t (&v)[8]) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
-               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+// A warp's 32 rows x 128 bytes (lane i holds row i) turned through shared memory so that eight lanes hold the 128 bytes of a
+// row: 16-byte piece lane % 8 of row 4 t + lane / 8. Accesses straight from the accumulator's layout touch 32 rows per
+// instruction, and residual rows fetched that way wait one by one (the epilogue of a 256 x 256 tile with a residual took
+// about 10 us; turned, down of 2,048 rows x 14,336 x 4,096 went from 248 to 201 us, gate/up from 410 to 331). `buf`: the warp's kStoreBytes, pieces placed by the row's low three bits so that neither side meets in a
+// bank. The accesses are volatile assembly: in the unrolled epilogue the compiler otherwise starts all pieces at once and
+// sends the totals to local memory.
+__device__ __forceinline__ void put_piece(uint32_t buf, int lane, int c, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + lane * 128 + ((c ^ (lane & 7)) << 4)), "r"(w0), "r"(w1), "r"(w2), "r"(w3)
                : "memory");
 }
-__device__ __forceinline__ void ld256(const void* p, uint32_t (&v)[8]) {
-  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "l"(p)
+__device__ __forceinline__ uint4 get_piece(uint32_t buf, int lane, int t) {
+  const int r = 4 * t + (lane >> 3);
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(buf + r * 128 + (((lane & 7) ^ (r & 7)) << 4))
                : "memory");
+  return v;
+}
+__device__ __forceinline__ void store_piece(char* p, uint4 v) {
+  asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ uint4 load_piece(const char* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+// The turned rows to global memory: `base` is the block's first byte of its first row, `pitch` bytes from row to row.
+__device__ __forceinline__ void store_turned(uint32_t buf, char* base, size_t pitch, int rows, int lane) {
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const uint4 v = get_piece(buf, lane, t);
+    const int r = 4 * t + (lane >> 3);
+    if (r < rows) store_piece(base + r * pitch + (lane & 7) * 16, v);
+  }
+  __syncwarp();  // the buffer may be written again
 }
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -364,7 +402,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const int bt = WIDE ? BNT : bn;           // columns of a work item's tile (bn: 16 .. 128 in steps of 16)
   const RingShape ring = ring_shape(A_ROWS, WIDE ? BNW : bn);
   const int kStages = ring.stages, kStageBytes = ring.stage_bytes, kTileBytesX = ring.tile_bytes_x;
-  Barriers* bars = reinterpret_cast<Barriers*>(tiles + ring.ring_bytes);
+  Barriers* bars = reinterpret_cast<Barriers*>(tiles + ring.ring_bytes + kEpiWarps * kStoreBytes);
   volatile uint32_t* failed = &bars->failed;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -449,108 +487,120 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   if (warp < kFirstEpiWarp) {
   if (WIDE) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
-    if (lane == 0) {
-      // The weights do not depend on the kernel before this one: the W tiles of the first
-      // round of the ring are requested at once, the wait for the previous kernel comes
-      // after, then the x tiles of those stages follow. Later stages load both together.
-      uint32_t it = 0;  // k-tiles issued so far, over all output tiles of this block
-      bool ok = true, waited = false;
-      // In a pair both blocks' loads are counted on the "full" barrier of rank 0, which
-      // expects the bytes of both; each block waits on its own "empty" barrier.
-      auto expect = [&](int s) {
-        if (!PAIR)
-          mbar_expect_tx(&bars->full[s], kStageBytes);
-        else if (rank == 0)
-          mbar_expect_tx(&bars->full[s], 2 * kStageBytes);
-      };
-      auto load = [&](void* dst, const CUtensorMap* map, int x, int y, int s) {
-        if (PAIR)
-          tma_load_2d_pair(dst, map, x, y, peer_addr(smem_u32(&bars->full[s]), 0));
-        else
-          tma_load_2d(dst, map, x, y, &bars->full[s]);
-      };
-      if (GROUPED) read_lists(), waited = true;
-      for (int tile = worker; tile < out_tiles && ok; tile += workers) {
-        int m0 = item_m0(tile), n0 = item_n0(tile) + (PAIR ? static_cast<int>(rank) * BN : 0);
-        if (GROUPED) {
-          int m_end, g;
-          group_tile(tile, m0, m_end, g);
-          n0 += g * N;  // the group's rows of W
-        }
-        const int kt0 = item_c0(tile) * kTilesPerChunk, kt1 = min(num_tiles, item_c1(tile) * kTilesPerChunk);
-        int kt = kt0;
-        if (!waited) {  // first item of this block
-          const int early = min(kt1 - kt0, kStages);
+    // The weights do not depend on the kernel before this one: the W tiles of the first
+    // round of the ring are requested at once, the wait for the previous kernel comes
+    // after, then the x tiles of those stages follow. Later stages load both together.
+    int s = 0;                       // stage of the next k-tile
+    uint32_t parity = 1;             // of the wait for that stage: passes at once in the first round
+    bool ok = true, waited = false;
+    // In a pair both blocks' loads are counted on the "full" barrier of rank 0, which
+    // expects the bytes of both; each block waits on its own "empty" barrier.
+    auto expect = [&](int st) {
+      if (!PAIR)
+        mbar_expect_tx(&bars->full[st], kStageBytes);
+      else if (rank == 0)
+        mbar_expect_tx(&bars->full[st], 2 * kStageBytes);
+    };
+    auto load = [&](void* dst, const CUtensorMap* map, int x, int y, int st) {
+      if (PAIR)
+        tma_load_2d_pair(dst, map, x, y, peer_addr(smem_u32(&bars->full[st]), 0));
+      else
+        tma_load_2d(dst, map, x, y, &bars->full[st]);
+    };
+    if (GROUPED) read_lists(), waited = true;
+    for (int tile = worker; tile < out_tiles && ok; tile += workers) {
+      int m0 = item_m0(tile), n0 = item_n0(tile) + (PAIR ? static_cast<int>(rank) * BN : 0);
+      if (GROUPED) {
+        int m_end, g;
+        group_tile(tile, m0, m_end, g);
+        n0 += g * N;  // the group's rows of W
+      }
+      const int kt0 = item_c0(tile) * kTilesPerChunk, kt1 = min(num_tiles, item_c1(tile) * kTilesPerChunk);
+      int kt = kt0;
+      if (!waited) {  // first item of this block
+        const int early = min(kt1 - kt0, kStages);
+        if (elect_one()) {
           for (int e = 0; e < early; ++e) {
-            unsigned char* a = tiles + e * kStageBytes;
             expect(e);
-            load(a + kTileBytesX, &map_w, (kt0 + e) * BK, n0, e);
+            load(tiles + e * kStageBytes + kTileBytesX, &map_w, (kt0 + e) * BK, n0, e);
           }
-          bw::pdl_wait();
-          waited = true;
-          for (int e = 0; e < early; ++e) load(tiles + e * kStageBytes, &map_x, (kt0 + e) * BK, m0, e);
-          kt += early;
-          it += early;
         }
-        for (; kt < kt1; ++kt, ++it) {
-          const int s = it % kStages;
-          const uint32_t round = it / kStages;
-          if (round > 0 && !mbar_wait(&bars->empty[s], (round - 1) & 1, failed)) {
-            ok = false;
-            break;
-          }
+        bw::pdl_wait();
+        waited = true;
+        __syncwarp();
+        if (elect_one())
+          for (int e = 0; e < early; ++e) load(tiles + e * kStageBytes, &map_x, (kt0 + e) * BK, m0, e);
+        __syncwarp();
+        kt += early;
+        s = early;
+        if (s == kStages) s = 0, parity ^= 1;
+      }
+      for (; kt < kt1; ++kt) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&bars->empty[s], parity, failed))) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           unsigned char* a = tiles + s * kStageBytes;
           expect(s);
           load(a, &map_x, kt * BK, m0, s);
           load(a + kTileBytesX, &map_w, kt * BK, n0, s);
         }
+        __syncwarp();
+        if (++s == kStages) s = 0, parity ^= 1;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {  // in a pair the block of rank 0 issues for both
-      uint32_t it = 0, gc = 0;  // k-tiles and chunks consumed so far
+    if (rank == 0) {  // in a pair the block of rank 0 issues for both
+      int s = 0;                     // stage of the next k-tile, and the parity of its arrival
+      uint32_t parity = 0;
+      uint32_t gc = 0;               // chunks begun so far
       bool ok = true;
       read_lists();
       for (int tile = worker; tile < out_tiles && ok; tile += workers) {
         for (int c = item_c0(tile); c < item_c1(tile) && ok; ++c, ++gc) {
           const int buf = gc & 1;
           const uint32_t use = gc >> 1;  // how often this accumulator was used before
-          if (use > 0 && !mbar_wait(&bars->acc_empty[buf], (use - 1) & 1, failed)) {
+          if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(&bars->acc_empty[buf], (use - 1) & 1, failed))) {
             ok = false;
             break;
           }
           fence_after_sync();
           const uint32_t d = tmem_base + buf * BNT;
           const int t_begin = c * kTilesPerChunk, t_end = min(num_tiles, t_begin + kTilesPerChunk);
-          for (int kt = t_begin; kt < t_end; ++kt, ++it) {
-            const int s = it % kStages;
-            if (!mbar_wait(&bars->full[s], (it / kStages) & 1, failed)) {
+          for (int kt = t_begin; kt < t_end; ++kt) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&bars->full[s], parity, failed))) {
               ok = false;
               break;
             }
             fence_after_sync();
             const uint32_t a_addr = smem_u32(tiles + s * kStageBytes);
             const uint64_t adesc = make_desc(a_addr), bdesc = make_desc(a_addr + kTileBytesX);
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k) {
-              // 16 k-elements are 32 bytes: the start address field moves by 2 (units of 16 bytes)
-              const uint32_t acc = (kt > t_begin || k > 0) ? 1u : 0u;
+              for (int k = 0; k < BK / 16; ++k) {
+                // 16 k-elements are 32 bytes: the start address field moves by 2 (units of 16 bytes)
+                const uint32_t acc = (kt > t_begin || k > 0) ? 1u : 0u;
+                if (PAIR)
+                  umma_pair(d, adesc + 2 * k, bdesc + 2 * k, instr_desc_pair(BNT), acc);
+                else
+                  umma(d, adesc + 2 * k, bdesc + 2 * k, instr_desc(bt), acc);
+              }
+              // the stage may be refilled once these MMAs are done; the chunk's last commit also
+              // hands the accumulator to the epilogue
               if (PAIR)
-                umma_pair(d, adesc + 2 * k, bdesc + 2 * k, instr_desc_pair(BNT), acc);
+                umma_commit_pair(&bars->empty[s]);
               else
-                umma(d, adesc + 2 * k, bdesc + 2 * k, instr_desc(bt), acc);
+                umma_commit(&bars->empty[s]);
+              if (kt + 1 == t_end) {
+                if (PAIR)
+                  umma_commit_pair(&bars->acc_full[buf]);
+                else
+                  umma_commit(&bars->acc_full[buf]);
+              }
             }
-            // the stage may be refilled once these MMAs are done
-            if (PAIR)
-              umma_commit_pair(&bars->empty[s]);
-            else
-              umma_commit(&bars->empty[s]);
-          }
-          if (ok) {
-            if (PAIR)
-              umma_commit_pair(&bars->acc_full[buf]);
-            else
-              umma_commit(&bars->acc_full[buf]);
+            __syncwarp();
+            if (++s == kStages) s = 0, parity ^= 1;
           }
         }
       }
@@ -567,12 +617,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     const int quarter = warp & 3;
     const int et = quarter * 32 + lane;  // 0..127: this thread's row of the tile
     const int blk = (warp - kFirstEpiWarp) >> 2;  // 0, or 0..1 in a wide tile
-    constexpr int half = 0;
+    const uint32_t store_buf = smem_u32(tiles + ring.ring_bytes) + (warp - kFirstEpiWarp) * kStoreBytes;
     const int off0 = blk * BN, off1 = off0 + BN / 2;  // column offsets of the pieces in the tile
-    float total[2 * PW];
     uint32_t gc = 0;
     bool ok = true;
     for (int tile = worker; tile < out_tiles && ok; tile += workers) {
+      // The running totals start at -0, which leaves whatever is added to it as it is: the first chunk sum is added like the
+      // others. (Choosing between "v" and "total + v" by the chunk made the compiler keep both, and sent half of the totals
+      // to local memory in the epilogues with SwiGLU or a residual.)
+      float total[2 * PW];
+#pragma unroll
+      for (int j = 0; j < 2 * PW; ++j) total[j] = -0.0f;
       int m0 = item_m0(tile), row_end = M;
       const int n0 = item_n0(tile);
       if (GROUPED) {
@@ -580,12 +635,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         group_tile(tile, m0, row_end, g);
       }
       const int row = m0 + et;
+      // rows of this warp's part of the tile, and whether its full blocks may go through shared memory in 16-byte accesses
+      const int first_row = m0 + quarter * 32, warp_rows = min(32, row_end - first_row);
+      const bool turned = (N & 7) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (reinterpret_cast<uintptr_t>(residual) & 15) == 0;
+      constexpr int kBlocks = 2 * PW / 32;  // blocks of 32 columns: 128 bytes of a float32 row
+      auto block_col = [&](int b) { return n0 + (b * 32 >= PW ? off1 + b * 32 - PW : off0 + b * 32); };
+      auto put_totals = [&](int b) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          put_piece(store_buf, lane, c, __float_as_uint(total[b * 32 + 4 * c]), __float_as_uint(total[b * 32 + 4 * c + 1]),
+                    __float_as_uint(total[b * 32 + 4 * c + 2]), __float_as_uint(total[b * 32 + 4 * c + 3]));
+      };
       for (int c = item_c0(tile); c < item_c1(tile) && ok; ++c, ++gc) {
         const int buf = gc & 1;
         if (!mbar_wait(&bars->acc_full[buf], (gc >> 1) & 1, failed)) {
           ok = false;
           break;
         }
+        __syncwarp();
         fence_after_sync();
         if (!SPLIT || quarter * 32 < M) {  // in split mode warps whose rows are all padding read nothing
           const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BNT;
@@ -599,7 +666,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
 #pragma unroll
               for (int j = 0; j < LDW; ++j) {
                 float& t = total[piece * PW + g * LDW + j];
-                t = (SPLIT || c == 0) ? v[j] : t + v[j];
+                t = SPLIT ? v[j] : t + v[j];
               }
             }
           }
@@ -613,28 +680,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             mbar_arrive(&bars->acc_empty[buf]);
         }
       }
-      if (!ok) break;
-      if (row >= row_end) continue;
+      if (!__all_sync(0xffffffffu, ok)) break;
+      if (warp_rows <= 0) continue;
       if (SPLIT && num_chunks > 1) {
         // this item's chunk sum goes to scratch; a second kernel adds the chunk sums in order
-        const int chunk = item_c0(tile);
+        float* plane = partials + static_cast<size_t>(item_c0(tile)) * M * N;
 #pragma unroll
-        for (int piece = 0; piece < 2; ++piece) {
-          const int col0 = n0 + (piece ? off1 : off0);
-          const int cols = min(PW, min(N, n0 + bt) - col0);
-          float* mine = partials + (static_cast<size_t>(chunk) * M + row) * N + col0;
-          if (cols == PW && (N & 7) == 0 && (reinterpret_cast<uintptr_t>(partials) & 31) == 0) {
+        for (int b = 0; b < kBlocks; ++b) {
+          const int col0 = block_col(b), cols = min(32, min(N, n0 + bt) - col0);
+          if (cols <= 0) continue;
+          if (cols == 32 && (N & 3) == 0 && (reinterpret_cast<uintptr_t>(partials) & 15) == 0) {
+            put_totals(b);
+            store_turned(store_buf, reinterpret_cast<char*>(plane + static_cast<size_t>(first_row) * N + col0), static_cast<size_t>(N) * 4, warp_rows, lane);
+          } else if (row < row_end) {
 #pragma unroll
-            for (int j = 0; j < PW; j += 8) {
-              uint32_t o[8];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(total[piece * PW + j + e]);
-              st256(mine + j, o);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < PW; ++j)
-              if (!WIDE && j < cols) __stcg(mine + j, total[piece * PW + j]);
+            for (int j = 0; j < 32; ++j)
+              if (!WIDE && j < cols) __stcg(plane + static_cast<size_t>(row) * N + col0 + j, total[b * 32 + j]);
           }
         }
         continue;
@@ -643,78 +704,99 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         // the first piece holds gate rows, the second the up rows of the same indices; both
         // are rounded to bfloat16 first, as if the product had been stored
         if (n0 + off0 >= N) continue;
-        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(Y) + static_cast<size_t>(row) * (N / 2) + (n0 + blk * BN) / 2 + half * PW;
-        const bool wide_store = (reinterpret_cast<uintptr_t>(Y) & 31) == 0;  // rows are N bytes, N % 128 == 0
+        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(Y) + static_cast<size_t>(first_row) * (N / 2) + (n0 + blk * BN) / 2;
+        // the activation is tested once, outside the unrolled code: a test per entry made the compiler keep both
+        // activations' intermediates of many entries alive, and they went to local memory (4 KB per thread and tile)
+        auto glu = [&](auto act_c) {
+          constexpr int act = decltype(act_c)::value;
 #pragma unroll
-        for (int j = 0; j < PW; j += 16) {
-          uint32_t o[8];
+          for (int c = 0; c < 8; ++c) {
+            uint32_t o[4];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float g0 = __bfloat162float(__float2bfloat16_rn(total[j + 2 * e]));
-            const float g1 = __bfloat162float(__float2bfloat16_rn(total[j + 2 * e + 1]));
-            const float u0 = __bfloat162float(__float2bfloat16_rn(total[PW + j + 2 * e]));
-            const float u1 = __bfloat162float(__float2bfloat16_rn(total[PW + j + 2 * e + 1]));
-            o[e] = pack_bf16(bw::glu_one(g0, u0, y_is_f32), bw::glu_one(g1, u1, y_is_f32));
+            for (int e = 0; e < 4; ++e) {
+              const int j = 8 * c + 2 * e;
+              const float g0 = __bfloat162float(__float2bfloat16_rn(total[j]));
+              const float g1 = __bfloat162float(__float2bfloat16_rn(total[j + 1]));
+              const float u0 = __bfloat162float(__float2bfloat16_rn(total[PW + j]));
+              const float u1 = __bfloat162float(__float2bfloat16_rn(total[PW + j + 1]));
+              o[e] = pack_bf16(bw::glu_one(g0, u0, act), bw::glu_one(g1, u1, act));
+            }
+            put_piece(store_buf, lane, c, o[0], o[1], o[2], o[3]);
           }
-          if (wide_store) {
-            st256(out + j, o);
-          } else {
-            *reinterpret_cast<uint4*>(out + j) = make_uint4(o[0], o[1], o[2], o[3]);
-            *reinterpret_cast<uint4*>(out + j + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+        };
+        if (y_is_f32 == bw::kGluGeluTanh)
+          glu(std::integral_constant<int, bw::kGluGeluTanh>{});
+        else
+          glu(std::integral_constant<int, bw::kGluSilu>{});
+        store_turned(store_buf, reinterpret_cast<char*>(out), static_cast<size_t>(N), warp_rows, lane);
+      } else if (EPI == 2) {
+#pragma unroll
+        for (int b = 0; b < kBlocks; ++b) {
+          const int col0 = block_col(b), cols = min(32, min(N, n0 + bt) - col0);  // may be <= 0 in a narrow or a last, partial tile
+          if (cols <= 0) continue;
+          const size_t at = static_cast<size_t>(first_row) * N + col0;
+          if (cols == 32 && turned) {
+            const size_t mine = at * 4 + (lane & 7) * 16, pitch = static_cast<size_t>(N) * 4;
+            char* base = reinterpret_cast<char*>(Y) + mine;
+            if (residual) {
+              // all eight pieces of the residual are asked for before the first is used
+              const char* rbase = reinterpret_cast<const char*>(residual) + mine;
+              uint4 res[8];
+#pragma unroll
+              for (int t = 0; t < 8; ++t) {
+                const int r = 4 * t + (lane >> 3);
+                res[t] = r < warp_rows ? load_piece(rbase + r * pitch) : make_uint4(0u, 0u, 0u, 0u);
+              }
+              put_totals(b);
+              __syncwarp();
+#pragma unroll
+              for (int t = 0; t < 8; ++t) {
+                const int r = 4 * t + (lane >> 3);
+                uint4 v = get_piece(store_buf, lane, t);
+                v.x = __float_as_uint(__uint_as_float(res[t].x) + __uint_as_float(v.x));
+                v.y = __float_as_uint(__uint_as_float(res[t].y) + __uint_as_float(v.y));
+                v.z = __float_as_uint(__uint_as_float(res[t].z) + __uint_as_float(v.z));
+                v.w = __float_as_uint(__uint_as_float(res[t].w) + __uint_as_float(v.w));
+                if (r < warp_rows) store_piece(base + r * pitch, v);
+              }
+              __syncwarp();
+            } else {
+              put_totals(b);
+              store_turned(store_buf, reinterpret_cast<char*>(static_cast<float*>(Y) + at), pitch, warp_rows, lane);
+            }
+          } else if (row < row_end) {
+            const size_t mine = at + static_cast<size_t>(lane) * N;
+#pragma unroll
+            for (int j = 0; j < 32; ++j)  // static indices keep the totals in registers
+              if (!WIDE && j < cols)
+                static_cast<float*>(Y)[mine + j] = residual ? residual[mine + j] + total[b * 32 + j] : total[b * 32 + j];
           }
         }
-        continue;
-      }
-      if (EPI == 0 && y_is_f32 == 2 * bw::kOutRelu2) {
+      } else {
+        if (y_is_f32 == 2 * bw::kOutRelu2) {
 #pragma unroll
-        for (int j = 0; j < 2 * PW; ++j) total[j] = bw::out_act(total[j], bw::kOutRelu2);
-      } else if (EPI == 0 && !GROUPED && y_is_f32 == 2 * bw::kOutTanh) {
+          for (int j = 0; j < 2 * PW; ++j) total[j] = bw::out_act(total[j], bw::kOutRelu2);
+        } else if (!GROUPED && y_is_f32 == 2 * bw::kOutTanh) {
 #pragma unroll
-        for (int j = 0; j < 2 * PW; ++j) total[j] = bw::out_act(total[j], bw::kOutTanh);
-      }
+          for (int j = 0; j < 2 * PW; ++j) total[j] = bw::out_act(total[j], bw::kOutTanh);
+        }
 #pragma unroll
-      for (int piece = 0; piece < 2; ++piece) {
-        const int col0 = n0 + (piece ? off1 : off0);
-        const int cols = min(PW, min(N, n0 + bt) - col0);  // may be <= 0 in a narrow or a last, partial tile
-        if (cols <= 0) continue;
-        const size_t base = static_cast<size_t>(row) * N + col0;
-        if (EPI == 2) {
-          float* out = static_cast<float*>(Y) + base;
-          const float* res = residual ? residual + base : nullptr;
-          if (cols == PW && (N & 7) == 0 && (reinterpret_cast<uintptr_t>(Y) & 31) == 0 &&
-              (reinterpret_cast<uintptr_t>(residual) & 31) == 0) {
+        for (int piece = 0; piece < 2; ++piece) {
+          const int col0 = n0 + (piece ? off1 : off0);
+          const int cols = min(PW, min(N, n0 + bt) - col0);  // may be <= 0 in a narrow or a last, partial tile
+          if (cols <= 0) continue;
+          __nv_bfloat16* out = static_cast<__nv_bfloat16*>(Y) + static_cast<size_t>(first_row) * N + col0;
+          if (cols == PW && turned) {
 #pragma unroll
-            for (int j = 0; j < PW; j += 8) {
-              uint32_t o[8];
-              if (res) {
-                ld256(res + j, o);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) + total[piece * PW + j + e]);
-              } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(total[piece * PW + j + e]);
-              }
-              st256(out + j, o);
+            for (int c = 0; c < 8; ++c) {
+              const float* t8 = total + piece * PW + 8 * c;
+              put_piece(store_buf, lane, c, pack_bf16(t8[0], t8[1]), pack_bf16(t8[2], t8[3]), pack_bf16(t8[4], t8[5]), pack_bf16(t8[6], t8[7]));
             }
-          } else {
-#pragma unroll
-            for (int j = 0; j < PW; ++j)  // static indices keep the totals in registers
-              if (!WIDE && j < cols) out[j] = res ? res[j] + total[piece * PW + j] : total[piece * PW + j];
-          }
-        } else {
-          __nv_bfloat16* out = static_cast<__nv_bfloat16*>(Y) + base;
-          if (cols == PW && (N & 15) == 0 && (reinterpret_cast<uintptr_t>(Y) & 31) == 0) {
-#pragma unroll
-            for (int j = 0; j < PW; j += 16) {
-              uint32_t o[8];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) o[e] = pack_bf16(total[piece * PW + j + 2 * e], total[piece * PW + j + 2 * e + 1]);
-              st256(out + j, o);
-            }
-          } else {
+            store_turned(store_buf, reinterpret_cast<char*>(out), static_cast<size_t>(N) * 2, warp_rows, lane);
+          } else if (row < row_end) {
 #pragma unroll
             for (int j = 0; j < PW; ++j)
-              if (!WIDE && j < cols) out[j] = __float2bfloat16_rn(total[piece * PW + j]);
+              if (!WIDE && j < cols) out[static_cast<size_t>(lane) * N + j] = __float2bfloat16_rn(total[piece * PW + j]);
           }
         }
       }
@@ -902,7 +984,8 @@ struct Fused {
 // asked. Neither allocates. Returns 0 or an error; *pairs receives the number of pairs.
 template <bool SPLIT, int A_ROWS, int EPI, bool WIDE, bool PAIR = false, bool GROUPED = false>
 int configure_tc(int* pairs = nullptr) {
-  constexpr int smem_max = kSmemBudget + sizeof(Barriers) + 1024;
+  constexpr int kEpi = WIDE ? 8 : 4;  // epilogue warps
+  constexpr int smem_max = kSmemBudget + kEpi * kStoreBytes + sizeof(Barriers) + 1024;
   constexpr int threads = WIDE ? 384 : 192;
   static_assert(smem_max <= 227 * 1024, "ring does not fit");
   static bool configured[kMaxDevices] = {false};
@@ -921,7 +1004,7 @@ int configure_tc(int* pairs = nullptr) {
       cudaLaunchConfig_t probe = {};
       probe.gridDim = dim3(2 * (sm_count_of_device() / 2));
       probe.blockDim = dim3(threads);
-      probe.dynamicSmemBytes = ring.ring_bytes + static_cast<int>(sizeof(Barriers)) + 1024;
+      probe.dynamicSmemBytes = ring.ring_bytes + kEpi * kStoreBytes + static_cast<int>(sizeof(Barriers)) + 1024;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
@@ -947,11 +1030,11 @@ int launch_tc(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_
   constexpr int BNT = WIDE ? 2 * BN : BN;
   constexpr int BNW = PAIR ? BN : BNT;
   constexpr int BMT = PAIR ? 2 * BM : BM;
-  constexpr int threads = WIDE ? 384 : 192;
+  constexpr int threads = WIDE ? 384 : 192, kEpi = WIDE ? 8 : 4;
   const int chunks = (k + kChunk - 1) / kChunk;
   const int bn = WIDE ? BNT : narrow_bn;
   const RingShape ring = ring_shape(A_ROWS, WIDE ? BNW : bn);
-  const int smem = ring.ring_bytes + static_cast<int>(sizeof(Barriers)) + 1024;
+  const int smem = ring.ring_bytes + kEpi * kStoreBytes + static_cast<int>(sizeof(Barriers)) + 1024;
   auto kernel = gemm_tc_kernel<SPLIT, A_ROWS, EPI, WIDE, PAIR>;
   int max_pairs = 0;
   if (const int rc = configure_tc<SPLIT, A_ROWS, EPI, WIDE, PAIR>(&max_pairs)) return rc;
@@ -989,9 +1072,9 @@ int launch_tc(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_
 template <int EPI>
 int launch_tc_grouped(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_f32, int rows, int n, int k,
                       const int* group_off, const int* tile_prefix, int groups, int* error_word, cudaStream_t stream) {
-  constexpr int BNT = 2 * BN, threads = 384;
+  constexpr int BNT = 2 * BN, threads = 384, kEpi = 8;
   const RingShape ring = ring_shape(BM, BNT);
-  const int smem = ring.ring_bytes + static_cast<int>(sizeof(Barriers)) + 1024;
+  const int smem = ring.ring_bytes + kEpi * kStoreBytes + static_cast<int>(sizeof(Barriers)) + 1024;
   auto kernel = gemm_tc_kernel<false, BM, EPI, true, false, true>;
   if (const int rc = configure_tc<false, BM, EPI, true, false, true>()) return rc;
   CUtensorMap map_x, map_w;
