@@ -18,12 +18,12 @@
 // a piece is one 128-byte swizzled line), the scores add up over the pieces' k-steps in order,
 // and the output takes one MMA per 16 keys over all 128 columns (the pieces of V are the
 // swizzle atoms of one MN-major operand, a piece apart).
-// What the tensor core does is handed out by one thread, and every instruction or barrier
-// operation costs that thread about a hundred cycles, which is what a tile's time is made of
-// (measured with time stamps: 21 such operations and 2,500 cycles per tile of 64 keys at head
-// size 128, where the arithmetic needs 500). So that thread waits only for what nothing else
-// implies (keys landed, weights written: the buffers of S and O are free by then, see below)
-// and announces the output and the freed stage with one commit.
+// What the tensor core does is handed out by one warp, whose operations are what a tile's time is
+// made of. So it waits only for what nothing else implies (keys landed, weights written: the
+// buffers of S and O are free by then, see below) and announces the output and the freed stage
+// with one commit; and all its lanes walk the loop with one elected to issue (a lone lane's
+// operation took about a hundred cycles, most of them moves of descriptors into uniform
+// registers).
 // At head size 64 two blocks share an SM (256 tensor-memory columns and about 100 KB each), so
 // one block's softmax overlaps the other's MMAs; at 128 a block has the SM to itself (384 of
 // the 512 columns, 170 KB) and overlaps its own stages. Every mbarrier wait is bounded
@@ -79,6 +79,13 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* failed) {
   return bw::mbar_wait_bounded(bar, parity, failed);
+}
+// One lane of a whole, converged warp: the code it guards runs with operands that the compiler knows to be the warp's, kept
+// in uniform registers (see bf16_gemm_tc.cu).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
                                             uint64_t* bar) {
@@ -252,19 +259,23 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = mbar_wait(&bars->q_full, 0, failed);
+    // all lanes walk the loop and wait, one of them issues
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, failed)) != 0; };
+    bool ok = wait(&bars->q_full, 0);
+    fence_after_sync();
+    const uint32_t q_addr = smem_u32(sq);
+    int qk_s = 0;                 // stage of the next tile of scores, and the parity of its arrival
+    uint32_t qk_parity = 0;
+    auto issue_qk = [&](int t) -> bool {
+      const int s = qk_s, b = t & 1;
+      if (!wait(&bars->kv_full[s], qk_parity)) return false;
+      if (++qk_s == kStages) qk_s = 0, qk_parity ^= 1;
+      // The scores' buffer was read by the softmax of tile t - 2 before that tile's weights were
+      // announced, and this warp saw that announcement before it formed tile t - 2's output:
+      // no barrier of its own.
       fence_after_sync();
-      const uint32_t q_addr = smem_u32(sq);
-      auto issue_qk = [&](int t) -> bool {
-        const int s = t % kStages, b = t & 1;
-        if (!mbar_wait(&bars->kv_full[s], (t / kStages) & 1, failed)) return false;
-        // The scores' buffer was read by the softmax of tile t - 2 before that tile's weights were
-        // announced, and this thread saw that announcement before it formed tile t - 2's output:
-        // no barrier of its own (a wait costs this thread a hundred cycles even when it is over,
-        // and the tensor core's work is handed out by this one thread).
-        fence_after_sync();
-        const uint32_t k_addr = smem_u32(skv + s * 2 * kKBytes);
+      const uint32_t k_addr = smem_u32(skv + s * 2 * kKBytes);
+      if (elect_one()) {
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {  // d ascending: piece after piece, 16 values a step
           const uint64_t qdesc = make_desc(q_addr + i * kQPiece), kdesc = make_desc(k_addr + i * kKPiece);
@@ -272,24 +283,30 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           for (int k = 0; k < 4; ++k) umma(tmem_base + b * 64, qdesc + 2 * k, kdesc + 2 * k, kDescQK, (i | k) > 0 ? 1u : 0u);
         }
         umma_commit(&bars->s_full[b]);
-        return true;
-      };
-      if (ok && ntiles > 0) ok = issue_qk(0);
-      for (int t = 0; t < ntiles && ok; ++t) {
-        const int s = t % kStages, b = t & 1;
-        if (t + 1 < ntiles) ok = issue_qk(t + 1);  // the next tile's scores are computed while this one's weights are formed
-        if (!ok) break;
-        if (!mbar_wait(&bars->p_ready[b], (t >> 1) & 1, failed)) break;
-        // the output buffer was merged (tile t - 2) before the softmax of this tile began: same argument
-        fence_after_sync();
-        const uint64_t pdesc = make_desc(smem_u32(sp + b * kPBytes));
-        const uint32_t v_addr = smem_u32(skv + s * 2 * kKBytes + kKBytes);
-        const uint64_t vdesc = kPieces == 1 ? make_desc(v_addr) : make_desc_wide(v_addr, kKPiece);
+      }
+      __syncwarp();
+      return true;
+    };
+    if (ok && ntiles > 0) ok = issue_qk(0);
+    int s = 0;
+    for (int t = 0; t < ntiles && ok; ++t) {
+      const int b = t & 1;
+      if (t + 1 < ntiles) ok = issue_qk(t + 1);  // the next tile's scores are computed while this one's weights are formed
+      if (!ok) break;
+      if (!wait(&bars->p_ready[b], (t >> 1) & 1)) break;
+      // the output buffer was merged (tile t - 2) before the softmax of this tile began: same argument
+      fence_after_sync();
+      const uint64_t pdesc = make_desc(smem_u32(sp + b * kPBytes));
+      const uint32_t v_addr = smem_u32(skv + s * 2 * kKBytes + kKBytes);
+      const uint64_t vdesc = kPieces == 1 ? make_desc(v_addr) : make_desc_wide(v_addr, kKPiece);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < kTileKV / 16; ++k)  // 16 keys: 32 bytes along a row of P, two 8-key groups (2048 bytes) of V
           umma(tmem_base + kOCol + b * HD, pdesc + 2 * k, vdesc + 128 * k, kDescPV, k > 0 ? 1u : 0u);
         umma_commit(&bars->pv_done[s]);  // the output is there, and the stage may be filled again
       }
+      __syncwarp();
+      if (++s == kStages) s = 0;
     }
   } else {
     // one thread per stacked row; warp w may touch tensor-memory lanes 32 * (w % 4) .. + 31
