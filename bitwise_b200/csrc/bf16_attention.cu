@@ -48,6 +48,13 @@ constexpr int kRowBytes = kSwizzle ? HD * 2 : HD * 2 + 16;
 __device__ __forceinline__ int piece_offset(int row, int piece) {
   return row * kRowBytes + (kSwizzle ? (((piece & ~7) | ((piece ^ row) & 7)) << 4) : (piece << 4));
 }
+// The same within a tile of ROWS rows that TMA brought (BOXES): a box is at most one 128-byte line wide, so a head of 128 lies
+// as two halves of 64 entries, each [ROWS][128 bytes] with the line's own swizzle. At 64 both layouts are the same.
+template <bool BOXES, int ROWS>
+__device__ __forceinline__ int tile_offset(int row, int piece) {
+  if (!BOXES) return piece_offset(row, piece);
+  return (piece >> 3) * (ROWS * 128) + row * 128 + (((piece ^ row) & 7) << 4);
+}
 constexpr int kQBytes = kTileM * kRowBytes;
 constexpr int kKVBytes = kTileKV * kRowBytes;
 constexpr int kPieces = HD / 8;             // 16-byte pieces per row
@@ -114,6 +121,7 @@ struct TileResult {
 // domain), mask, maximum, weights, sum, o = P V from zero. sq points at the warp's 16 rows of
 // Q, sk / sv at the tile's keys and values in shared memory (padded rows of kRowBytes).
 // Both modes call this one function, so a tile gives the same bits in both.
+template <bool BOXES>
 __device__ __forceinline__ void attend_tile(const unsigned char* sq, const unsigned char* sk, const unsigned char* sv,
                                             int lane, int j0, int pos_lo, int pos_hi, int first_lo, int first_hi,
                                             float scale_log2, TileResult& r) {
@@ -129,13 +137,13 @@ __device__ __forceinline__ void attend_tile(const unsigned char* sq, const unsig
     uint32_t a[4];
     {
       const int row = (lane & 7) + ((lane >> 3) & 1) * 8;
-      ldmatrix_x4(a, smem_u32(sq + piece_offset(row, kk * 2 + (lane >> 4))));
+      ldmatrix_x4(a, smem_u32(sq + tile_offset<BOXES, 16>(row, kk * 2 + (lane >> 4))));
     }
     uint32_t b[kTileKV / 16][4];
 #pragma unroll
     for (int np = 0; np < kTileKV / 16; ++np) {
       const int key = np * 16 + (lane & 7) + (lane >> 4) * 8;
-      ldmatrix_x4(b[np], smem_u32(sk + piece_offset(key, kk * 2 + ((lane >> 3) & 1))));
+      ldmatrix_x4(b[np], smem_u32(sk + tile_offset<BOXES, kTileKV>(key, kk * 2 + ((lane >> 3) & 1))));
     }
 #pragma unroll
     for (int np = 0; np < kTileKV / 16; ++np) {
@@ -208,7 +216,7 @@ __device__ __forceinline__ void attend_tile(const unsigned char* sq, const unsig
       for (int dd = 0; dd < 4; ++dd) {
         if (d0 + dd < HD / 16) {
           const int key = kp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-          ldmatrix_x4_trans(b[dd], smem_u32(sv + piece_offset(key, (d0 + dd) * 2 + (lane >> 4))));
+          ldmatrix_x4_trans(b[dd], smem_u32(sv + tile_offset<BOXES, kTileKV>(key, (d0 + dd) * 2 + (lane >> 4))));
         }
       }
 #pragma unroll
@@ -335,7 +343,7 @@ attention_whole_kernel(const __nv_bfloat16* __restrict__ qkv, int q_stride, cons
     __syncthreads();
     if (warp_active) {
       TileResult r;
-      attend_tile(sq + warp * 16 * kRowBytes, stage_k(t & 1), stage_k(t & 1) + kKVBytes, lane, kv_lo + t * kTileKV, pos_lo,
+      attend_tile<false>(sq + warp * 16 * kRowBytes, stage_k(t & 1), stage_k(t & 1) + kKVBytes, lane, kv_lo + t * kTileKV, pos_lo,
                   pos_hi, first_lo, first_hi, scale_log2, r);
       const MergeWeights wl = merge_weights(M_lo, r.max_lo), wh = merge_weights(M_hi, r.max_hi);
       M_lo = wl.mx;
@@ -423,7 +431,7 @@ attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_stride, cons
   if (!mine) return;
 
   TileResult r;
-  attend_tile(sq, sk, sv, lane, t * kTileKV, p, p, first, first, scale_log2, r);
+  attend_tile<false>(sq, sk, sv, lane, t * kTileKV, p, p, first, first, scale_log2, r);
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int m = (lane >> 2) + half * 8;
@@ -448,12 +456,13 @@ attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_stride, cons
 // and values is eight copies instead of a thousand 16-byte ones, and the query row is one
 // more. Tiles that earlier steps stored are requested before the wait for the kernel before
 // this one. The arithmetic and the records are those of attention_split_kernel (same bits).
-#if BW_HEAD_DIM == 64
+#if BW_HEAD_DIM == 64 || BW_HEAD_DIM == 128
+constexpr int kHalves = HD / 64;      // boxes across a head
 constexpr int kStreamWarps = 6;
 constexpr int kStreamStages = 2;
 constexpr int kStreamMaxRows = 512;  // rows of a step whose positions fit into shared memory beside the rings
-constexpr int kStreamQBytes = 16 * 128;                       // 16 stacked rows; a step's row fills `group` of them
-constexpr int kStreamItemBytes = kStreamQBytes + 2 * kKVBytes;  // 18 KB, a multiple of 1024
+constexpr int kStreamQBytes = 16 * HD * 2;                    // 16 stacked rows; a step's row fills `group` of them
+constexpr int kStreamItemBytes = kStreamQBytes + 2 * kKVBytes;  // 18 or 36 KB, a multiple of 1024
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
@@ -470,13 +479,34 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity, int* failure) {
   bw::mbar_wait_bounded(bar, parity, reinterpret_cast<volatile uint32_t*>(failure));
 }
-__device__ __forceinline__ void tma_box_4d(void* dst, const CUtensorMap* map, int c2, int c3, uint64_t* bar) {
+__device__ __forceinline__ void tma_box_4d(void* dst, const CUtensorMap* map, int c0, int c2, int c3, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(0), "r"(c2), "r"(c3), "r"(smem_u32(bar))
+      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(0), "r"(c2), "r"(c3), "r"(smem_u32(bar))
       : "memory");
 }
 
+// Requests a tile's keys (at sk) and values (kKVBytes behind), given the pages that lanes 0 .. pages_per_tile - 1 hold: a box
+// per page and half of a head, a lane each (a request holds its thread for a hundred cycles).
+__device__ __forceinline__ void request_tile(unsigned char* sk, const CUtensorMap* map_k, const CUtensorMap* map_v, int page,
+                                             int pages_per_tile, int g, int my_page, int lane, uint64_t* bar) {
+  const int boxes = pages_per_tile * 2 * kHalves;  // at most 32: pages of 8 keys or more
+  const int c = lane < boxes ? lane : 0;
+  const int pg = c / (2 * kHalves), i = (c >> 1) % kHalves;
+  const int blk = __shfl_sync(0xffffffffu, my_page, pg);
+  if (lane < boxes)
+    tma_box_4d(sk + (c & 1) * kKVBytes + i * kTileKV * 128 + pg * page * 128, (c & 1) ? map_v : map_k, 64 * i, g, blk, bar);
+}
+// A row's last tile: values behind its position are whatever the page's last holder left, and their weights are zero; they
+// become zero as well, so that an infinity left there cannot reach the sum.
+__device__ __forceinline__ void clear_values(unsigned char* sv, int first_row, int lane) {
+  for (int c = first_row * 8 + lane; c < kTileKV * 8; c += 32)
+#pragma unroll
+    for (int i = 0; i < kHalves; ++i) *reinterpret_cast<uint4*>(sv + i * kTileKV * 128 + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+}
+
+#if BW_HEAD_DIM == 64
 // map_q: [row][kv head][head of the group][64], box = the group's heads of one row and kv head.
 // map_k / map_v: [page][kv head][slot][64], box = one page of one kv head.
 //
@@ -559,13 +589,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   };
   // requests keys and values of an item, given the pages that lanes 0 .. pages_per_tile - 1 hold
   auto request_kv = [&](const Item& it, int my_page, unsigned char* buf, uint64_t* bar) {
-    for (int pg = 0; pg < pages_per_tile; ++pg) {
-      const int blk = __shfl_sync(0xffffffffu, my_page, pg);
-      if (lane == 0) {
-        tma_box_4d(buf + kStreamQBytes + pg * page * 128, &map_k, it.g, blk, bar);
-        tma_box_4d(buf + kStreamQBytes + kKVBytes + pg * page * 128, &map_v, it.g, blk, bar);
-      }
-    }
+    request_tile(buf + kStreamQBytes, &map_k, &map_v, page, pages_per_tile, it.g, my_page, lane, bar);
   };
   const uint32_t q_bytes = static_cast<uint32_t>(group) * 128, kv_bytes = 2 * kKVBytes;
 
@@ -594,7 +618,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     unsigned char* buf = ring + s * kStreamItemBytes;
     if (lane == 0) {
       mbar_arrive_expect_tx(bars + s, early[s] ? q_bytes : q_bytes + kv_bytes);
-      tma_box_4d(buf, &map_q, it.g, it.row, bars + s);
+      tma_box_4d(buf, &map_q, 0, it.g, it.row, bars + s);
     }
     __syncwarp();
     if (!early[s]) request_kv(it, first_pages[s], buf, bars + s);
@@ -617,16 +641,19 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     const int stage = used % kStreamStages;
     unsigned char* buf = ring + stage * kStreamItemBytes;
     mbar_wait_bounded(bars + stage, (used / kStreamStages) & 1, failure);
+    const bool cut = (it.t + 1) * kTileKV > it.p + 1;  // the tile ends behind the row's position
+    if (cut) clear_values(buf + kStreamQBytes + kKVBytes, it.p + 1 - it.t * kTileKV, lane);
     TileResult r;
-    attend_tile(buf, buf + kStreamQBytes, buf + kStreamQBytes + kKVBytes, lane, it.t * kTileKV, it.p, it.p, first, first,
+    attend_tile<true>(buf, buf + kStreamQBytes, buf + kStreamQBytes + kKVBytes, lane, it.t * kTileKV, it.p, it.p, first, first,
                 scale_log2, r);
     // the buffer is free (every ldmatrix of the item has delivered): the next item of the ring
     // takes it; the pages of the one after are looked up now and used a whole item later
+    if (cut) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the zeros before the copies that follow them
     __syncwarp();
     if (nx_ok) {
       if (lane == 0) {
         mbar_arrive_expect_tx(bars + stage, q_bytes + kv_bytes);
-        tma_box_4d(buf, &map_q, nx.g, nx.row, bars + stage);
+        tma_box_4d(buf, &map_q, 0, nx.g, nx.row, bars + stage);
       }
       __syncwarp();
       request_kv(nx, nx_page, buf, bars + stage);
@@ -653,12 +680,17 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   }
 }
 
+#endif  // BW_HEAD_DIM == 64
+
 // The per-tile blocks of attention_split_kernel (one warp, one key tile, a dozen blocks on an SM)
 // with the tile's keys and values fetched as TMA boxes: a page of a head is one box, eight
 // boxes a tile, asked for by one lane, instead of 32 warp-wide cp.async of four lines each
 // (whose issue was a third of a block's time). The query row still comes by cp.async, the
-// arithmetic and the record are attend_tile's: same bits. For steps of fewer rows than the
-// streaming kernel above is worth its set-up for.
+// arithmetic and the record are attend_tile's: same bits. At head size 64 for steps of fewer rows
+// than the streaming kernel above is worth its set-up for. At head size 128 for all steps: a tile
+// is 32 KB, persistent blocks have room for three warps with two of them each, and six blocks of
+// one warp keep the memory busier (64 rows, 32/8 heads, 900 to 4,090 keys, with the merge: 159 us
+// by cp.async, 146 persistent, 127 here, for keys and values that take 100 at the copy bandwidth).
 __global__ void __launch_bounds__(32)
 attention_tile_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                           const __nv_bfloat16* __restrict__ qkv, int q_stride, const int* __restrict__ block_table,
@@ -693,13 +725,7 @@ attention_tile_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
   auto request = [&]() {
     if (lane == 0) mbar_arrive_expect_tx(bar, 2 * kKVBytes);
     __syncwarp();
-    for (int pg = 0; pg < pages_per_tile; ++pg) {
-      const int blk = __shfl_sync(0xffffffffu, my_page, pg);
-      if (lane == 0) {
-        tma_box_4d(sk + pg * page * 128, &map_k, g, blk, bar);
-        tma_box_4d(sv + pg * page * 128, &map_v, g, blk, bar);
-      }
-    }
+    request_tile(sk, &map_k, &map_v, page, pages_per_tile, g, my_page, lane, bar);
   };
   if (settled) request();  // before the wait for the kernel that rotates q and stores this step's key and value
   bw::pdl_enter();
@@ -707,16 +733,17 @@ attention_tile_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
     const int m = idx / kPieces, piece = idx - m * kPieces;
     const bool ok = m < group;
     const __nv_bfloat16* src = qkv + static_cast<size_t>(row) * q_stride + (g * group + (ok ? m : 0)) * HD + piece * 8;
-    cp_async16(smem_u32(sq + piece_offset(m, piece)), src, ok);
+    cp_async16(smem_u32(sq + tile_offset<true, 16>(m, piece)), src, ok);
   }
   cp_async_commit();
   if (!settled) request();
   cp_async_wait<0>();
   if (!bw::mbar_wait_bounded(bar, 0, reinterpret_cast<volatile uint32_t*>(failure))) return;
   __syncwarp();
+  if ((t + 1) * kTileKV > p + 1) clear_values(sv, p + 1 - t * kTileKV, lane);
 
   TileResult r;
-  attend_tile(sq, sk, sv, lane, t * kTileKV, p, p, first, first, scale_log2, r);
+  attend_tile<true>(sq, sk, sv, lane, t * kTileKV, p, p, first, first, scale_log2, r);
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int m = (lane >> 2) + half * 8;
@@ -731,7 +758,7 @@ attention_tile_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
     }
   }
 }
-#endif  // BW_HEAD_DIM == 64
+#endif  // BW_HEAD_DIM == 64 || BW_HEAD_DIM == 128
 
 // Second half of split mode: per (row, head) the tile results are merged in ascending tile
 // order with the same formula as in whole mode; thread d carries output element d. The records
@@ -843,7 +870,7 @@ BW_API int bw_bf16_attention(const __nv_bfloat16* qkv, int q_stride, const __nv_
   return bw::launch_status();
 }
 
-#if BW_HEAD_DIM == 64
+#if BW_HEAD_DIM == 64 || BW_HEAD_DIM == 128
 namespace {
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -869,21 +896,24 @@ bool stream_map(CUtensorMap* map, const void* base, const cuuint64_t (&dims)[4],
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 int g_stream_mode = 1;  // 0 never, 1 for steps of many rows, 2 whenever the shape allows
-constexpr int kStreamMinRows = 32;
+constexpr int kStreamMinHeads = 2048;  // rows x key/value heads
 }  // namespace
 
 // How decode steps fetch the cache where the shape allows TMA boxes: 0 never (the cp.async blocks
-// of attention_split_kernel), 1 (the default) the streaming kernel for steps of 32 rows or more
-// and a block per key tile fed by boxes for fewer (measured on B200: with few rows the set-up of
-// a persistent block costs more than its steadier stream of loads gains), 2 the streaming kernel
-// whenever the shape allows. Returns the previous setting. Tests compare the kernels bit for bit.
+// of attention_split_kernel), 1 (the default) at head size 64 the streaming kernel where rows x
+// key/value heads are 2,048 or more, and else a block per key tile fed by boxes, 2 the streaming
+// kernel whenever the shape allows, 3 the blocks. The set-up of a persistent block costs more than
+// its steadier stream of loads gains until there is much to stream (measured on B200, streaming /
+// blocks, with the merge: 64 rows x 32 heads 212 / 227 us at 900 to 4,090 keys and 47.4 / 48.8 at
+// 200 to 600; 32 x 32 92.4 / 88.1 at 2,000; 64 x 5 49.9 / 46.5 and 17.8 / 12.3; 32 x 5 26.7 / 22.6).
+// Returns the previous setting. Tests compare the kernels bit for bit.
 BW_API int bw_bf16_attention_stream_mode(int mode) {
   const int before = g_stream_mode;
-  if (mode >= 0 && mode <= 2) g_stream_mode = mode;
+  if (mode >= 0 && mode <= 3) g_stream_mode = mode;
   return before;
 }
 
-// Whether decode steps of this shape can take bw_bf16_attention_stream: head size 64, pages of 8
+// Whether decode steps of this shape can take bw_bf16_attention_stream: head size 64 or 128, pages of 8
 // keys or more that divide a tile of 64, a group of at most 16 heads, rows that start on 16
 // bytes, and a step of at most 512 rows.
 BW_API int bw_bf16_attention_stream_usable(int n, int heads, int kv_heads, int hd, int page, int q_stride) {
@@ -910,6 +940,36 @@ BW_API int bw_bf16_attention_stream(const __nv_bfloat16* qkv, int q_stride, cons
     bw::set_error("attention (stream): %lld work items exceed the limit", items);
     return -1;
   }
+  CUtensorMap map_k, map_v;
+  {  // cache: [page][kv head][slot][d], box = one page of one kv head
+    const cuuint64_t dims[4] = {HD, static_cast<cuuint64_t>(page), static_cast<cuuint64_t>(kv_heads),
+                                static_cast<cuuint64_t>(num_pages)};
+    const cuuint64_t strides[3] = {HD * 2, static_cast<cuuint64_t>(page) * HD * 2,
+                                   static_cast<cuuint64_t>(kv_heads) * page * HD * 2};
+    const cuuint32_t box[4] = {64, static_cast<cuuint32_t>(page), 1, 1};
+    if (!stream_map(&map_k, kcache, dims, strides, box) || !stream_map(&map_v, vcache, dims, strides, box)) {
+      bw::set_error("attention (stream): cuTensorMapEncodeTiled refused the cache map");
+      return -1;
+    }
+  }
+  int* word = bw::failure_word();
+  if (!word) return -1;
+  const float scale_log2 = scale * 1.44269504088896341f;
+  const bool stream_it = HD == 64 && (g_stream_mode == 2 || (g_stream_mode == 1 && static_cast<long long>(n) * kv_heads >= kStreamMinHeads));
+  if (!stream_it) {  // a block per key tile
+    constexpr int tile_smem = kStreamItemBytes + 8 + 1008;  // dynamic shared memory starts on 16 bytes; six blocks fit an SM at head size 128
+    if (key_tiles > 65535 || kv_heads > 65535) {
+      bw::set_error("attention: %d key tiles or %d key/value heads exceed the grid limit", key_tiles, kv_heads);
+      return -1;
+    }
+    bw::launch_pdl(attention_tile_tma_kernel, dim3(n, kv_heads, key_tiles), dim3(32), tile_smem, stream, map_k, map_v, qkv,
+                   q_stride, block_table, max_blocks, row_seq, pos, heads, kv_heads, page, window, scale_log2, scratch,
+                   key_tiles, word);
+    bw::launch_pdl(merge_tiles_kernel, dim3(dim3(n, heads)), dim3(kMergeThreads), 0, stream, scratch, key_tiles, pos, out,
+                   out_stride, heads, window);
+    return bw::launch_status();
+  }
+#if BW_HEAD_DIM == 64
   const int group = heads / kv_heads;
   const int smem = kStreamWarps * kStreamStages * (kStreamItemBytes + 8) + (3 * n + 1) * 4 + 1024;
   constexpr int smem_max = kStreamWarps * kStreamStages * (kStreamItemBytes + 8) + (3 * kStreamMaxRows + 1) * 4 + 1024;
@@ -927,53 +987,28 @@ BW_API int bw_bf16_attention_stream(const __nv_bfloat16* qkv, int q_stride, cons
     if (sms <= 0) sms = 148;
     configured = true;
   }
-  CUtensorMap map_q, map_k, map_v;
+  CUtensorMap map_q;
   {  // queries: [row][kv head][head of the group][d], box = the group's heads of one row
     const cuuint64_t dims[4] = {HD, static_cast<cuuint64_t>(group), static_cast<cuuint64_t>(kv_heads),
                                 static_cast<cuuint64_t>(n)};
     const cuuint64_t strides[3] = {HD * 2, static_cast<cuuint64_t>(group) * HD * 2, static_cast<cuuint64_t>(q_stride) * 2};
-    const cuuint32_t box[4] = {HD, static_cast<cuuint32_t>(group), 1, 1};
+    const cuuint32_t box[4] = {64, static_cast<cuuint32_t>(group), 1, 1};
     if (!stream_map(&map_q, qkv, dims, strides, box)) {
       bw::set_error("attention (stream): cuTensorMapEncodeTiled refused the query map");
       return -1;
     }
   }
-  {  // cache: [page][kv head][slot][d], box = one page of one kv head
-    const cuuint64_t dims[4] = {HD, static_cast<cuuint64_t>(page), static_cast<cuuint64_t>(kv_heads),
-                                static_cast<cuuint64_t>(num_pages)};
-    const cuuint64_t strides[3] = {HD * 2, static_cast<cuuint64_t>(page) * HD * 2,
-                                   static_cast<cuuint64_t>(kv_heads) * page * HD * 2};
-    const cuuint32_t box[4] = {HD, static_cast<cuuint32_t>(page), 1, 1};
-    if (!stream_map(&map_k, kcache, dims, strides, box) || !stream_map(&map_v, vcache, dims, strides, box)) {
-      bw::set_error("attention (stream): cuTensorMapEncodeTiled refused the cache map");
-      return -1;
-    }
-  }
-  int* word = bw::failure_word();
-  if (!word) return -1;
-  const float scale_log2 = scale * 1.44269504088896341f;
-  if (g_stream_mode == 1 && n < kStreamMinRows) {  // few rows: a block per key tile, fed by the same boxes
-    constexpr int tile_smem = kStreamItemBytes + 8 + 1024;
-    if (key_tiles > 65535 || kv_heads > 65535) {
-      bw::set_error("attention: %d key tiles or %d key/value heads exceed the grid limit", key_tiles, kv_heads);
-      return -1;
-    }
-    bw::launch_pdl(attention_tile_tma_kernel, dim3(n, kv_heads, key_tiles), dim3(32), tile_smem, stream, map_k, map_v, qkv,
-                   q_stride, block_table, max_blocks, row_seq, pos, heads, kv_heads, page, window, scale_log2, scratch,
-                   key_tiles, word);
-    bw::launch_pdl(merge_tiles_kernel, dim3(dim3(n, heads)), dim3(kMergeThreads), 0, stream, scratch, key_tiles, pos, out,
-                   out_stride, heads, window);
-    return bw::launch_status();
-  }
-  const long long warps_needed = (items + 0) / 1;
   const unsigned grid = static_cast<unsigned>(
-      warps_needed < static_cast<long long>(sms) * kStreamWarps ? (warps_needed + kStreamWarps - 1) / kStreamWarps : sms);
+      items < static_cast<long long>(sms) * kStreamWarps ? (items + kStreamWarps - 1) / kStreamWarps : sms);
   bw::launch_pdl(attention_stream_kernel, dim3(grid), dim3(kStreamWarps * 32), smem, stream, map_q, map_k, map_v,
                  block_table, max_blocks, row_seq, pos, n, heads, kv_heads, page, window, scale_log2, scratch, key_tiles,
                  word);
   bw::launch_pdl(merge_tiles_kernel, dim3(dim3(n, heads)), dim3(kMergeThreads), 0, stream, scratch, key_tiles, pos, out,
                  out_stride, heads, window);
   return bw::launch_status();
+#else
+  return -1;
+#endif
 }
 #else
 BW_API int bw_bf16_attention_stream_mode(int) { return 0; }

@@ -230,7 +230,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     for (int i = lane; i < staged; i += 32) spages[i] = table[first_page + i];
     __syncwarp();
     if (lane == 0) {
-      mbar_expect_tx(&bars->q_full, kQBytes);
+      mbar_expect_tx(&bars->q_full, kPieces * (kTileM / group) * group * 128);  // a group that does not divide 128 leaves rows empty
       for (int i = 0; i < kPieces; ++i) tma_load_4d(sq + i * kQPiece, &map_q, 64 * i, 0, g, row0, &bars->q_full);
     }
     // A tile of keys and values is pages x pieces x 2 copies (16 at head size 128 with pages of 16),
@@ -299,6 +299,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const uint64_t pdesc = make_desc(smem_u32(sp + b * kPBytes));
       const uint32_t v_addr = smem_u32(skv + s * 2 * kKBytes + kKBytes);
       const uint64_t vdesc = kPieces == 1 ? make_desc(v_addr) : make_desc_wide(v_addr, kKPiece);
+      // Behind the block's last key lies whatever the page's last holder left. Its weights are zero; its values become zero as
+      // well, so that an infinity left there cannot reach a sum.
+      if (t + 1 == ntiles && kv_lo + ntiles * kTileKV > kv_hi) {
+        unsigned char* sv = skv + s * 2 * kKBytes + kKBytes;
+        for (int c = (kv_hi - kv_lo - t * kTileKV) * 8 + lane; c < kTileKV * 8; c += 32)
+#pragma unroll
+          for (int i = 0; i < kPieces; ++i) *reinterpret_cast<uint4*>(sv + i * kKPiece + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+      }
       if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < kTileKV / 16; ++k)  // 16 keys: 32 bytes along a row of P, two 8-key groups (2048 bytes) of V
@@ -475,12 +485,20 @@ bool make_map4(CUtensorMap* map, const void* base, const cuuint64_t (&dims)[4], 
 }  // namespace
 
 // Query rows per block, or 0 when this kernel cannot take the shape: head size 64 or 128, a page size
-// that divides 64, a group of heads that divides 128, rows that start on 16 bytes.
-BW_API int bw_bf16_attention_tc_tile_rows(int heads, int kv_heads, int hd, int page, int q_stride) {
+// that divides 64, rows that start on 16 bytes. A group of heads that does not divide 128 leaves the
+// last one or more of a block's 128 stacked rows empty: what their lanes compute from whatever lies in
+// shared memory there stays in their rows and is never stored. (Groups of 3 used to run on the mma.sync
+// kernel: a mixed step of the SmolLM2-360M shape spent 36 us a layer there.)
+BW_API int bw_bf16_attention_tc_query_rows(int heads, int kv_heads, int hd, int page, int q_stride) {
   if (hd != HD || kv_heads <= 0 || heads % kv_heads) return 0;
   const int group = heads / kv_heads;
-  if (group > kTileM || kTileM % group || page <= 0 || kTileKV % page || q_stride % 8 || !encoder()) return 0;
+  if (group > kTileM || page <= 0 || kTileKV % page || q_stride % 8 || !encoder()) return 0;
   return kTileM / group;
+}
+// The same for groups that fill a block's rows exactly, else 0.
+BW_API int bw_bf16_attention_tc_tile_rows(int heads, int kv_heads, int hd, int page, int q_stride) {
+  const int rows = bw_bf16_attention_tc_query_rows(heads, kv_heads, hd, page, q_stride);
+  return rows && kTileM % (heads / kv_heads) == 0 ? rows : 0;
 }
 
 BW_API int bw_bf16_attention_tc(const __nv_bfloat16* qkv, int q_stride, const __nv_bfloat16* kcache,
@@ -494,7 +512,7 @@ BW_API int bw_bf16_attention_tc(const __nv_bfloat16* qkv, int q_stride, const __
     bw::set_error("attention (tcgen05): %d query tiles exceed the grid limit", num_tiles);
     return -1;
   }
-  const int tile_rows_q = bw_bf16_attention_tc_tile_rows(heads, kv_heads, hd, page, q_stride);
+  const int tile_rows_q = bw_bf16_attention_tc_query_rows(heads, kv_heads, hd, page, q_stride);
   if (!tile_rows_q || out_stride % 8) {
     bw::set_error("attention (tcgen05): unsupported shape (heads %d/%d, head size %d, page %d)", heads, kv_heads, hd, page);
     return -1;
@@ -542,6 +560,7 @@ BW_API int bw_bf16_attention_tc(const __nv_bfloat16* qkv, int q_stride, const __
 
 #else  // other head sizes use the kernels of bf16_attention.cu
 
+BW_API int bw_bf16_attention_tc_query_rows(int, int, int, int, int) { return 0; }
 BW_API int bw_bf16_attention_tc_tile_rows(int, int, int, int, int) { return 0; }
 
 #endif

@@ -335,6 +335,12 @@ class KernelOps:
         if self.kind == "f32":
             self.lib.bw_f32_force_rows_plan(_c_int(tile_cols), _c_int(stages))
 
+    def force_f32_tile(self, tile: int = -1) -> None:
+        """Tests and measurements of the 32-bit path: force the tile that products of more than 16 rows take (0 .. 6; -1:
+        chosen from the shape).  Every one gives the same bits."""
+        if self.kind == "f32":
+            self.lib.bw_f32_force_tile(_c_int(tile))
+
     def pair_tiles(self, on: bool) -> bool:
         """Large batches run two thread blocks per 256 x 256 tile of a product (the default) or
         one per 128 x 256 tile; same bits either way.  Returns the previous setting."""
@@ -419,8 +425,8 @@ class KernelOps:
             return [16]
         group = max(1, heads // kv_heads)
         rows = [max(1, 64 // group)]
-        if 128 % group == 0:
-            rows.append(128 // group)  # the tcgen05 prefill kernel stacks 128 rows per block
+        if 128 // group > rows[0]:
+            rows.append(128 // group)  # the tcgen05 prefill kernel stacks up to 128 rows per block
         return rows
 
     def _attention_scratch(self, lib, device, n: int, heads: int, max_keys: int) -> torch.Tensor:
@@ -576,9 +582,9 @@ class KernelOps:
                 shape_key = (heads, kv_heads, head_dim, page, qkv.shape[1])
                 rows_tc = self._tc_tile_rows.get(shape_key)
                 if rows_tc is None:
-                    rows_tc = int(lib.bw_bf16_attention_tc_tile_rows(_c_int(heads), _c_int(kv_heads),
-                                                                     _c_int(head_dim), _c_int(page),
-                                                                     _c_int(qkv.shape[1])))
+                    rows_tc = int(lib.bw_bf16_attention_tc_query_rows(_c_int(heads), _c_int(kv_heads),
+                                                                      _c_int(head_dim), _c_int(page),
+                                                                      _c_int(qkv.shape[1])))
                     self._tc_tile_rows[shape_key] = rows_tc
                 sets = getattr(batch, "tile_sets", None)
                 if rows_tc > 0 and (sets is None or rows_tc in sets) and n > t_count:

@@ -98,6 +98,28 @@ def test_f32_linear_of_few_rows_every_tile_width_gives_the_chain(m):
     assert not ops.device_failure(), "a kernel gave up a bounded wait"
 
 
+@pytest.mark.parametrize("m,n,k", [(17, 1, 4), (33, 40, 36), (64, 130, 100), (65, 129, 32), (130, 257, 292), (129, 64, 1024)])
+def test_f32_linear_of_more_rows_every_tile_gives_the_chain(m, n, k):
+    """Products of more than 16 rows run on one of seven tiles, chosen for speed; every one must give the plain chain's bits:
+    edges of tiles in both directions, a k that ends inside a line of 32 and inside the ring, more lines than stages."""
+    rng = np.random.default_rng(m + n + k)
+    ops = _ops("float32")
+    x, w, res = rnd(rng, m, k), rnd(rng, n, k, scale=0.1), rnd(rng, m, n)
+    want = P.linear(x, w)
+    try:
+        for tile in range(-1, 7):
+            ops.force_f32_tile(tile)
+            out = torch.empty(m, n, device=DEV)
+            ops.linear(t(x), t(w), out)
+            assert_same_bits(out.cpu().numpy(), want, f"tile {tile}")
+            acc = t(res).clone()
+            ops.linear(t(x), t(w), acc, residual=acc)
+            assert_same_bits(acc.cpu().numpy(), (res + want).astype(np.float32), f"tile {tile}, residual in place")
+    finally:
+        ops.force_f32_tile(-1)
+    assert not ops.device_failure(), "a kernel gave up a bounded wait"
+
+
 def test_f32_linear_row_alone_equals_row_in_batch():
     rng = np.random.default_rng(5)
     x, w = rnd(rng, 50, 200), rnd(rng, 77, 200)
@@ -724,6 +746,59 @@ def test_bf16_attention_streaming_decode_kernel_gives_the_same_bits():
                 ops.stream_attention(hd, before)
         assert_same_bits(outs[2], outs[0], f"streaming: heads {heads}/{kv_heads} page {page} window {window}")
         assert_same_bits(outs[1], outs[0], f"a block per tile with TMA boxes: heads {heads}/{kv_heads} page {page} window {window}")
+    assert not ops.device_failure()
+
+
+@pytest.mark.parametrize("hd,heads,kv_heads,page,window", [(64, 3, 1, 16, 0), (64, 15, 5, 16, 0), (64, 5, 1, 8, 60), (64, 14, 2, 16, 0),
+                                                           (128, 6, 2, 16, 0), (128, 33, 1, 16, 0), (64, 64, 1, 16, 0)])
+def test_bf16_attention_tcgen05_takes_groups_that_leave_rows_of_a_block_empty(hd, heads, kv_heads, page, window):
+    """Groups of heads that do not divide a block's 128 stacked rows: the bits of the mma.sync kernel, whole prompts, portions
+    that end inside a block, and single rows beside them."""
+    rng = np.random.default_rng(heads)
+    ops = _ops("bfloat16")
+    lens = [200, 70, 129, 66]
+    k, v, table, _, _ = _paged(rng, lens, kv_heads, hd, page)
+    rows_by_seq = [(0, 200), (10, 60), (128, 1), (65, 1)]
+    q = bf(rnd(rng, sum(c for _, c in rows_by_seq), heads, hd))
+    k, v = bf(k), bf(v)
+    for s, n in enumerate(lens):  # what an earlier holder of the page left behind the last key must not be seen
+        last = table[s][(n - 1) // page]
+        k[last, :, (n - 1) % page + 1:], v[last, :, (n - 1) % page + 1:] = np.inf, np.inf
+    new, _, _ = _run_bf16_attention(q, rows_by_seq, k, v, table, heads, kv_heads, hd, window)
+    ops.legacy_attention = True
+    try:
+        old, _, _ = _run_bf16_attention(q, rows_by_seq, k, v, table, heads, kv_heads, hd, window)
+    finally:
+        ops.legacy_attention = False
+    assert np.isfinite(new).all()
+    assert_same_bits(new, old, f"heads {heads}/{kv_heads}")
+    assert not ops.device_failure()
+
+
+@pytest.mark.parametrize("heads,kv_heads,page,window", [(4, 1, 16, 0), (2, 2, 8, 0), (32, 2, 64, 0), (6, 2, 32, 130), (8, 8, 16, 0)])
+def test_bf16_attention_decode_of_wide_heads_through_boxes_gives_the_same_bits(heads, kv_heads, page, window):
+    """Head size 128: persistent blocks, a block per key tile, and the cp.async blocks; rows that end on a tile's first and last
+    key among them.  What an earlier holder of a page left behind a row's last key (infinities here) must not be seen."""
+    hd = 128
+    rng = np.random.default_rng(heads + page)
+    ops = _ops("bfloat16")
+    lens = [300, 129, 192, 193, 640]
+    k, v, table, _, _ = _paged(rng, lens, kv_heads, hd, page)
+    k, v = bf(k), bf(v)
+    rows = [(n - 1, 1) for n in lens]
+    q = bf(rnd(rng, len(lens), heads, hd))
+    for s, n in enumerate(lens):
+        last = table[s][(n - 1) // page]
+        k[last, :, (n - 1) % page + 1:], v[last, :, (n - 1) % page + 1:] = np.inf, np.inf
+    outs = {}
+    for mode in (0, 1, 2, 3):
+        before = ops.stream_attention(hd, mode)
+        try:
+            outs[mode], _, _ = _run_bf16_attention(q, rows, k, v, table, heads, kv_heads, hd, window)
+        finally:
+            ops.stream_attention(hd, before)
+        assert np.isfinite(outs[mode]).all(), f"mode {mode}"
+        assert_same_bits(outs[mode], outs[0], f"mode {mode}")
     assert not ops.device_failure()
 
 
