@@ -174,88 +174,6 @@ gemm_exact_kernel(const float* __restrict__ X, const float* __restrict__ W, floa
 }
 
 // ---------------------------------------------------------------------------------------
-// The same product for large batches (prefill) whose rows start on 16 bytes: tiles of
-// 128 x 128 outputs, a thread carries 8 x 8 of them (each still one chain, k ascending), so that
-// four 16-byte reads from shared memory feed 64 multiply-adds; the next k-tile is fetched
-// into registers while this one is used, and two buffers in shared memory leave one barrier
-// per k-tile.
-constexpr int kBigBM = 128, kBigBN = 128, kBigBK = 16;
-
-__global__ void __launch_bounds__(256, 2)
-gemm_exact_big_kernel(const float* __restrict__ X, const float* __restrict__ W, float* Y, const float* residual, int M,
-                      int N, int K) {
-  __shared__ __align__(16) float As[2][kBigBK][kBigBM + 4];
-  __shared__ __align__(16) float Bs[2][kBigBK][kBigBN + 4];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;  // columns 4 tx .. + 3 and 64 + 4 tx .. + 3, rows 8 ty .. + 7
-  const int m0 = blockIdx.y * kBigBM, n0 = blockIdx.x * kBigBN;
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-  // a thread fetches two 16-byte pieces of x and two of W per k-tile: piece p = tid + 256 i is
-  // row p / 4, k-quarter p % 4
-  float4 xa[2], wb[2];
-  auto fetch = [&](int k0) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int pc = tid + 256 * i, row = pc >> 2, gk = k0 + (pc & 3) * 4;
-      const int gm = m0 + row, gn = n0 + row;
-      xa[i] = (gm < M && gk < K) ? *reinterpret_cast<const float4*>(X + static_cast<size_t>(gm) * K + gk)
-                                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // K is a multiple of 4
-      wb[i] = (gn < N && gk < K) ? *reinterpret_cast<const float4*>(W + static_cast<size_t>(gn) * K + gk)
-                                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-  };
-  auto stash = [&](int buf) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int pc = tid + 256 * i, row = pc >> 2, kq = (pc & 3) * 4;
-      As[buf][kq + 0][row] = xa[i].x, As[buf][kq + 1][row] = xa[i].y;
-      As[buf][kq + 2][row] = xa[i].z, As[buf][kq + 3][row] = xa[i].w;
-      Bs[buf][kq + 0][row] = wb[i].x, Bs[buf][kq + 1][row] = wb[i].y;
-      Bs[buf][kq + 2][row] = wb[i].z, Bs[buf][kq + 3][row] = wb[i].w;
-    }
-  };
-  fetch(0);
-  stash(0);
-  __syncthreads();
-  const int tiles = (K + kBigBK - 1) / kBigBK;
-  for (int t = 0; t < tiles; ++t) {
-    const int buf = t & 1;
-    if (t + 1 < tiles) fetch((t + 1) * kBigBK);
-#pragma unroll
-    for (int k = 0; k < kBigBK; ++k) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][k][ty * 8]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][k][ty * 8 + 4]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[buf][k][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[buf][k][64 + tx * 4]);
-      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = __fmaf_rn(a[i], b[j], acc[i][j]);
-    }
-    if (t + 1 < tiles) stash(buf ^ 1);  // nobody reads that buffer: its tile was used before the last barrier
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gm = m0 + ty * 8 + i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int gn = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-      if (gn >= N) continue;
-      const size_t o = static_cast<size_t>(gm) * N + gn;
-      Y[o] = residual ? __fadd_rn(residual[o], acc[i][j]) : acc[i][j];
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------------------
 // The same product for steps of few rows (decode steps, up to 16 rows), where the weights are
 // all that is read: one chain per output as above (k ascending, fma after fma). The tiles of W
 // and x come through a ring of stages that a warp of its own requests; blocks stay for the
@@ -1255,11 +1173,228 @@ int launch_rows(const CUtensorMap& map_x, const CUtensorMap& map_w, float* y, co
   }
   return bw::launch_status();
 }
+
+// ---------------------------------------------------------------------------------------
+// The same product for more than 16 rows (prompt portions, large decode batches) whose rows start on 16 bytes: every output
+// is still one chain, k ascending.
+//
+// Bound by how the multiply-adds are fed: a warp's read of 16 bytes per lane holds its scheduler's register port for 16 cycles,
+// so a lane with TR x TC outputs spends 4 (TR + TC) cycles per value of k on reads beside TR TC on multiply-adds, and the two
+// overlap only as far as registers are left to read ahead. 8 x 8 outputs (64 to 64; 255 registers, two blocks of four warps on
+// an SM) and 4 x 8 (48 to 32, but 12 warps) come out alike at 48 to 50 TFLOP/s of the 74 that the cores offer; 8 x 16, 6 x 8 and
+// pairs of multiply-adds (fma.rn.f32x2) were no better or worse. A lane's values are four consecutive k of a row, so both
+// matrices stay as they lie in memory: a stage is one line of 32 values of k for the tile's rows of x and of W, two TMA boxes
+// with the 128-byte swizzle; no value passes through registers on its way to shared memory, and warps meet only at the ring's
+// barriers. Lane (ty, tx) of a warp (4 x 8) has rows ty + 4 i and columns tx + 8 j of the warp's part, so that the eight lanes
+// of a quarter warp read eight neighbouring rows of W (no bank twice) and the four values of ty four neighbouring rows of x.
+//
+// Small products have too few large tiles for the SMs, and a tile's chain of k steps is their time (8,192 steps of a block alone
+// with 8 x 8 outputs per lane: 730 us, with 2 x 2: 125); smaller tiles read more per multiply-add but fill the machine.
+// tile_plan below picks. Before, with tiles of 128 x 128 (64 x 64 up to 64 rows) fetched through registers, and now:
+// 2,048 x 2,048 x 16,384 3,105 -> 2,760 us; 512 x 8,192 x 2,048 1,063 -> 445; 128 x 2,048 x 6,144 279 -> 98;
+// 53 x 8,192 x 2,048 632 -> 152.
+template <int TR, int TC, int WR, int WC, int BLOCKS>
+struct TileShape {
+  static constexpr int BM = 4 * TR * WR, BN = 8 * TC * WC;
+  static constexpr int kWarps = WR * WC;
+  static constexpr int kThreads = kWarps * 32;  // (a fifth warp for the copies would cost a scheduler a third of its registers)
+  static constexpr int kXBytes = BM * 128, kStageBytes = (BM + BN) * 128;
+  static constexpr int kBlocks = BLOCKS;  // blocks that share an SM
+  static constexpr int kFit = (224 * 1024 / kBlocks - 1024 - 256) / kStageBytes;
+  static constexpr int kStages = kFit > 6 ? 6 : kFit;
+  static constexpr int kSmem = kStages * (kStageBytes + 16) + 1024;
+  static_assert(BM % 8 == 0 && BN % 8 == 0 && BM <= 256 && BN <= 256 && kStages >= 2, "tile shape");
+};
+
+template <int TR, int TC, int WR, int WC, int BLOCKS>
+__global__ void __launch_bounds__(TileShape<TR, TC, WR, WC, BLOCKS>::kThreads, TileShape<TR, TC, WR, WC, BLOCKS>::kBlocks)
+gemm_exact_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, float* Y,
+                       const float* residual, int M, int N, int K, int* failure) {
+  using S = TileShape<TR, TC, WR, WC, BLOCKS>;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* ring = bw::smem_align_1024(smem_raw);
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + S::kStages * S::kStageBytes);
+  uint64_t* empty = full + S::kStages;
+  volatile uint32_t* gave_up = reinterpret_cast<volatile uint32_t*>(failure);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.y * S::BM, n0 = blockIdx.x * S::BN;
+  const int lines = (K + kRowsTileK - 1) / kRowsTileK;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S::kStages; ++s) bar_init(full + s, 1), bar_init(empty + s, S::kWarps);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  // Warp 0 asks for the lines: the first round at once (the weights before the wait for the kernel before this one, which they
+  // do not depend on), later ones when the stage's last line has been used by all warps, a line after it was: no warp waits
+  // for the slowest one, and the lines in between are on their way.
+  auto box = [&](void* dst, const CUtensorMap* map, int line, int row, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(smem_addr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(line * kRowsTileK), "r"(row), "r"(smem_addr(bar))
+        : "memory");
+  };
+  const int early = min(lines, S::kStages);
+  if (threadIdx.x == 0)
+    for (int t = 0; t < early; ++t) {
+      bar_expect(full + t, S::kStageBytes);
+      box(ring + t * S::kStageBytes + S::kXBytes, &map_w, t, n0, full + t);
+    }
+  bw::pdl_wait();
+  if (threadIdx.x == 0)
+    for (int t = 0; t < early; ++t) box(ring + t * S::kStageBytes, &map_x, t, m0, full + t);
+  __syncwarp();
+  const int tx = lane & 7, ty = lane >> 3;
+  const int r0 = (warp / WC) * 4 * TR + ty, c0 = (warp % WC) * 8 * TC + tx;  // this lane's first row and column of the tile
+  float acc[TR][TC];
+#pragma unroll
+  for (int i = 0; i < TR; ++i)
+#pragma unroll
+    for (int j = 0; j < TC; ++j) acc[i][j] = 0.0f;
+  constexpr int JB = TC < 4 ? TC : 4;  // columns whose values are held at a time
+  // 16-byte piece p of a swizzled line sits at piece p ^ (row % 8): rows ty + 4 i and columns tx + 8 j of the tile
+  auto piece = [&](const unsigned char* xs, const unsigned char* ws, int p) {
+    float4 a[TR];
+#pragma unroll
+    for (int i = 0; i < TR; ++i) a[i] = *reinterpret_cast<const float4*>(xs + i * 512 + ((p ^ (ty + 4 * (i & 1))) << 4));
+#pragma unroll
+    for (int j0 = 0; j0 < TC; j0 += JB) {
+      float4 b[JB];
+#pragma unroll
+      for (int j = 0; j < JB; ++j) b[j] = *reinterpret_cast<const float4*>(ws + (j0 + j) * 1024 + ((p ^ tx) << 4));
+#pragma unroll
+      for (int i = 0; i < TR; ++i)
+#pragma unroll
+        for (int j = 0; j < JB; ++j) acc[i][j0 + j] = __fmaf_rn(a[i].x, b[j].x, acc[i][j0 + j]);
+#pragma unroll
+      for (int i = 0; i < TR; ++i)
+#pragma unroll
+        for (int j = 0; j < JB; ++j) acc[i][j0 + j] = __fmaf_rn(a[i].y, b[j].y, acc[i][j0 + j]);
+#pragma unroll
+      for (int i = 0; i < TR; ++i)
+#pragma unroll
+        for (int j = 0; j < JB; ++j) acc[i][j0 + j] = __fmaf_rn(a[i].z, b[j].z, acc[i][j0 + j]);
+#pragma unroll
+      for (int i = 0; i < TR; ++i)
+#pragma unroll
+        for (int j = 0; j < JB; ++j) acc[i][j0 + j] = __fmaf_rn(a[i].w, b[j].w, acc[i][j0 + j]);
+    }
+  };
+  int s = 0, before = 0;  // stage of this line, and of the one before
+  uint32_t parity = 0, before_parity = 0;
+  for (int t = 0; t < lines; ++t) {
+    if (!bar_try(full + s, parity)) bw::mbar_wait_bounded(full + s, parity, gave_up);
+    if (warp == 0 && t > 0 && t - 1 + S::kStages < lines) {
+      const bool free = bw::mbar_wait_bounded(empty + before, before_parity, gave_up);
+      if (lane == 0 && free) {
+        bar_expect(full + before, S::kStageBytes);
+        box(ring + before * S::kStageBytes, &map_x, t - 1 + S::kStages, m0, full + before);
+        box(ring + before * S::kStageBytes + S::kXBytes, &map_w, t - 1 + S::kStages, n0, full + before);
+      }
+      __syncwarp();
+    }
+    before = s, before_parity = parity;
+    const unsigned char* xs = ring + s * S::kStageBytes + r0 * 128;
+    const unsigned char* ws = ring + s * S::kStageBytes + S::kXBytes + c0 * 128;
+    const int left = (K - t * kRowsTileK) / 4;  // K is a multiple of 4: pieces beyond it are not walked
+    if (left >= 8) {
+#pragma unroll
+      for (int p = 0; p < 8; ++p) piece(xs, ws, p);
+    } else {
+      for (int p = 0; p < left; ++p) piece(xs, ws, p);
+    }
+    __syncwarp();
+    if (lane == 0) bar_arrive(empty + s);
+    if (++s == S::kStages) s = 0, parity ^= 1;
+  }
+#pragma unroll
+  for (int i = 0; i < TR; ++i) {
+    const int gm = m0 + r0 + 4 * i;
+    if (gm >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TC; ++j) {
+      const int gn = n0 + c0 + 8 * j;
+      if (gn >= N) continue;
+      const size_t o = static_cast<size_t>(gm) * N + gn;
+      Y[o] = residual ? __fadd_rn(residual[o], acc[i][j]) : acc[i][j];
+    }
+  }
+}
+
+// row-major rows x k floats (k a multiple of 4), boxes of box_rows rows x 32 values, 128-byte swizzle, zeros outside
+bool f32_tile_map(CUtensorMap* map, const void* base, int rows, int k, int box_rows) {
+  EncodeTiledF32 enc = f32_encoder();
+  if (!enc) return false;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k) * 4};
+  const cuuint32_t box[2] = {kRowsTileK, static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t elem[2] = {1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int TR, int TC, int WR, int WC, int BLOCKS>
+int launch_tile(const float* x, const float* w, float* y, const float* residual, int m, int n, int k, cudaStream_t stream) {
+  using S = TileShape<TR, TC, WR, WC, BLOCKS>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_exact_tile_kernel<TR, TC, WR, WC, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
+    if (e != cudaSuccess) {
+      bw::set_error("linear (32-bit): cannot raise shared memory: %s", cudaGetErrorString(e));
+      return static_cast<int>(e);
+    }
+    configured = true;
+  }
+  int* word = bw::failure_word();
+  if (!word) return -1;
+  CUtensorMap map_x, map_w;
+  if (!f32_tile_map(&map_x, x, m, k, S::BM) || !f32_tile_map(&map_w, w, n, k, S::BN)) {
+    bw::set_error("linear (32-bit): cuTensorMapEncodeTiled refused [%d x %d] / [%d x %d]", m, k, n, k);
+    return -1;
+  }
+  const unsigned gy = (m + S::BM - 1) / S::BM;
+  if (gy > 65535u) {
+    bw::set_error("linear: %d rows exceed the grid limit", m);
+    return -1;
+  }
+  bw::launch_pdl(gemm_exact_tile_kernel<TR, TC, WR, WC, BLOCKS>, dim3((n + S::BN - 1) / S::BN, gy), dim3(S::kThreads), static_cast<size_t>(S::kSmem),
+                 stream, map_x, map_w, y, residual, m, n, k, word);
+  return bw::launch_status();
+}
+
+// The tile of a product of more than 16 rows: 0 the kernel of 128 x 128 tiles, else by index into BW_F32_TILES; the one whose
+// estimated time is least. Cycles per value of k as measured on a B200: a block alone on its SM (its chain's own time), and its
+// share where its SM has as many blocks as fit.
+#define BW_F32_TILES(X_) X_(0, 8, 8, 2, 2, 2) X_(1, 4, 8, 4, 1, 3) X_(2, 4, 4, 4, 1, 3) X_(3, 4, 2, 4, 1, 3) X_(4, 4, 4, 2, 2, 3) X_(5, 4, 2, 2, 2, 3) X_(6, 2, 2, 4, 1, 3)
+struct TileCost {
+  int bm, bn, fit, alone, share;  // rows, columns, blocks per SM, cycles per value of k alone and as one of many
+};
+constexpr TileCost kTileCosts[] = {{64, 128, 2, 179, 95}, {64, 64, 3, 72, 50}, {64, 32, 3, 50, 29}, {64, 16, 3, 39, 19},
+                                   {32, 64, 3, 50, 29},    {32, 32, 3, 39, 18}, {32, 16, 3, 32, 13}};
+int g_forced_tile = -1;
+
+int tile_plan(int m, int n) {
+  if (g_forced_tile >= 0) return g_forced_tile;
+  const int sms = sm_count();
+  int best = 0;
+  long long best_cost = -1;
+  for (int i = 0; i < 7; ++i) {
+    const TileCost& c = kTileCosts[i];
+    const long long blocks = static_cast<long long>((m + c.bm - 1) / c.bm) * ((n + c.bn - 1) / c.bn);
+    const long long per_sm = (blocks + sms - 1) / sms, rounds = per_sm / c.fit, rest = per_sm % c.fit;
+    auto together = [&](long long count) { return count * c.share > c.alone ? count * c.share : c.alone; };
+    const long long cost = rounds * together(c.fit) + (rest ? together(rest) : 0);
+    if (best_cost < 0 || cost < best_cost) best = i, best_cost = cost;
+  }
+  return best;
+}
 }  // namespace
 
 // For measurements and tests: fixes the streaming tile's width (16, 32, 64 or 128 columns) and
 // the stages of its ring for the products that follow (0: the library's own choice).
 BW_API void bw_f32_force_rows_plan(int tile_cols, int stages) { g_forced_tile_cols = tile_cols, g_forced_stages = stages; }
+
+// The same for the tile of products of more than 16 rows (0..6; -1: the library's own choice).
+BW_API void bw_f32_force_tile(int tile) { g_forced_tile = tile >= 0 && tile <= 6 ? tile : -1; }
 
 // ---------------------------------------------------------------------------------------
 // Exported entry points.
@@ -1327,13 +1462,14 @@ BW_API int bw_f32_linear(const float* x, const float* w, float* y, const float* 
     return -1;
   } else if (m <= 16) {
     gemm_exact_kernel<16><<<dim3(gx, (m + 15) / 16), 256, 0, stream>>>(x, w, y, residual, m, n, k);
-  } else if (m > 64 && k % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
-    const unsigned gy = (m + kBigBM - 1) / kBigBM;
-    if (gy > 65535u) {
-      bw::set_error("linear: %d rows exceed the grid limit", m);
-      return -1;
+  } else if (k % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && f32_encoder() != nullptr) {
+    switch (tile_plan(m, n)) {
+#define BW_CASE(I_, TR_, TC_, WR_, WC_, BLOCKS_) \
+  case I_: return launch_tile<TR_, TC_, WR_, WC_, BLOCKS_>(x, w, y, residual, m, n, k, stream);
+      BW_F32_TILES(BW_CASE)
+#undef BW_CASE
     }
-    gemm_exact_big_kernel<<<dim3((n + kBigBN - 1) / kBigBN, gy), 256, 0, stream>>>(x, w, y, residual, m, n, k);
+    return -1;
   } else {
     const unsigned gy = (m + 63) / 64;
     if (gy > 65535u) {
