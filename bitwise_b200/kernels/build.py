@@ -29,7 +29,7 @@ BASE_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompil
 KERNEL_SETS: Dict[str, List[tuple]] = {
     "f32": [("common.cu", []), ("sampling.cu", []), ("exact_f32.cu", ["-fmad=false"])],
     "bf16": [("common.cu", []), ("sampling.cu", []), ("bf16_ops.cu", []), ("bf16_gemm.cu", []), ("bf16_gemm_tc.cu", []),
-             ("bf16_gemm_rows.cu", [])],
+             ("bf16_gemm_rows.cu", []), ("block_step.cu", [])],
     # compiled once per head size, with -DBW_HEAD_DIM=<n>
     "bf16_attn": [("common.cu", []), ("bf16_attention.cu", []), ("bf16_attention_tc.cu", [])],
     # parts that only some architectures have (layer norm, latent attention, routed feed-forward):

@@ -7,6 +7,7 @@ constructor raises, and every call checks that its tensors live on a CUDA device
 """
 from __future__ import annotations
 
+import array
 import ctypes
 from typing import Optional
 
@@ -61,6 +62,7 @@ class KernelOps:
 
     OUT_ACTIVATIONS = (None, "relu2", "tanh")  # what a product's outputs can pass before they are stored, by index
     FUSED_ACTIVATIONS = ("silu", "gelu_tanh")  # what the gate/up product can apply in its epilogue, by index
+    BLOCK_CALL_MEMBERS = 53  # 64-bit members of the library's block call (block_step.cu)
 
     def __init__(self, dtype: str, verbose_build: bool = True):
         if dtype not in ("float32", "bfloat16"):
@@ -88,6 +90,7 @@ class KernelOps:
         self._retired = []
         self._attn_scratch: Optional[torch.Tensor] = None
         self._fns = {}
+        self._block_fns = {}  # head size -> the attention library's entry points, as addresses
         self._dev_index: Optional[int] = None
         self._scratch_sizes = {}
         self._kernel_counts = {}
@@ -628,6 +631,80 @@ class KernelOps:
                 raise KernelError(f"bw_bf16_attention failed ({rc}): "
                                   + lib.bw_last_error().decode("utf-8", "replace"))
             self.launches += 2 if split else 1
+
+    def prenorm_block(self, ctx, x: torch.Tensor, cache, block) -> bool:
+        """All launches of one pre-norm block (RMSNorm, grouped-query attention, RMSNorm, dense SwiGLU) in one call of the
+        library, as the block's parts would make them one by one; ``block`` = (norm1, mixer, norm2, feed_forward).  False,
+        with nothing launched, for what the call does not take: the parts then run, with their own checks."""
+        if self.kind != "bf16" or self.legacy_attention:
+            return False
+        norm1, mixer, norm2, ffn = block
+        n, width, heads, kv_heads, hd = ctx.n, mixer.width, mixer.heads, mixer.kv_heads, mixer.head_dim
+        q_dim, qkv_dim, inter, bf16 = mixer.q_dim, mixer.q_dim + 2 * mixer.kv_dim, ffn.intermediate, torch.bfloat16
+        k, v, table = cache.k, cache.v, cache.block_table
+        if k.dim() != 4:
+            return False
+        pages, page = k.shape[0], k.shape[2]
+        w_qkv, w_o, w_gu, w_down = mixer.w_qkv, mixer.w_o, ffn.w_gate_up, ffn.w_down
+        tables = mixer.position.rotary_tables(x.device) if mixer.position is not None else None
+        cos, sin = tables if tables is not None else (None, None)
+        if hd % 16 or not 16 <= hd <= 256 or heads % kv_heads or norm1.width != width or norm2.width != width or ffn.width != width:
+            return False
+        for t_, dtype, shape in ((x, torch.float32, (n, width)), (k, bf16, (pages, kv_heads, page, hd)), (v, bf16, (pages, kv_heads, page, hd)),
+                                 (w_qkv, bf16, (qkv_dim, width)), (w_o, bf16, (width, q_dim)), (w_gu, bf16, (2 * inter, width)),
+                                 (w_down, bf16, (width, inter)), (norm1.weight, torch.float32, (width,)),
+                                 (norm2.weight, torch.float32, (width,))):
+            if t_ is None or t_.dtype is not dtype or t_.shape != shape or not t_.is_cuda or not t_.is_contiguous():
+                return False
+        if table.dtype is not torch.int32 or table.dim() != 2 or not table.is_contiguous():
+            return False
+        if cos is not None and (cos.dtype is not torch.float32 or cos.shape[1] != hd // 2 or cos.shape != sin.shape
+                                or not cos.is_contiguous() or not sin.is_contiguous()):
+            return False
+        lib = self._attention_lib(hd)
+        fns = self._block_fns.get(hd)
+        if fns is None:
+            if int(self.lib.bw_bf16_block_members()) != self.BLOCK_CALL_MEMBERS:
+                raise KernelError("the library's block call has other members than this binding")
+            names = ("bw_bf16_attention", "bw_bf16_attention_tc", "bw_bf16_attention_tc_query_rows", "bw_bf16_attention_stream",
+                     "bw_bf16_attention_stream_usable")
+            # (a head size without a kernel has no entry point for it, and its query says so)
+            fns = self._block_fns[hd] = tuple(ctypes.cast(getattr(lib, f), ctypes.c_void_p).value if hasattr(lib, f) else 0 for f in names)
+        group = heads // kv_heads
+        sets = ctx.tile_sets
+        rows, rows_tc = max(1, 64 // group), 128 // group
+        if rows not in sets:
+            return False
+        t_seq, t_row0, t_rows, t_count = sets[rows]
+        c_seq, c_row0, c_rows, c_count = sets.get(rows_tc, (None, None, None, 0))
+        has_tc = rows_tc if c_seq is not None else 0
+        workspace = ctx.workspace
+        buffers = [workspace.rows("normed", n, width, bf16), workspace.rows("qkv", n, qkv_dim, bf16), workspace.rows("attn", n, q_dim, bf16),
+                   workspace.rows("ffn_h", n, inter, bf16)]
+        gate_up = 0 if ffn.fused else workspace.rows("gate_up", n, 2 * inter, bf16).data_ptr()
+        partials = counters = attn_scratch = 0
+        if n <= self._split_rows:
+            for out, inner in ((qkv_dim, width), (width, q_dim), (2 * inter, width), (width, inter)):
+                self._linear_scratch(x.device, out, inner)
+            partials, counters = self._partials.data_ptr() if self._partials is not None else 0, self._counters.data_ptr()
+        if t_count == n and ctx.max_keys > 128:
+            attn_scratch = self._attention_scratch(lib, x.device, n, heads, ctx.max_keys).data_ptr()
+        ptr = lambda t_: 0 if t_ is None else t_.data_ptr()
+        call = array.array("q", (
+            x.data_ptr(), *(b.data_ptr() for b in buffers), gate_up, partials, counters, attn_scratch,
+            norm1.weight.data_ptr(), norm2.weight.data_ptr(), w_qkv.data_ptr(), w_o.data_ptr(), w_gu.data_ptr(), w_down.data_ptr(),
+            int(ffn.fused), width, heads, kv_heads, hd, inter, mixer.window or 0, ptr(cos), ptr(sin),
+            k.data_ptr(), v.data_ptr(), pages, page, int(cache.writable), table.data_ptr(), table.shape[1],
+            n, ctx.max_keys, ctx.pos.data_ptr(), ctx.row_seq.data_ptr(), ctx.seq_pos0.data_ptr(), ctx.seq_row0.data_ptr(),
+            t_seq.data_ptr(), t_row0.data_ptr(), t_rows.data_ptr(), t_count, has_tc, ptr(c_seq), ptr(c_row0), ptr(c_rows), c_count,
+            *fns, 0, 0))
+        rc = self.lib.bw_bf16_block(ctypes.c_void_p(call.buffer_info()[0]), _c_float(norm1.eps), _c_float(norm2.eps),
+                                    _c_float(mixer.scale), self._stream())
+        if rc != 0:
+            failed = lib if call[-1] else self.lib
+            raise KernelError(f"bw_bf16_block failed ({rc}): " + failed.bw_last_error().decode("utf-8", "replace"))
+        self.launches += call[-2]
+        return True
 
     def swiglu(self, gate_up: torch.Tensor, out: torch.Tensor) -> None:
         """out = silu(gate) * up for rows laid out [gate | up]."""

@@ -13,7 +13,10 @@ from typing import Dict, List, Optional
 import torch
 
 from ..weights.loader import KEEP32, ParamSpec
-from .base import FeedForward, Mixer, Norm, Part, SlotStateNeed, StepContext
+from .attention import GQAAttention
+from .base import FeedForward, Mixer, Norm, PagedKVView, Part, SlotStateNeed, StepContext
+from .mlp import SwiGLU
+from .norm import RMSNorm
 
 
 class PreNormBlock(Part):
@@ -63,6 +66,8 @@ class PreNormBlock(Part):
 
     def forward(self, ctx: StepContext, x: torch.Tensor, cache) -> None:
         """Run the block on the float32 stream ``x`` in place."""
+        if self._in_one_call(ctx, x, cache):
+            return
         xn = ctx.workspace.rows("normed", ctx.n, self.width, ctx.act_dtype)
         if not self.opened:
             self.mixer_norm.forward(ctx, x, xn)
@@ -76,6 +81,19 @@ class PreNormBlock(Part):
             self.mixer.forward(ctx, xn, x, cache)
             self.ffn_norm.forward(ctx, x, xn)
         self.feed_forward.forward(ctx, xn, x, **last)
+
+
+    def _in_one_call(self, ctx: StepContext, x: torch.Tensor, cache) -> bool:
+        """The plain arrangement of exactly these parts goes to the kernel library as one call, where the library offers it
+        and takes the sizes: the launches are those that the parts make below."""
+        call = getattr(ctx.ops, "prenorm_block", None)
+        if call is None or self.opened or self.next_norm is not None or type(cache) is not PagedKVView:
+            return False
+        if type(self.mixer) is not GQAAttention or type(self.feed_forward) is not SwiGLU or self.feed_forward.activation != "silu":
+            return False
+        if type(self.mixer_norm) is not RMSNorm or type(self.ffn_norm) is not RMSNorm:
+            return False
+        return call(ctx, x, cache, (self.mixer_norm, self.mixer, self.ffn_norm, self.feed_forward))
 
 
 def chain_norms(blocks) -> None:
