@@ -26,6 +26,7 @@
 // memory and the block drains and returns instead of hanging; the host reports the flag.
 #include <cuda.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "bw_common.cuh"
@@ -48,15 +49,23 @@ constexpr int kStoreBytes = 32 * 128;          // per epilogue warp: 32 rows x 1
 // The W tile of a stage holds w_rows rows: 128 (256 for a wide tile), or fewer, in steps of
 // 16, when a product has too few columns to give every SM a 128-column tile: a decode step
 // then runs more, narrower tiles instead of cutting k further.
-constexpr int kMaxStages = 32;
+//
+// A stage of a narrow tile holds up to kMaxTilesPerStage k-tiles, as many as leave three stages: a turn of the loops that ask
+// for a stage and use it costs their warps some 300 cycles of barrier operations whatever it holds, and the four MMAs of a
+// narrow k-tile take 120 (64 rows x 8,192 x 2,048 in tiles of 32 columns: 42 -> 27 us, of 64: 45 -> 36). Wide tiles keep one:
+// their MMAs take 500 cycles, and a ring of few large stages covers less of the memory's latency.
+constexpr int kMaxStages = 32, kMaxTilesPerStage = 4;
 struct RingShape {
-  int tile_bytes_x, stage_bytes, stages, pad_bytes, ring_bytes;
+  int tile_bytes_x, tile_bytes, per_stage, stage_bytes, stages, pad_bytes, ring_bytes;
 };
-__host__ __device__ inline RingShape ring_shape(int a_rows, int w_rows) {
+__host__ __device__ inline RingShape ring_shape(int a_rows, int w_rows, bool wide) {
   RingShape r;
   r.tile_bytes_x = a_rows * BK * 2;
-  r.stage_bytes = r.tile_bytes_x + w_rows * BK * 2;
+  r.tile_bytes = r.tile_bytes_x + w_rows * BK * 2;
   r.pad_bytes = (BM - a_rows) * BK * 2;  // behind the last stage
+  r.per_stage = wide ? 1 : kMaxTilesPerStage;
+  while (r.per_stage > 1 && (kSmemBudget - r.pad_bytes) / (r.per_stage * r.tile_bytes) < 3) r.per_stage >>= 1;
+  r.stage_bytes = r.per_stage * r.tile_bytes;
   const int fit = (kSmemBudget - r.pad_bytes) / r.stage_bytes;
   r.stages = fit > kMaxStages ? kMaxStages : fit;
   r.ring_bytes = r.stages * r.stage_bytes + r.pad_bytes;
@@ -195,19 +204,6 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[64]) {
   uint32_t r[64];
   asm volatile(
@@ -400,8 +396,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   constexpr int LDW = WIDE ? 64 : 32;       // columns per tcgen05.ld (what the register budget allows)
   constexpr int kTmemColsT = 2 * BNT;  // two accumulators
   const int bt = WIDE ? BNT : bn;           // columns of a work item's tile (bn: 16 .. 128 in steps of 16)
-  const RingShape ring = ring_shape(A_ROWS, WIDE ? BNW : bn);
-  const int kStages = ring.stages, kStageBytes = ring.stage_bytes, kTileBytesX = ring.tile_bytes_x;
+  const RingShape ring = ring_shape(A_ROWS, WIDE ? BNW : bn, WIDE);
+  const int kStages = ring.stages, kPer = ring.per_stage, kStageBytes = ring.stage_bytes, kTileBytes = ring.tile_bytes,
+            kTileBytesX = ring.tile_bytes_x;
   Barriers* bars = reinterpret_cast<Barriers*>(tiles + ring.ring_bytes + kEpiWarps * kStoreBytes);
   volatile uint32_t* failed = &bars->failed;
 
@@ -495,11 +492,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     bool ok = true, waited = false;
     // In a pair both blocks' loads are counted on the "full" barrier of rank 0, which
     // expects the bytes of both; each block waits on its own "empty" barrier.
-    auto expect = [&](int st) {
+    auto expect = [&](int st, int count) {
       if (!PAIR)
-        mbar_expect_tx(&bars->full[st], kStageBytes);
+        mbar_expect_tx(&bars->full[st], count * kTileBytes);
       else if (rank == 0)
-        mbar_expect_tx(&bars->full[st], 2 * kStageBytes);
+        mbar_expect_tx(&bars->full[st], 2 * count * kTileBytes);
     };
     auto load = [&](void* dst, const CUtensorMap* map, int x, int y, int st) {
       if (PAIR)
@@ -518,33 +515,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       const int kt0 = item_c0(tile) * kTilesPerChunk, kt1 = min(num_tiles, item_c1(tile) * kTilesPerChunk);
       int kt = kt0;
       if (!waited) {  // first item of this block
-        const int early = min(kt1 - kt0, kStages);
+        const int early = min(kt1 - kt0, kStages * kPer);
         if (elect_one()) {
           for (int e = 0; e < early; ++e) {
-            expect(e);
-            load(tiles + e * kStageBytes + kTileBytesX, &map_w, (kt0 + e) * BK, n0, e);
+            if (e % kPer == 0) expect(e / kPer, min(kPer, early - e));
+            load(tiles + e * kTileBytes + kTileBytesX, &map_w, (kt0 + e) * BK, n0, e / kPer);
           }
         }
         bw::pdl_wait();
         waited = true;
         __syncwarp();
         if (elect_one())
-          for (int e = 0; e < early; ++e) load(tiles + e * kStageBytes, &map_x, (kt0 + e) * BK, m0, e);
+          for (int e = 0; e < early; ++e) load(tiles + e * kTileBytes, &map_x, (kt0 + e) * BK, m0, e / kPer);
         __syncwarp();
         kt += early;
-        s = early;
+        s = (early + kPer - 1) / kPer;
         if (s == kStages) s = 0, parity ^= 1;
       }
-      for (; kt < kt1; ++kt) {
+      for (; kt < kt1; kt += kPer) {
         if (!__all_sync(0xffffffffu, mbar_wait(&bars->empty[s], parity, failed))) {
           ok = false;
           break;
         }
         if (elect_one()) {
-          unsigned char* a = tiles + s * kStageBytes;
-          expect(s);
-          load(a, &map_x, kt * BK, m0, s);
-          load(a + kTileBytesX, &map_w, kt * BK, n0, s);
+          const int count = min(kPer, kt1 - kt);
+          expect(s, count);
+          for (int j = 0; j < count; ++j) {
+            unsigned char* a = tiles + s * kStageBytes + j * kTileBytes;
+            load(a, &map_x, (kt + j) * BK, m0, s);
+            load(a + kTileBytesX, &map_w, (kt + j) * BK, n0, s);
+          }
         }
         __syncwarp();
         if (++s == kStages) s = 0, parity ^= 1;
@@ -568,23 +568,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           fence_after_sync();
           const uint32_t d = tmem_base + buf * BNT;
           const int t_begin = c * kTilesPerChunk, t_end = min(num_tiles, t_begin + kTilesPerChunk);
-          for (int kt = t_begin; kt < t_end; ++kt) {
+          for (int kt = t_begin; kt < t_end; kt += kPer) {
             if (!__all_sync(0xffffffffu, mbar_wait(&bars->full[s], parity, failed))) {
               ok = false;
               break;
             }
             fence_after_sync();
-            const uint32_t a_addr = smem_u32(tiles + s * kStageBytes);
-            const uint64_t adesc = make_desc(a_addr), bdesc = make_desc(a_addr + kTileBytesX);
+            const uint32_t stage_addr = smem_u32(tiles + s * kStageBytes);
             if (elect_one()) {
+              const int count = min(kPer, t_end - kt);
+              for (int j = 0; j < count; ++j) {
+                const uint32_t a_addr = stage_addr + j * kTileBytes;
+                const uint64_t adesc = make_desc(a_addr), bdesc = make_desc(a_addr + kTileBytesX);
 #pragma unroll
-              for (int k = 0; k < BK / 16; ++k) {
-                // 16 k-elements are 32 bytes: the start address field moves by 2 (units of 16 bytes)
-                const uint32_t acc = (kt > t_begin || k > 0) ? 1u : 0u;
-                if (PAIR)
-                  umma_pair(d, adesc + 2 * k, bdesc + 2 * k, instr_desc_pair(BNT), acc);
-                else
-                  umma(d, adesc + 2 * k, bdesc + 2 * k, instr_desc(bt), acc);
+                for (int k = 0; k < BK / 16; ++k) {
+                  // 16 k-elements are 32 bytes: the start address field moves by 2 (units of 16 bytes)
+                  const uint32_t acc = (kt + j > t_begin || k > 0) ? 1u : 0u;
+                  if (PAIR)
+                    umma_pair(d, adesc + 2 * k, bdesc + 2 * k, instr_desc_pair(BNT), acc);
+                  else
+                    umma(d, adesc + 2 * k, bdesc + 2 * k, instr_desc(bt), acc);
+                }
               }
               // the stage may be refilled once these MMAs are done; the chunk's last commit also
               // hands the accumulator to the epilogue
@@ -592,7 +596,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                 umma_commit_pair(&bars->empty[s]);
               else
                 umma_commit(&bars->empty[s]);
-              if (kt + 1 == t_end) {
+              if (kt + kPer >= t_end) {
                 if (PAIR)
                   umma_commit_pair(&bars->acc_full[buf]);
                 else
@@ -895,44 +899,72 @@ int sm_count_of_device() {
   return sm_count[dev];
 }
 
-// How a product with one block of rows (m <= 128) runs. A tcgen05.mma that adds to the
-// accumulator of the one before it starts only when that one is done, about 100 ns later
-// whatever the tile's width, so a block's time is the number of such steps it issues one
-// after the other: 32 per chunk of 512. The plan minimises (rounds of the SMs over the work
-// items) x (steps per item): items are output tiles (all chunks inside, "whole") or (tile,
-// chunk) pairs ("split", which adds a second kernel and the traffic of the chunk sums);
-// tiles are 16 .. 128 columns wide in steps of 16, or 256. Of equal plans the one with the
-// narrower tiles wins (more SMs stream weights). Every plan gives the same bits.
+// How a product with few tiles runs. The plan is the one of least estimated time, from times measured on a B200 (us):
+//   whole   items are output tiles with all their chunks; a chunk of a tile takes kChunkUs by the tile's width, rounds of the SMs
+//           over the items follow each other, and a launch costs about 6 us around them
+//   split   items are (tile, chunk) pairs; the second kernel costs about 2 us (little up to 16 rows), and the chunk sums are written and read
+//           (8 bytes each) at about 5 TB/s. One block of rows only: beyond it the chunk sums outgrow what they save
+//   pairs   more than 128 rows: 256 x 256 tiles on pairs of blocks, 2.45 us a chunk, 8.5 us around them (10.5 where a
+//           residual is read or SwiGLU applied)
+// and none is faster than its operands arrive: a chunk's rows of x and W at about 83 KB a us for a block, and at about 9.5 TB/s
+// over all SMs. Tiles are 16 .. 128
+// columns wide in steps of 16, or 256 with one block of rows. Of equal plans the one with the narrower tiles wins (more SMs
+// stream weights). Every plan gives the same bits. What the estimate changed against counting steps of the tensor core:
+// 128 rows x 2,048 x 6,144 23.3 -> 14.9 us, 512 x 960 x 960 15.6 -> 10.5, 512 x 2,560 x 960 25 -> 17.
 struct Plan {
   bool split;
   int bn;
+  bool pair;
 };
 int g_tile_width = 0;  // 0: chosen from the shape; else forced (tests, measurements)
 int g_force_mode = 0;  // 0: chosen; 1: whole; 2: split where it is possible
 
 constexpr int kMaxSplitColumns = 16384;  // bounds the scratch of the chunk sums
 
-Plan plan_rows(int m, int n, int k, bool swiglu, int sms, bool allow_wide = true) {
+// a chunk of a narrow or wide tile, by its width / 16
+double chunk_us(int bn) {
+  constexpr double us[] = {1.25, 1.25, 1.5, 1.8, 1.95, 2.05, 2.2, 2.3};
+  return bn > BN ? 3.3 : us[bn / 16 - 1];
+}
+
+Plan plan_rows(int m, int n, int k, bool swiglu, bool reads, int sms, bool allow_wide = true) {
   const int chunks = (k + kChunk - 1) / kChunk;
-  const int steps_chunk = kChunk / 16;
-  const bool may_split = m <= BM && chunks > 1 && n <= kMaxSplitColumns;
-  Plan best{false, BN};
+  const bool one_block = m <= BM;
+  const bool may_split = one_block && chunks > 1 && n <= kMaxSplitColumns;
+  const int a_rows = m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : BM;  // rows of x in a stage
+  const int m_blocks = (m + BM - 1) / BM;
+  const double us_per_kb = 1.024e3 / 9.5e6, block_us_per_kb = 1.0 / 83.0;
+  Plan best{false, BN, false};
   double best_cost = -1.0;
+  if (!one_block && allow_wide && (!g_tile_width || g_tile_width > BN)) {
+    const long long items = static_cast<long long>((m + 2 * BM - 1) / (2 * BM)) * ((n + 2 * BN - 1) / (2 * BN));
+    const long long pairs = sms / 2;
+    best = Plan{false, 2 * BN, true};
+    best_cost = (swiglu || reads ? 10.5 : 8.5) + static_cast<double>((items + pairs - 1) / pairs) * chunks * 2.45;
+  }
   for (int mode = 0; mode < 2; ++mode) {
     if (mode == 1 && !may_split) continue;
-    if (g_force_mode == 1 && mode == 1) continue;
+    if (one_block && g_force_mode == 1 && mode == 1) continue;
     if (g_force_mode == 2 && mode == 0 && may_split) continue;
     for (int bn = 16; bn <= 2 * BN; bn = (bn < BN ? bn + 16 : 2 * bn)) {
       if (swiglu && bn < BN) continue;  // gate and up of an output lie 64 columns apart
-      if (bn > BN && (!allow_wide || n % 64)) continue;
-      if (g_tile_width && bn != g_tile_width && !(swiglu && g_tile_width < BN && bn == BN)) continue;
-      const long long tiles = (n + bn - 1) / bn;
+      // a tile much narrower than its rows brings more x than W: slower wherever measured (128 rows x 2,048 x 6,144 in tiles
+      // of 32 columns 30 us, of 64 15) but at one size
+      if (2 * bn < a_rows && !g_tile_width) continue;
+      // of several row blocks only tiles of 64 and 128 columns: 200 rows x 2,048 x 6,144 took 25 us in tiles of 112, 19 in pairs
+      if (!one_block && bn != BN / 2 && bn != BN && !g_tile_width) continue;
+      if (bn > BN && (!allow_wide || n % 64 || !one_block)) continue;
+      if (g_tile_width && bn != g_tile_width && !(swiglu && g_tile_width < BN && bn == BN) && !(!one_block && g_tile_width > BN && !best.pair)) continue;
+      const long long tiles = static_cast<long long>((n + bn - 1) / bn) * m_blocks;
       const long long items = mode ? tiles * chunks : tiles;
       const long long rounds = (items + sms - 1) / sms;
-      double cost = static_cast<double>(rounds) * (mode ? steps_chunk : steps_chunk * chunks);
-      // the second kernel, and writing and reading the chunk sums (8 bytes each at about 3 TB/s)
-      if (mode) cost += 20.0 + 2.67e-5 * chunks * static_cast<double>(m) * n;
-      if (best_cost < 0 || cost < best_cost - 1e-9) best = Plan{mode == 1, bn}, best_cost = cost;
+      const double step = std::max(chunk_us(bn), (a_rows + bn) * block_us_per_kb);
+      double cost = static_cast<double>(rounds) * step * (mode ? 1 : chunks);
+      const double arrive = static_cast<double>(tiles) * chunks * (a_rows + bn) * us_per_kb;
+      if (cost < arrive) cost = arrive;
+      cost += mode ? (m <= 16 ? 5.5 : 8.2) + 1.6e-6 * chunks * static_cast<double>(m) * n : 6.0;
+      // pairs give way only to a clearly lower estimate (it is good to about a tenth)
+      if (best_cost < 0 || cost < best_cost * (best.pair ? 0.9 : 1.0) - 1e-9) best = Plan{mode == 1, bn, false}, best_cost = cost;
     }
   }
   return best;
@@ -951,7 +983,7 @@ bool rows_path_takes(int m, int n, int k, int swiglu, const void* x = nullptr, c
 }
 }  // namespace
 
-// Forces the width of the output tiles of small batches (a multiple of 16 up to 128, or 256;
+// Forces the width of the output tiles (a multiple of 16 up to 128, or 256;
 // 0: chosen from the shape) and the mode (0 chosen, 1 whole, 2 split where possible). Every
 // combination gives the same bits. For tests and measurements.
 BW_API void bw_bf16_linear_tc_force(int bn, int mode) {
@@ -961,14 +993,14 @@ BW_API void bw_bf16_linear_tc_force(int bn, int mode) {
 
 // Whether a plain product of this shape is split along k (then it needs scratch).
 BW_API int bw_bf16_linear_tc_splits(int m, int n, int k) {
-  return m <= BM && plan_rows(m, n, k, false, sm_count_of_device()).split;
+  return m <= BM && plan_rows(m, n, k, false, false, sm_count_of_device()).split;
 }
 // Whether some plan may split it (what callers size the scratch by).
 BW_API int bw_bf16_linear_tc_may_split(int m, int n, int k) { return m <= BM && k > kChunk && n <= kMaxSplitColumns; }
 // Kernels that one call launches (1, or 2 when the product is split): callers count launches.
 BW_API int bw_bf16_linear_tc_kernels(int m, int n, int k, int swiglu, int has_scratch) {
   if (rows_path_takes(m, n, k, swiglu)) return 1;
-  return (m <= BM && has_scratch && plan_rows(m, n, k, swiglu != 0, sm_count_of_device()).split) ? 2 : 1;
+  return (m <= BM && has_scratch && plan_rows(m, n, k, swiglu != 0, false, sm_count_of_device()).split) ? 2 : 1;
 }
 
 namespace {
@@ -1000,7 +1032,7 @@ int configure_tc(int* pairs = nullptr) {
     }
     if (PAIR) {
       constexpr int BNW = BN;
-      const RingShape ring = ring_shape(A_ROWS, BNW);
+      const RingShape ring = ring_shape(A_ROWS, BNW, true);
       cudaLaunchConfig_t probe = {};
       probe.gridDim = dim3(2 * (sm_count_of_device() / 2));
       probe.blockDim = dim3(threads);
@@ -1033,7 +1065,7 @@ int launch_tc(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_
   constexpr int threads = WIDE ? 384 : 192, kEpi = WIDE ? 8 : 4;
   const int chunks = (k + kChunk - 1) / kChunk;
   const int bn = WIDE ? BNT : narrow_bn;
-  const RingShape ring = ring_shape(A_ROWS, WIDE ? BNW : bn);
+  const RingShape ring = ring_shape(A_ROWS, WIDE ? BNW : bn, WIDE);
   const int smem = ring.ring_bytes + kEpi * kStoreBytes + static_cast<int>(sizeof(Barriers)) + 1024;
   auto kernel = gemm_tc_kernel<SPLIT, A_ROWS, EPI, WIDE, PAIR>;
   int max_pairs = 0;
@@ -1073,7 +1105,7 @@ template <int EPI>
 int launch_tc_grouped(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_f32, int rows, int n, int k,
                       const int* group_off, const int* tile_prefix, int groups, int* error_word, cudaStream_t stream) {
   constexpr int BNT = 2 * BN, threads = 384, kEpi = 8;
-  const RingShape ring = ring_shape(BM, BNT);
+  const RingShape ring = ring_shape(BM, BNT, true);
   const int smem = ring.ring_bytes + kEpi * kStoreBytes + static_cast<int>(sizeof(Barriers)) + 1024;
   auto kernel = gemm_tc_kernel<false, BM, EPI, true, false, true>;
   if (const int rc = configure_tc<false, BM, EPI, true, false, true>()) return rc;
@@ -1105,17 +1137,17 @@ int launch_tc_rows(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int 
   // wide tiles want whole pieces of 64 columns and 32-byte stores
   const bool wide_ok = n % 64 == 0 && reinterpret_cast<uintptr_t>(y) % 32 == 0 &&
                        reinterpret_cast<uintptr_t>(residual) % 32 == 0 && reinterpret_cast<uintptr_t>(partials) % 32 == 0;
+  Plan plan = plan_rows(m, n, k, fused.mode == 2, residual != nullptr, sm_count_of_device(), wide_ok);
   if (m <= BM) {
-    Plan plan = plan_rows(m, n, k, fused.mode == 2, sm_count_of_device(), wide_ok);
-    if (!partials) plan = Plan{false, plan.split ? BN : plan.bn};
+    if (!partials) plan = Plan{false, plan.split ? BN : plan.bn, false};
     const bool wide = plan.bn > BN;
     if (plan.split) return wide ? BW_LAUNCH_ROWS(true, 0, true) : BW_LAUNCH_ROWS(true, 0, false);
     return wide ? BW_LAUNCH_ROWS(false, EPI, true) : BW_LAUNCH_ROWS(false, EPI, false);
   }
 #undef BW_LAUNCH_ROWS
 #undef BW_LAUNCH
-  if (!wide_ok)
-    return launch_tc<false, 128, EPI, false>(x, w, y, y_is_f32, residual, m, n, k, error_word, nullptr, fused, stream);
+  if (!wide_ok || !plan.pair)
+    return launch_tc<false, 128, EPI, false>(x, w, y, y_is_f32, residual, m, n, k, error_word, nullptr, fused, stream, plan.bn);
   if (g_pair_tiles)
     return launch_tc<false, 128, EPI, true, true>(x, w, y, y_is_f32, residual, m, n, k, error_word, nullptr, fused, stream);
   return launch_tc<false, 128, EPI, true>(x, w, y, y_is_f32, residual, m, n, k, error_word, nullptr, fused, stream);

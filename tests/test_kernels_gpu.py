@@ -407,6 +407,38 @@ def test_bf16_linear_two_blocks_per_tile_give_the_same_bits():
     assert not ops.device_failure()
 
 
+@pytest.mark.parametrize("m,n,k", [(129, 40, 64), (200, 264, 520), (257, 128, 1544), (512, 960, 960), (385, 1000, 2568)])
+def test_bf16_linear_narrow_tiles_of_many_rows_give_the_same_bits(m, n, k):
+    """More than 128 rows with few tiles run on tiles of 128 rows and 16 .. 128 columns: the bits of pairs and of the legacy
+    kernel, for rows and columns that end inside a tile, k that ends inside a stage of four k-tiles, a product that is plain,
+    adds a residual, or applies SwiGLU."""
+    rng = np.random.default_rng(m + n)
+    ops = _ops("bfloat16")
+    b16 = torch.bfloat16
+    x, w, res = t(bf(rnd(rng, m, k)), b16), t(bf(rnd(rng, n, k, scale=0.05)), b16), rnd(rng, m, n)
+    inter = 192
+    w_gu = ops.interleave_gate_up(t(bf(rnd(rng, inter, k, scale=0.05)), b16), t(bf(rnd(rng, inter, k, scale=0.05)), b16))
+
+    def run(legacy=False):
+        acc, out, h = t(res).clone(), torch.empty(m, n, device=DEV, dtype=b16), torch.empty(m, inter, device=DEV, dtype=b16)
+        ops.linear(x, w, acc, residual=acc, legacy=legacy)
+        ops.linear(x, w, out, legacy=legacy)
+        ops.linear_swiglu(x, w_gu, h)
+        return acc, out, h
+    try:
+        ops.force_linear_plan(256, 0)
+        want = run()
+        legacy = run(legacy=True)
+        assert torch.equal(want[0], legacy[0]) and torch.equal(want[1], legacy[1])
+        for width in (0, 16, 48, 64, 112, 128):
+            ops.force_linear_plan(width, 0)
+            for got, ref, what in zip(run(), want, ("residual", "plain", "SwiGLU")):
+                assert torch.equal(got, ref), f"width {width}, {what}"
+    finally:
+        ops.force_linear_plan(0, 0)
+    assert not ops.device_failure()
+
+
 def test_bf16_linear_few_rows_kernel_gives_the_same_bits():
     """Steps of up to 16 rows run their products on the streaming kernel (a warp per 8 columns
     and chunk, chunk sums added inside the kernel, clusters of blocks when k is long). Same bits
