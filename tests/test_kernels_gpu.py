@@ -265,6 +265,31 @@ def test_sample_rows_over_the_vocabulary(vocab):
     assert got[1] == vocab // 2 and got[2] == vocab - 2
 
 
+@pytest.mark.parametrize("vocab", [4096, 5000, 49152])
+def test_sample_rows_at_running_sums(vocab):
+    """Targets on, just below and just above a running sum, where sums in another order may not be trusted: equal weights (a
+    target of exactly k of them), a long tail of weights too small to move the sum, and logits that are no number."""
+    rng = np.random.default_rng(vocab + 1)
+    marks = [1, vocab // 512, vocab // 2, vocab - 1]
+    us = [0.0, 1.0 - 2.0 ** -53] + [f(k / vocab) for k in marks for f in (lambda v: v, lambda v: np.nextafter(v, 0.0), lambda v: np.nextafter(v, 1.0))]
+    us += list(rng.random(6))
+    rows = len(us) + 3
+    logits = np.zeros((rows, vocab), dtype=np.float32)
+    logits[len(us) - 6:] = rnd(rng, rows - len(us) + 6, vocab, scale=4.0)
+    logits[-3, 1:] -= 60.0           # one weight of about 1 and a tail of 1e-26 each
+    logits[-3, 0] = 0.0
+    logits[-2, vocab // 3] = np.nan
+    logits[-1, 7] = np.inf
+    us = np.array(us + [0.9999999, 0.5, 0.5], dtype=np.float64)
+    temps = np.ones(rows, dtype=np.float32)
+    out = torch.empty(rows, dtype=torch.int32, device=DEV)
+    _ops("bfloat16").sample_rows(t(logits), t(temps), torch.from_numpy(us).to(DEV), out)
+    got = out.cpu().numpy()
+    for r in range(rows - 2):
+        assert got[r] == P.sample_row(logits[r], temps[r], us[r], exp="det"), f"row {r}"
+    assert ((got >= 0) & (got < vocab)).all()
+
+
 def test_fingerprint_rows():
     rng = np.random.default_rng(7)
     for vocab in (256, 385):
