@@ -500,9 +500,16 @@ BW_API int bw_bf16_linear_rows_tanh(const __nv_bfloat16* x, const __nv_bfloat16*
 }
 
 // Whether the fused q/k/v projection of a step can rotate and store its outputs itself
-// (bw_bf16_linear_rows_rope): a shape of this path whose tiles hold both halves of a head.
+// (bw_bf16_linear_rows_rope): a shape of this path whose tiles hold both halves of a head, or one that
+// the tcgen05 kernel takes (block pairs, heads of 64).
+BW_API int bw_bf16_linear_tc_rope_usable(const void* x, const void* w, int m, int n, int k, int hd);
+BW_API int bw_bf16_linear_tc_rope(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* qkv, int m, int n, int k,
+                                  const int* pos, const int* row_seq, const float* cos_t, const float* sin_t,
+                                  const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache, int heads,
+                                  int kv_heads, int hd, int page, int write_kv, cudaStream_t stream);
 BW_API int bw_bf16_linear_rows_rope_usable(const void* x, const void* w, int m, int n, int k, int heads, int kv_heads,
                                            int hd) {
+  if (m > 16) return heads > 0 && kv_heads > 0 && n == (heads + 2 * kv_heads) * hd && bw_bf16_linear_tc_rope_usable(x, w, m, n, k, hd);
   RowsShape s;
   return g_rows_enabled && hd >= 16 && hd % 16 == 0 && heads > 0 && kv_heads > 0 && n == (heads + 2 * kv_heads) * hd &&
          (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (reinterpret_cast<uintptr_t>(w) % 16 == 0) &&
@@ -518,6 +525,9 @@ BW_API int bw_bf16_linear_rows_rope(const __nv_bfloat16* x, const __nv_bfloat16*
                                     const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache,
                                     int heads, int kv_heads, int hd, int page, int write_kv, cudaStream_t stream) {
   if (m <= 0 || n <= 0) return 0;
+  if (m > 16)
+    return bw_bf16_linear_tc_rope(x, w, qkv, m, n, k, pos, row_seq, cos_t, sin_t, block_table, max_blocks, kcache, vcache, heads, kv_heads,
+                                  hd, page, write_kv, stream);
   RowsShape s;
   if (!bw_bf16_linear_rows_rope_usable(x, w, m, n, k, heads, kv_heads, hd) || !rows_shape(m, n, k, true, &s) || page <= 0) {
     bw::set_error("linear with rotation (few rows): shape [%d x %d] x [%d x %d], %d/%d heads of %d is not for this path", m,

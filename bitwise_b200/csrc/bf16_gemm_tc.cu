@@ -9,15 +9,15 @@
 // adds them in the same ascending order.
 //
 // One thread block computes one 128 x 128 output tile with six warps:
-//   warp 0   one thread issues the TMA loads of the x tile and the W tile, 64 k-elements per
-//            stage (128-byte rows, 128-byte swizzle), into a ring of stages
-//   warp 1   one thread issues tcgen05.mma (M 128, N 128, K 16, four per stage) into one of
+//   warp 0   an elected lane issues the TMA loads of the x tile and the W tile, 64 k-elements
+//            per k-tile (128-byte rows, 128-byte swizzle), into a ring of stages
+//   warp 1   an elected lane issues tcgen05.mma (M 128, N 128, K 16, four per k-tile) into one of
 //            two accumulators in tensor memory; a commit frees the stage, and at the end of a
 //            chunk another commit hands the accumulator to the epilogue
 //   warps 2-5  read the finished chunk sum from tensor memory (each thread one row, 32 columns
 //            at a time) and add it to the running total in registers, while the tensor core
 //            already works on the next chunk in the other accumulator; after the last chunk
-//            they add the residual and store.
+//            they add the residual, apply SwiGLU or rotate the heads, and store.
 // The kernel is persistent: one block per SM (6 stages of 32 KB) takes output tiles round-robin,
 // and because loads, MMAs and the epilogue each walk the tile sequence on their own, the store
 // of one tile overlaps the main loop of the next.
@@ -371,6 +371,18 @@ __global__ void reduce_swiglu_kernel(const float* __restrict__ partials, int num
 // rows of W, the epilogue stores the rows up to the group's end. Rows that a tile reads beyond
 // its group are the next group's or zeros, and their results are never stored. The lists are
 // written by a kernel of the same step, so every role waits for it before it reads them.
+// EPI 3: what the epilogue of the fused q/k/v product does with it (see there).
+struct RopeOut {
+  const int* pos;            // position of every row
+  const int* row_seq;        // its sequence's row of the block table
+  const float* cos_t;        // [positions][hd / 2], or null: nothing is rotated
+  const float* sin_t;
+  const int* block_table;
+  int max_blocks;
+  __nv_bfloat16* kcache;     // [pages][kv_heads][page][hd]
+  __nv_bfloat16* vcache;
+  int heads, kv_heads, page, write_kv;
+};
 struct GroupItems {
   const int* group_off;
   const int* tile_prefix;
@@ -381,7 +393,8 @@ template <bool SPLIT, int A_ROWS, int EPI, bool WIDE, bool PAIR, bool GROUPED = 
 __global__ void __launch_bounds__(WIDE ? 384 : 192, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, void* Y,
                int y_is_f32, const float* residual, int M, int N, int K, int* error_flag, float* partials, int bn,
-               GroupItems gi) {
+               GroupItems gi, RopeOut rp) {
+  static_assert(EPI != 3 || PAIR, "the rotating epilogue belongs to pairs");
   static_assert(!GROUPED || (!SPLIT && !PAIR && A_ROWS == BM && EPI != 1), "grouped products run whole, single-block tiles");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // the swizzled tiles want 1024-byte alignment
@@ -639,6 +652,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         group_tile(tile, m0, row_end, g);
       }
       const int row = m0 + et;
+      int rope_pos = 0;
+      long long rope_slot = 0;  // this row's place in the cache, in rows of a head, of the first kv head
+      if (EPI == 3 && row < M) {
+        rope_pos = rp.pos[row];
+        if (rp.write_kv) {
+          const long long block = rp.block_table[static_cast<size_t>(rp.row_seq[row]) * rp.max_blocks + rope_pos / rp.page];
+          rope_slot = block * rp.kv_heads * rp.page + rope_pos % rp.page;
+        }
+      }
       // rows of this warp's part of the tile, and whether its full blocks may go through shared memory in 16-byte accesses
       const int first_row = m0 + quarter * 32, warp_rows = min(32, row_end - first_row);
       const bool turned = (N & 7) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (reinterpret_cast<uintptr_t>(residual) & 15) == 0;
@@ -733,6 +755,71 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         else
           glu(std::integral_constant<int, bw::kGluSilu>{});
         store_turned(store_buf, reinterpret_cast<char*>(out), static_cast<size_t>(N), warp_rows, lane);
+      } else if (EPI == 3) {
+        // The fused q/k/v product rotates and stores itself: a thread owns a row, and with it both partners of every rotation
+        // of its heads (a piece of 64 columns is a head). Rounded to bfloat16 as the stored product would be, rotated with rope_cache_bf16_kernel's arithmetic (same bits), turned
+        // through shared memory, q goes to Y and k and v to their row of a page. The kernel that did this from the stored
+        // product read and wrote it once more: attention of 2,047 rows at 32 heads of 64, products included, 129.5 -> 125 us.
+        // (Rotating behind the turn, where eight lanes read a row's tables together, took 130: the exchange of partners costs
+        // more than the tables.)
+        constexpr int HD = 64;
+        const float* cos_row = rp.cos_t ? rp.cos_t + static_cast<size_t>(rope_pos) * (HD / 2) : nullptr;
+        const float* sin_row = rp.cos_t ? rp.sin_t + static_cast<size_t>(rope_pos) * (HD / 2) : nullptr;
+        // the 64 columns of head `head` that lie turned in the warp's buffer
+        auto store = [&](int head) {
+          if (head < rp.heads) {
+            __nv_bfloat16* out = static_cast<__nv_bfloat16*>(Y) + static_cast<size_t>(first_row) * N + head * HD;
+            store_turned(store_buf, reinterpret_cast<char*>(out), static_cast<size_t>(N) * 2, warp_rows, lane);
+            return;
+          }
+          const bool is_k = head < rp.heads + rp.kv_heads;
+          const int kvh = head - rp.heads - (is_k ? 0 : rp.kv_heads);
+          char* base = reinterpret_cast<char*>((is_k ? rp.kcache : rp.vcache) + static_cast<size_t>(kvh) * rp.page * HD);
+          __syncwarp();
+#pragma unroll
+          for (int t = 0; t < 8; ++t) {
+            const uint4 v = get_piece(store_buf, lane, t);
+            const int r = 4 * t + (lane >> 3);
+            const long long slot = __shfl_sync(0xffffffffu, rope_slot, r);
+            if (r < warp_rows) store_piece(base + slot * (HD * 2) + (lane & 7) * 16, v);
+          }
+          __syncwarp();
+        };
+        // eight rotations: x1 and x2 become the first and second partners
+        auto rotate = [&](float* x1, float* x2, int i, bool turn) {
+          if (!turn) return;
+          float c[8], sn[8];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint4 cv = load_piece(reinterpret_cast<const char*>(cos_row + i + 4 * h));
+            const uint4 sv = load_piece(reinterpret_cast<const char*>(sin_row + i + 4 * h));
+            c[4 * h] = __uint_as_float(cv.x), c[4 * h + 1] = __uint_as_float(cv.y), c[4 * h + 2] = __uint_as_float(cv.z), c[4 * h + 3] = __uint_as_float(cv.w);
+            sn[4 * h] = __uint_as_float(sv.x), sn[4 * h + 1] = __uint_as_float(sv.y), sn[4 * h + 2] = __uint_as_float(sv.z), sn[4 * h + 3] = __uint_as_float(sv.w);
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float a = __bfloat162float(__float2bfloat16_rn(x1[e])), b = __bfloat162float(__float2bfloat16_rn(x2[e]));
+            x1[e] = __fsub_rn(__fmul_rn(a, c[e]), __fmul_rn(b, sn[e]));
+            x2[e] = __fadd_rn(__fmul_rn(b, c[e]), __fmul_rn(a, sn[e]));
+          }
+        };
+        auto put8 = [&](int c, const float* v) {
+          put_piece(store_buf, lane, c, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+        };
+#pragma unroll
+        for (int piece = 0; piece < 2; ++piece) {
+          const int head = (n0 + (piece ? off1 : off0)) >> 6;
+          if (head * HD >= N || (head >= rp.heads && !rp.write_kv)) continue;
+          const bool turn = cos_row && head < rp.heads + rp.kv_heads;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            float *x1 = total + piece * PW + 8 * c, *x2 = x1 + 32;
+            rotate(x1, x2, 8 * c, turn);
+            put8(c, x1);
+            put8(c + 4, x2);
+          }
+          store(head);
+        }
       } else if (EPI == 2) {
 #pragma unroll
         for (int b = 0; b < kBlocks; ++b) {
@@ -1058,7 +1145,7 @@ int configure_tc(int* pairs = nullptr) {
 
 template <bool SPLIT, int A_ROWS, int EPI, bool WIDE, bool PAIR = false>
 int launch_tc(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_f32, const float* residual, int m, int n,
-              int k, int* error_word, float* partials, const Fused& fused, cudaStream_t stream, int narrow_bn = BN) {
+              int k, int* error_word, float* partials, const Fused& fused, cudaStream_t stream, int narrow_bn = BN, const RopeOut& rope = RopeOut{}) {
   constexpr int BNT = WIDE ? 2 * BN : BN;
   constexpr int BNW = PAIR ? BN : BNT;
   constexpr int BMT = PAIR ? 2 * BM : BM;
@@ -1080,13 +1167,13 @@ int launch_tc(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_
   if (PAIR) {
     const unsigned pairs = static_cast<unsigned>(items < max_pairs ? items : max_pairs);
     bw::launch_pdl_cluster(2, kernel, dim3(2 * pairs), dim3(threads), smem, stream, map_x, map_w, y, y_is_f32, residual, m,
-                            n, k, error_word, partials, bn, GroupItems{nullptr, nullptr, 0});
+                            n, k, error_word, partials, bn, GroupItems{nullptr, nullptr, 0}, rope);
     return bw::launch_status();
   }
   const int sms = sm_count_of_device();
   const unsigned grid = static_cast<unsigned>(items < sms ? items : sms);
   bw::launch_pdl(kernel, dim3(grid), dim3(threads), smem, stream, map_x, map_w, y, y_is_f32, residual, m, n, k,
-                 error_word, partials, bn, GroupItems{nullptr, nullptr, 0});
+                 error_word, partials, bn, GroupItems{nullptr, nullptr, 0}, rope);
   if (SPLIT) {
     const size_t outputs = static_cast<size_t>(m) * n;
     if (fused.mode == 2)
@@ -1119,7 +1206,7 @@ int launch_tc_grouped(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, i
   const unsigned grid = static_cast<unsigned>(items < sms ? items : sms);
   bw::launch_pdl(kernel, dim3(grid), dim3(threads), smem, stream, map_x, map_w, y, y_is_f32,
                  static_cast<const float*>(nullptr), rows, n, k, error_word, static_cast<float*>(nullptr), BNT,
-                 GroupItems{group_off, tile_prefix, groups});
+                 GroupItems{group_off, tile_prefix, groups}, RopeOut{});
   return bw::launch_status();
 }
 
@@ -1190,6 +1277,41 @@ BW_API int bw_bf16_linear_tc(const __nv_bfloat16* x, const __nv_bfloat16* w, voi
   const Fused none;
   if (y_is_f32 == 1) return launch_tc_rows<2>(x, w, y, 1, residual, m, n, k, word, partials, none, stream);
   return launch_tc_rows<0>(x, w, y, y_is_f32, nullptr, m, n, k, word, partials, none, stream);
+}
+
+// The fused q/k/v product on block pairs that rotates and stores its outputs itself, for heads of 64 (what
+// bw_bf16_linear_rows_rope is for few rows: the same arguments and the same results). Elsewhere the rotation stays a kernel
+// of its own: where narrow tiles are the better plan each block has one tile, whose epilogue nothing overlaps (a step of 512
+// rows through 32 layers of width 960: 2,264 us, with rotating narrow tiles 2,273), and heads of 128 spread a row's tables
+// over twice the lines (attention of 1,200 rows at 32 heads of 128: 203 us, with this epilogue 207).
+BW_API int bw_bf16_linear_tc_rope_usable(const void* x, const void* w, int m, int n, int k, int hd) {
+  return m > BM && n > 0 && hd == 64 && bw_bf16_linear_tc_usable(x, w, k) && plan_rows(m, n, k, false, false, sm_count_of_device()).pair;
+}
+
+BW_API int bw_bf16_rope_cache(__nv_bfloat16* qkv, int row_stride, const int* pos, const int* row_seq, const float* cos_t,
+                              const float* sin_t, const int* block_table, int max_blocks, __nv_bfloat16* kcache,
+                              __nv_bfloat16* vcache, int n, int heads, int kv_heads, int hd, int page, int write_kv,
+                              cudaStream_t stream);
+
+BW_API int bw_bf16_linear_tc_rope(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* qkv, int m, int n, int k,
+                                  const int* pos, const int* row_seq, const float* cos_t, const float* sin_t,
+                                  const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache, int heads,
+                                  int kv_heads, int hd, int page, int write_kv, cudaStream_t stream) {
+  if (m <= 0 || n <= 0) return 0;
+  if (!bw_bf16_linear_tc_rope_usable(x, w, m, n, k, hd) || n != (heads + 2 * kv_heads) * hd || page <= 0) {
+    bw::set_error("linear with rotation (tcgen05): shape [%d x %d] x [%d x %d], %d/%d heads of %d is not for this path", m, k, n, k, heads, kv_heads, hd);
+    return -1;
+  }
+  auto off16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 != 0; };
+  if (reinterpret_cast<uintptr_t>(qkv) % 32 || off16(kcache) || off16(vcache) || off16(cos_t) || off16(sin_t)) {
+    const int rc = bw_bf16_linear_tc(x, w, qkv, 0, nullptr, m, n, k, nullptr, nullptr, stream);
+    return rc ? rc : bw_bf16_rope_cache(qkv, n, pos, row_seq, cos_t, sin_t, block_table, max_blocks, kcache, vcache, m, heads, kv_heads, hd, page, write_kv, stream);
+  }
+  int* word = bw::failure_word();
+  if (!word) return -1;
+  const RopeOut rope{pos, row_seq, cos_t, sin_t, block_table, max_blocks, kcache, vcache, heads, kv_heads, page, write_kv};
+  const Fused none;
+  return launch_tc<false, 128, 3, true, true>(x, w, qkv, 0, nullptr, m, n, k, word, nullptr, none, stream, 2 * BN, rope);
 }
 
 // Grouped products on the tcgen05 kernel: y[i] = x[i] W_g^T for the rows i of group g, x holding

@@ -324,8 +324,8 @@ class KernelOps:
         return self._partials, self._counters
 
     def force_linear_plan(self, width: int = 0, mode: int = 0) -> None:
-        """Tests and measurements: force the tile width of small batches (16 .. 128 in steps of
-        16, or 256; 0: chosen from the shape) and the mode (0 chosen, 1 one block walks k,
+        """Tests and measurements: force the tile width (16 .. 128 in steps of 16, or 256, above
+        128 rows on block pairs; 0: chosen from the shape) and the mode (0 chosen, 1 one block walks k,
         2 split along k where possible).  Every combination gives the same bits."""
         if self.kind == "bf16":
             self._kernel_counts.clear()
@@ -361,11 +361,12 @@ class KernelOps:
         return bool(self.lib.bw_bf16_linear_rows_enable(_c_int(int(on))))
 
     def stream_attention(self, head_dim: int, mode: int) -> int:
-        """How decode steps with head size 64 fetch the cache where TMA boxes fit (pages of 8 keys
-        or more that divide 64): 0 never (a thread block per key tile that copies with cp.async),
-        1 (the default) the streaming kernel (persistent blocks, TMA rings) for steps of 32 rows
-        or more and a block per key tile fed by TMA boxes for fewer, 2 the streaming kernel
-        whenever the shape allows.  Same bits every way.  Returns the previous setting."""
+        """How decode steps with head sizes 64 and 128 fetch the cache where TMA boxes fit (pages of 8
+        keys or more that divide 64): 0 never (a thread block per key tile that copies with cp.async),
+        1 (the default) a block per key tile fed by TMA boxes, and at head size 64 the streaming kernel
+        (persistent blocks, TMA rings) for steps of 2,048 (row, kv head) pairs or more, 2 the streaming
+        kernel whenever the shape allows (head size 128: as 1).  Same bits every way.  Returns the
+        previous setting."""
         if self.kind != "bf16":
             return 0
         return int(self._attention_lib(head_dim).bw_bf16_attention_stream_mode(_c_int(int(mode))))
@@ -486,8 +487,8 @@ class KernelOps:
 
     def fuses_rope(self, m: int, width: int, heads: int, kv_heads: int, head_dim: int) -> bool:
         """Whether ``linear_rope_cache`` takes a step of m rows: then the fused q/k/v product
-        rotates q and k and stores k and v in the cache itself (steps of up to 16 rows on the
-        serving precision)."""
+        rotates q and k and stores k and v in the cache itself (on the serving precision steps of up
+        to 16 rows, and those whose product runs on block pairs, with heads of 64)."""
         if self.kind != "bf16":
             return False
         key = ("rope", m, width, heads, kv_heads, head_dim)
@@ -606,7 +607,7 @@ class KernelOps:
                     return
             if split:
                 scratch = self._attention_scratch(lib, qkv.device, n, heads, max_keys)
-                # head size 64: the cache streams through TMA rings, one block per SM (same bits)
+                # head sizes 64 and 128: the cache arrives as TMA page boxes (same bits)
                 if lib.bw_bf16_attention_stream_usable(_c_int(n), _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(page),
                                                        _c_int(qkv.shape[1])):
                     fn = lib.bw_bf16_attention_stream

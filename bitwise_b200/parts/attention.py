@@ -74,7 +74,7 @@ class GQAAttention(Mixer):
         cos, sin = tables if tables is not None else (None, None)
         fuses = getattr(ops, "fuses_rope", None)
         if fuses and fuses(n, self.width, self.heads, self.kv_heads, self.head_dim):
-            # a step of few rows: the projection rotates and stores its outputs itself
+            # the projection rotates and stores its outputs itself
             ops.linear_rope_cache(xn, self.w_qkv, qkv, ctx.pos, ctx.row_seq, cos, sin, cache.block_table, cache.k,
                                   cache.v, self.heads, self.kv_heads, self.head_dim, write_kv=cache.writable)
         else:

@@ -562,6 +562,43 @@ def test_bf16_qkv_product_that_rotates_and_stores_equals_product_then_rope():
     assert not ops.device_failure()
 
 
+@pytest.mark.parametrize("m,width,heads,kv_heads,hd,page", [
+    (300, 2048, 32, 32, 64, 16), (1031, 1024, 33, 9, 64, 64), (1025, 520, 40, 4, 64, 32),
+    (513, 64, 78, 9, 64, 16), (2047, 256, 8, 8, 64, 8)])
+def test_bf16_qkv_product_of_many_rows_that_rotates_and_stores(m, width, heads, kv_heads, hd, page):
+    """Block pairs, the last tiles and rows partly filled: the bits of the product followed by the rotation kernel."""
+    rng = np.random.default_rng(m)
+    ops = _ops("bfloat16")
+    from bitwise_b200.parts.rope import RotaryEncoding
+    assert ops.fuses_rope(m, width, heads, kv_heads, hd)
+    n = (heads + 2 * kv_heads) * hd
+    x = t(bf(rnd(rng, m, width)), torch.bfloat16)
+    w = t(bf(rnd(rng, n, width, scale=0.05)), torch.bfloat16)
+    tables = RotaryEncoding(hd, 10000.0, None, positions=2048).rotary_tables(DEV)
+    seqs = 3
+    seq = np.sort(rng.integers(0, seqs, m)).astype(np.int32)
+    pos = np.concatenate([5 + 11 * s + np.arange((seq == s).sum()) for s in range(seqs)]).astype(np.int32)
+    per_seq = 2048 // page
+    pages = seqs * per_seq + 2
+    table = rng.permutation(pages)[:seqs * per_seq].reshape(seqs, -1).astype(np.int32)
+    for (cos, sin), write, lead in ((tables, True, 0), ((None, None), True, 0), (tables, False, 0), (tables, True, 8)):
+        outs = []
+        for fused in (False, True):
+            k = torch.full((pages, kv_heads, page, hd), 0.5, device=DEV, dtype=torch.bfloat16)
+            v = torch.full((pages, kv_heads, page, hd), -0.25, device=DEV, dtype=torch.bfloat16)
+            qkv = torch.zeros(m * n + lead, device=DEV, dtype=torch.bfloat16)[lead:].view(m, n)  # lead 8: starts on 16 bytes only
+            args = (t(pos, torch.int32), t(seq, torch.int32), cos, sin, t(table, torch.int32), k, v, heads, kv_heads, hd)
+            if fused:
+                ops.linear_rope_cache(x, w, qkv, *args, write_kv=write)
+            else:
+                ops.linear(x, w, qkv)
+                ops.rope_cache(qkv, *args, write_kv=write)
+            outs.append((qkv[:, :heads * hd].contiguous(), k, v))
+        for got, want, what in zip(outs[1], outs[0], ("q", "key cache", "value cache")):
+            assert torch.equal(got.view(torch.int16), want.view(torch.int16)), f"{what}: rotate {cos is not None}, store {write}, lead {lead}"
+    assert not ops.device_failure()
+
+
 def test_bf16_rmsnorm_and_swiglu():
     """Tolerance: one bfloat16 rounding of a float32 result (2^-8 relative) plus 1e-6 absolute."""
     rng = np.random.default_rng(9)
