@@ -46,6 +46,11 @@ def _need(t: torch.Tensor, dtype, what: str, dims: Optional[int] = None) -> None
         raise KernelError(f"{what}: expected {dims} dimensions, got {tuple(t.shape)}")
 
 
+def _fits(t: torch.Tensor, dtype) -> bool:
+    """What ``_need`` asks of a tensor, as an answer instead of an error."""
+    return t.is_cuda and t.dtype is dtype and t.is_contiguous()
+
+
 def _need_rows(t: torch.Tensor, dtype, what: str) -> None:
     """A matrix whose rows are contiguous; the rows may lie apart (columns sliced out of wider rows)."""
     if not t.is_cuda:
@@ -579,6 +584,8 @@ class KernelOps:
                 raise KernelError(f"attention (bfloat16): head size {head_dim} is not a multiple of 16 up to 256")
             lib = self._attention_lib(head_dim)
             t_seq, t_row0, t_rows, t_count = batch.query_tiles(self.attention_tile_rows(heads, kv_heads))
+            for t_ in (batch.seq_pos0, batch.seq_row0, t_seq, t_row0, t_rows):
+                _need(t_, torch.int32, "attention step arrays")
             scratch = None
             split = t_count == n and max_keys > 128  # a decode step: one tile of keys per warp
             if not split and not self.legacy_attention:
@@ -593,6 +600,8 @@ class KernelOps:
                 sets = getattr(batch, "tile_sets", None)
                 if rows_tc > 0 and (sets is None or rows_tc in sets) and n > t_count:
                     q_seq, q_row0, q_rows, q_count = batch.query_tiles(rows_tc)
+                    for t_ in (q_seq, q_row0, q_rows):
+                        _need(t_, torch.int32, "attention step arrays")
                     fn = lib.bw_bf16_attention_tc
                     fn.restype = _c_int
                     rc = fn(_p(qkv), _c_int(qkv.shape[1]), _p(kcache), _p(vcache), _c_int(kcache.shape[0]),
@@ -636,7 +645,8 @@ class KernelOps:
     def prenorm_block(self, ctx, x: torch.Tensor, cache, block) -> bool:
         """All launches of one pre-norm block (RMSNorm, grouped-query attention, RMSNorm, dense SwiGLU) in one call of the
         library, as the block's parts would make them one by one; ``block`` = (norm1, mixer, norm2, feed_forward).  False,
-        with nothing launched, for what the call does not take: the parts then run, with their own checks."""
+        with nothing launched, for what the call does not take: the parts then run, with their own checks.  Whatever a part
+        would have checked before its launch is checked here in every call: the library sees addresses only."""
         if self.kind != "bf16" or self.legacy_attention:
             return False
         norm1, mixer, norm2, ffn = block
@@ -655,12 +665,24 @@ class KernelOps:
                                  (w_qkv, bf16, (qkv_dim, width)), (w_o, bf16, (width, q_dim)), (w_gu, bf16, (2 * inter, width)),
                                  (w_down, bf16, (width, inter)), (norm1.weight, torch.float32, (width,)),
                                  (norm2.weight, torch.float32, (width,))):
-            if t_ is None or t_.dtype is not dtype or t_.shape != shape or not t_.is_cuda or not t_.is_contiguous():
+            if t_ is None or t_.shape != shape or not _fits(t_, dtype):
                 return False
-        if table.dtype is not torch.int32 or table.dim() != 2 or not table.is_contiguous():
+        if table.dim() != 2:
             return False
-        if cos is not None and (cos.dtype is not torch.float32 or cos.shape[1] != hd // 2 or cos.shape != sin.shape
-                                or not cos.is_contiguous() or not sin.is_contiguous()):
+        if cos is not None:
+            if cos.dim() != 2 or cos.shape[1] != hd // 2 or cos.shape != sin.shape:
+                return False
+            if not (_fits(cos, torch.float32) and _fits(sin, torch.float32)):
+                return False
+        group = heads // kv_heads
+        rows, rows_tc = max(1, 64 // group), 128 // group
+        sets = ctx.tile_sets
+        if rows not in sets:
+            return False
+        t_seq, t_row0, t_rows, t_count = sets[rows]
+        c_seq, c_row0, c_rows, c_count = sets.get(rows_tc, (None, None, None, 0))
+        arrays = (table, ctx.pos, ctx.row_seq, ctx.seq_pos0, ctx.seq_row0, t_seq, t_row0, t_rows)
+        if not all(_fits(t_, torch.int32) for t_ in arrays + ((c_seq, c_row0, c_rows) if c_seq is not None else ())):
             return False
         lib = self._attention_lib(hd)
         fns = self._block_fns.get(hd)
@@ -671,18 +693,15 @@ class KernelOps:
                      "bw_bf16_attention_stream_usable")
             # (a head size without a kernel has no entry point for it, and its query says so)
             fns = self._block_fns[hd] = tuple(ctypes.cast(getattr(lib, f), ctypes.c_void_p).value if hasattr(lib, f) else 0 for f in names)
-        group = heads // kv_heads
-        sets = ctx.tile_sets
-        rows, rows_tc = max(1, 64 // group), 128 // group
-        if rows not in sets:
-            return False
-        t_seq, t_row0, t_rows, t_count = sets[rows]
-        c_seq, c_row0, c_rows, c_count = sets.get(rows_tc, (None, None, None, 0))
         has_tc = rows_tc if c_seq is not None else 0
         workspace = ctx.workspace
         buffers = [workspace.rows("normed", n, width, bf16), workspace.rows("qkv", n, qkv_dim, bf16), workspace.rows("attn", n, q_dim, bf16),
                    workspace.rows("ffn_h", n, inter, bf16)]
-        gate_up = 0 if ffn.fused else workspace.rows("gate_up", n, 2 * inter, bf16).data_ptr()
+        if not ffn.fused:
+            buffers.append(workspace.rows("gate_up", n, 2 * inter, bf16))
+        if not all(_fits(b, bf16) for b in buffers):
+            return False
+        gate_up = 0 if ffn.fused else buffers[4].data_ptr()
         partials = counters = attn_scratch = 0
         if n <= self._split_rows:
             for out, inner in ((qkv_dim, width), (width, q_dim), (2 * inter, width), (width, inter)):
@@ -692,7 +711,7 @@ class KernelOps:
             attn_scratch = self._attention_scratch(lib, x.device, n, heads, ctx.max_keys).data_ptr()
         ptr = lambda t_: 0 if t_ is None else t_.data_ptr()
         call = array.array("q", (
-            x.data_ptr(), *(b.data_ptr() for b in buffers), gate_up, partials, counters, attn_scratch,
+            x.data_ptr(), *(b.data_ptr() for b in buffers[:4]), gate_up, partials, counters, attn_scratch,
             norm1.weight.data_ptr(), norm2.weight.data_ptr(), w_qkv.data_ptr(), w_o.data_ptr(), w_gu.data_ptr(), w_down.data_ptr(),
             int(ffn.fused), width, heads, kv_heads, hd, inter, mixer.window or 0, ptr(cos), ptr(sin),
             k.data_ptr(), v.data_ptr(), pages, page, int(cache.writable), table.data_ptr(), table.shape[1],

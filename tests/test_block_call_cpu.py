@@ -1,0 +1,115 @@
+"""What a pre-norm block hands to the library's one call, and what it does not: tensors that only say they are on the device, and a
+library that records its calls instead of launching."""
+import ctypes
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from bitwise_b200.kernels.ops import KernelOps
+from bitwise_b200.parts.attention import GQAAttention
+from bitwise_b200.parts.base import PagedKVView, Workspace
+from bitwise_b200.parts.mlp import SwiGLU
+from bitwise_b200.parts.norm import RMSNorm
+
+WIDTH, HEADS, KV, HD, INTER, N, PAGE = 64, 4, 2, 16, 64, 3, 16
+
+
+class OnDevice(torch.Tensor):
+    is_cuda = property(lambda self: True)
+
+
+def dev(*shape, dtype=torch.float32):
+    return torch.zeros(*shape, dtype=dtype).as_subclass(OnDevice)
+
+
+def ints(*shape):
+    return dev(*shape, dtype=torch.int32)
+
+
+class Library:
+    """Answers as the kernel libraries do, and counts the block calls."""
+    def __init__(self):
+        self.calls = 0
+
+    def bw_bf16_block_members(self):
+        return KernelOps.BLOCK_CALL_MEMBERS
+
+    def bw_bf16_block(self, call, *rest):
+        self.calls += 1
+        return 0
+
+
+class DeviceWorkspace(Workspace):
+    def rows(self, name, n, width, dtype, growable=False):
+        return super().rows(name, n, width, dtype, growable).as_subclass(OnDevice)
+
+
+def _setup(fused=True):
+    ops = object.__new__(KernelOps)
+    ops.kind, ops.dtype, ops.act_dtype, ops.legacy_attention, ops.launches = "bf16", "bfloat16", torch.bfloat16, False, 0
+    ops.lib, ops._attn_libs, ops._block_fns, ops._split_rows = Library(), {HD: object()}, {}, 0
+    ops._stream = lambda: ctypes.c_void_p(0)
+    bf = torch.bfloat16
+    norm1, norm2 = RMSNorm(WIDTH, 1e-5), RMSNorm(WIDTH, 1e-5)
+    norm1.weight, norm2.weight = dev(WIDTH), dev(WIDTH)
+    position = SimpleNamespace(tables=[dev(64, HD // 2), dev(64, HD // 2)])
+    position.rotary_tables = lambda device: tuple(position.tables)
+    mixer = GQAAttention(WIDTH, HEADS, KV, HD, position)
+    mixer.w_qkv, mixer.w_o = dev((HEADS + 2 * KV) * HD, WIDTH, dtype=bf), dev(WIDTH, HEADS * HD, dtype=bf)
+    ffn = SwiGLU(WIDTH, INTER)
+    ffn.w_gate_up, ffn.w_down, ffn.fused = dev(2 * INTER, WIDTH, dtype=bf), dev(WIDTH, INTER, dtype=bf), fused
+    view = PagedKVView(dev(4, KV, PAGE, HD, dtype=bf), dev(4, KV, PAGE, HD, dtype=bf), ints(1, 4), PAGE)
+    ctx = SimpleNamespace(ops=ops, workspace=DeviceWorkspace("cpu", 8), n=N, pos=ints(N), row_seq=ints(N), seq_pos0=ints(1), seq_row0=ints(2),
+                          max_keys=64, act_dtype=bf, tile_sets={32: (ints(1), ints(1), ints(1), 1), 64: (ints(1), ints(1), ints(1), 1)})
+    return SimpleNamespace(ops=ops, ctx=ctx, x=dev(N, WIDTH), view=view, position=position, parts=(norm1, mixer, norm2, ffn))
+
+
+def _tile(s, height, i, t):
+    s.ctx.tile_sets[height] = tuple(t if j == i else v for j, v in enumerate(s.ctx.tile_sets[height]))
+
+
+HOST, LONG, APART = "on the host", "64-bit", "not contiguous"
+
+
+def _spoil(how, t):
+    if how == HOST:
+        return torch.zeros(t.shape, dtype=t.dtype)
+    if how == LONG:
+        return dev(*t.shape, dtype=torch.int64 if t.dtype == torch.int32 else torch.float64)
+    return dev(*[2 * n for n in t.shape], dtype=t.dtype)[tuple(slice(None, None, 2) for _ in t.shape)]
+
+
+@pytest.mark.parametrize("fused", [True, False])
+def test_a_plain_block_is_taken(fused):
+    s = _setup(fused)
+    assert s.ops.prenorm_block(s.ctx, s.x, s.view, s.parts) and s.ops.lib.calls == 1
+
+
+@pytest.mark.parametrize("how", [HOST, LONG, APART])
+@pytest.mark.parametrize("what", ["pos", "row_seq", "seq_pos0", "seq_row0", "block_table", "cos", "sin", "tile 32 0", "tile 32 1", "tile 32 2",
+                                  "tile 64 0", "tile 64 1", "tile 64 2"])
+def test_what_the_parts_would_refuse_is_not_handed_over_as_an_address(what, how):
+    s = _setup()
+    if what.startswith("tile"):
+        _, height, i = what.split()
+        if how == APART and s.ctx.tile_sets[int(height)][int(i)].numel() < 2:
+            _tile(s, int(height), int(i), ints(3))  # (a single entry is always contiguous)
+        _tile(s, int(height), int(i), _spoil(how, s.ctx.tile_sets[int(height)][int(i)]))
+    elif what == "block_table":
+        s.view.block_table = _spoil(how, s.view.block_table)
+    elif what in ("cos", "sin"):
+        i = ("cos", "sin").index(what)
+        s.position.tables[i] = _spoil(how, s.position.tables[i])
+    else:
+        if how == APART and getattr(s.ctx, what).numel() < 2:
+            setattr(s.ctx, what, ints(3))
+        setattr(s.ctx, what, _spoil(how, getattr(s.ctx, what)))
+    assert not s.ops.prenorm_block(s.ctx, s.x, s.view, s.parts)
+    assert s.ops.lib.calls == 0
+
+
+def test_a_workspace_on_the_host_is_not_handed_over():
+    s = _setup()
+    s.ctx.workspace = Workspace("cpu", 8)
+    assert not s.ops.prenorm_block(s.ctx, s.x, s.view, s.parts) and s.ops.lib.calls == 0

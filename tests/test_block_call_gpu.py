@@ -48,7 +48,10 @@ def test_one_call_gives_the_bits_of_the_parts(hidden, heads, kv_heads, head_dim,
     assert not model.ops.device_failure()
 
 
-def test_what_the_call_does_not_take_goes_to_the_parts_and_their_checks():
+@pytest.mark.parametrize("what", ["cache type", "64-bit positions", "positions on the host", "rows' sequences on the host", "block table on the host",
+                                  "tiles on the host"])
+def test_what_the_call_does_not_take_goes_to_the_parts_and_their_checks(what):
+    """(What the one call hands over without these checks is shown in test_block_call_cpu.py, where nothing reads it.)"""
     from bitwise_b200.kernels.ops import KernelError
     cfg = LlamaConfig(vocab_size=64, hidden_size=64, num_hidden_layers=1, num_attention_heads=4, num_key_value_heads=2, head_dim=16,
                       intermediate_size=64, tie_word_embeddings=True, max_position_embeddings=64)
@@ -57,6 +60,17 @@ def test_what_the_call_does_not_take_goes_to_the_parts_and_their_checks():
     st = Stepper(model.decoder, manager, storage, model.ops, max_rows=32, max_seqs=2, max_tokens_per_request=64, use_graphs=False)
     ctx, _ = st.prepare([StepEntry("a", [1, 2, 3], [2])])
     view = ctx.cache_views[0]
-    view.k = view.k.float()  # no cache of this precision
+    if what == "cache type":
+        view.k = view.k.float()  # no cache of this precision
+    elif what == "64-bit positions":
+        ctx.pos = ctx.pos.long()
+    elif what == "positions on the host":
+        ctx.pos = ctx.pos.cpu()
+    elif what == "rows' sequences on the host":
+        ctx.row_seq = ctx.row_seq.cpu()
+    elif what == "block table on the host":
+        view.block_table = view.block_table.cpu()
+    else:
+        ctx.tile_sets = {h: (s, r0.cpu(), r, c) for h, (s, r0, r, c) in ctx.tile_sets.items()}
     with pytest.raises(KernelError):
         model.decoder.forward(ctx, ctx.cache_views)
