@@ -89,11 +89,20 @@ class PreNormBlock(Part):
         call = getattr(ctx.ops, "prenorm_block", None)
         if call is None or self.opened or self.next_norm is not None or type(cache) is not PagedKVView:
             return False
-        if type(self.mixer) is not GQAAttention or type(self.feed_forward) is not SwiGLU or self.feed_forward.activation != "silu":
+        if not (_is_plain(self.mixer, GQAAttention) and _is_plain(self.feed_forward, SwiGLU) and self.feed_forward.activation == "silu"):
             return False
-        if type(self.mixer_norm) is not RMSNorm or type(self.ffn_norm) is not RMSNorm:
+        if not (_is_plain(self.mixer_norm, RMSNorm) and _is_plain(self.ffn_norm, RMSNorm)):
             return False
         return call(ctx, x, cache, (self.mixer_norm, self.mixer, self.ffn_norm, self.feed_forward))
+
+
+# what the library's block call stands for; a part whose ``forward`` is another one (a subclass's, or one that a program put in
+# its place to watch or change what passes) runs it
+_PLAIN_FORWARD = {kind: kind.forward for kind in (GQAAttention, SwiGLU, RMSNorm)}
+
+
+def _is_plain(part, kind) -> bool:
+    return type(part) is kind and getattr(part.forward, "__func__", None) is _PLAIN_FORWARD[kind]
 
 
 def chain_norms(blocks) -> None:

@@ -9,6 +9,7 @@ import torch
 from bitwise_b200.kernels.ops import KernelOps
 from bitwise_b200.parts.attention import GQAAttention
 from bitwise_b200.parts.base import PagedKVView, Workspace
+from bitwise_b200.parts.block import PreNormBlock
 from bitwise_b200.parts.mlp import SwiGLU
 from bitwise_b200.parts.norm import RMSNorm
 
@@ -113,3 +114,22 @@ def test_a_workspace_on_the_host_is_not_handed_over():
     s = _setup()
     s.ctx.workspace = Workspace("cpu", 8)
     assert not s.ops.prenorm_block(s.ctx, s.x, s.view, s.parts) and s.ops.lib.calls == 0
+
+
+def test_a_part_whose_forward_a_program_replaced_is_not_passed_by(monkeypatch):
+    s = _setup()
+    norm1, mixer, norm2, ffn = s.parts
+    block = PreNormBlock(WIDTH, mixer, ffn, norm1, norm2, {})
+    assert block._in_one_call(s.ctx, s.x, s.view)
+    for part in s.parts:  # on the object
+        before = part.forward
+        part.forward = lambda *a, **k: before(*a, **k)
+        assert not block._in_one_call(s.ctx, s.x, s.view), type(part).__name__
+        del part.forward
+        assert block._in_one_call(s.ctx, s.x, s.view)
+    for kind in (GQAAttention, SwiGLU, RMSNorm):  # on the class
+        plain = kind.forward
+        with monkeypatch.context() as m:
+            m.setattr(kind, "forward", lambda self, *a, **k: plain(self, *a, **k))
+            assert not block._in_one_call(s.ctx, s.x, s.view), kind.__name__
+    assert block._in_one_call(s.ctx, s.x, s.view)
