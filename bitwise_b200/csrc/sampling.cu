@@ -3,7 +3,8 @@
 
 // ---------------------------------------------------------------------------------------
 // Sampling. One block per logits row.
-//   temperature <= 0: the first index of the maximum (src/engine.cpp:40-45).
+//   temperature <= 0: the first index of the maximum (src/engine.cpp:40-45). A logit that is no number is never larger than
+//   another, so it is passed over, and nothing is larger than one at index 0, which therefore stays.
 //   otherwise: w_i = exp((l_i - max) / T) in 32-bit, total and running sums in 64-bit in
 //   vocabulary order, the first i with cum > u * total, skipping w_i <= 0, else the last
 //   positive one (src/engine.cpp:50-80).  The 64-bit sums are formed per contiguous
@@ -30,11 +31,12 @@ sample_rows_kernel(const float* __restrict__ logits, int vocab, const float* __r
   int best_i = -1;
   for (int i = tid; i < vocab; i += kSampleThreads) {
     const float v = l[i];
-    if (best_i < 0 || v > best) {  // indices come in increasing order: ">" keeps the first maximum
+    if (v > best || (best_i < 0 && v == v)) {  // indices come in increasing order: ">" keeps the first maximum
       best = v;
       best_i = i;
     }
   }
+  if (tid == 0 && l[0] != l[0]) best = l[0], best_i = 0;
   s_val[tid] = best;
   s_idx[tid] = best_i;
   __syncthreads();
@@ -176,7 +178,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
   for (int j = tid; j < count; j += kSampleBlockThreads) {
     const float v = l[first + j];
     seg_values[j] = v;
-    if (best_i < 0 || v > best) best = v, best_i = first + j;  // a thread's indices come in increasing order
+    if (v > best || (best_i < 0 && v == v)) best = v, best_i = first + j;  // a thread's indices come in increasing order
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
@@ -189,6 +191,8 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
   if (tid == 0) {
     for (int w = 1; w < kWarps; ++w)
       if (sample_better(w_val[w], w_idx[w], best, best_i)) best = w_val[w], best_i = w_idx[w];
+    const float head = seg_values[0];  // (this thread's own store)
+    if (rank == 0 && head != head) best = head, best_i = 0;
     b_val = best, b_idx = best_i;
   }
   sample_cluster_sync();

@@ -265,6 +265,37 @@ def test_sample_rows_over_the_vocabulary(vocab):
     assert got[1] == vocab // 2 and got[2] == vocab - 2
 
 
+@pytest.mark.parametrize("vocab", [700, 4095, 4096, 5000, 49152])
+def test_sample_rows_passes_over_logits_that_are_no_number(vocab):
+    """A logit that is no number is never the maximum unless it is the first one, wherever the maximum lies beside it: further on in the
+    same thread's part, in a neighbouring lane's or warp's, in another block's.  With a temperature its weight makes the total no
+    number, and the last positive weight is taken."""
+    rng = np.random.default_rng(vocab)
+    base = min(64 * ((vocab + 511) // 512), vocab // 2)  # where the second of a cluster's blocks begins
+    pairs = [(0, 3), (5, 261), (5, vocab - 1), (vocab - 1, 0)]
+    pairs += [(base + 5, base + d) for d in (0, 4, 7, 13, 21, 29, 37, 5 + 64)] + [(base, 1), (base + 5, 1)]
+    pairs = [(bad, top) for bad, top in pairs if bad < vocab and top < vocab]
+    logits = rnd(rng, len(pairs) + 3, vocab)
+    for r, (bad, top) in enumerate(pairs):
+        logits[r, bad], logits[r, top] = np.nan, 30.0
+    logits[-3] = np.nan
+    logits[-2, 1:] = np.nan
+    logits[-1, :vocab // 2] = np.nan
+    logits[-1, 0] = -np.inf
+    rows = len(logits)
+    out = torch.empty(rows, dtype=torch.int32, device=DEV)
+    u = torch.full((rows,), 0.5, dtype=torch.float64, device=DEV)
+    _ops("bfloat16").sample_rows(t(logits), torch.zeros(rows, device=DEV), u, out)
+    want = [P.argmax_row(row) for row in logits]
+    assert want[:len(pairs)] == [0 if bad == 0 else top for bad, top in pairs]
+    assert out.cpu().tolist() == want
+    flat = np.zeros((2, vocab), dtype=np.float32)
+    flat[0, base + 5] = flat[1, vocab - 1] = np.nan
+    out = torch.empty(2, dtype=torch.int32, device=DEV)
+    _ops("bfloat16").sample_rows(t(flat), torch.ones(2, device=DEV), u[:2].contiguous(), out)
+    assert out.cpu().tolist() == [vocab - 1, vocab - 2]
+
+
 @pytest.mark.parametrize("vocab", [4096, 5000, 49152])
 def test_sample_rows_at_running_sums(vocab):
     """Targets on, just below and just above a running sum, where sums in another order may not be trusted: equal weights (a
