@@ -1217,7 +1217,8 @@ gemm_exact_tile_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
   uint64_t* empty = full + S::kStages;
   volatile uint32_t* gave_up = reinterpret_cast<volatile uint32_t*>(failure);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.y * S::BM, n0 = blockIdx.x * S::BN;
+  const int m0 = static_cast<int>(blockIdx.z * gridDim.y + blockIdx.y) * S::BM, n0 = blockIdx.x * S::BN;
+  if (m0 >= M) return;  // row blocks beyond what one dimension of a grid holds go on along z
   const int lines = (K + kRowsTileK - 1) / kRowsTileK;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::kStages; ++s) bar_init(full + s, 1), bar_init(empty + s, S::kWarps);
@@ -1351,13 +1352,9 @@ int launch_tile(const float* x, const float* w, float* y, const float* residual,
     bw::set_error("linear (32-bit): cuTensorMapEncodeTiled refused [%d x %d] / [%d x %d]", m, k, n, k);
     return -1;
   }
-  const unsigned gy = (m + S::BM - 1) / S::BM;
-  if (gy > 65535u) {
-    bw::set_error("linear: %d rows exceed the grid limit", m);
-    return -1;
-  }
-  bw::launch_pdl(gemm_exact_tile_kernel<TR, TC, WR, WC, BLOCKS>, dim3((n + S::BN - 1) / S::BN, gy), dim3(S::kThreads), static_cast<size_t>(S::kSmem),
-                 stream, map_x, map_w, y, residual, m, n, k, word);
+  const unsigned row_blocks = (m + S::BM - 1) / S::BM, gy = row_blocks < 65535u ? row_blocks : 65535u;
+  bw::launch_pdl(gemm_exact_tile_kernel<TR, TC, WR, WC, BLOCKS>, dim3((n + S::BN - 1) / S::BN, gy, (row_blocks + gy - 1) / gy), dim3(S::kThreads),
+                 static_cast<size_t>(S::kSmem), stream, map_x, map_w, y, residual, m, n, k, word);
   return bw::launch_status();
 }
 
@@ -1463,6 +1460,10 @@ BW_API int bw_f32_linear(const float* x, const float* w, float* y, const float* 
   } else if (m <= 16) {
     gemm_exact_kernel<16><<<dim3(gx, (m + 15) / 16), 256, 0, stream>>>(x, w, y, residual, m, n, k);
   } else if (k % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && f32_encoder() != nullptr) {
+    if (m > 65535 * 128) {
+      bw::set_error("linear: %d rows exceed the grid limit", m);
+      return -1;
+    }
     switch (tile_plan(m, n)) {
 #define BW_CASE(I_, TR_, TC_, WR_, WC_, BLOCKS_) \
   case I_: return launch_tile<TR_, TC_, WR_, WC_, BLOCKS_>(x, w, y, residual, m, n, k, stream);

@@ -120,6 +120,31 @@ def test_f32_linear_of_more_rows_every_tile_gives_the_chain(m, n, k):
     assert not ops.device_failure(), "a kernel gave up a bounded wait"
 
 
+def test_f32_linear_takes_as_many_rows_as_tiles_of_128_would():
+    """More row blocks than one dimension of a grid holds (65,535, of 32 or 64 rows): the bits of the same rows in smaller products,
+    and the limit stays that of 65,535 blocks of 128."""
+    from bitwise_b200.kernels.ops import KernelError
+    ops = _ops("float32")
+    m, k, n = 64 * 65535 + 65, 4, 3
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(1)
+    x, w = torch.randn(m, k, generator=gen, device=DEV), torch.randn(n, k, generator=gen, device=DEV)
+    want = torch.empty(m, n, device=DEV)
+    for i in range(0, m, 1 << 20):
+        ops.linear(x[i:i + (1 << 20)], w, want[i:i + (1 << 20)])
+    try:
+        for tile in (-1, 0, 6):
+            ops.force_f32_tile(tile)
+            out = torch.zeros(m, n, device=DEV)
+            ops.linear(x, w, out)
+            assert torch.equal(out.view(torch.int32), want.view(torch.int32)), f"tile {tile}"
+    finally:
+        ops.force_f32_tile(-1)
+    with pytest.raises(KernelError):
+        ops.linear(torch.zeros(128 * 65535 + 1, k, device=DEV), w[:1], torch.empty(128 * 65535 + 1, 1, device=DEV))
+    assert not ops.device_failure()
+
+
 def test_f32_linear_row_alone_equals_row_in_batch():
     rng = np.random.default_rng(5)
     x, w = rnd(rng, 50, 200), rnd(rng, 77, 200)
