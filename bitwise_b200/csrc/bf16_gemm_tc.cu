@@ -1288,6 +1288,8 @@ BW_API int bw_bf16_linear_tc_rope_usable(const void* x, const void* w, int m, in
   return m > BM && n > 0 && hd == 64 && bw_bf16_linear_tc_usable(x, w, k) && plan_rows(m, n, k, false, false, sm_count_of_device()).pair;
 }
 
+BW_API int bw_bf16_linear(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_f32, const float* residual, int m, int n,
+                          int k, float* partials, int* counters, int use_legacy, cudaStream_t stream);
 BW_API int bw_bf16_rope_cache(__nv_bfloat16* qkv, int row_stride, const int* pos, const int* row_seq, const float* cos_t,
                               const float* sin_t, const int* block_table, int max_blocks, __nv_bfloat16* kcache,
                               __nv_bfloat16* vcache, int n, int heads, int kv_heads, int hd, int page, int write_kv,
@@ -1298,13 +1300,15 @@ BW_API int bw_bf16_linear_tc_rope(const __nv_bfloat16* x, const __nv_bfloat16* w
                                   const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache, int heads,
                                   int kv_heads, int hd, int page, int write_kv, cudaStream_t stream) {
   if (m <= 0 || n <= 0) return 0;
-  if (!bw_bf16_linear_tc_rope_usable(x, w, m, n, k, hd) || n != (heads + 2 * kv_heads) * hd || page <= 0) {
+  if (!bw_bf16_linear_tc_rope_usable(nullptr, nullptr, m, n, k, hd) || n != (heads + 2 * kv_heads) * hd || page <= 0) {
     bw::set_error("linear with rotation (tcgen05): shape [%d x %d] x [%d x %d], %d/%d heads of %d is not for this path", m, k, n, k, heads, kv_heads, hd);
     return -1;
   }
+  // The shape alone brought the call here (whether a step is fused is asked before there are tensors): x or weights that TMA does
+  // not take, and outputs that the epilogue's stores do not, run as the product and the rotation kernel.
   auto off16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 != 0; };
-  if (reinterpret_cast<uintptr_t>(qkv) % 32 || off16(kcache) || off16(vcache) || off16(cos_t) || off16(sin_t)) {
-    const int rc = bw_bf16_linear_tc(x, w, qkv, 0, nullptr, m, n, k, nullptr, nullptr, stream);
+  if (off16(x) || off16(w) || reinterpret_cast<uintptr_t>(qkv) % 32 || off16(kcache) || off16(vcache) || off16(cos_t) || off16(sin_t)) {
+    const int rc = bw_bf16_linear(x, w, qkv, 0, nullptr, m, n, k, nullptr, nullptr, 0, stream);
     return rc ? rc : bw_bf16_rope_cache(qkv, n, pos, row_seq, cos_t, sin_t, block_table, max_blocks, kcache, vcache, m, heads, kv_heads, hd, page, write_kv, stream);
   }
   int* word = bw::failure_word();

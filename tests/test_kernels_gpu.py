@@ -655,6 +655,35 @@ def test_bf16_qkv_product_of_many_rows_that_rotates_and_stores(m, width, heads, 
     assert not ops.device_failure()
 
 
+def test_bf16_qkv_product_of_many_rows_takes_weights_of_any_start():
+    """x and weights that do not start on 16 bytes are no operands of TMA; the call takes them all the same."""
+    rng = np.random.default_rng(2)
+    ops = _ops("bfloat16")
+    from bitwise_b200.parts.rope import RotaryEncoding
+    m, width, heads, kv_heads, hd, page = 300, 2048, 32, 32, 64, 16
+    assert ops.fuses_rope(m, width, heads, kv_heads, hd)
+    n, b16 = (heads + 2 * kv_heads) * hd, torch.bfloat16
+    x, w = t(bf(rnd(rng, m, width)), b16), t(bf(rnd(rng, n, width, scale=0.05)), b16)
+    cos, sin = RotaryEncoding(hd, 10000.0, None, positions=512).rotary_tables(DEV)
+    pos = torch.arange(m, dtype=torch.int32, device=DEV)
+    table = torch.arange((m + page - 1) // page, dtype=torch.int32, device=DEV).view(1, -1)
+
+    def moved(a, lead):
+        flat = torch.empty(a.numel() + lead, device=DEV, dtype=b16)
+        flat[lead:] = a.reshape(-1)
+        return flat[lead:].view(a.shape)
+    outs = []
+    for lead_x, lead_w in ((0, 0), (0, 4), (2, 0)):
+        k, v = (torch.zeros(table.shape[1], kv_heads, page, hd, device=DEV, dtype=b16) for _ in range(2))
+        qkv = torch.zeros(m, n, device=DEV, dtype=b16)
+        ops.linear_rope_cache(moved(x, lead_x), moved(w, lead_w), qkv, pos, torch.zeros_like(pos), cos, sin, table, k, v, heads, kv_heads, hd)
+        outs.append((qkv[:, :heads * hd].contiguous(), k, v))
+    for other in outs[1:]:
+        for got, want in zip(other, outs[0]):
+            assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    assert not ops.device_failure()
+
+
 def test_bf16_rmsnorm_and_swiglu():
     """Tolerance: one bfloat16 rounding of a float32 result (2^-8 relative) plus 1e-6 absolute."""
     rng = np.random.default_rng(9)
