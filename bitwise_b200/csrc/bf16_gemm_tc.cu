@@ -754,7 +754,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           glu(std::integral_constant<int, bw::kGluGeluTanh>{});
         else
           glu(std::integral_constant<int, bw::kGluSilu>{});
-        store_turned(store_buf, reinterpret_cast<char*>(out), static_cast<size_t>(N), warp_rows, lane);
+        if (WIDE || turned) {
+          store_turned(store_buf, reinterpret_cast<char*>(out), static_cast<size_t>(N), warp_rows, lane);
+        } else {  // outputs that do not start on 16 bytes, as the second kernel of a split product takes them
+          __syncwarp();
+          for (int t = 0; t < 8; ++t) {
+            const uint4 v = get_piece(store_buf, lane, t);
+            const int r = 4 * t + (lane >> 3);
+            if (r >= warp_rows) continue;
+            uint16_t* to = reinterpret_cast<uint16_t*>(out + static_cast<size_t>(r) * (N / 2) + (lane & 7) * 8);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) to[2 * e] = static_cast<uint16_t>(w[e]), to[2 * e + 1] = static_cast<uint16_t>(w[e] >> 16);
+          }
+          __syncwarp();
+        }
       } else if (EPI == 3) {
         // The fused q/k/v product rotates and stores itself: a thread owns a row, and with it both partners of every rotation
         // of its heads (a piece of 64 columns is a head). Rounded to bfloat16 as the stored product would be, rotated with rope_cache_bf16_kernel's arithmetic (same bits), turned

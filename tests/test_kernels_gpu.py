@@ -520,6 +520,29 @@ def test_bf16_linear_narrow_tiles_of_many_rows_give_the_same_bits(m, n, k):
     assert not ops.device_failure()
 
 
+@pytest.mark.parametrize("m,inter,k", [(20, 192, 1544), (100, 128, 512), (128, 64, 4096), (40, 320, 64)])
+def test_bf16_linear_swiglu_into_an_output_of_any_start(m, inter, k):
+    """Whole or split, the gate/up product of a batch writes an output that does not start on 16 bytes, with the same bits."""
+    rng = np.random.default_rng(m + inter)
+    ops = _ops("bfloat16")
+    b16 = torch.bfloat16
+    x = t(bf(rnd(rng, m, k)), b16)
+    w = ops.interleave_gate_up(t(bf(rnd(rng, inter, k, scale=0.05)), b16), t(bf(rnd(rng, inter, k, scale=0.05)), b16))
+    want = torch.empty(m, inter, device=DEV, dtype=b16)
+    ops.linear_swiglu(x, w, want)
+    try:
+        for mode in (0, 1, 2):
+            ops.force_linear_plan(128 if mode else 0, mode)
+            for lead in (1, 2, 4):
+                flat = torch.full((m * inter + lead + 8,), 7.0, device=DEV, dtype=b16)
+                ops.linear_swiglu(x, w, flat[lead:lead + m * inter].view(m, inter))
+                assert torch.equal(flat[lead:lead + m * inter].view(m, inter).view(torch.int16), want.view(torch.int16)), (mode, lead)
+                assert (flat[:lead] == 7.0).all() and (flat[lead + m * inter:] == 7.0).all()
+    finally:
+        ops.force_linear_plan(0, 0)
+    assert not ops.device_failure()
+
+
 def test_bf16_linear_few_rows_kernel_gives_the_same_bits():
     """Steps of up to 16 rows run their products on the streaming kernel (a warp per 8 columns
     and chunk, chunk sums added inside the kernel, clusters of blocks when k is long). Same bits
