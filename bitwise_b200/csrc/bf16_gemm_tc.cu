@@ -1299,7 +1299,8 @@ BW_API int bw_bf16_linear_tc(const __nv_bfloat16* x, const __nv_bfloat16* w, voi
 // rows through 32 layers of width 960: 2,264 us, with rotating narrow tiles 2,273), and heads of 128 spread a row's tables
 // over twice the lines (attention of 1,200 rows at 32 heads of 128: 203 us, with this epilogue 207).
 BW_API int bw_bf16_linear_tc_rope_usable(const void* x, const void* w, int m, int n, int k, int hd) {
-  return m > BM && n > 0 && hd == 64 && bw_bf16_linear_tc_usable(x, w, k) && plan_rows(m, n, k, false, false, sm_count_of_device()).pair;
+  return g_pair_tiles && m > BM && n > 0 && hd == 64 && bw_bf16_linear_tc_usable(x, w, k) &&
+         plan_rows(m, n, k, false, false, sm_count_of_device()).pair;
 }
 
 BW_API int bw_bf16_linear(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_f32, const float* residual, int m, int n,

@@ -354,6 +354,7 @@ class KernelOps:
         one per 128 x 256 tile; same bits either way.  Returns the previous setting."""
         if self.kind != "bf16":
             return False
+        self._kernel_counts.clear()
         return bool(self.lib.bw_bf16_linear_tc_pair_tiles(_c_int(int(on))))
 
     def rows_path(self, on: bool) -> bool:

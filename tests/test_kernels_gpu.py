@@ -707,6 +707,19 @@ def test_bf16_qkv_product_of_many_rows_takes_weights_of_any_start():
     assert not ops.device_failure()
 
 
+def test_bf16_single_block_tiles_cover_the_product_that_rotates():
+    """With block pairs switched off no product runs on them, the fused q/k/v product of many rows included."""
+    ops = _ops("bfloat16")
+    assert ops.fuses_rope(300, 2048, 32, 32, 64)
+    before = ops.pair_tiles(False)
+    try:
+        assert not ops.fuses_rope(300, 2048, 32, 32, 64)
+        assert ops.fuses_rope(8, 2048, 32, 32, 64)
+    finally:
+        ops.pair_tiles(before)
+    assert ops.fuses_rope(300, 2048, 32, 32, 64)
+
+
 def test_bf16_rmsnorm_and_swiglu():
     """Tolerance: one bfloat16 rounding of a float32 result (2^-8 relative) plus 1e-6 absolute."""
     rng = np.random.default_rng(9)
