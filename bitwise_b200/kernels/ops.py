@@ -599,7 +599,8 @@ class KernelOps:
                                                                       _c_int(qkv.shape[1])))
                     self._tc_tile_rows[shape_key] = rows_tc
                 sets = getattr(batch, "tile_sets", None)
-                if rows_tc > 0 and (sets is None or rows_tc in sets) and n > t_count:
+                # (it stores 16 bytes at a time; outputs that do not start there go to the kernel below)
+                if rows_tc > 0 and (sets is None or rows_tc in sets) and n > t_count and out.data_ptr() % 16 == 0:
                     q_seq, q_row0, q_rows, q_count = batch.query_tiles(rows_tc)
                     for t_ in (q_seq, q_row0, q_rows):
                         _need(t_, torch.int32, "attention step arrays")

@@ -1017,6 +1017,34 @@ def test_bf16_attention_decode_of_wide_heads_through_boxes_gives_the_same_bits(h
     assert not ops.device_failure()
 
 
+@pytest.mark.parametrize("hd,heads,kv_heads", [(64, 3, 1), (128, 6, 2), (64, 4, 2)])
+def test_bf16_attention_of_many_rows_into_an_output_of_any_start(hd, heads, kv_heads):
+    """The tcgen05 kernel stores 16 bytes at a time; an output that starts elsewhere gets the same bits from the other kernel."""
+    rng = np.random.default_rng(hd + heads)
+    ops = _ops("bfloat16")
+    lens = [70, 33]
+    k, v, table, _, _ = _paged(rng, lens, kv_heads, hd, 16)
+    n, b16 = sum(lens), torch.bfloat16
+    qkv = t(bf(rnd(rng, n, (heads + 2 * kv_heads) * hd)), b16)
+    I = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+
+    class Batch:
+        seq_row0, seq_pos0 = I([0, 70, 103]), I([0, 0])
+        tile_sets = {rows: None for rows in ops.attention_tile_heights(heads, kv_heads, hd)}
+
+        def query_tiles(self, rows):
+            tiles = [(s, (0, 70)[s] + a, min(rows, c - a)) for s, c in enumerate(lens) for a in range(0, c, rows)]
+            return I([x[0] for x in tiles]), I([x[1] for x in tiles]), I([x[2] for x in tiles]), len(tiles)
+    outs = []
+    for lead in (0, 2, 4):
+        out = torch.zeros(n * heads * hd + lead, device=DEV, dtype=b16)[lead:].view(n, heads * hd)
+        ops.attention(qkv, t(k, b16), t(v, b16), I(table), I([0] * 70 + [1] * 33), I(list(range(70)) + list(range(33))), out, heads, kv_heads,
+                      hd, 0, 70, 0.125, batch=Batch())
+        outs.append(out.contiguous().view(torch.int16).cpu())
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    assert not ops.device_failure()
+
+
 def test_bf16_attention_tensor_core_generations_agree_bit_for_bit():
     """The tcgen05 prefill kernel (head sizes 64 and 128) and the mma.sync kernels give the same
     bits: whole prompts, late portions, with a window, grouped heads, several sequences in a step."""
