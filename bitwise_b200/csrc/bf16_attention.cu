@@ -691,12 +691,13 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 // is 32 KB, persistent blocks have room for three warps with two of them each, and six blocks of
 // one warp keep the memory busier (64 rows, 32/8 heads, 900 to 4,090 keys, with the merge: 159 us
 // by cp.async, 146 persistent, 127 here, for keys and values that take 100 at the copy bandwidth).
+constexpr int kTileGridZ = 65535;
 __global__ void __launch_bounds__(32)
 attention_tile_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                           const __nv_bfloat16* __restrict__ qkv, int q_stride, const int* __restrict__ block_table,
                           int max_blocks, const int* __restrict__ row_seq, const int* __restrict__ pos, int heads,
                           int kv_heads, int page, int window, float scale_log2, float* __restrict__ tile_out, int max_tiles,
-                          int* failure) {
+                          int n, int* failure) {
   extern __shared__ __align__(1024) unsigned char tile_raw[];
   unsigned char* base = bw::smem_align_1024(tile_raw);
   unsigned char* sq = base;                  // 16 stacked rows of 128 bytes
@@ -704,7 +705,9 @@ attention_tile_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
   unsigned char* sv = sk + kKVBytes;
   uint64_t* bar = reinterpret_cast<uint64_t*>(sv + kKVBytes);
   const int lane = threadIdx.x;
-  const int row = blockIdx.x, g = blockIdx.y, t = blockIdx.z;
+  int row = blockIdx.x, t = blockIdx.z;
+  const int g = blockIdx.y;
+  if (row >= n) t += row / n * kTileGridZ, row %= n;  // key tiles beyond what a grid's z holds go on along x
   const int group = heads / kv_heads;
   const int p = pos[row];
   const int first = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
@@ -958,13 +961,10 @@ BW_API int bw_bf16_attention_stream(const __nv_bfloat16* qkv, int q_stride, cons
   const bool stream_it = HD == 64 && (g_stream_mode == 2 || (g_stream_mode == 1 && static_cast<long long>(n) * kv_heads >= kStreamMinHeads));
   if (!stream_it) {  // a block per key tile
     constexpr int tile_smem = kStreamItemBytes + 8 + 1008;  // dynamic shared memory starts on 16 bytes; six blocks fit an SM at head size 128
-    if (key_tiles > 65535 || kv_heads > 65535) {
-      bw::set_error("attention: %d key tiles or %d key/value heads exceed the grid limit", key_tiles, kv_heads);
-      return -1;
-    }
-    bw::launch_pdl(attention_tile_tma_kernel, dim3(n, kv_heads, key_tiles), dim3(32), tile_smem, stream, map_k, map_v, qkv,
-                   q_stride, block_table, max_blocks, row_seq, pos, heads, kv_heads, page, window, scale_log2, scratch,
-                   key_tiles, word);
+    const int slices = (key_tiles + kTileGridZ - 1) / kTileGridZ;
+    bw::launch_pdl(attention_tile_tma_kernel, dim3(n * slices, kv_heads, key_tiles < kTileGridZ ? key_tiles : kTileGridZ), dim3(32),
+                   tile_smem, stream, map_k, map_v, qkv, q_stride, block_table, max_blocks, row_seq, pos, heads, kv_heads, page, window,
+                   scale_log2, scratch, key_tiles, n, word);
     bw::launch_pdl(merge_tiles_kernel, dim3(dim3(n, heads)), dim3(kMergeThreads), 0, stream, scratch, key_tiles, pos, out,
                    out_stride, heads, window);
     return bw::launch_status();

@@ -1045,6 +1045,43 @@ def test_bf16_attention_of_many_rows_into_an_output_of_any_start(hd, heads, kv_h
     assert not ops.device_failure()
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+def test_bf16_attention_decode_over_more_key_tiles_than_a_grid_holds(hd):
+    """A row of 4.2 million keys has more tiles of 64 than one dimension of a grid.  Its pages stand for three in turn, so that the
+    softmax is that of three pages' keys, each as often as its pages come."""
+    rng = np.random.default_rng(hd)
+    ops = _ops("bfloat16")
+    heads, kv_heads, page, n = 2, 1, 64, 2
+    last = [64 * 65535 + 70, 130]
+    blocks = last[0] // page + 1
+    k, v = bf(rnd(rng, 3, kv_heads, page, hd)), bf(rnd(rng, 3, kv_heads, page, hd))
+    q = bf(rnd(rng, n, heads, hd))
+    qkv = np.zeros((n, (heads + 2 * kv_heads) * hd), dtype=np.float32)
+    qkv[:, :heads * hd] = q.reshape(n, -1)
+    I = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    table = (torch.arange(blocks, device=DEV, dtype=torch.int32) % 3).repeat(n, 1).contiguous()
+
+    class Batch:
+        seq_row0, seq_pos0, tile_sets = I([0, 1, 2]), I(last), {}
+
+        def query_tiles(self, rows):
+            return I([0, 1]), I([0, 1]), I([1, 1]), 2
+    out = torch.zeros(n, heads * hd, device=DEV, dtype=torch.bfloat16)
+    ops.attention(t(qkv, torch.bfloat16), t(k, torch.bfloat16), t(v, torch.bfloat16), table, I([0, 1]), I(last), out, heads, kv_heads, hd, 0,
+                  last[0] + 1, 1.0 / np.sqrt(hd), batch=Batch())
+    got = out.float().cpu().numpy().reshape(n, heads, hd)
+    keys, values = k[:, 0].reshape(-1, hd).astype(np.float64), v[:, 0].reshape(-1, hd).astype(np.float64)
+    for r in range(n):
+        times = np.array([(last[r] + 1) // 192] * 192) + (np.arange(192) < (last[r] + 1) % 192)
+        for h in range(heads):
+            s = keys @ q[r, h].astype(np.float64) / np.sqrt(hd)
+            w = times * np.exp(s - s.max())
+            want = w @ values / w.sum()
+            # 2^-9 each for weights and result in bfloat16, up to 65,537 / 2^24 for the merge of the tiles one after the other
+            assert np.abs(got[r, h] - want).max() <= 2.0 ** -7 * np.abs(values).max(), (r, h)
+    assert not ops.device_failure()
+
+
 def test_bf16_attention_tensor_core_generations_agree_bit_for_bit():
     """The tcgen05 prefill kernel (head sizes 64 and 128) and the mma.sync kernels give the same
     bits: whole prompts, late portions, with a window, grouped heads, several sequences in a step."""
