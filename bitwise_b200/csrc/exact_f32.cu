@@ -1336,14 +1336,17 @@ bool f32_tile_map(CUtensorMap* map, const void* base, int rows, int k, int box_r
 template <int TR, int TC, int WR, int WC, int BLOCKS>
 int launch_tile(const float* x, const float* w, float* y, const float* residual, int m, int n, int k, cudaStream_t stream) {
   using S = TileShape<TR, TC, WR, WC, BLOCKS>;
-  static bool configured = false;
-  if (!configured) {
+  constexpr int kMaxDevices = 64;
+  static bool configured[kMaxDevices] = {false};  // a kernel's limit is raised for one device
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = 0;
+  if (!configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(gemm_exact_tile_kernel<TR, TC, WR, WC, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
     if (e != cudaSuccess) {
       bw::set_error("linear (32-bit): cannot raise shared memory: %s", cudaGetErrorString(e));
       return static_cast<int>(e);
     }
-    configured = true;
+    configured[dev] = true;
   }
   int* word = bw::failure_word();
   if (!word) return -1;

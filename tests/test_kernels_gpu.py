@@ -145,6 +145,26 @@ def test_f32_linear_takes_as_many_rows_as_tiles_of_128_would():
     assert not ops.device_failure()
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs a second device")
+def test_f32_linear_of_more_rows_on_a_second_device():
+    """A kernel's shared-memory limit is raised for one device at a time.  (A process of its own: a library has one failure word.)"""
+    import subprocess
+    import sys
+    child = """
+import torch
+from bitwise_b200.kernels.ops import KernelOps
+x, w = torch.arange(70 * 64).view(70, 64).remainder(13).float(), torch.arange(130 * 64).view(130, 64).remainder(7).float()
+kept = []
+for dev in (0, 1):
+    torch.cuda.set_device(dev)
+    kept.append(KernelOps("float32"))
+    out = torch.empty(70, 130, device="cuda")
+    kept[-1].linear(x.cuda(), w.cuda(), out)
+    assert torch.equal(out.cpu(), x @ w.T), dev  # whole numbers: exact in any order
+"""
+    subprocess.run([sys.executable, "-c", child], check=True, timeout=600)
+
+
 def test_f32_linear_row_alone_equals_row_in_batch():
     rng = np.random.default_rng(5)
     x, w = rnd(rng, 50, 200), rnd(rng, 77, 200)
