@@ -293,14 +293,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const int b = t & 1;
       if (t + 1 < ntiles) ok = issue_qk(t + 1);  // the next tile's scores are computed while this one's weights are formed
       if (!ok) break;
-      if (!wait(&bars->p_ready[b], (t >> 1) & 1)) break;
-      // the output buffer was merged (tile t - 2) before the softmax of this tile began: same argument
-      fence_after_sync();
-      const uint64_t pdesc = make_desc(smem_u32(sp + b * kPBytes));
-      const uint32_t v_addr = smem_u32(skv + s * 2 * kKBytes + kKBytes);
-      const uint64_t vdesc = kPieces == 1 ? make_desc(v_addr) : make_desc_wide(v_addr, kKPiece);
       // Behind the block's last key lies whatever the page's last holder left. Its weights are zero; its values become zero as
-      // well, so that an infinity left there cannot reach a sum.
+      // well, so that an infinity left there cannot reach a sum. (The tile landed before its scores were formed, so
+      // this goes on beside its softmax.)
       if (t + 1 == ntiles && kv_lo + ntiles * kTileKV > kv_hi) {
         unsigned char* sv = skv + s * 2 * kKBytes + kKBytes;
         for (int c = (kv_hi - kv_lo - t * kTileKV) * 8 + lane; c < kTileKV * 8; c += 32)
@@ -309,6 +304,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
       }
+      if (!wait(&bars->p_ready[b], (t >> 1) & 1)) break;
+      // the output buffer was merged (tile t - 2) before the softmax of this tile began: same argument
+      fence_after_sync();
+      const uint64_t pdesc = make_desc(smem_u32(sp + b * kPBytes));
+      const uint32_t v_addr = smem_u32(skv + s * 2 * kKBytes + kKBytes);
+      const uint64_t vdesc = kPieces == 1 ? make_desc(v_addr) : make_desc_wide(v_addr, kKPiece);
       if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < kTileKV / 16; ++k)  // 16 keys: 32 bytes along a row of P, two 8-key groups (2048 bytes) of V
