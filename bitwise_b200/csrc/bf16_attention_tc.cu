@@ -496,11 +496,6 @@ BW_API int bw_bf16_attention_tc_query_rows(int heads, int kv_heads, int hd, int 
   if (group > kTileM || page <= 0 || kTileKV % page || q_stride % 8 || !encoder()) return 0;
   return kTileM / group;
 }
-// The same for groups that fill a block's rows exactly, else 0.
-BW_API int bw_bf16_attention_tc_tile_rows(int heads, int kv_heads, int hd, int page, int q_stride) {
-  const int rows = bw_bf16_attention_tc_query_rows(heads, kv_heads, hd, page, q_stride);
-  return rows && kTileM % (heads / kv_heads) == 0 ? rows : 0;
-}
 
 BW_API int bw_bf16_attention_tc(const __nv_bfloat16* qkv, int q_stride, const __nv_bfloat16* kcache,
                                 const __nv_bfloat16* vcache, int num_pages, const int* block_table, int max_blocks,
@@ -562,6 +557,5 @@ BW_API int bw_bf16_attention_tc(const __nv_bfloat16* qkv, int q_stride, const __
 #else  // other head sizes use the kernels of bf16_attention.cu
 
 BW_API int bw_bf16_attention_tc_query_rows(int, int, int, int, int) { return 0; }
-BW_API int bw_bf16_attention_tc_tile_rows(int, int, int, int, int) { return 0; }
 
 #endif

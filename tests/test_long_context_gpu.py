@@ -145,12 +145,20 @@ def test_bfloat16_batch_of_different_lengths_replays_graphs(name, tiny_folders):
 
 
 def test_bfloat16_many_requests_through_the_streaming_kernel(tiny_folders):
-    """34 live requests (the streaming decode kernel takes steps of 32 rows or more at head size
-    64) whose contexts pass 128, 192 and 256 keys while they decode together."""
+    """34 live requests through the streaming decode kernel (head size 64; asked for, as it would be chosen for more rows) whose
+    contexts pass 128, 192 and 256 keys while they decode together."""
     name = "tiny_long"
     model = _model(tiny_folders[name], "bfloat16")
     c = model.decoder.config
     lib = model.ops._attention_lib(c.head_dim)
+    before = model.ops.stream_attention(c.head_dim, 2)
+    try:
+        _many_requests(model, c, lib, name, tiny_folders)
+    finally:
+        model.ops.stream_attention(c.head_dim, before)
+
+
+def _many_requests(model, c, lib, name, tiny_folders):
     assert lib.bw_bf16_attention_stream_usable(34, c.num_attention_heads, c.num_key_value_heads, c.head_dim, 16,
                                                (c.num_attention_heads + 2 * c.num_key_value_heads) * c.head_dim)
     reqs, heads = {}, {}
