@@ -1019,17 +1019,24 @@ int sm_count_of_device() {
 }
 
 // How a product with few tiles runs. The plan is the one of least estimated time, from times measured on a B200 (us):
-//   whole   items are output tiles with all their chunks; a chunk of a tile takes kChunkUs by the tile's width, rounds of the SMs
+//   whole   items are output tiles with all their chunks; a chunk of a tile takes chunk_us by the tile's width, rounds of the SMs
 //           over the items follow each other, and a launch costs about 6 us around them
-//   split   items are (tile, chunk) pairs; the second kernel costs about 2 us (little up to 16 rows), and the chunk sums are written and read
-//           (8 bytes each) at about 5 TB/s. One block of rows only: beyond it the chunk sums outgrow what they save
+//   split   items are (tile, chunk) pairs; the second kernel costs about 2 us (little up to 16 rows), and the chunk sums are written
+//           and read (8 bytes each) at about 5 TB/s. One block of rows only: beyond it the chunk sums outgrow what they save
 //   pairs   more than 128 rows: 256 x 256 tiles on pairs of blocks, 2.45 us a chunk, 8.5 us around them (10.5 where a
 //           residual is read or SwiGLU applied)
 // and none is faster than its operands arrive: a chunk's rows of x and W at about 83 KB a us for a block, and at about 9.5 TB/s
 // over all SMs. Tiles are 16 .. 128
-// columns wide in steps of 16, or 256 with one block of rows. Of equal plans the one with the narrower tiles wins (more SMs
-// stream weights). Every plan gives the same bits. What the estimate changed against counting steps of the tensor core:
-// 128 rows x 2,048 x 6,144 23.3 -> 14.9 us, 512 x 960 x 960 15.6 -> 10.5, 512 x 2,560 x 960 25 -> 17.
+// columns wide in steps of 16, or 256 with one block of rows (split along k only where one round of the SMs takes all its
+// items: nothing hides such an item's fill and drain). Of equal plans the one with the narrower tiles wins (more SMs stream
+// weights). Every plan gives the same bits.
+//
+// The times are those of 17 to 128 rows at 14 shapes from 960 x 960 to 28,672 x 4,096, every width and mode of each; the plan
+// chosen is on average 3 % behind the best one. Tiles of 16 to 48 columns were first taken as faster than they are (64 rows x
+// 2,048 x 6,144: 48 columns 17.5 us, 64 columns 14.5; 32 and 48 rows 15.6 and 16.4, 12.8 and 14.4; 48 rows x 4,096 x 6,144 in 48
+// columns 22.3, now 20.4). Against counting steps of the tensor core: 128 rows x 2,048 x 6,144 28.2 -> 14.6 us, 512 x 960 x
+// 960 15.6 -> 10.5, 512 x 2,560 x 960 25 -> 17; up to 33 rows x 8,192 x 2,048 and x 4,096 x 4,096 are 2 to 5 % slower than with
+// the kernel of that rule, at the same plans (17 rows: 16.8 -> 17.5 us, 16.3 -> 16.6).
 struct Plan {
   bool split;
   int bn;
@@ -1042,9 +1049,11 @@ constexpr int kMaxSplitColumns = 16384;  // bounds the scratch of the chunk sums
 
 // a chunk of a narrow or wide tile, by its width / 16
 double chunk_us(int bn) {
-  constexpr double us[] = {1.25, 1.25, 1.5, 1.8, 1.95, 2.05, 2.2, 2.3};
+  constexpr double us[] = {1.5, 1.55, 2.1, 1.8, 1.95, 2.05, 2.2, 2.35};
   return bn > BN ? 3.3 : us[bn / 16 - 1];
 }
+
+constexpr double kWideChunkAloneUs = 4.6;  // of a split product in tiles of 256 columns
 
 Plan plan_rows(int m, int n, int k, bool swiglu, bool reads, int sms, bool allow_wide = true) {
   const int chunks = (k + kChunk - 1) / kChunk;
@@ -1073,15 +1082,18 @@ Plan plan_rows(int m, int n, int k, bool swiglu, bool reads, int sms, bool allow
       // of several row blocks only tiles of 64 and 128 columns: 200 rows x 2,048 x 6,144 took 25 us in tiles of 112, 19 in pairs
       if (!one_block && bn != BN / 2 && bn != BN && !g_tile_width) continue;
       if (bn > BN && (!allow_wide || n % 64 || !one_block)) continue;
-      if (g_tile_width && bn != g_tile_width && !(swiglu && g_tile_width < BN && bn == BN) && !(!one_block && g_tile_width > BN && !best.pair)) continue;
+      if (g_tile_width && bn != g_tile_width && !(swiglu && g_tile_width < BN && bn == BN) &&
+          !(!one_block && g_tile_width > BN && !best.pair))
+        continue;
       const long long tiles = static_cast<long long>((n + bn - 1) / bn) * m_blocks;
       const long long items = mode ? tiles * chunks : tiles;
       const long long rounds = (items + sms - 1) / sms;
-      const double step = std::max(chunk_us(bn), (a_rows + bn) * block_us_per_kb);
+      if (mode == 1 && bn > BN && rounds > 1 && !g_tile_width) continue;
+      const double step = std::max(mode == 1 && bn > BN ? kWideChunkAloneUs : chunk_us(bn), (a_rows + bn) * block_us_per_kb);
       double cost = static_cast<double>(rounds) * step * (mode ? 1 : chunks);
       const double arrive = static_cast<double>(tiles) * chunks * (a_rows + bn) * us_per_kb;
       if (cost < arrive) cost = arrive;
-      cost += mode ? (m <= 16 ? 5.5 : 8.2) + 1.6e-6 * chunks * static_cast<double>(m) * n : 6.0;
+      cost += mode ? (m <= 16 ? 5.5 : 8.5) + 1.6e-6 * chunks * static_cast<double>(m) * n : 6.0;
       // pairs give way only to a clearly lower estimate (it is good to about a tenth)
       if (best_cost < 0 || cost < best_cost * (best.pair ? 0.9 : 1.0) - 1e-9) best = Plan{mode == 1, bn, false}, best_cost = cost;
     }
