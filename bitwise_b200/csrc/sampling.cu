@@ -12,30 +12,73 @@
 //   reference adds strictly one by one, which differs from this by 64-bit rounding only.
 constexpr int kSampleThreads = 512;
 
-__global__ void __launch_bounds__(kSampleThreads)
+// The weight of a logit.
+__device__ __forceinline__ float sample_weight(float l, float mx, float temp) {
+  return bw::det_expf(__fdiv_rn(__fsub_rn(l, mx), temp));
+}
+// Sums taken as trees differ from the serial ones by rounding only, and by no more than a known bound: a sum of n positive terms
+// in any order of additions of which each term passes through at most a is off by at most a / 2^53 of the sum. The serial
+// running sums have a <= 2 seg + 512 and their target seg + 512, those of the kernels below less than seg / 4 + 64 each. With
+// the rounding of the comparisons, twice the serial bound is the distance from which a tree sum tells on which side of the
+// target its serial one lies.
+__device__ __forceinline__ double sample_near(double total, int seg) {
+  return total * (2 * seg + kSampleThreads + 128) * 2.220446049250313e-16;
+}
+// One warp: the first of a segment's `len` weights whose running sum (`base` before the segment) passes the target; -1 when
+// there is none or a sum is too near to tell.
+template <typename Weight>
+__device__ __forceinline__ int sample_scan(int len, Weight weight, double base, double target, double near, int lane) {
+  for (int j0 = 0; j0 < len; j0 += 32) {
+    const float w = j0 + lane < len ? weight(j0 + lane) : 0.0f;
+    double run = static_cast<double>(w);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const double o = __shfl_up_sync(0xffffffffu, run, d);
+      if (lane >= d) run += o;
+    }
+    const double cum = base + run;
+    const uint32_t over = __ballot_sync(0xffffffffu, w > 0.0f && cum > target);
+    if (over) {
+      const int at = __ffs(over) - 1;
+      const bool clear = cum - target > near && target - (cum - static_cast<double>(w)) > near;
+      return __shfl_sync(0xffffffffu, clear ? 1 : 0, at) ? j0 + at : -1;
+    }
+    base = __shfl_sync(0xffffffffu, cum, 31);
+  }
+  return -1;
+}
+
+// A block per row: steps of many rows, whose blocks fill the machine, and small vocabularies. Four lanes share a segment, eight
+// segments are in flight in a warp; where the tree sums do not settle the token (see below) it is found again with one
+// thread per segment and every sum in order. Bound by the exponentials and the reads behind them: with serial sums alone 512
+// rows of 8,192 logits took 27 us at a temperature, with trees 21; 64 rows of 128,256 156 and 64. 32 registers, four blocks an SM.
+__global__ void __launch_bounds__(kSampleThreads, 4)
 sample_rows_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
                    const double* __restrict__ uniform, int* __restrict__ out_token) {
   bw::pdl_enter();
   const int row = blockIdx.x;
   const float* l = logits + static_cast<size_t>(row) * vocab;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int kWarps = kSampleThreads / 32;
   __shared__ float s_val[kSampleThreads];
   __shared__ int s_idx[kSampleThreads];
   __shared__ double s_sum[kSampleThreads];
+  __shared__ double w_sum[kWarps];
   __shared__ double s_total;
   __shared__ int s_pick;
   __shared__ int s_last;
 
-  // maximum and its first index
+  // maximum and its first index (indices come in increasing order: ">" keeps the first maximum)
   float best = -INFINITY;
   int best_i = -1;
+#pragma unroll 8
   for (int i = tid; i < vocab; i += kSampleThreads) {
     const float v = l[i];
-    if (v > best || (best_i < 0 && v == v)) {  // indices come in increasing order: ">" keeps the first maximum
-      best = v;
-      best_i = i;
-    }
+    if (v > best) best = v, best_i = i;
   }
+  if (best_i < 0)  // nothing above minus infinity here: the first that is a number
+    for (int i = tid; i < vocab && best_i < 0; i += kSampleThreads)
+      if (l[i] == l[i]) best_i = i;
   if (tid == 0 && l[0] != l[0]) best = l[0], best_i = 0;
   s_val[tid] = best;
   s_idx[tid] = best_i;
@@ -60,14 +103,71 @@ sample_rows_kernel(const float* __restrict__ logits, int vocab, const float* __r
     if (tid == 0) out_token[row] = arg;
     return;
   }
-
-  // contiguous segment of this thread
   const int seg = (vocab + kSampleThreads - 1) / kSampleThreads;
+
+  // tree sums: of every segment, and of what lies before it
+  for (int s = warp * 32 + (lane >> 2); s < warp * 32 + 32; s += 8) {
+    const int from = min(vocab, s * seg), len = min(vocab, from + seg) - from;
+    double local = 0.0;
+    for (int j0 = lane & 3; j0 < len; j0 += 4 * 4) {
+      float v[4];  // asked for together
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = j0 + 4 * e < len ? l[from + j0 + 4 * e] : -INFINITY;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (j0 + 4 * e < len) local += static_cast<double>(sample_weight(v[e], mx, temp));
+    }
+    local += __shfl_xor_sync(0xffffffffu, local, 1);
+    local += __shfl_xor_sync(0xffffffffu, local, 2);
+    if ((lane & 3) == 0) s_sum[s] = local;
+  }
+  __syncwarp();
+  const double mine = s_sum[tid];  // by this warp
+  double run = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const double o = __shfl_up_sync(0xffffffffu, run, d);
+    if (lane >= d) run += o;
+  }
+  if (lane == 31) w_sum[warp] = run;
+  double before = __shfl_up_sync(0xffffffffu, run, 1);
+  if (lane == 0) before = 0.0;
+  __syncthreads();
+  {
+    double base = 0.0, total = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      if (w == warp) base = total;
+      total += w_sum[w];
+    }
+    const double near = sample_near(total, seg), target = uniform[row] * total;
+    const double lo = base + before, hi = lo + mine;
+    // whether the target lies in or near this segment (also if anything is no number)
+    const bool candidate = !(lo > target + near) && !(hi < target - near);
+    if (candidate) s_pick = tid, s_total = lo;  // used when there is one
+    if (__syncthreads_count(candidate) == 1) {
+      const int s = s_pick;
+      const double start = s_total;
+      if (warp == 0) {
+        const int from = min(vocab, s * seg), len = min(vocab, from + seg) - from;
+        const int at = sample_scan(len, [&](int j) { return sample_weight(l[from + j], mx, temp); }, start, target, near, lane);
+        if (lane == 0) s_last = at < 0 ? -1 : from + at;
+      }
+      __syncthreads();
+      if (s_last >= 0) {
+        if (tid == 0) out_token[row] = s_last;
+        return;
+      }
+    }
+  }
+  __syncthreads();
+
+  // near a running sum: contiguous segment of this thread
   const int lo = min(vocab, tid * seg), hi = min(vocab, lo + seg);
   double local = 0.0;
   int last_pos = -1;
   for (int i = lo; i < hi; ++i) {
-    const float w = bw::det_expf(__fdiv_rn(__fsub_rn(l[i], mx), temp));
+    const float w = sample_weight(l[i], mx, temp);
     if (w > 0.0f) last_pos = i;
     local += static_cast<double>(w);
   }
@@ -92,7 +192,7 @@ sample_rows_kernel(const float* __restrict__ logits, int vocab, const float* __r
   const double target = uniform[row] * total;
   double cum = s_sum[tid];
   for (int i = lo; i < hi; ++i) {
-    const float w = bw::det_expf(__fdiv_rn(__fsub_rn(l[i], mx), temp));
+    const float w = sample_weight(l[i], mx, temp);
     if (w <= 0.0f) continue;
     cum += static_cast<double>(w);
     if (cum > target) {
@@ -111,9 +211,9 @@ sample_rows_kernel(const float* __restrict__ logits, int vocab, const float* __r
 // difference is known, so the token is the serial kernel's wherever the target lies further than the bound from the two
 // running sums it falls between. Where it does not (a uniform number of 0 or nearly 1, a logit that is no number, or a chance
 // of some 1e-9 a row) the row is done again with one thread per segment and every sum in the serial kernel's order.
-// Head and sampler together for 64 rows of 128,256 logits, half of them greedy: 550 us with the kernel above, 258 us with
-// serial sums here, 229 us with trees (the product alone takes 185 us). The sampler alone: 64 rows 71 -> 39 us, one row of
-// 49,152 23 -> 12 us.
+// Head and sampler together for 64 rows of 128,256 logits, half of them greedy: 550 us with a block per row and serial sums,
+// 258 us with serial sums here, 229 us with trees (the product alone takes 185 us). The sampler alone: 64 rows 71 -> 39 us, one
+// row of 49,152 23 -> 12 us.
 constexpr int kSampleBlocks = 8, kSampleBlockThreads = 256, kSegmentsPerBlock = kSampleThreads / kSampleBlocks;
 
 __device__ __forceinline__ void sample_cluster_sync() {
@@ -218,7 +318,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
     double local = 0.0;
 #pragma unroll 4
     for (int j = lane; j < len; j += 32) {
-      const float w = bw::det_expf(__fdiv_rn(__fsub_rn(v[j], mx), temp));
+      const float w = sample_weight(v[j], mx, temp);
       v[j] = w;
       local += static_cast<double>(w);
     }
@@ -256,10 +356,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
   }
   __syncthreads();
   {
-    // A sum of n positive terms in any order of additions of which each term passes through at most a is off by at most
-    // a / 2^53 of the sum: the serial sums have a <= 2 seg + 512, those here a < 128. With the rounding of the target and of
-    // the comparisons, the distance that tells is taken as twice that.
-    const double near = total * (2 * seg + kSampleThreads + 128) * 2.220446049250313e-16;
+    const double near = sample_near(total, seg);
     const double target = uniform[row] * total;
     // whether the target lies in or near one of this block's segments (also if anything is no number)
     bool candidate = false;
@@ -274,27 +371,8 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
     } else if (candidates == 1 && warp == 0) {
       const int s = b_last[0], len = max(0, min(seg, count - s * seg));
       const float* v = seg_values + s * seg;
-      double base = all_sum[seg0 + s];
-      int pick = -1;
-      for (int j0 = 0; j0 < len; j0 += 32) {
-        const float w = j0 + lane < len ? v[j0 + lane] : 0.0f;
-        double run = static_cast<double>(w);
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const double o = __shfl_up_sync(0xffffffffu, run, d);
-          if (lane >= d) run += o;
-        }
-        const double cum = base + run;
-        const uint32_t over = __ballot_sync(0xffffffffu, w > 0.0f && cum > target);
-        if (over) {
-          const int at = __ffs(over) - 1;
-          const bool clear = cum - target > near && target - (cum - static_cast<double>(w)) > near;
-          if (__shfl_sync(0xffffffffu, clear ? 1 : 0, at)) pick = first + s * seg + j0 + at;
-          break;
-        }
-        base = __shfl_sync(0xffffffffu, cum, 31);
-      }
-      if (lane == 0) b_pick = pick;
+      const int at = sample_scan(len, [&](int j) { return v[j]; }, all_sum[seg0 + s], target, near, lane);
+      if (lane == 0) b_pick = at < 0 ? -1 : first + s * seg + at;
     }
   }
   sample_cluster_sync();
@@ -372,6 +450,15 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
   sample_cluster_sync();
 }
 
+// Which kernel a row goes to: 0 chosen from the sizes, 1 a block, 2 a cluster where the segments fit. Both give the same tokens.
+// Returns the previous setting. For tests and measurements.
+static int g_sample_kernel = 0;
+BW_API int bw_sample_rows_kernel(int kernel) {
+  const int before = g_sample_kernel;
+  if (kernel >= 0 && kernel <= 2) g_sample_kernel = kernel;
+  return before;
+}
+
 BW_API int bw_sample_rows(const float* logits, int rows, int vocab, const float* temperature,
                           const double* uniform, int* out_token, cudaStream_t stream) {
   if (rows <= 0) return 0;
@@ -379,11 +466,16 @@ BW_API int bw_sample_rows(const float* logits, int rows, int vocab, const float*
     bw::set_error("sample_rows: vocabulary size %d", vocab);
     return -1;
   }
-  // A cluster per row from kClusterVocab logits on, as far as the segments fit into shared memory.
-  constexpr int kClusterVocab = 4096, kMaxSmem = 200 * 1024, kMaxDevices = 64;
+  // A cluster per row where the blocks of all rows run at once or nearly so, the row is long enough for eight blocks to gain on
+  // one, and the segments fit into shared memory. Beyond that a block per row is as fast or faster. Cluster / block, us, all rows
+  // greedy and all rows at a temperature: 1 row of 8,192 logits 5.6 / 4.2, 10.3 / 8.9; 16,000: 6.2 / 6.2, 10.3 / 12.4;
+  // 128,256: 8.3 / 14.5, 22.4 / 55.4; 64 rows of 16,000: 8.3 / 6.3, 14.4 / 14.4; 49,152: 8.3 / 8.3, 18.5 / 26.2; 128,256: 24.1 /
+  // 28.8, 55.9 / 63.7; 128 rows of 49,152: 12.4 / 8.3, 28.9 / 26.7; 512 rows of 8,192: 28.8 / 8.3, 65.6 / 20.6.
+  constexpr int kClusterVocab = 12288, kLongVocab = 24576, kMaxSmem = 200 * 1024, kMaxDevices = 64;
   const int seg = (vocab + kSampleThreads - 1) / kSampleThreads;
   const long long smem = 4ll * kSegmentsPerBlock * seg;
-  if (vocab >= kClusterVocab && smem <= kMaxSmem && rows <= 0x7fffffff / kSampleBlocks) {
+  const bool cluster = g_sample_kernel == 2 || (g_sample_kernel == 0 && vocab >= kClusterVocab && rows <= (vocab >= kLongVocab ? 64 : 32));
+  if (cluster && smem <= kMaxSmem && rows <= 0x7fffffff / kSampleBlocks) {
     static bool configured[kMaxDevices] = {false};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = 0;

@@ -169,6 +169,11 @@ class KernelOps:
         self._call("bw_sample_rows", _p(logits), _c_int(rows), _c_int(vocab), _p(temperature), _p(uniform),
                    _p(out_tokens), self._stream())
 
+    def sampler_kernel(self, kernel: int = 0) -> int:
+        """Tests and measurements: which kernel samples (0 chosen from the sizes, 1 a block per row, 2 a cluster per row where the
+        vocabulary fits).  Same tokens either way.  Returns the previous setting."""
+        return int(self.lib.bw_sample_rows_kernel(_c_int(kernel)))
+
     def fingerprint_rows(self, logits: torch.Tensor, slot: torch.Tensor, state: torch.Tensor) -> None:
         """state[slot[r]] = chained hash of logits row r's raw bits (one row per slot per call)."""
         rows, vocab = logits.shape

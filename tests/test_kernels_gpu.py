@@ -366,6 +366,39 @@ def test_sample_rows_at_running_sums(vocab):
     assert ((got >= 0) & (got < vocab)).all()
 
 
+@pytest.mark.parametrize("kernel", [1, 2])
+@pytest.mark.parametrize("vocab", [1, 3, 511, 512, 513, 4095, 4096, 6143, 32000, 49153])
+def test_sample_rows_block_and_cluster_give_the_plain_samplers_tokens(vocab, kernel):
+    """Both kernels over sizes on either side of the choice between them (a step's rows decide it too, and a row's token may not
+    depend on its neighbours): uniform numbers inside, at both ends, on and beside running sums, one positive weight, ties."""
+    rng = np.random.default_rng(vocab)
+    us = [0.0, 1.0 - 2.0 ** -53, 0.5, np.nextafter(0.5, 0.0), np.nextafter(0.5, 1.0), 1.0 / vocab] + list(rng.random(10))
+    rows = len(us)
+    logits = rnd(rng, rows, vocab, scale=3.0)
+    logits[:6] = 0.0                       # equal weights: every multiple of 1 / vocab is a running sum
+    logits[6, :] = -np.inf
+    logits[6, vocab // 3] = 1.0
+    logits[7, :] = -np.inf                 # no weight at all
+    logits[8, vocab // 2:] = -np.inf
+    logits[9, 0] = 90.0                    # all others vanish beside it
+    temps = np.array([1.0] * 11 + [0.0, -1.0] + [0.02, 5.0, 0.7], dtype=np.float32)
+    us = np.array(us, dtype=np.float64)
+    ops = _ops("bfloat16")
+    out = torch.full((rows,), -7, dtype=torch.int32, device=DEV)
+    before = ops.sampler_kernel(kernel)
+    try:
+        ops.sample_rows(t(logits), t(temps), torch.from_numpy(us).to(DEV), out)
+    finally:
+        ops.sampler_kernel(before)
+    got = out.cpu().numpy()
+    for r in range(rows):
+        if r == 7:  # the plain sampler's maximum of nothing has no weights to walk
+            assert got[r] == 0
+            continue
+        want = P.argmax_row(logits[r]) if temps[r] <= 0 else P.sample_row(logits[r], temps[r], us[r], exp="det")
+        assert got[r] == want, f"row {r}: {got[r]}, plain sampler {want}"
+
+
 def test_fingerprint_rows():
     rng = np.random.default_rng(7)
     for vocab in (256, 385):
