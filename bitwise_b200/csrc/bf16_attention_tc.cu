@@ -116,8 +116,8 @@ __device__ __forceinline__ uint64_t make_desc_wide(uint32_t smem_addr, uint32_t 
   d |= static_cast<uint64_t>(2) << 61;
   return d;
 }
-// kind::f16, D float32, A and B bfloat16, M 128, N 64; bit 16 set: B is MN-major (N = HD: all of
-// a head's columns in one instruction, an instruction's issue costs its thread about a hundred cycles)
+// kind::f16, D float32, A and B bfloat16, M 128, N 64; bit 16 set: B is MN-major (N = HD: all of a head's columns in one
+// instruction)
 constexpr uint32_t kDescQK = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
 constexpr uint32_t kDescPV = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((static_cast<uint32_t>(HD) >> 3) << 17) | ((128u >> 4) << 24);
 

@@ -18,7 +18,7 @@
 //            at a time) and add it to the running total in registers, while the tensor core
 //            already works on the next chunk in the other accumulator; after the last chunk
 //            they add the residual, apply SwiGLU or rotate the heads, and store.
-// The kernel is persistent: one block per SM (6 stages of 32 KB) takes output tiles round-robin,
+// The kernel is persistent: one block per SM (a ring of up to 192 KB) takes output tiles round-robin,
 // and because loads, MMAs and the epilogue each walk the tile sequence on their own, the store
 // of one tile overlaps the main loop of the next.
 //
@@ -246,11 +246,13 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[32]) {
 // A warp's 32 rows x 128 bytes (lane i holds row i) turned through shared memory so that eight lanes hold the 128 bytes of a
 // row: 16-byte piece lane % 8 of row 4 t + lane / 8. Accesses straight from the accumulator's layout touch 32 rows per
 // instruction, and residual rows fetched that way wait one by one (the epilogue of a 256 x 256 tile with a residual took
-// about 10 us; turned, down of 2,048 rows x 14,336 x 4,096 went from 248 to 201 us, gate/up from 410 to 331). `buf`: the warp's kStoreBytes, pieces placed by the row's low three bits so that neither side meets in a
-// bank. The accesses are volatile assembly: in the unrolled epilogue the compiler otherwise starts all pieces at once and
-// sends the totals to local memory.
+// about 10 us; turned, down of 2,048 rows x 14,336 x 4,096 went from 248 to 201 us, gate/up from 410 to 331). `buf`: the
+// warp's kStoreBytes, pieces placed by the row's low three bits so that neither side meets in a bank. The accesses are
+// volatile assembly: in the unrolled epilogue the compiler otherwise starts all pieces at once and sends the totals to local
+// memory.
 __device__ __forceinline__ void put_piece(uint32_t buf, int lane, int c, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + lane * 128 + ((c ^ (lane & 7)) << 4)), "r"(w0), "r"(w1), "r"(w2), "r"(w3)
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + lane * 128 + ((c ^ (lane & 7)) << 4)), "r"(w0), "r"(w1), "r"(w2),
+               "r"(w3)
                : "memory");
 }
 __device__ __forceinline__ uint4 get_piece(uint32_t buf, int lane, int t) {
@@ -362,11 +364,11 @@ __global__ void reduce_swiglu_kernel(const float* __restrict__ partials, int num
 // 32 bytes (the path costs registers that the totals need): the host gives wide tiles only
 // products with n a multiple of 64 and outputs that start on 32 bytes.
 //
-// WIDE: the output tile is 128 x 256 instead of 128 x 128 and sixteen epilogue warps share it
-// (one row x 64 columns per thread). A wide tile needs a third less operand traffic per flop.
+// WIDE: the output tile is 128 x 256 instead of 128 x 128 and eight epilogue warps share it
+// (one row x 128 columns per thread). A wide tile needs a third less operand traffic per flop.
 // Large batches are bound by how fast a chunk sum leaves tensor memory: the tensor core may
 // start chunk c + 2 only when the epilogue has read chunk c out of that accumulator, so the
-// read is spread over many warps, 32 columns per tcgen05.ld, and the totals of a thread (64)
+// read is spread over both warpgroups, 64 columns per tcgen05.ld, and the totals of a thread (128)
 // stay in registers.
 //
 // PAIR (with WIDE, whole mode): two blocks of a cluster share a 256 x 256 tile, see above.
@@ -670,7 +672,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
       // rows of this warp's part of the tile, and whether its full blocks may go through shared memory in 16-byte accesses
       const int first_row = m0 + quarter * 32, warp_rows = min(32, row_end - first_row);
-      const bool turned = (N & 7) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (reinterpret_cast<uintptr_t>(residual) & 15) == 0;
+      const bool turned =
+          (N & 7) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (reinterpret_cast<uintptr_t>(residual) & 15) == 0;
       constexpr int kBlocks = 2 * PW / 32;  // blocks of 32 columns: 128 bytes of a float32 row
       auto block_col = [&](int b) { return n0 + (b * 32 >= PW ? off1 + b * 32 - PW : off0 + b * 32); };
       auto put_totals = [&](int b) {
@@ -789,8 +792,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         }
       } else if (EPI == 3) {
         // The fused q/k/v product rotates and stores itself: a thread owns a row, and with it both partners of every rotation
-        // of its heads (a piece of 64 columns is a head). Rounded to bfloat16 as the stored product would be, rotated with rope_cache_bf16_kernel's arithmetic (same bits), turned
-        // through shared memory, q goes to Y and k and v to their row of a page. The kernel that did this from the stored
+        // of its heads (a piece of 64 columns is a head). Rounded to bfloat16 as the stored product would be, rotated with
+        // rope_cache_bf16_kernel's arithmetic (same bits), turned through shared memory, q goes to Y and k and v to their row
+        // of a page. The kernel that did this from the stored
         // product read and wrote it once more: attention of 2,047 rows at 32 heads of 64, products included, 129.5 -> 125 us.
         // (Rotating behind the turn, where eight lanes read a row's tables together, took 130: the exchange of partners costs
         // more than the tables.)
@@ -825,8 +829,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           for (int h = 0; h < 2; ++h) {
             const uint4 cv = load_piece(reinterpret_cast<const char*>(cos_row + i + 4 * h));
             const uint4 sv = load_piece(reinterpret_cast<const char*>(sin_row + i + 4 * h));
-            c[4 * h] = __uint_as_float(cv.x), c[4 * h + 1] = __uint_as_float(cv.y), c[4 * h + 2] = __uint_as_float(cv.z), c[4 * h + 3] = __uint_as_float(cv.w);
-            sn[4 * h] = __uint_as_float(sv.x), sn[4 * h + 1] = __uint_as_float(sv.y), sn[4 * h + 2] = __uint_as_float(sv.z), sn[4 * h + 3] = __uint_as_float(sv.w);
+            c[4 * h] = __uint_as_float(cv.x), c[4 * h + 1] = __uint_as_float(cv.y);
+            c[4 * h + 2] = __uint_as_float(cv.z), c[4 * h + 3] = __uint_as_float(cv.w);
+            sn[4 * h] = __uint_as_float(sv.x), sn[4 * h + 1] = __uint_as_float(sv.y);
+            sn[4 * h + 2] = __uint_as_float(sv.z), sn[4 * h + 3] = __uint_as_float(sv.w);
           }
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
@@ -1189,7 +1195,8 @@ int configure_tc(int* pairs = nullptr) {
 
 template <bool SPLIT, int A_ROWS, int EPI, bool WIDE, bool PAIR = false>
 int launch_tc(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_f32, const float* residual, int m, int n,
-              int k, int* error_word, float* partials, const Fused& fused, cudaStream_t stream, int narrow_bn = BN, const RopeOut& rope = RopeOut{}) {
+              int k, int* error_word, float* partials, const Fused& fused, cudaStream_t stream, int narrow_bn = BN,
+              const RopeOut& rope = RopeOut{}) {
   constexpr int BNT = WIDE ? 2 * BN : BN;
   constexpr int BNW = PAIR ? BN : BNT;
   constexpr int BMT = PAIR ? 2 * BM : BM;
@@ -1346,7 +1353,8 @@ BW_API int bw_bf16_linear_tc_rope(const __nv_bfloat16* x, const __nv_bfloat16* w
                                   int kv_heads, int hd, int page, int write_kv, cudaStream_t stream) {
   if (m <= 0 || n <= 0) return 0;
   if (!bw_bf16_linear_tc_rope_usable(nullptr, nullptr, m, n, k, hd) || n != (heads + 2 * kv_heads) * hd || page <= 0) {
-    bw::set_error("linear with rotation (tcgen05): shape [%d x %d] x [%d x %d], %d/%d heads of %d is not for this path", m, k, n, k, heads, kv_heads, hd);
+    bw::set_error("linear with rotation (tcgen05): shape [%d x %d] x [%d x %d], %d/%d heads of %d is not for this path", m, k, n, k,
+                  heads, kv_heads, hd);
     return -1;
   }
   // The shape alone brought the call here (whether a step is fused is asked before there are tensors): x or weights that TMA does
@@ -1354,7 +1362,9 @@ BW_API int bw_bf16_linear_tc_rope(const __nv_bfloat16* x, const __nv_bfloat16* w
   auto off16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 != 0; };
   if (off16(x) || off16(w) || reinterpret_cast<uintptr_t>(qkv) % 32 || off16(kcache) || off16(vcache) || off16(cos_t) || off16(sin_t)) {
     const int rc = bw_bf16_linear(x, w, qkv, 0, nullptr, m, n, k, nullptr, nullptr, 0, stream);
-    return rc ? rc : bw_bf16_rope_cache(qkv, n, pos, row_seq, cos_t, sin_t, block_table, max_blocks, kcache, vcache, m, heads, kv_heads, hd, page, write_kv, stream);
+    return rc ? rc
+              : bw_bf16_rope_cache(qkv, n, pos, row_seq, cos_t, sin_t, block_table, max_blocks, kcache, vcache, m, heads, kv_heads, hd,
+                                   page, write_kv, stream);
   }
   int* word = bw::failure_word();
   if (!word) return -1;

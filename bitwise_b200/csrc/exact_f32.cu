@@ -1341,7 +1341,8 @@ int launch_tile(const float* x, const float* w, float* y, const float* residual,
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = 0;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_exact_tile_kernel<TR, TC, WR, WC, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_exact_tile_kernel<TR, TC, WR, WC, BLOCKS>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
     if (e != cudaSuccess) {
       bw::set_error("linear (32-bit): cannot raise shared memory: %s", cudaGetErrorString(e));
       return static_cast<int>(e);
@@ -1356,15 +1357,18 @@ int launch_tile(const float* x, const float* w, float* y, const float* residual,
     return -1;
   }
   const unsigned row_blocks = (m + S::BM - 1) / S::BM, gy = row_blocks < 65535u ? row_blocks : 65535u;
-  bw::launch_pdl(gemm_exact_tile_kernel<TR, TC, WR, WC, BLOCKS>, dim3((n + S::BN - 1) / S::BN, gy, (row_blocks + gy - 1) / gy), dim3(S::kThreads),
-                 static_cast<size_t>(S::kSmem), stream, map_x, map_w, y, residual, m, n, k, word);
+  const dim3 grid((n + S::BN - 1) / S::BN, gy, (row_blocks + gy - 1) / gy);
+  bw::launch_pdl(gemm_exact_tile_kernel<TR, TC, WR, WC, BLOCKS>, grid, dim3(S::kThreads), static_cast<size_t>(S::kSmem), stream, map_x,
+                 map_w, y, residual, m, n, k, word);
   return bw::launch_status();
 }
 
-// The tile of a product of more than 16 rows: 0 the kernel of 128 x 128 tiles, else by index into BW_F32_TILES; the one whose
-// estimated time is least. Cycles per value of k as measured on a B200: a block alone on its SM (its chain's own time), and its
-// share where its SM has as many blocks as fit.
-#define BW_F32_TILES(X_) X_(0, 8, 8, 2, 2, 2) X_(1, 4, 8, 4, 1, 3) X_(2, 4, 4, 4, 1, 3) X_(3, 4, 2, 4, 1, 3) X_(4, 4, 4, 2, 2, 3) X_(5, 4, 2, 2, 2, 3) X_(6, 2, 2, 4, 1, 3)
+// The tile of a product of more than 16 rows, by index into BW_F32_TILES (64 x 128 down to 32 x 16): the one whose estimated
+// time is least. Cycles per value of k as measured on a B200: a block alone on its SM (its chain's own time), and its share
+// where its SM has as many blocks as fit.
+#define BW_F32_TILES(X_)                                                                         \
+  X_(0, 8, 8, 2, 2, 2) X_(1, 4, 8, 4, 1, 3) X_(2, 4, 4, 4, 1, 3) X_(3, 4, 2, 4, 1, 3) \
+  X_(4, 4, 4, 2, 2, 3) X_(5, 4, 2, 2, 2, 3) X_(6, 2, 2, 4, 1, 3)
 struct TileCost {
   int bm, bn, fit, alone, share;  // rows, columns, blocks per SM, cycles per value of k alone and as one of many
 };
@@ -1462,7 +1466,8 @@ BW_API int bw_f32_linear(const float* x, const float* w, float* y, const float* 
     return -1;
   } else if (m <= 16) {
     gemm_exact_kernel<16><<<dim3(gx, (m + 15) / 16), 256, 0, stream>>>(x, w, y, residual, m, n, k);
-  } else if (k % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && f32_encoder() != nullptr) {
+  } else if (k % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
+             f32_encoder() != nullptr) {
     if (m > 65535 * 128) {
       bw::set_error("linear: %d rows exceed the grid limit", m);
       return -1;
