@@ -51,7 +51,7 @@ __device__ __forceinline__ int sample_scan(int len, Weight weight, double base, 
 // A block per row: steps of many rows, whose blocks fill the machine, and small vocabularies. Four lanes share a segment, eight
 // segments are in flight in a warp; where the tree sums do not settle the token (see below) it is found again with one
 // thread per segment and every sum in order. Bound by the exponentials and the reads behind them: with serial sums alone 512
-// rows of 8,192 logits took 27 us at a temperature, with trees 21; 64 rows of 128,256 156 and 64. 32 registers, four blocks an SM.
+// rows of 8,192 logits took 27 us at a temperature, with trees 17; 64 rows of 128,256 156 and 67. 32 registers, four blocks an SM.
 __global__ void __launch_bounds__(kSampleThreads, 4)
 sample_rows_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
                    const double* __restrict__ uniform, int* __restrict__ out_token) {
@@ -468,9 +468,9 @@ BW_API int bw_sample_rows(const float* logits, int rows, int vocab, const float*
   }
   // A cluster per row where the blocks of all rows run at once or nearly so, the row is long enough for eight blocks to gain on
   // one, and the segments fit into shared memory. Beyond that a block per row is as fast or faster. Cluster / block, us, all rows
-  // greedy and all rows at a temperature: 1 row of 8,192 logits 5.6 / 4.2, 10.3 / 8.9; 16,000: 6.2 / 6.2, 10.3 / 12.4;
-  // 128,256: 8.3 / 14.5, 22.4 / 55.4; 64 rows of 16,000: 8.3 / 6.3, 14.4 / 14.4; 49,152: 8.3 / 8.3, 18.5 / 26.2; 128,256: 24.1 /
-  // 28.8, 55.9 / 63.7; 128 rows of 49,152: 12.4 / 8.3, 28.9 / 26.7; 512 rows of 8,192: 28.8 / 8.3, 65.6 / 20.6.
+  // greedy and all rows at a temperature: 1 row of 8,192 logits 5.6 / 4.2, 10.3 / 8.3; 16,000: 6.2 / 6.2, 10.3 / 12.4;
+  // 128,256: 8.3 / 12.4, 21.2 / 58.9; 64 rows of 16,000: 8.3 / 6.2, 14.4 / 12.8; 49,152: 8.3 / 8.2, 18.5 / 26.7; 128,256: 24.1 /
+  // 26.7, 56.5 / 66.8; 128 rows of 49,152: 12.4 / 8.3, 29.1 / 26.9; 512 rows of 8,192: 28.8 / 6.3, 65.6 / 16.6.
   constexpr int kClusterVocab = 12288, kLongVocab = 24576, kMaxSmem = 200 * 1024, kMaxDevices = 64;
   const int seg = (vocab + kSampleThreads - 1) / kSampleThreads;
   const long long smem = 4ll * kSegmentsPerBlock * seg;
