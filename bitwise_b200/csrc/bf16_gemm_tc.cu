@@ -1054,9 +1054,10 @@ int g_force_mode = 0;  // 0: chosen; 1: whole; 2: split where it is possible
 constexpr int kMaxSplitColumns = 16384;  // bounds the scratch of the chunk sums
 
 // a chunk of a narrow or wide tile, by its width / 16
-double chunk_us(int bn) {
+double chunk_us(int bn, bool few) {
   constexpr double us[] = {1.5, 1.55, 2.1, 1.8, 1.95, 2.05, 2.2, 2.35};
-  return bn > BN ? 3.3 : us[bn / 16 - 1];
+  constexpr double few_us[] = {1.25, 1.25, 1.5, 1.8, 1.95, 2.05, 2.2, 2.3};  // up to 16 rows, which mostly run elsewhere
+  return bn > BN ? 3.3 : few ? few_us[bn / 16 - 1] : us[bn / 16 - 1];
 }
 
 constexpr double kWideChunkAloneUs = 4.6;  // of a split product in tiles of 256 columns
@@ -1094,8 +1095,9 @@ Plan plan_rows(int m, int n, int k, bool swiglu, bool reads, int sms, bool allow
       const long long tiles = static_cast<long long>((n + bn - 1) / bn) * m_blocks;
       const long long items = mode ? tiles * chunks : tiles;
       const long long rounds = (items + sms - 1) / sms;
-      if (mode == 1 && bn > BN && rounds > 1 && !g_tile_width) continue;
-      const double step = std::max(mode == 1 && bn > BN ? kWideChunkAloneUs : chunk_us(bn), (a_rows + bn) * block_us_per_kb);
+      const bool few = m <= 16, wide_alone = mode == 1 && bn > BN && !few;
+      if (wide_alone && rounds > 1 && !g_tile_width) continue;
+      const double step = std::max(wide_alone ? kWideChunkAloneUs : chunk_us(bn, few), (a_rows + bn) * block_us_per_kb);
       double cost = static_cast<double>(rounds) * step * (mode ? 1 : chunks);
       const double arrive = static_cast<double>(tiles) * chunks * (a_rows + bn) * us_per_kb;
       if (cost < arrive) cost = arrive;
