@@ -3,32 +3,38 @@
 // Same arithmetic, in the same order, as attention_whole_kernel / attention_split_kernel in
 // bf16_attention.cu (key tiles of 64 at fixed positions; per tile and row the maximum, the sum
 // of the weights and the unnormalised output with bfloat16 weights; ordered merge), so the
-// three kernels give the same bits. What changes is where the work runs:
-//   warp 0     brings Q (once) and the key/value tiles of the paged cache into shared memory
-//              with TMA (128-byte swizzle), one box per page and piece, the lanes asking for
-//              one box each
-//   warp 1     one thread issues tcgen05.mma: S = Q K^T (128 stacked rows x 64 keys, K-major
-//              operands) into one of two S buffers in tensor memory, and O_t = P V (P from
-//              shared memory, V as an MN-major operand) into one of two O buffers
-//   warps 2-5  one thread per stacked row: read the S row from tensor memory, scale, mask,
-//              maximum, weights, sum; write the bfloat16 weights as the next A operand into
-//              shared memory; later read the O_t row and merge it into the running state in
-//              registers; finally normalise and store
+// three kernels give the same bits. What changes is where the work runs. A block per SM walks work items (128 stacked query rows
+// of one kv head) one after the other; its sixteen warps:
+//   warp 0     scores: issues S = Q K^T (128 stacked rows x 64 keys, K-major operands) into one of four S buffers in tensor memory,
+//              up to three key tiles ahead of their use, and asks for the item's Q
+//   warp 1     outputs: issues O_t = P V (P in tensor memory, over the scores it was made from; V as an MN-major operand in
+//              shared memory) into one of two O buffers
+//   warps 2-3  bring the keys and the values of the paged cache into shared memory with TMA (128-byte swizzle), one box per
+//              page and piece, the lanes asking for one box each
+//   warps 4-7, 8-11  the softmax of every other key tile, one thread per stacked row: read the S row from tensor memory, scale,
+//              mask, maximum, weights, sum; write the bfloat16 weights back as the next A operand, and (maximum, sum) to shared memory
+//   warps 12-15  one thread per stacked row: merge the O_t row of each key tile, in order, into the running state in
+//              registers; after the item's last tile normalise and store
 // A head of 128 is two pieces of 64 along d: Q, K and V tiles are kept piece by piece (a row of
 // a piece is one 128-byte swizzled line), the scores add up over the pieces' k-steps in order,
 // and the output takes one MMA per 16 keys over all 128 columns (the pieces of V are the
 // swizzle atoms of one MN-major operand, a piece apart).
-// What the tensor core does is handed out by one warp, whose operations are what a tile's time is
-// made of. So it waits only for what nothing else implies (keys landed, weights written: the
-// buffers of S and O are free by then, see below) and announces the output and the freed stage
-// with one commit; and all its lanes walk the loop with one elected to issue (a lone lane's
-// operation took about a hundred cycles, most of them moves of descriptors into uniform
-// registers).
-// At head size 64 two blocks share an SM (256 tensor-memory columns and about 100 KB each), so
-// one block's softmax overlaps the other's MMAs; at 128 a block has the SM to itself (384 of
-// the 512 columns, 170 KB) and overlaps its own stages. Every mbarrier wait is bounded
-// (bw_common.cuh).
+//
+// What bounds it: the special-function unit gives 16 exponentials a cycle and SM, 512 cycles for a tile of 128 x 64; beside it
+// the chains of single warps. One warp that did a row's softmax and its merge took 1,600 cycles a key tile (two waits,
+// 700 for the weights, 440 for the merge), whether one or two of them shared a scheduler, and a warp that issued all MMAs of two
+// tiles 2,700. So each chain is cut up: softmax by two groups of warps in turn, the merge by a third, scores and outputs issued
+// by a warp each, keys and values asked for by a warp each (a turn of a loading warp takes 430 cycles and 53 more for each box where
+// its lanes ask side by side; one elected lane with the operands in its registers asks for four in 200). Several barriers are
+// waited for in one poll (15 cycles each; a poll and the branch on it 75 to 100, twice that through a vote).
+// Weights go straight to tensor memory; scaling, sums and merge run two values per instruction (f32x2, the same roundings).
+// A key tile now takes about 950 cycles at head size 64 and 1,300 at 128, exponentials half of it at 64; what is left is the merge's chain.
+// Measured, attention alone: 2,047 rows at 32 heads of 64, 47 -> 39 us; rows 848 .. 2,047 at 32 / 8 heads of 128, 87 -> 50;
+// 24 single rows of up to 1,270 keys beside 488 rows at 15 / 5 heads of 64, 24 -> 13.8 (the longest row's chain of key tiles).
+// Every mbarrier wait is bounded (bw_common.cuh).
 #include <cuda.h>
+
+#include <algorithm>
 
 #include "bw_common.cuh"
 
@@ -42,28 +48,39 @@ namespace {
 
 constexpr int HD = BW_HEAD_DIM;
 constexpr int kPieces = HD / 64;  // 64-wide pieces of a head along d
-constexpr int kTileM = 128;   // stacked rows per block
+constexpr int kTileM = 128;   // stacked rows per tile
 constexpr int kTileKV = 64;   // keys per tile
-constexpr int kStages = 3;    // key/value tiles in flight (a fourth at head size 128 fits and was slower end to end)  // key/value tiles in flight (at 64 two blocks share an SM's shared memory)
-constexpr int kThreads = 192;
-constexpr int kQPiece = kTileM * 128;          // 16 KB: one piece of the Q tile
+constexpr int kQPiece = kTileM * 128;          // 16 KB: one piece of a Q tile
 constexpr int kKPiece = kTileKV * 128;         // 8 KB: one piece of a K (or V) tile
 constexpr int kQBytes = kPieces * kQPiece;
 constexpr int kKBytes = kPieces * kKPiece;
-constexpr int kPBytes = kTileM * 128;          // 16 KB per weight buffer
-constexpr int kOCol = 128;                     // S0 S1 at columns 0 and 64, O0 O1 at 128 and 128 + HD
-constexpr int kTmemCols = HD == 64 ? 256 : 512;
+constexpr int kThreads = 512;
+constexpr int kQBuffers = HD == 64 ? 2 : 1;
+constexpr int kStages = HD == 64 ? 6 : 5;      // key tiles, and value tiles, in flight
+constexpr int kSBuffers = 4;
+constexpr int kOCol = kSBuffers * kTileKV;     // O0, O1 behind the four S buffers
+constexpr int kTmemCols = 512;
+constexpr int kMaxItems = 64;                  // of a block: its list lies in shared memory
+// registers by warpgroup: issuing and loading warps, softmax (two groups), merge; together what 512 threads start with (128 each)
+constexpr int kRegsIssue = 56, kRegsSoftmax = HD == 64 ? 152 : 128, kRegsMerge = HD == 64 ? 152 : 200;
+static_assert(kRegsIssue + 2 * kRegsSoftmax + kRegsMerge == 512, "registers of the warpgroups");
 
+struct __align__(16) Item {
+  int seq, row0, rows, g;  // sequence, first row, rows, kv head
+  int pos0, kv_lo, tiles;  // position of the first row, first key, key tiles
+  int pad;
+};
 struct __align__(8) Barriers {
-  uint64_t q_full;
-  uint64_t kv_full[kStages], pv_done[kStages];  // a tile's keys and values have landed; its output is formed
-  uint64_t s_full[2], p_ready[2];
+  uint64_t q_full[kQBuffers], q_empty[kQBuffers];
+  uint64_t k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages];
+  uint64_t s_full[kSBuffers], p_ready[kSBuffers], pv_done[kSBuffers];  // scores formed; weights written; output formed
+  uint64_t o_free[kSBuffers];                                          // output merged
   uint32_t tmem_base;
   uint32_t failed;
 };
-constexpr int kMaxTablePages = 2048;  // page ids of the block's key range, staged in shared memory
 
-constexpr int kSmemBytes = kQBytes + kStages * 2 * kKBytes + 2 * kPBytes + sizeof(Barriers) + kMaxTablePages * 4 + 1024;
+constexpr int kSmemBytes = kQBuffers * kQBytes + kStages * 2 * kKBytes + kMaxItems * static_cast<int>(sizeof(Item)) +
+                           kSBuffers * kTileM * 8 + static_cast<int>(sizeof(Barriers)) + 1024;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -79,6 +96,48 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* failed) {
   return bw::mbar_wait_bounded(bar, parity, failed);
+}
+// Several barriers in one wait: their polls overlap (15 cycles each, where a poll and the branch on it take 75 to 100).
+__device__ __forceinline__ bool mbar_wait2(uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1, volatile uint32_t* failed) {
+  const uint32_t a0 = smem_u32(bar0), a1 = smem_u32(bar1);
+  for (uint32_t spin = 0; spin < bw::kSpinLimit; ++spin) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+        "and.pred p, p, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(a0), "r"(parity0), "r"(a1), "r"(parity1)
+        : "memory");
+    if (done) return true;
+    if ((spin & 1023u) == 1023u && *failed) return false;
+  }
+  *failed = 1;
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait3(uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1, uint64_t* bar2, uint32_t parity2,
+                                           volatile uint32_t* failed) {
+  const uint32_t a0 = smem_u32(bar0), a1 = smem_u32(bar1), a2 = smem_u32(bar2);
+  for (uint32_t spin = 0; spin < bw::kSpinLimit; ++spin) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p, q, r;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 r, [%5], %6;\n\t"
+        "and.pred p, p, q;\n\t"
+        "and.pred p, p, r;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(a0), "r"(parity0), "r"(a1), "r"(parity1), "r"(a2), "r"(parity2)
+        : "memory");
+    if (done) return true;
+    if ((spin & 1023u) == 1023u && *failed) return false;
+  }
+  *failed = 1;
+  return false;
 }
 // One lane of a whole, converged warp: the code it guards runs with operands that the compiler knows to be the warp's, kept
 // in uniform registers (see bf16_gemm_tc.cu).
@@ -129,6 +188,15 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t b
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// the same with A in tensor memory: 16 values of a row in 8 columns of 32 bits
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
@@ -145,6 +213,47 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64]) {
       : "memory");
 #pragma unroll
   for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
+}
+// 32 consecutive columns asked for, and the wait for two such blocks (whose operands keep every use behind it)
+__device__ __forceinline__ void tmem_ask(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_have(uint32_t (&r)[32], uint32_t (&q)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]),
+                 "+r"(q[0]), "+r"(q[1]), "+r"(q[2]), "+r"(q[3]), "+r"(q[4]), "+r"(q[5]), "+r"(q[6]), "+r"(q[7]), "+r"(q[8]), "+r"(q[9]), "+r"(q[10]), "+r"(q[11]), "+r"(q[12]), "+r"(q[13]), "+r"(q[14]), "+r"(q[15]), "+r"(q[16]), "+r"(q[17]), "+r"(q[18]), "+r"(q[19]), "+r"(q[20]), "+r"(q[21]), "+r"(q[22]), "+r"(q[23]), "+r"(q[24]), "+r"(q[25]), "+r"(q[26]), "+r"(q[27]), "+r"(q[28]), "+r"(q[29]), "+r"(q[30]), "+r"(q[31])
+               :
+               : "memory");
+}
+// 16 consecutive columns of this thread's lane written (tmem_written: they are)
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+               ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_written() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// Two float32 operations in one instruction, each rounded as the single one.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
 }
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -165,37 +274,61 @@ __device__ __forceinline__ float merge_value(float X, float x, const MergeWeight
   return __fmaf_rn(x, w.b, __fmul_rn(X, w.a));
 }
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table, int max_blocks,
                     const int* __restrict__ tile_seq, const int* __restrict__ tile_row0,
-                    const int* __restrict__ tile_rows, const int* __restrict__ seq_pos0,
+                    const int* __restrict__ tile_rows, int total, const int* __restrict__ seq_pos0,
                     const int* __restrict__ seq_row0, __nv_bfloat16* __restrict__ out, int out_stride, int heads,
                     int kv_heads, int page, int window, float scale_log2, int* error_flag) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* base = bw::smem_align_1024(smem_raw);
-  unsigned char* sq = base;
-  unsigned char* skv = sq + kQBytes;                    // stage s: K at skv + s * 2 * kKBytes, V kKBytes behind
-  unsigned char* sp = skv + kStages * 2 * kKBytes;      // two weight buffers
-  Barriers* bars = reinterpret_cast<Barriers*>(sp + 2 * kPBytes);
-  int* spages = reinterpret_cast<int*>(bars + 1);
+  unsigned char* sq = bw::smem_align_1024(smem_raw);
+  unsigned char* sk = sq + kQBuffers * kQBytes;
+  unsigned char* sv = sk + kStages * kKBytes;
+  Item* items = reinterpret_cast<Item*>(sv + kStages * kKBytes);
+  float2* stats = reinterpret_cast<float2*>(items + kMaxItems);  // [kSBuffers][kTileM]: maximum and sum of a row's key tile
+  Barriers* bars = reinterpret_cast<Barriers*>(stats + kSBuffers * kTileM);
   volatile uint32_t* failed = &bars->failed;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int group = heads / kv_heads;
+  // The host lists the tiles with the most keys first; with the heads running fastest the items of all tiles are dealt to the blocks
+  // forwards and backwards in turn, which evens out their keys. Item j of a block is number
+  auto number = [&](int j) { return j * static_cast<int>(gridDim.x) + static_cast<int>((j & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x); };
+  int count = 0;  // of this block's items
+  while (number(count) < total) ++count;
+  if (static_cast<int>(threadIdx.x) < count) {
+    const int i = number(threadIdx.x), tile = i / kv_heads;
+    Item it;
+    it.g = i - tile * kv_heads;
+    it.seq = tile_seq[tile], it.row0 = tile_row0[tile], it.rows = tile_rows[tile];
+    it.pos0 = seq_pos0[it.seq] + (it.row0 - seq_row0[it.seq]);
+    it.kv_lo = (window > 0 && it.pos0 - window + 1 > 0) ? ((it.pos0 - window + 1) / kTileKV) * kTileKV : 0;
+    it.tiles = (it.pos0 + it.rows - it.kv_lo + kTileKV - 1) / kTileKV;
+    it.pad = 0;
+    items[threadIdx.x] = it;
+  }
   if (threadIdx.x == 0) {
-    mbar_init(&bars->q_full, 1);
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(&bars->kv_full[s], 1);
-      mbar_init(&bars->pv_done[s], 1);
+    for (int i = 0; i < kQBuffers; ++i) {
+      mbar_init(&bars->q_full[i], 1);
+      mbar_init(&bars->q_empty[i], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&bars->s_full[b], 1);
-      mbar_init(&bars->p_ready[b], 4);
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(&bars->k_full[i], 1);
+      mbar_init(&bars->k_empty[i], 1);
+      mbar_init(&bars->v_full[i], 1);
+      mbar_init(&bars->v_empty[i], 1);
+    }
+    for (int i = 0; i < kSBuffers; ++i) {
+      mbar_init(&bars->s_full[i], 1);
+      mbar_init(&bars->p_ready[i], 4);
+      mbar_init(&bars->pv_done[i], 1);
+      mbar_init(&bars->o_free[i], 4);
     }
     bars->failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
+  if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
                  "n"(kTmemCols)
                  : "memory");
@@ -207,250 +340,307 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const uint32_t tmem_base = bars->tmem_base;
   bw::pdl_enter();
 
-  // The host lists the tiles with the most keys first, and blocks are handed out with
-  // blockIdx.x running fastest: the heads of the longest tile start first, then those of the
-  // next one, so the long blocks do not start late and stretch the tail of the launch.
-  const int tile = blockIdx.y, g = blockIdx.x;
-  const int group = heads / kv_heads;
-  const int seq = tile_seq[tile], row0 = tile_row0[tile], nrows = tile_rows[tile];
-  const int mrows = nrows * group;
-  const int p_first = seq_pos0[seq] + (row0 - seq_row0[seq]);
-  const int p_last = p_first + nrows - 1;
-  const int kv_lo = (window > 0 && p_first - window + 1 > 0) ? ((p_first - window + 1) / kTileKV) * kTileKV : 0;
-  const int kv_hi = p_last + 1;
-  const int ntiles = (kv_hi - kv_lo + kTileKV - 1) / kTileKV;
-  const int pages_per_tile = kTileKV / page;
-
-  if (warp == 0) {
-    // the page ids of this block's key range go to shared memory first (one coalesced read),
-    // so that the loop below does not wait for a table entry per page
-    const int* table = block_table + static_cast<size_t>(seq) * max_blocks;
-    const int first_page = kv_lo / page, last_page = (kv_hi - 1) / page;
-    const int staged = min(last_page - first_page + 1, kMaxTablePages);
-    for (int i = lane; i < staged; i += 32) spages[i] = table[first_page + i];
-    __syncwarp();
-    if (lane == 0) {
-      mbar_expect_tx(&bars->q_full, kPieces * (kTileM / group) * group * 128);  // a group that does not divide 128 leaves rows empty
-      for (int i = 0; i < kPieces; ++i) tma_load_4d(sq + i * kQPiece, &map_q, 64 * i, 0, g, row0, &bars->q_full);
-    }
-    // A tile of keys and values is pages x pieces x 2 copies (16 at head size 128 with pages of 16),
-    // and the issue of one holds its thread for a hundred cycles or more: the lanes issue one each,
-    // side by side, or the copies of a tile would take longer to ask for than the tile takes to use.
-    const int copies = pages_per_tile * kPieces * 2;
-    for (int t = 0; t < ntiles; ++t) {
-      const int s = t % kStages;
-      int ok = 1;
-      if (lane == 0) {
-        if (t >= kStages && !mbar_wait(&bars->pv_done[s], ((t / kStages) - 1) & 1, failed)) ok = 0;
-        if (ok) mbar_expect_tx(&bars->kv_full[s], 2 * kKBytes);
-      }
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
-      unsigned char* k = skv + s * 2 * kKBytes;
-      const int j0 = kv_lo + t * kTileKV;
-      for (int c = lane; c < copies; c += 32) {
-        const int pg = c / (kPieces * 2), i = (c >> 1) % kPieces, is_v = c & 1;
-        const int j = j0 + pg * page;
-        // pages wholly beyond the last key are not in the table: any valid page will do, its keys are masked
-        const int pi = min(j / page, last_page) - first_page;
-        const int blk = pi < staged ? spages[pi] : table[first_page + pi];
-        tma_load_4d(k + is_v * kKBytes + i * kKPiece + pg * page * 128, is_v ? &map_v : &map_k, 64 * i, 0, g, blk,
-                    &bars->kv_full[s]);
-      }
-    }
-  } else if (warp == 1) {
-    // all lanes walk the loop and wait, one of them issues
-    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, failed)) != 0; };
-    bool ok = wait(&bars->q_full, 0);
-    fence_after_sync();
-    const uint32_t q_addr = smem_u32(sq);
-    int qk_s = 0;                 // stage of the next tile of scores, and the parity of its arrival
-    uint32_t qk_parity = 0;
-    auto issue_qk = [&](int t) -> bool {
-      const int s = qk_s, b = t & 1;
-      if (!wait(&bars->kv_full[s], qk_parity)) return false;
-      if (++qk_s == kStages) qk_s = 0, qk_parity ^= 1;
-      // The scores' buffer was read by the softmax of tile t - 2 before that tile's weights were
-      // announced, and this warp saw that announcement before it formed tile t - 2's output:
-      // no barrier of its own.
-      fence_after_sync();
-      const uint32_t k_addr = smem_u32(skv + s * 2 * kKBytes);
-      if (elect_one()) {
-#pragma unroll
-        for (int i = 0; i < kPieces; ++i) {  // d ascending: piece after piece, 16 values a step
-          const uint64_t qdesc = make_desc(q_addr + i * kQPiece), kdesc = make_desc(k_addr + i * kKPiece);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) umma(tmem_base + b * 64, qdesc + 2 * k, kdesc + 2 * k, kDescQK, (i | k) > 0 ? 1u : 0u);
+  // Every role walks the items and their key tiles in the same order; c counts the key tiles of all of them. All lanes of a warp
+  // walk the loops and wait, one of them issues (a lone lane's operation took about a hundred cycles, most of them moves of
+  // descriptors into uniform registers).
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, failed); };
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
+    if (warp == 0) {
+      const uint32_t q_bytes = kPieces * (kTileM / group) * group * 128;  // a group that does not divide 128 leaves rows empty
+      auto ask_q = [&](int j) {
+        const int qb = j % kQBuffers;
+        const Item& it = items[j];
+        const int g = it.g, row0 = it.row0;
+        if (elect_one()) {
+          mbar_expect_tx(&bars->q_full[qb], q_bytes);
+          for (int i = 0; i < kPieces; ++i)
+            tma_load_4d(sq + qb * kQBytes + i * kQPiece, &map_q, 64 * i, 0, g, row0, &bars->q_full[qb]);
         }
-        umma_commit(&bars->s_full[b]);
-      }
-      __syncwarp();
-      return true;
-    };
-    if (ok && ntiles > 0) ok = issue_qk(0);
-    int s = 0;
-    for (int t = 0; t < ntiles && ok; ++t) {
-      const int b = t & 1;
-      if (t + 1 < ntiles) ok = issue_qk(t + 1);  // the next tile's scores are computed while this one's weights are formed
-      if (!ok) break;
-      // Behind the block's last key lies whatever the page's last holder left. Its weights are zero; its values become zero as
-      // well, so that an infinity left there cannot reach a sum. (The tile landed before its scores were formed, so
-      // this goes on beside its softmax.)
-      if (t + 1 == ntiles && kv_lo + ntiles * kTileKV > kv_hi) {
-        unsigned char* sv = skv + s * 2 * kKBytes + kKBytes;
-        for (int c = (kv_hi - kv_lo - t * kTileKV) * 8 + lane; c < kTileKV * 8; c += 32)
-#pragma unroll
-          for (int i = 0; i < kPieces; ++i) *reinterpret_cast<uint4*>(sv + i * kKPiece + c * 16) = make_uint4(0u, 0u, 0u, 0u);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-      }
-      if (!wait(&bars->p_ready[b], (t >> 1) & 1)) break;
-      // the output buffer was merged (tile t - 2) before the softmax of this tile began: same argument
-      fence_after_sync();
-      const uint64_t pdesc = make_desc(smem_u32(sp + b * kPBytes));
-      const uint32_t v_addr = smem_u32(skv + s * 2 * kKBytes + kKBytes);
-      const uint64_t vdesc = kPieces == 1 ? make_desc(v_addr) : make_desc_wide(v_addr, kKPiece);
-      if (elect_one()) {
+      };
+      int c = 0, s = 0;
+      uint32_t parity = 0;
+      bool ok = true;
+      if (kQBuffers == 2) ask_q(0);
+      for (int j = 0; j < count && ok; ++j) {
+        // Q of the next item (with one buffer: of this one) once the scores that used its place are formed
+        const int ahead = j + kQBuffers - 1;
+        if (ahead < count) {
+          if (ahead >= kQBuffers) ok = wait(&bars->q_empty[ahead % kQBuffers], ((ahead / kQBuffers) - 1) & 1);
+          if (!ok) break;
+          ask_q(ahead);
+        }
+        const int qb = j % kQBuffers, tiles = items[j].tiles;
+        if (!wait(&bars->q_full[qb], (j / kQBuffers) & 1)) break;
+        const uint32_t q_addr = smem_u32(sq) + qb * kQBytes;
+        for (int t = 0; t < tiles; ++t, ++c) {
+          const int b = c % kSBuffers;
+          // The scores go over the weights of four key tiles ago, once their output is formed and merged. (Formed alone would do
+          // for the weights; merged as well keeps the maximum and sum that lie beside them until they have been read.)
+          // (In the first round the barrier's phase before the first passes at once.)
+          if (!(ok = mbar_wait2(&bars->o_free[b], ((c / kSBuffers) & 1) ^ 1, &bars->k_full[s], parity, failed))) break;
+          __syncwarp();
+          fence_after_sync();
+          const uint32_t k_addr = smem_u32(sk) + s * kKBytes;
+          if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < kTileKV / 16; ++k)  // 16 keys: 32 bytes along a row of P, two 8-key groups (2048 bytes) of V
-          umma(tmem_base + kOCol + b * HD, pdesc + 2 * k, vdesc + 128 * k, kDescPV, k > 0 ? 1u : 0u);
-        umma_commit(&bars->pv_done[s]);  // the output is there, and the stage may be filled again
+            for (int i = 0; i < kPieces; ++i) {  // d ascending: piece after piece, 16 values a step
+              const uint64_t qdesc = make_desc(q_addr + i * kQPiece), kdesc = make_desc(k_addr + i * kKPiece);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) umma(tmem_base + b * kTileKV, qdesc + 2 * k, kdesc + 2 * k, kDescQK, (i | k) > 0 ? 1u : 0u);
+            }
+            umma_commit(&bars->s_full[b]);
+            umma_commit(&bars->k_empty[s]);
+            if (t + 1 == tiles) umma_commit(&bars->q_empty[qb]);
+          }
+          __syncwarp();
+          if (++s == kStages) s = 0, parity ^= 1;
+        }
       }
-      __syncwarp();
-      if (++s == kStages) s = 0;
+    } else if (warp == 1) {
+      int c = 0, s = 0;
+      uint32_t parity = 0;
+      bool ok = true;
+      for (int j = 0; j < count && ok; ++j) {
+        const int tiles = items[j].tiles, end = items[j].pos0 + items[j].rows - items[j].kv_lo;  // keys of the item
+        for (int t = 0; t < tiles; ++t, ++c) {
+          // Behind the item's last key lies whatever the page's last holder left. Its weights are zero; its values become zero as
+          // well, so that an infinity left there cannot reach a sum. (This goes on beside the tile's softmax.)
+          if (t + 1 == tiles && tiles * kTileKV > end) {
+            if (!(ok = wait(&bars->v_full[s], parity))) break;
+            for (int e = (end - t * kTileKV) * 8 + lane; e < kTileKV * 8; e += 32)
+#pragma unroll
+              for (int i = 0; i < kPieces; ++i)
+                *reinterpret_cast<uint4*>(sv + s * kKBytes + i * kKPiece + e * 16) = make_uint4(0u, 0u, 0u, 0u);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+          }
+          // the output goes over that of two key tiles ago, once it is merged
+          const int c2 = c + kSBuffers - 2;  // (of the round before for the first two, whose phase passes at once)
+          if (!(ok = mbar_wait3(&bars->v_full[s], parity, &bars->o_free[c2 % kSBuffers], (c2 / kSBuffers - 1) & 1,
+                                &bars->p_ready[c % kSBuffers], (c / kSBuffers) & 1, failed)))
+            break;
+          __syncwarp();
+          fence_after_sync();
+          const uint32_t v_addr = smem_u32(sv) + s * kKBytes;
+          const uint64_t vdesc = kPieces == 1 ? make_desc(v_addr) : make_desc_wide(v_addr, kKPiece);
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < kTileKV / 16; ++k)  // 16 keys: 8 columns of P, two 8-key groups (2048 bytes) of V
+              umma_ts(tmem_base + kOCol + (c & 1) * HD, tmem_base + (c % kSBuffers) * kTileKV + 8 * k, vdesc + 128 * k, kDescPV,
+                      k > 0 ? 1u : 0u);
+            umma_commit(&bars->pv_done[c % kSBuffers]);
+            umma_commit(&bars->v_empty[s]);
+          }
+          __syncwarp();
+          if (++s == kStages) s = 0, parity ^= 1;
+        }
+      }
+    } else {
+      // keys (warp 2) or values (warp 3): a tile is pages x pieces boxes
+      auto bring = [&](const CUtensorMap* map, unsigned char* ring, uint64_t* full, uint64_t* empty) {
+        const int pages_per_tile = kTileKV / page;
+        int s = 0;
+        uint32_t parity = 1;  // the first round passes at once
+        for (int j = 0; j < count; ++j) {
+          const Item it = items[j];
+          // page ids: a lane holds one of 32, the next 32 are on their way
+          const int* table = block_table + static_cast<size_t>(it.seq) * max_blocks;
+          // (pages wholly beyond the last key are not in the table: any valid page will do, its keys are masked)
+          const int first_page = it.kv_lo / page, last_page = (it.pos0 + it.rows - 1) / page;
+          auto fetch = [&](int block) { return table[min(first_page + 32 * block + lane, last_page)]; };
+          int block = 0, ids = fetch(0), next = fetch(1);
+          for (int t = 0; t < it.tiles; ++t) {
+            const int q0 = t * pages_per_tile;  // first page of the tile, from the item's first
+            if (pages_per_tile <= 32 && (q0 >> 5) != block) block = q0 >> 5, ids = next, next = fetch(block + 1);
+            int id4[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) id4[p] = __shfl_sync(0xffffffffu, ids, (q0 + p) & 31);
+            if (!wait(&empty[s], parity)) return;
+            __syncwarp();
+            unsigned char* to = ring + s * kKBytes;
+            if (pages_per_tile == 4) {  // the ordinary page of 16 keys: one lane asks for all
+              if (elect_one()) {
+                mbar_expect_tx(&full[s], kKBytes);
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+#pragma unroll
+                  for (int i = 0; i < kPieces; ++i)
+                    tma_load_4d(to + i * kKPiece + p * (kTileKV / 4) * 128, map, 64 * i, 0, it.g, id4[p], &full[s]);
+              }
+            } else {
+              if (elect_one()) mbar_expect_tx(&full[s], kKBytes);
+              for (int e = lane; e < pages_per_tile * kPieces; e += 32) {
+                const int pg = e / kPieces, i = e % kPieces;
+                const int id = table[min(first_page + q0 + pg, last_page)];
+                tma_load_4d(to + i * kKPiece + pg * page * 128, map, 64 * i, 0, it.g, id, &full[s]);
+              }
+            }
+            __syncwarp();
+            if (++s == kStages) s = 0, parity ^= 1;
+          }
+        }
+      };
+      if (warp == 2)
+        bring(&map_k, sk, bars->k_full, bars->k_empty);
+      else
+        bring(&map_v, sv, bars->v_full, bars->v_empty);
     }
-  } else {
+  } else if (warp < 12) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
     // one thread per stacked row; warp w may touch tensor-memory lanes 32 * (w % 4) .. + 31
-    const int quarter = warp & 3;
+    const int turn = (warp - 4) >> 2, quarter = warp & 3;
     const int m = quarter * 32 + lane;
-    const int pos = (m < mrows) ? p_first + m / group : p_last;
-    const int first = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    float o_tot[HD];
-#pragma unroll
-    for (int i = 0; i < HD; ++i) o_tot[i] = 0.0f;
-    float M = -INFINITY, L = 0.0f, prev_max = -INFINITY, prev_sum = 0.0f;
+    int c0 = 0;  // key tiles of the items before
     bool ok = true;
-    for (int t = 0; t < ntiles && ok; ++t) {
-      const int b = t & 1;
-      const int j0 = kv_lo + t * kTileKV;
-      if (!mbar_wait(&bars->s_full[b], (t >> 1) & 1, failed)) {
-        ok = false;
-        break;
-      }
-      fence_after_sync();
-      float s[kTileKV];
-      tmem_ld64(lane_addr + b * 64, s);
-      fence_before_sync();
-      // mask, maximum of the raw scores (the mask test is skipped for tiles inside the row's
-      // range), then weights e = 2^(s * scale - ref) with one fused multiply-add per key
-      float tmax = -INFINITY;
-      const bool inside = j0 + kTileKV - 1 <= pos && j0 >= first;
-      if (!inside) {
-#pragma unroll
-        for (int i = 0; i < kTileKV; ++i) {
-          const int j = j0 + i;
-          s[i] = (j <= pos && j >= first) ? s[i] : -INFINITY;
-        }
-      }
-      {  // the maximum is exact in any order: four independent chains instead of one of 64
-        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int i = 0; i < kTileKV; i += 4) {
-          m4[0] = fmaxf(m4[0], s[i]);
-          m4[1] = fmaxf(m4[1], s[i + 1]);
-          m4[2] = fmaxf(m4[2], s[i + 2]);
-          m4[3] = fmaxf(m4[3], s[i + 3]);
-        }
-        tmax = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-      }
-      tmax = __fmul_rn(tmax, scale_log2);
-      const float nref = (tmax == -INFINITY) ? 0.0f : -tmax;
-      // their sum in the order of the other kernels: key j belongs to quad lane (j % 8) / 2; a
-      // quad lane adds its pairs for j / 8 ascending; then (a0 + a1) + (a2 + a3)
-      float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      uint32_t packed[kTileKV / 2];
-#pragma unroll
-      for (int nb = 0; nb < kTileKV / 8; ++nb)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float e0 = bw::exp2_approx(__fmaf_rn(s[nb * 8 + 2 * q], scale_log2, nref));
-          const float e1 = bw::exp2_approx(__fmaf_rn(s[nb * 8 + 2 * q + 1], scale_log2, nref));
-          part[q] = __fadd_rn(part[q], __fadd_rn(e0, e1));
-          __nv_bfloat162 pr = __floats2bfloat162_rn(e0, e1);
-          packed[nb * 4 + q] = *reinterpret_cast<uint32_t*>(&pr);
-        }
-      const float tsum = __fadd_rn(__fadd_rn(part[0], part[1]), __fadd_rn(part[2], part[3]));
-      // the row of P: 64 bfloat16 = eight 16-byte pieces, swizzled like a TMA-written tile
-      unsigned char* prow = sp + b * kPBytes + m * 128;
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        *reinterpret_cast<uint4*>(prow + ((c ^ (m & 7)) << 4)) =
-            make_uint4(packed[c * 4], packed[c * 4 + 1], packed[c * 4 + 2], packed[c * 4 + 3]);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // make the writes visible to the tensor core
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->p_ready[b]);
-
-      // the output of the tile before this one is merged now, while the tensor core forms this
-      // tile's output from the weights just written
-      if (t > 0) {
-        const int pb = (t - 1) & 1;
-        if (!mbar_wait(&bars->pv_done[(t - 1) % kStages], ((t - 1) / kStages) & 1, failed)) {
+    for (int j = 0; j < count && ok; ++j) {
+      const int pos0 = items[j].pos0, rows = items[j].rows, kv_lo = items[j].kv_lo, tiles = items[j].tiles;
+      const int pos = (m < rows * group) ? pos0 + m / group : pos0 + rows - 1;
+      const int low_key = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+      const bool used = quarter * 32 < rows * group;  // else no lane of this warp holds a row
+      for (int t = (turn ^ c0) & 1; t < tiles; t += 2) {
+        const int c = c0 + t, b = c % kSBuffers;
+        const int j0 = kv_lo + t * kTileKV;
+        if (!mbar_wait(&bars->s_full[b], (c / kSBuffers) & 1, failed)) {
           ok = false;
           break;
         }
+        __syncwarp();
         fence_after_sync();
-        const MergeWeights w = merge_weights(M, prev_max);
-        M = w.mx;
-        L = merge_value(L, prev_sum, w);
+        if (used) {
+          float s[kTileKV];
+          tmem_ld64(lane_addr + b * kTileKV, s);
+          // mask, maximum of the raw scores (the mask test is skipped for tiles inside the row's
+          // range), then weights e = 2^(s * scale - ref) with one fused multiply-add per key
+          const bool inside = j0 + kTileKV - 1 <= pos && j0 >= low_key;
+          if (!inside) {
 #pragma unroll
-        for (int pc = 0; pc < kPieces; ++pc) {
-          float v[64];
-          tmem_ld64(lane_addr + kOCol + pb * HD + 64 * pc, v);
+            for (int i = 0; i < kTileKV; ++i) {
+              const int k = j0 + i;
+              s[i] = (k <= pos && k >= low_key) ? s[i] : -INFINITY;
+            }
+          }
+          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // the maximum is exact in any order
 #pragma unroll
-          for (int i = 0; i < 64; ++i) o_tot[64 * pc + i] = merge_value(o_tot[64 * pc + i], v[i], w);
+          for (int i = 0; i < kTileKV; i += 8) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) m4[e] = fmaxf(m4[e], fmaxf(s[i + e], s[i + 4 + e]));
+          }
+          const float tmax = __fmul_rn(fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])), scale_log2);
+          const float nref = (tmax == -INFINITY) ? 0.0f : -tmax;
+          // their sum in the order of the other kernels: key j belongs to quad lane (j % 8) / 2; a
+          // quad lane adds its pairs for j / 8 ascending; then (a0 + a1) + (a2 + a3)
+          float2 part[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};  // quad lanes 0 and 1, 2 and 3
+          const float2 scale2 = make_float2(scale_log2, scale_log2), nref2 = make_float2(nref, nref);
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t packed[16];
+#pragma unroll
+            for (int e8 = 0; e8 < 4; ++e8)  // eight keys
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                float2 e[2];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                  const int i = half * 32 + e8 * 8 + 4 * h + 2 * q;
+                  const float2 z = fma2(make_float2(s[i], s[i + 1]), scale2, nref2);
+                  e[q] = make_float2(bw::exp2_approx(z.x), bw::exp2_approx(z.y));
+                  __nv_bfloat162 pr = __floats2bfloat162_rn(e[q].x, e[q].y);
+                  packed[(i / 2) & 15] = *reinterpret_cast<uint32_t*>(&pr);
+                }
+                part[h] = add2(part[h], add2(make_float2(e[0].x, e[1].x), make_float2(e[0].y, e[1].y)));
+              }
+            tmem_st16(lane_addr + b * kTileKV + 16 * half, packed);  // over the scores this warp has read
+          }
+          stats[b * kTileM + m] = make_float2(tmax, __fadd_rn(__fadd_rn(part[0].x, part[0].y), __fadd_rn(part[1].x, part[1].y)));
+          tmem_written();
         }
         fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->p_ready[b]);
       }
-      prev_max = tmax;
-      prev_sum = tsum;
+      c0 += tiles;
     }
-    if (ok && ntiles > 0) {  // the last tile's output
-      const int pb = (ntiles - 1) & 1;
-      if (mbar_wait(&bars->pv_done[(ntiles - 1) % kStages], ((ntiles - 1) / kStages) & 1, failed)) {
-        fence_after_sync();
-        const MergeWeights w = merge_weights(M, prev_max);
-        M = w.mx;
-        L = merge_value(L, prev_sum, w);
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsMerge));
+    const int quarter = warp & 3;
+    const int m = quarter * 32 + lane;
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    int c = 0;
+    bool ok = true;
+    for (int j = 0; j < count && ok; ++j) {
+      const int rows = items[j].rows, tiles = items[j].tiles;
+      const bool used = quarter * 32 < rows * group;
+      float2 o_tot[HD / 2];
 #pragma unroll
-        for (int pc = 0; pc < kPieces; ++pc) {
-          float v[64];
-          tmem_ld64(lane_addr + kOCol + pb * HD + 64 * pc, v);
-#pragma unroll
-          for (int i = 0; i < 64; ++i) o_tot[64 * pc + i] = merge_value(o_tot[64 * pc + i], v[i], w);
+      for (int i = 0; i < HD / 2; ++i) o_tot[i] = make_float2(0.0f, 0.0f);
+      float M = -INFINITY, L = 0.0f;
+      for (int t = 0; t < tiles; ++t, ++c) {
+        const int b = c % kSBuffers;
+        const uint32_t parity = (c / kSBuffers) & 1;
+        // the maximum and sum are there when the weights are
+        if (!mbar_wait2(&bars->p_ready[b], parity, &bars->pv_done[b], parity, failed)) {
+          ok = false;
+          break;
         }
-      } else {
-        ok = false;
+        __syncwarp();
+        fence_after_sync();
+        const uint32_t from = lane_addr + kOCol + (c & 1) * HD;
+        uint32_t v0[32], v1[32];
+        if (used) {
+          tmem_ask(from, v0);
+          tmem_ask(from + 32, v1);
+          const float2 st = stats[b * kTileM + m];
+          const MergeWeights w = merge_weights(M, st.x);
+          M = w.mx;
+          L = merge_value(L, st.y, w);
+          const float2 wa = make_float2(w.a, w.a), wb = make_float2(w.b, w.b);
+          auto merge = [&](int first, const uint32_t (&v)[32]) {  // merge_value of two entries at a time
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              float2& o = o_tot[first / 2 + i];
+              o = fma2(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), wb, mul2(o, wa));
+            }
+          };
+          tmem_have(v0, v1);
+          if (HD == 128) {
+            merge(0, v0);
+            tmem_ask(from + 64, v0);
+            merge(32, v1);
+            tmem_ask(from + 96, v1);
+            tmem_have(v0, v1);
+          }
+          fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->o_free[b]);  // the output is in registers: the one after the next may go over it
+          merge(HD - 64, v0);
+          merge(HD - 32, v1);
+        } else {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->o_free[b]);
+        }
       }
-    }
-    if (ok && m < mrows) {
-      const int qr = m / group, hq = m - qr * group;
-      __nv_bfloat16* dst = out + static_cast<size_t>(row0 + qr) * out_stride + (g * group + hq) * HD;
-      const float inv = __fdiv_rn(1.0f, L);
+      if (ok && m < rows * group) {
+        const int qr = m / group, hq = m - qr * group;
+        __nv_bfloat16* dst = out + static_cast<size_t>(items[j].row0 + qr) * out_stride + (items[j].g * group + hq) * HD;
+        const float inv = __fdiv_rn(1.0f, L);
 #pragma unroll
-      for (int c = 0; c < HD / 8; ++c) {
-        __align__(16) __nv_bfloat162 o[4];
+        for (int e8 = 0; e8 < HD / 8; ++e8) {
+          __align__(16) __nv_bfloat162 o[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          o[e] = __floats2bfloat162_rn(__fmul_rn(o_tot[c * 8 + 2 * e], inv), __fmul_rn(o_tot[c * 8 + 2 * e + 1], inv));
-        *reinterpret_cast<uint4*>(dst + c * 8) = *reinterpret_cast<const uint4*>(o);
+          for (int e = 0; e < 4; ++e)
+            o[e] = __floats2bfloat162_rn(__fmul_rn(o_tot[e8 * 4 + e].x, inv), __fmul_rn(o_tot[e8 * 4 + e].y, inv));
+          *reinterpret_cast<uint4*>(dst + e8 * 8) = *reinterpret_cast<const uint4*>(o);
+        }
       }
     }
   }
 
   fence_before_sync();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 0) {
     __syncwarp();
     fence_after_sync();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(kTmemCols) : "memory");
@@ -485,7 +675,7 @@ bool make_map4(CUtensorMap* map, const void* base, const cuuint64_t (&dims)[4], 
 
 }  // namespace
 
-// Query rows per block, or 0 when this kernel cannot take the shape: head size 64 or 128, a page size
+// Query rows per tile, or 0 when this kernel cannot take the shape: head size 64 or 128, a page size
 // that divides 64, rows that start on 16 bytes. A group of heads that does not divide 128 leaves the
 // last one or more of a block's 128 stacked rows empty: what their lanes compute from whatever lies in
 // shared memory there stays in their rows and is never stored. (Groups of 3 used to run on the mma.sync
@@ -516,15 +706,6 @@ BW_API int bw_bf16_attention_tc(const __nv_bfloat16* qkv, int q_stride, const __
   const int group = heads / kv_heads;
   int* word = bw::failure_word();
   if (!word) return -1;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) {
-      bw::set_error("attention (tcgen05): cannot raise shared memory: %s", cudaGetErrorString(e));
-      return static_cast<int>(e);
-    }
-    configured = true;
-  }
   CUtensorMap map_q, map_k, map_v;
   {  // queries: [token][kv head][head of the group][d], box = 128 stacked rows of one kv head
     const cuuint64_t dims[4] = {HD, static_cast<cuuint64_t>(group), static_cast<cuuint64_t>(kv_heads),
@@ -548,9 +729,26 @@ BW_API int bw_bf16_attention_tc(const __nv_bfloat16* qkv, int q_stride, const __
     }
   }
   const float scale_log2 = scale * 1.44269504088896341f;
-  bw::launch_pdl(attention_tc_kernel, dim3(kv_heads, num_tiles), dim3(kThreads), kSmemBytes, stream, map_q, map_k, map_v,
-                 block_table, max_blocks, tile_seq, tile_row0, tile_rows, seq_pos0, seq_row0, out, out_stride, heads,
-                 kv_heads, page, window, scale_log2, word);
+  static bool configured[64] = {false};  // by device
+  static int sm_count[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  if (!configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (e != cudaSuccess) {
+      bw::set_error("attention (tcgen05): cannot raise shared memory: %s", cudaGetErrorString(e));
+      return static_cast<int>(e);
+    }
+    cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
+    if (sm_count[dev] <= 0) sm_count[dev] = 148;
+    configured[dev] = true;
+  }
+  // a block per SM, and whole rounds of them more where a block's list would not hold its items
+  const int total = num_tiles * kv_heads, sms = sm_count[dev];
+  const int blocks = std::min(total, sms * ((total + kMaxItems * sms - 1) / (kMaxItems * sms)));
+  bw::launch_pdl(attention_tc_kernel, dim3(blocks), dim3(kThreads), kSmemBytes, stream, map_q, map_k, map_v, block_table, max_blocks,
+                 tile_seq, tile_row0, tile_rows, total, seq_pos0, seq_row0, out, out_stride, heads, kv_heads, page, window,
+                 scale_log2, word);
   return bw::launch_status();
 }
 

@@ -1045,6 +1045,28 @@ def test_bf16_attention_tcgen05_takes_groups_that_leave_rows_of_a_block_empty(hd
     assert not ops.device_failure()
 
 
+@pytest.mark.parametrize("hd,heads,kv_heads,page,window", [(64, 40, 40, 16, 0), (64, 42, 14, 1, 0), (64, 48, 48, 64, 130), (128, 128, 32, 16, 0),
+                                                           (128, 40, 40, 8, 70)])
+def test_bf16_attention_tcgen05_blocks_that_walk_several_tiles(hd, heads, kv_heads, page, window):
+    """More query tiles than SMs: a block takes several one after the other, of different lengths, and hands buffers on from one to the
+    next.  The bits of the mma.sync kernel."""
+    rng = np.random.default_rng(heads + page)
+    ops = _ops("bfloat16")
+    lens = [700, 557, 6, 1000, 64]
+    k, v, table, _, _ = _paged(rng, lens, kv_heads, hd, page)
+    rows_by_seq = [(0, 700), (300, 257), (5, 1), (999, 1), (0, 64)]
+    q = bf(rnd(rng, sum(c for _, c in rows_by_seq), heads, hd))
+    k, v = bf(k), bf(v)
+    new, _, _ = _run_bf16_attention(q, rows_by_seq, k, v, table, heads, kv_heads, hd, window)
+    ops.legacy_attention = True
+    try:
+        old, _, _ = _run_bf16_attention(q, rows_by_seq, k, v, table, heads, kv_heads, hd, window)
+    finally:
+        ops.legacy_attention = False
+    assert_same_bits(new, old, f"heads {heads}/{kv_heads} page {page} window {window}")
+    assert not ops.device_failure()
+
+
 @pytest.mark.parametrize("heads,kv_heads,page,window", [(4, 1, 16, 0), (2, 2, 8, 0), (32, 2, 64, 0), (6, 2, 32, 130), (8, 8, 16, 0)])
 def test_bf16_attention_decode_of_wide_heads_through_boxes_gives_the_same_bits(heads, kv_heads, page, window):
     """Head size 128: a block per key tile fed by TMA boxes, and the cp.async blocks; rows that end on a tile's first and last
