@@ -305,7 +305,9 @@ BW_API int bw_bf16_linear_counters(int n) { return (n + kSplitBN - 1) / kSplitBN
 
 BW_API int bw_bf16_linear_split_rows() { return 128; }
 
-// One entry for every bfloat16 product. `y_is_f32`: 1 float32 outputs, 0 bfloat16, 2 a bfloat16 after the activation
+// One entry for every bfloat16 product. `partials` and `counters`: up to bw_bf16_linear_split_rows() rows the scratch of a split
+// product; above them `partials` is bw_bf16_linear_tc_cut_floats() floats that start out zero, one such scratch for each stream
+// (or null). `y_is_f32`: 1 float32 outputs, 0 bfloat16, 2 a bfloat16 after the activation
 // a (bw::out_act). `use_legacy` != 0 forces the mma.sync tile (tests
 // compare the two variants bit for bit); otherwise the tcgen05 kernel runs whenever the rows
 // start on 16 bytes, and the legacy tile takes the remaining shapes (an inner size that is no

@@ -506,7 +506,7 @@ BW_API int bw_bf16_linear_tc_rope_usable(const void* x, const void* w, int m, in
 BW_API int bw_bf16_linear_tc_rope(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* qkv, int m, int n, int k,
                                   const int* pos, const int* row_seq, const float* cos_t, const float* sin_t,
                                   const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache, int heads,
-                                  int kv_heads, int hd, int page, int write_kv, cudaStream_t stream);
+                                  int kv_heads, int hd, int page, int write_kv, float* partials, cudaStream_t stream);
 BW_API int bw_bf16_linear_rows_rope_usable(const void* x, const void* w, int m, int n, int k, int heads, int kv_heads,
                                            int hd) {
   if (m > 16) return heads > 0 && kv_heads > 0 && n == (heads + 2 * kv_heads) * hd && bw_bf16_linear_tc_rope_usable(x, w, m, n, k, hd);
@@ -519,15 +519,16 @@ BW_API int bw_bf16_linear_rows_rope_usable(const void* x, const void* w, int m, 
 // qkv = x W^T for the fused q/k/v weights, then what bw_bf16_rope_cache does to it, in the same
 // kernel: q rotated into qkv[:, :heads * hd]; k rotated and v as it is into the pages
 // block_table[row_seq[r]][pos[r] / page] of the cache (not when write_kv is 0; the k and v
-// columns of qkv are not written). cos_t / sin_t null: nothing is rotated.
+// columns of qkv are not written). cos_t / sin_t null: nothing is rotated. partials: scratch as for bw_bf16_linear.
 BW_API int bw_bf16_linear_rows_rope(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* qkv, int m, int n, int k,
                                     const int* pos, const int* row_seq, const float* cos_t, const float* sin_t,
                                     const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache,
-                                    int heads, int kv_heads, int hd, int page, int write_kv, cudaStream_t stream) {
+                                    int heads, int kv_heads, int hd, int page, int write_kv, float* partials,
+                                    cudaStream_t stream) {
   if (m <= 0 || n <= 0) return 0;
   if (m > 16)
     return bw_bf16_linear_tc_rope(x, w, qkv, m, n, k, pos, row_seq, cos_t, sin_t, block_table, max_blocks, kcache, vcache, heads, kv_heads,
-                                  hd, page, write_kv, stream);
+                                  hd, page, write_kv, partials, stream);
   RowsShape s;
   if (!bw_bf16_linear_rows_rope_usable(x, w, m, n, k, heads, kv_heads, hd) || !rows_shape(m, n, k, true, &s) || page <= 0) {
     bw::set_error("linear with rotation (few rows): shape [%d x %d] x [%d x %d], %d/%d heads of %d is not for this path", m,

@@ -55,6 +55,7 @@ constexpr int kDirectRows = 40;                // up to these rows chunk sums ar
 // for a stage and use it costs their warps some 300 cycles of barrier operations whatever it holds, and the four MMAs of a
 // narrow k-tile take 120 (64 rows x 8,192 x 2,048 in tiles of 32 columns: 42 -> 27 us, of 64: 45 -> 36). Wide tiles keep one:
 // their MMAs take 500 cycles, and a ring of few large stages covers less of the memory's latency.
+constexpr uint32_t kFlagPolls = 4000000u;  // of about 100 ns and more, for what another pair leaves
 constexpr int kMaxStages = 32, kMaxTilesPerStage = 4;
 struct RingShape {
   int tile_bytes_x, tile_bytes, per_stage, stage_bytes, stages, pad_bytes, ring_bytes;
@@ -371,7 +372,13 @@ __global__ void reduce_swiglu_kernel(const float* __restrict__ partials, int num
 // read is spread over both warpgroups, 64 columns per tcgen05.ld, and the totals of a thread (128)
 // stay in registers.
 //
-// PAIR (with WIDE, whole mode): two blocks of a cluster share a 256 x 256 tile, see above.
+// PAIR (with WIDE, whole mode): two blocks of a cluster share a 256 x 256 tile, see above. With scratch (`partials`, see
+// kCutFloats) the tiles of the last two rounds are cut along k so that every pair gets as many chunks as the others: they are
+// laid end to end and each pair takes an equal stretch, at least a tile long. A stretch begins inside a tile whose first
+// chunks end the stretch of the pair before. That pair does them first of all and leaves the running totals in scratch; this
+// one does its part of the tile last, with those totals to start from: the order of the additions, and so the bits, are those of
+// a whole tile, and nobody waits in practice. Pairs wait for pairs with lower numbers only, which are placed before them.
+// (1,200 rows x 4,096 x 4,096: 80 tiles on 74 pairs, two rounds of 8 chunks become stretches of 8 or 9.)
 //
 // GROUPED (whole mode): one product per group over lists of rows. x holds the rows group by group
 // (group g owns rows group_off[g] .. group_off[g + 1] - 1), W is [groups * N][K], y row i is x row
@@ -392,6 +399,10 @@ struct RopeOut {
   __nv_bfloat16* vcache;
   int heads, kv_heads, page, write_kv;
 };
+// Scratch of the tiles that are cut: the totals of a tile by pair, block of the pair, epilogue warp, then 32 blocks of 16 bytes a
+// lane; behind them a flag (an int) for each warp, zero between launches.
+constexpr int kCutWarps = 16;                          // epilogue warps of a pair
+constexpr int kCutFloats = kCutWarps * 32 * (2 * BN / 2);  // a pair's
 struct GroupItems {
   const int* group_off;
   const int* tile_prefix;
@@ -463,6 +474,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   auto item_n0 = [&](int t) { return SPLIT ? (t / num_chunks) * bt : (t / (GROUPED ? row_tiles : m_blocks)) * bt; };
   auto item_c0 = [&](int t) { return SPLIT ? t % num_chunks : 0; };
   auto item_c1 = [&](int t) { return SPLIT ? t % num_chunks + 1 : num_chunks; };
+  // A pair's items where tiles are cut: `full` rounds of whole tiles, then its stretch u0 .. u1 of the chunks of the others.
+  const bool cut = PAIR && partials != nullptr;
+  const int full = cut ? out_tiles / workers - 1 : 0, base = full * workers;
+  const int u0 = cut ? static_cast<int>(static_cast<long long>(worker) * (out_tiles - base) * num_chunks / workers) : 0;
+  const int u1 = cut ? static_cast<int>(static_cast<long long>(worker + 1) * (out_tiles - base) * num_chunks / workers) : 0;
+  // the i-th item of this worker: its output tile and chunks
+  auto item = [&](int i, int& tile, int& c0, int& c1) -> bool {
+    if (PAIR && cut && i >= full) {
+      i -= full;
+      const int head = u1 % num_chunks;  // chunks of a tile that the next pair finishes
+      if (head > 0 && i-- == 0) {
+        tile = base + u1 / num_chunks, c0 = 0, c1 = head;
+        return true;
+      }
+      const int first = (u0 + num_chunks - 1) / num_chunks, count = u1 / num_chunks - first;
+      if (i < count) {
+        tile = base + first + i, c0 = 0, c1 = num_chunks;
+        return true;
+      }
+      tile = base + u0 / num_chunks, c0 = u0 % num_chunks, c1 = num_chunks;
+      return i == count && c0 > 0;
+    }
+    tile = worker + i * workers;
+    c0 = item_c0(tile), c1 = item_c1(tile);
+    return tile < out_tiles;
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -527,14 +564,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         tma_load_2d(dst, map, x, y, &bars->full[st]);
     };
     if (GROUPED) read_lists(), waited = true;
-    for (int tile = worker; tile < out_tiles && ok; tile += workers) {
+    for (int i = 0, tile, c0, c1; ok && item(i, tile, c0, c1); ++i) {
       int m0 = item_m0(tile), n0 = item_n0(tile) + (PAIR ? static_cast<int>(rank) * BN : 0);
       if (GROUPED) {
         int m_end, g;
         group_tile(tile, m0, m_end, g);
         n0 += g * N;  // the group's rows of W
       }
-      const int kt0 = item_c0(tile) * kTilesPerChunk, kt1 = min(num_tiles, item_c1(tile) * kTilesPerChunk);
+      const int kt0 = c0 * kTilesPerChunk, kt1 = min(num_tiles, c1 * kTilesPerChunk);
       int kt = kt0;
       if (!waited) {  // first item of this block
         const int early = min(kt1 - kt0, kStages * kPer);
@@ -579,8 +616,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       uint32_t gc = 0;               // chunks begun so far
       bool ok = true;
       read_lists();
-      for (int tile = worker; tile < out_tiles && ok; tile += workers) {
-        for (int c = item_c0(tile); c < item_c1(tile) && ok; ++c, ++gc) {
+      for (int i = 0, tile, c0, c1; ok && item(i, tile, c0, c1); ++i) {
+        for (int c = c0; c < c1 && ok; ++c, ++gc) {
           const int buf = gc & 1;
           const uint32_t use = gc >> 1;  // how often this accumulator was used before
           if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(&bars->acc_empty[buf], (use - 1) & 1, failed))) {
@@ -647,7 +684,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     const int off0 = blk * BN, off1 = off0 + BN / 2;  // column offsets of the pieces in the tile
     uint32_t gc = 0;
     bool ok = true;
-    for (int tile = worker; tile < out_tiles && ok; tile += workers) {
+    for (int i = 0, tile, c0, c1; ok && item(i, tile, c0, c1); ++i) {
       // The running totals start at -0, which leaves whatever is added to it as it is: the first chunk sum is added like the
       // others. (Choosing between "v" and "total + v" by the chunk made the compiler keep both, and sent half of the totals
       // to local memory in the epilogues with SwiGLU or a residual.)
@@ -682,7 +719,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           put_piece(store_buf, lane, c, __float_as_uint(total[b * 32 + 4 * c]), __float_as_uint(total[b * 32 + 4 * c + 1]),
                     __float_as_uint(total[b * 32 + 4 * c + 2]), __float_as_uint(total[b * 32 + 4 * c + 3]));
       };
-      for (int c = item_c0(tile); c < item_c1(tile) && ok; ++c, ++gc) {
+      if (PAIR && c0 > 0 && warp_rows > 0) {  // the tile's first chunks were added up by the pair before
+        const int slot = ((worker - 1) * 2 + static_cast<int>(rank)) * (kCutWarps / 2) + warp - kFirstEpiWarp;
+        int* flag = reinterpret_cast<int*>(partials + static_cast<size_t>(workers) * kCutFloats) + slot;
+        if (lane == 0) {
+          uint32_t spin = 0;
+          int seen = 0;
+          while (!seen && spin++ < kFlagPolls) {
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
+            if (!seen) __nanosleep(100);
+          }
+          if (!seen) *failed = 1;
+          *flag = 0;  // for the next launch
+        }
+        __syncwarp();
+        const char* from = reinterpret_cast<const char*>(partials + static_cast<size_t>(slot) * (32 * 2 * PW)) + lane * 16;
+#pragma unroll
+        for (int j = 0; j < 2 * PW / 4; ++j) {
+          const float4 v = __ldcg(reinterpret_cast<const float4*>(from + j * 512));
+          total[4 * j] = v.x, total[4 * j + 1] = v.y, total[4 * j + 2] = v.z, total[4 * j + 3] = v.w;
+        }
+      }
+      for (int c = c0; c < c1 && ok; ++c, ++gc) {
         const int buf = gc & 1;
         if (!mbar_wait(&bars->acc_full[buf], (gc >> 1) & 1, failed)) {
           ok = false;
@@ -718,6 +776,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
       if (!__all_sync(0xffffffffu, ok)) break;
       if (warp_rows <= 0) continue;
+      if (PAIR && c1 < num_chunks) {  // the next pair goes on from these totals
+        const int slot = (worker * 2 + static_cast<int>(rank)) * (kCutWarps / 2) + warp - kFirstEpiWarp;
+        char* to = reinterpret_cast<char*>(partials + static_cast<size_t>(slot) * (32 * 2 * PW)) + lane * 16;
+#pragma unroll
+        for (int j = 0; j < 2 * PW / 4; ++j)
+          __stcg(reinterpret_cast<float4*>(to + j * 512), make_float4(total[4 * j], total[4 * j + 1], total[4 * j + 2], total[4 * j + 3]));
+        __syncwarp();
+        if (lane == 0) {
+          __threadfence();
+          asm volatile("st.release.gpu.global.s32 [%0], %1;"
+                       ::"l"(reinterpret_cast<int*>(partials + static_cast<size_t>(workers) * kCutFloats) + slot), "r"(1)
+                       : "memory");
+        }
+        continue;
+      }
       if (SPLIT && num_chunks > 1) {
         // this item's chunk sum goes to scratch; a second kernel adds the chunk sums in order
         float* plane = partials + static_cast<size_t>(item_c0(tile)) * M * N;
@@ -1000,6 +1073,9 @@ BW_API int bw_bf16_linear_tc_pair_tiles(int on) {
 BW_API long long bw_bf16_linear_tc_scratch_floats(int m, int n, int k) {
   return static_cast<long long>((k + kChunk - 1) / kChunk) * m * n;
 }
+// Scratch of products of more than 128 rows whose last tiles are cut (see PAIR): floats, all of them zero at first and
+// each product's own until it is done. The entry points below take it as `partials` (null: tiles stay whole).
+BW_API long long bw_bf16_linear_tc_cut_floats();
 BW_API int bw_bf16_linear_tc_counters(int n) { return (n + BN - 1) / BN; }
 
 // Split mode is chosen from the shape alone: one block of rows, more than one chunk, and too
@@ -1024,13 +1100,21 @@ int sm_count_of_device() {
   return sm_count[dev];
 }
 
+}  // namespace
+
+BW_API long long bw_bf16_linear_tc_cut_floats() {
+  return static_cast<long long>(sm_count_of_device() / 2) * (kCutFloats + kCutWarps);
+}
+
+namespace {
+
 // How a product with few tiles runs. The plan is the one of least estimated time, from times measured on a B200 (us):
 //   whole   items are output tiles with all their chunks; a chunk of a tile takes chunk_us by the tile's width, rounds of the SMs
 //           over the items follow each other, and a launch costs about 6 us around them
 //   split   items are (tile, chunk) pairs; the second kernel costs about 2 us (little up to 16 rows), and the chunk sums are written
 //           and read (8 bytes each) at about 5 TB/s. One block of rows only: beyond it the chunk sums outgrow what they save
 //   pairs   more than 128 rows: 256 x 256 tiles on pairs of blocks, 2.45 us a chunk, 8.5 us around them (10.5 where a
-//           residual is read or SwiGLU applied)
+//           residual is read or SwiGLU applied); the last rounds are cut along k where that evens them out
 // and none is faster than its operands arrive: a chunk's rows of x and W at about 83 KB a us for a block, and at about 9.5 TB/s
 // over all SMs. Tiles are 16 .. 128
 // columns wide in steps of 16, or 256 with one block of rows (split along k only where one round of the SMs takes all its
@@ -1062,6 +1146,22 @@ double chunk_us(int bn, bool few) {
 
 constexpr double kWideChunkAloneUs = 4.6;  // of a split product in tiles of 256 columns
 
+// Chunks of the pair that has the most of them, over `items` tiles of `chunks` each: whole rounds, or with the last ones cut (see
+// the kernel). They are cut where that saves a pair a quarter of its chunks: near full rounds the GPU runs at its power limit, and
+// what one pair does less the others do slower (us, whole and cut, chunks of a pair before and after: 1,200 x 4,096 x 4,096
+// 53.9 -> 41.8, 16 and 9; 1,200 x 14,336 x 4,096 196 -> 121, 56 and 31; but 1,200 x 4,096 x 6,144 50.2 -> 50.8, 16 and 13; 2,047 x 2,048 x
+// 6,144 41.3 -> 48.7, 12 and 11; 2,047 x 14,336 x 4,096 204 -> 214, 56 and 49).
+bool pairs_cut(long long items, long long pairs, int chunks, long long* most) {
+  const long long rounds = (items + pairs - 1) / pairs, whole = rounds * chunks;
+  *most = whole;
+  if (items <= pairs || items % pairs == 0) return false;
+  const long long full = items / pairs - 1, rest = items - full * pairs;
+  const long long even = full * chunks + (rest * chunks + pairs - 1) / pairs;
+  if (4 * even > 3 * whole) return false;
+  *most = even;
+  return true;
+}
+
 Plan plan_rows(int m, int n, int k, bool swiglu, bool reads, int sms, bool allow_wide = true) {
   const int chunks = (k + kChunk - 1) / kChunk;
   const bool one_block = m <= BM;
@@ -1075,7 +1175,9 @@ Plan plan_rows(int m, int n, int k, bool swiglu, bool reads, int sms, bool allow
     const long long items = static_cast<long long>((m + 2 * BM - 1) / (2 * BM)) * ((n + 2 * BN - 1) / (2 * BN));
     const long long pairs = sms / 2;
     best = Plan{false, 2 * BN, true};
-    best_cost = (swiglu || reads ? 10.5 : 8.5) + static_cast<double>((items + pairs - 1) / pairs) * chunks * 2.45;
+    long long most = 0;
+    pairs_cut(items, pairs, chunks, &most);
+    best_cost = (swiglu || reads ? 10.5 : 8.5) + static_cast<double>(most) * 2.45;
   }
   for (int mode = 0; mode < 2; ++mode) {
     if (mode == 1 && !may_split) continue;
@@ -1219,8 +1321,10 @@ int launch_tc(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int y_is_
   const long long items = SPLIT ? static_cast<long long>(n_blocks) * chunks : static_cast<long long>(n_blocks) * m_blocks;
   if (PAIR) {
     const unsigned pairs = static_cast<unsigned>(items < max_pairs ? items : max_pairs);
+    long long most;
+    const bool cut = partials && static_cast<int>(pairs) <= sm_count_of_device() / 2 && pairs_cut(items, pairs, chunks, &most);
     bw::launch_pdl_cluster(2, kernel, dim3(2 * pairs), dim3(threads), smem, stream, map_x, map_w, y, y_is_f32, residual, m,
-                            n, k, error_word, partials, bn, GroupItems{nullptr, nullptr, 0}, rope);
+                            n, k, error_word, cut ? partials : nullptr, bn, GroupItems{nullptr, nullptr, 0}, rope);
     return bw::launch_status();
   }
   const int sms = sm_count_of_device();
@@ -1289,7 +1393,7 @@ int launch_tc_rows(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, int 
   if (!wide_ok || !plan.pair)
     return launch_tc<false, 128, EPI, false>(x, w, y, y_is_f32, residual, m, n, k, error_word, nullptr, fused, stream, plan.bn);
   if (g_pair_tiles)
-    return launch_tc<false, 128, EPI, true, true>(x, w, y, y_is_f32, residual, m, n, k, error_word, nullptr, fused, stream);
+    return launch_tc<false, 128, EPI, true, true>(x, w, y, y_is_f32, residual, m, n, k, error_word, partials, fused, stream);
   return launch_tc<false, 128, EPI, true>(x, w, y, y_is_f32, residual, m, n, k, error_word, nullptr, fused, stream);
 }
 
@@ -1352,7 +1456,7 @@ BW_API int bw_bf16_rope_cache(__nv_bfloat16* qkv, int row_stride, const int* pos
 BW_API int bw_bf16_linear_tc_rope(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* qkv, int m, int n, int k,
                                   const int* pos, const int* row_seq, const float* cos_t, const float* sin_t,
                                   const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache, int heads,
-                                  int kv_heads, int hd, int page, int write_kv, cudaStream_t stream) {
+                                  int kv_heads, int hd, int page, int write_kv, float* partials, cudaStream_t stream) {
   if (m <= 0 || n <= 0) return 0;
   if (!bw_bf16_linear_tc_rope_usable(nullptr, nullptr, m, n, k, hd) || n != (heads + 2 * kv_heads) * hd || page <= 0) {
     bw::set_error("linear with rotation (tcgen05): shape [%d x %d] x [%d x %d], %d/%d heads of %d is not for this path", m, k, n, k,
@@ -1363,7 +1467,7 @@ BW_API int bw_bf16_linear_tc_rope(const __nv_bfloat16* x, const __nv_bfloat16* w
   // not take, and outputs that the epilogue's stores do not, run as the product and the rotation kernel.
   auto off16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 != 0; };
   if (off16(x) || off16(w) || reinterpret_cast<uintptr_t>(qkv) % 32 || off16(kcache) || off16(vcache) || off16(cos_t) || off16(sin_t)) {
-    const int rc = bw_bf16_linear(x, w, qkv, 0, nullptr, m, n, k, nullptr, nullptr, 0, stream);
+    const int rc = bw_bf16_linear(x, w, qkv, 0, nullptr, m, n, k, partials, nullptr, 0, stream);
     return rc ? rc
               : bw_bf16_rope_cache(qkv, n, pos, row_seq, cos_t, sin_t, block_table, max_blocks, kcache, vcache, m, heads, kv_heads, hd,
                                    page, write_kv, stream);
@@ -1372,7 +1476,7 @@ BW_API int bw_bf16_linear_tc_rope(const __nv_bfloat16* x, const __nv_bfloat16* w
   if (!word) return -1;
   const RopeOut rope{pos, row_seq, cos_t, sin_t, block_table, max_blocks, kcache, vcache, heads, kv_heads, page, write_kv};
   const Fused none;
-  return launch_tc<false, 128, 3, true, true>(x, w, qkv, 0, nullptr, m, n, k, word, nullptr, none, stream, 2 * BN, rope);
+  return launch_tc<false, 128, 3, true, true>(x, w, qkv, 0, nullptr, m, n, k, word, partials, none, stream, 2 * BN, rope);
 }
 
 // Grouped products on the tcgen05 kernel: y[i] = x[i] W_g^T for the rows i of group g, x holding

@@ -23,7 +23,7 @@ BW_API int bw_bf16_linear_rows_rope_usable(const void* x, const void* w, int m, 
 BW_API int bw_bf16_linear_rows_rope(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* qkv, int m, int n, int k,
                                     const int* pos, const int* row_seq, const float* cos_t, const float* sin_t,
                                     const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache, int heads,
-                                    int kv_heads, int hd, int page, int write_kv, cudaStream_t stream);
+                                    int kv_heads, int hd, int page, int write_kv, float* partials, cudaStream_t stream);
 
 namespace {
 
@@ -80,19 +80,19 @@ BW_API int bw_bf16_block(void* call, float eps1, float eps2, float scale, cudaSt
   const int window = static_cast<int>(c.window), pages = static_cast<int>(c.num_pages), writable = static_cast<int>(c.writable);
   const int q_dim = heads * hd, qkv_dim = (heads + 2 * kv_heads) * hd;
   const bool scratch = n <= bw_bf16_linear_split_rows();
-  float* partials = scratch ? c.partials : nullptr;
+  float* partials = c.partials;  // the caller gives each range of rows the scratch it takes
   int* counters = scratch ? c.counters : nullptr;
   c.launches = 0, c.attention_failed = 0;
   int rc;
 #define BW_DO(KERNELS_, CALL_)        \
   if ((rc = (CALL_)) != 0) return rc; \
   c.launches += (KERNELS_)
-  auto kernels = [&](int m, int out, int in, int swiglu) { return bw_bf16_linear_tc_kernels(m, out, in, swiglu, partials != nullptr); };
+  auto kernels = [&](int m, int out, int in, int swiglu) { return bw_bf16_linear_tc_kernels(m, out, in, swiglu, scratch && partials != nullptr); };
 
   BW_DO(1, bw_bf16_rmsnorm(c.x, c.norm1, c.normed, nullptr, n, width, eps1, stream));
   if (bw_bf16_linear_rows_rope_usable(nullptr, nullptr, n, qkv_dim, width, heads, kv_heads, hd)) {
     BW_DO(1, bw_bf16_linear_rows_rope(c.normed, c.w_qkv, c.qkv, n, qkv_dim, width, c.pos, c.row_seq, c.cos_t, c.sin_t, c.block_table,
-                                      max_blocks, c.k, c.v, heads, kv_heads, hd, page, writable, stream));
+                                      max_blocks, c.k, c.v, heads, kv_heads, hd, page, writable, partials, stream));
   } else {
     BW_DO(kernels(n, qkv_dim, width, 0),
           bw_bf16_linear(c.normed, c.w_qkv, c.qkv, 0, nullptr, n, qkv_dim, width, partials, counters, 0, stream));

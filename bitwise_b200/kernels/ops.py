@@ -104,6 +104,7 @@ class KernelOps:
         if self.kind == "bf16":
             self.lib.bw_bf16_linear_scratch_floats.restype = ctypes.c_longlong
             self._split_rows = int(self.lib.bw_bf16_linear_split_rows())
+            self._cut = {}
         # One word of device memory that every kernel of this object's libraries raises when a
         # bounded wait runs out, and its pinned mirror on the host (filled by failure_poll).
         self._failure_word: Optional[torch.Tensor] = None
@@ -241,13 +242,11 @@ class KernelOps:
             if out.dtype not in (torch.float32, torch.bfloat16):
                 raise KernelError("linear: out must be float32 or bfloat16")
             _need(out, out.dtype, "linear out", 2)
-            partials = counters = None
-            if m <= self._split_rows:
-                partials, counters = self._linear_scratch(x.device, n, k)
+            partials, counters = self._linear_scratch(x.device, n, k) if m <= self._split_rows else (self._cut_scratch(x.device), None)
             self._call("bw_bf16_linear", _p(x), _p(w), _p(out), _c_int(2 * act + int(out.dtype == torch.float32)),
                        _p(residual), _c_int(m), _c_int(n), _c_int(k), _p(partials), _p(counters),
                        _c_int(int(legacy)), self._stream(),
-                       launches=1 if legacy else self._linear_kernels(m, n, k, False, partials is not None))
+                       launches=1 if legacy else self._linear_kernels(m, n, k, False, counters is not None and partials is not None))
 
     def _linear_then(self, x, w, out, residual, then) -> bool:
         """``linear`` with the norm that follows in one kernel; False where the shape takes another path."""
@@ -297,12 +296,11 @@ class KernelOps:
         _need(out, self.act_dtype, "linear_swiglu out", 2)
         if self.kind != "bf16" or n % 128 or k % 8 or tuple(out.shape) != (m, n // 2) or w_interleaved.shape[1] != k:
             raise KernelError("linear_swiglu: unsupported shapes or precision")
-        partials = None
-        if m <= self._split_rows:
-            partials, _ = self._linear_scratch(x.device, n, k)
+        split = m <= self._split_rows
+        partials = self._linear_scratch(x.device, n, k)[0] if split else self._cut_scratch(x.device)
         self._call("bw_bf16_linear_tc_swiglu", _p(x), _p(w_interleaved), _p(out), _c_int(m), _c_int(n), _c_int(k),
                    _p(partials), _c_int(self.FUSED_ACTIVATIONS.index(activation)), self._stream(),
-                   launches=self._linear_kernels(m, n, k, True, partials is not None))
+                   launches=self._linear_kernels(m, n, k, True, split and partials is not None))
 
     def _linear_kernels(self, m: int, n: int, k: int, swiglu: bool, scratch: bool) -> int:
         """Kernels that a product of this shape launches (2 when it is split along k)."""
@@ -332,6 +330,36 @@ class KernelOps:
             self._retired.append(self._counters)
             self._counters = torch.zeros(max(tiles, 1024), dtype=torch.int32, device=device)
         return self._partials, self._counters
+
+    _cut: Optional[dict] = None  # stream -> scratch of its products of many rows (serving precision)
+    CUT_STREAMS = 8  # streams that get a scratch of their own for products whose last tiles are cut
+
+    def _cut_scratch(self, device) -> Optional[torch.Tensor]:
+        """Scratch of a product of more than 128 rows (running totals of tiles that two pairs of blocks share, and flags that are
+        zero between launches): one for each stream, since products of different streams may run side by side.  None, and
+        the tiles stay whole, for streams beyond the first few and while a stream captures (a graph may be replayed beside
+        another one that was captured on the same stream)."""
+        if self._cut is None:
+            return None
+        stream = self._stream().value
+        if torch.cuda.is_current_stream_capturing():
+            return None
+        got = self._cut.get(stream)
+        if got is None:
+            if len(self._cut) >= self.CUT_STREAMS:
+                return None
+            self.lib.bw_bf16_linear_tc_cut_floats.restype = ctypes.c_longlong
+            got = torch.zeros(int(self.lib.bw_bf16_linear_tc_cut_floats()), dtype=torch.float32, device=device)
+            return self._cut.setdefault(stream, got)
+        return got
+
+    def _clear_cut_scratch(self) -> None:
+        """After a bounded wait ran out: flags that nobody waited for any more go back to zero."""
+        if self._cut:
+            torch.cuda.synchronize()
+            for scratch in list(self._cut.values()):
+                scratch.zero_()
+            torch.cuda.synchronize()
 
     def force_linear_plan(self, width: int = 0, mode: int = 0) -> None:
         """Tests and measurements: force the tile width (16 .. 128 in steps of 16, or 256, above
@@ -405,6 +433,7 @@ class KernelOps:
             return False
         self._failure_host[0] = 0
         self._failure_word.zero_()
+        self._clear_cut_scratch()
         return True
 
     def device_failure(self) -> bool:
@@ -414,6 +443,7 @@ class KernelOps:
         bad = bool(int(word.item()))
         if bad:
             word.zero_()
+            self._clear_cut_scratch()
         return bad
 
     def selftest_bounded_wait(self, polls: int = 4096) -> int:
@@ -541,7 +571,7 @@ class KernelOps:
         self._call("bw_bf16_linear_rows_rope", _p(x), _p(w_qkv), _p(qkv), _c_int(m), _c_int(n), _c_int(k), _p(pos),
                    _p(row_seq), _p(cos), _p(sin), _p(block_table), _c_int(block_table.shape[1]), _p(kcache), _p(vcache),
                    _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(kcache.shape[2]), _c_int(int(write_kv)),
-                   self._stream())
+                   _p(self._cut_scratch(x.device) if m > self._split_rows else None), self._stream())
 
     def attention(self, qkv: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor,
                   block_table: torch.Tensor, row_seq: torch.Tensor, pos: torch.Tensor, out: torch.Tensor,
@@ -714,6 +744,9 @@ class KernelOps:
             for out, inner in ((qkv_dim, width), (width, q_dim), (2 * inter, width), (width, inter)):
                 self._linear_scratch(x.device, out, inner)
             partials, counters = self._partials.data_ptr() if self._partials is not None else 0, self._counters.data_ptr()
+        else:
+            scratch = self._cut_scratch(x.device)
+            partials = scratch.data_ptr() if scratch is not None else 0
         if t_count == n and ctx.max_keys > 128:
             attn_scratch = self._attention_scratch(lib, x.device, n, heads, ctx.max_keys).data_ptr()
         ptr = lambda t_: 0 if t_ is None else t_.data_ptr()

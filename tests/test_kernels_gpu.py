@@ -762,6 +762,46 @@ def test_bf16_qkv_product_of_many_rows_takes_weights_of_any_start():
     assert not ops.device_failure()
 
 
+@pytest.mark.parametrize("m,n,k", [(1200, 4096, 4096), (700, 6464, 1096), (300, 9984, 2048), (513, 12928, 1032), (257, 19136, 4104),
+                                   (1536, 3520, 5128)])
+def test_bf16_products_of_many_rows_whose_last_tiles_are_cut(m, n, k):
+    """More tiles than block pairs, and a last round that is not full: two pairs share a tile along k, the second going on from the first
+    one's totals.  The bits of whole tiles on single blocks, call after call, and from two streams at a time."""
+    ops = _ops("bfloat16")
+    gen = torch.Generator(device=DEV).manual_seed(m + n + k)
+    draw = lambda *shape, dtype=torch.bfloat16: torch.randn(*shape, generator=gen, device=DEV).to(dtype)
+    x, w, res = draw(m, k), draw(n, k) * 0.05, draw(m, n, dtype=torch.float32)
+    glu = n % 128 == 0
+
+    def all_three():
+        y, z = torch.empty(m, n, device=DEV, dtype=torch.bfloat16), res.clone()
+        ops.linear(x, w, y)
+        ops.linear(x, w, z, residual=z)
+        h = torch.empty(m, n // 2, device=DEV, dtype=torch.bfloat16)
+        if glu:
+            ops.linear_swiglu(x, w, h)
+        return [y.view(torch.int16), z.view(torch.int32)] + ([h.view(torch.int16)] if glu else [])
+    before = ops.pair_tiles(False)
+    try:
+        want = all_three()
+    finally:
+        ops.pair_tiles(before)
+    for _ in range(3):
+        for got, exp in zip(all_three(), want):
+            assert torch.equal(got, exp)
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in range(2)], []
+    for _ in range(3):
+        for s in streams:
+            with torch.cuda.stream(s):
+                got.append(all_three())
+    torch.cuda.synchronize()
+    for g in got:
+        for a, b in zip(g, want):
+            assert torch.equal(a, b)
+    assert not ops.device_failure()
+
+
 def test_bf16_single_block_tiles_cover_the_product_that_rotates():
     """With block pairs switched off no product runs on them, the fused q/k/v product of many rows included."""
     ops = _ops("bfloat16")
