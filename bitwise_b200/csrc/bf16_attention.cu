@@ -381,15 +381,15 @@ attention_whole_kernel(const __nv_bfloat16* __restrict__ qkv, int q_stride, cons
 // ---------------------------------------------------------------------------------------
 // Split mode (decode steps: one query row per sequence, at most 16 stacked rows): a block
 // takes (row, key/value head, kSplitWarps consecutive key tiles), each warp one tile of its
-// own: it loads the tile, computes the tile result and stores it. Record layout per (row,
-// head, tile): o[HD], maximum, sum.
+// own: it loads the tile, computes the tile result and stores it: o[HD] per (row, head, tile), and behind
+// all of those (maximum, sum) per (row, head, tile).
 constexpr int kSplitQBytes = 16 * kRowBytes;
 
 __global__ void __launch_bounds__(kSplitWarps * 32)
 attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_stride, const __nv_bfloat16* __restrict__ kcache,
                        const __nv_bfloat16* __restrict__ vcache, const int* __restrict__ block_table, int max_blocks,
                        const int* __restrict__ row_seq, const int* __restrict__ pos, int heads, int kv_heads, int page,
-                       int page_shift, int window, float scale_log2, float* __restrict__ tile_out, int max_tiles) {
+                       int page_shift, int window, float scale_log2, float* __restrict__ tile_out, float2* __restrict__ tile_stats, int max_tiles) {
   // The step's index arrays (positions, row -> sequence, block tables) were copied to the
   // device before the step's first kernel, and the keys and values of a tile that ends before
   // the row's own position were stored by earlier steps: those loads are issued before the
@@ -436,14 +436,12 @@ attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_stride, cons
   for (int half = 0; half < 2; ++half) {
     const int m = (lane >> 2) + half * 8;
     if (m >= group) continue;
-    float* dst = tile_out + ((static_cast<size_t>(row) * heads + (g * group + m)) * max_tiles + t) * (HD + 2);
+    const size_t rec = (static_cast<size_t>(row) * heads + (g * group + m)) * max_tiles + t;
+    float* dst = tile_out + rec * HD;
 #pragma unroll
     for (int i = 0; i < HD / 8; ++i)
       *reinterpret_cast<float2*>(dst + i * 8 + 2 * (lane & 3)) = make_float2(r.o[i][half * 2], r.o[i][half * 2 + 1]);
-    if ((lane & 3) == 0) {
-      dst[HD] = half ? r.max_hi : r.max_lo;
-      dst[HD + 1] = half ? r.sum_hi : r.sum_lo;
-    }
+    if ((lane & 3) == 0) tile_stats[rec] = half ? make_float2(r.max_hi, r.sum_hi) : make_float2(r.max_lo, r.sum_lo);
   }
 }
 
@@ -486,6 +484,17 @@ __device__ __forceinline__ void tma_box_4d(void* dst, const CUtensorMap* map, in
       : "memory");
 }
 
+// The same for what is read once and then the first to leave L2: keys and values of a decode step, so that the tile
+// results they give (a fifteenth of their bytes) are still there when they are merged.
+__device__ __forceinline__ void tma_box_4d_once(void* dst, const CUtensorMap* map, int c0, int c2, int c3, uint64_t* bar) {
+  uint64_t policy;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4, %5}], [%6], %7;"
+      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(0), "r"(c2), "r"(c3), "r"(smem_u32(bar)), "l"(policy)
+      : "memory");
+}
+
 // Requests a tile's keys (at sk) and values (kKVBytes behind), given the pages that lanes 0 .. pages_per_tile - 1 hold: a box
 // per page and half of a head, a lane each (a request holds its thread for a hundred cycles).
 __device__ __forceinline__ void request_tile(unsigned char* sk, const CUtensorMap* map_k, const CUtensorMap* map_v, int page,
@@ -495,7 +504,7 @@ __device__ __forceinline__ void request_tile(unsigned char* sk, const CUtensorMa
   const int pg = c / (2 * kHalves), i = (c >> 1) % kHalves;
   const int blk = __shfl_sync(0xffffffffu, my_page, pg);
   if (lane < boxes)
-    tma_box_4d(sk + (c & 1) * kKVBytes + i * kTileKV * 128 + pg * page * 128, (c & 1) ? map_v : map_k, 64 * i, g, blk, bar);
+    tma_box_4d_once(sk + (c & 1) * kKVBytes + i * kTileKV * 128 + pg * page * 128, (c & 1) ? map_v : map_k, 64 * i, g, blk, bar);
 }
 // A row's last tile: values behind its position are whatever the page's last holder left, and their weights are zero; they
 // become zero as well, so that an infinity left there cannot reach the sum.
@@ -520,8 +529,8 @@ __global__ void __launch_bounds__(kStreamWarps * 32)
 attention_stream_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table, int max_blocks,
                         const int* __restrict__ row_seq, const int* __restrict__ pos, int n, int heads, int kv_heads,
-                        int page, int window, float scale_log2, float* __restrict__ tile_out, int max_tiles,
-                        int* failure) {
+                        int page, int window, float scale_log2, float* __restrict__ tile_out, float2* __restrict__ tile_stats,
+                        int max_tiles, int* failure) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = bw::smem_align_1024(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -668,14 +677,12 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     for (int half = 0; half < 2; ++half) {
       const int m = (lane >> 2) + half * 8;
       if (m >= group) continue;
-      float* dst = tile_out + ((static_cast<size_t>(it.row) * heads + (it.g * group + m)) * max_tiles + it.t) * (HD + 2);
+      const size_t rec = (static_cast<size_t>(it.row) * heads + (it.g * group + m)) * max_tiles + it.t;
+      float* dst = tile_out + rec * HD;
 #pragma unroll
       for (int i = 0; i < HD / 8; ++i)
         *reinterpret_cast<float2*>(dst + i * 8 + 2 * (lane & 3)) = make_float2(r.o[i][half * 2], r.o[i][half * 2 + 1]);
-      if ((lane & 3) == 0) {
-        dst[HD] = half ? r.max_hi : r.max_lo;
-        dst[HD + 1] = half ? r.sum_hi : r.sum_lo;
-      }
+      if ((lane & 3) == 0) tile_stats[rec] = half ? make_float2(r.max_hi, r.sum_hi) : make_float2(r.max_lo, r.sum_lo);
     }
   }
 }
@@ -696,8 +703,8 @@ __global__ void __launch_bounds__(32)
 attention_tile_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                           const __nv_bfloat16* __restrict__ qkv, int q_stride, const int* __restrict__ block_table,
                           int max_blocks, const int* __restrict__ row_seq, const int* __restrict__ pos, int heads,
-                          int kv_heads, int page, int window, float scale_log2, float* __restrict__ tile_out, int max_tiles,
-                          int n, int* failure) {
+                          int kv_heads, int page, int window, float scale_log2, float* __restrict__ tile_out,
+                          float2* __restrict__ tile_stats, int max_tiles, int n, int* failure) {
   extern __shared__ __align__(1024) unsigned char tile_raw[];
   unsigned char* base = bw::smem_align_1024(tile_raw);
   unsigned char* sq = base;                  // 16 stacked rows of 128 bytes
@@ -751,52 +758,130 @@ attention_tile_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
   for (int half = 0; half < 2; ++half) {
     const int m = (lane >> 2) + half * 8;
     if (m >= group) continue;
-    float* dst = tile_out + ((static_cast<size_t>(row) * heads + (g * group + m)) * max_tiles + t) * (HD + 2);
+    const size_t rec = (static_cast<size_t>(row) * heads + (g * group + m)) * max_tiles + t;
+    float* dst = tile_out + rec * HD;
 #pragma unroll
     for (int i = 0; i < HD / 8; ++i)
       *reinterpret_cast<float2*>(dst + i * 8 + 2 * (lane & 3)) = make_float2(r.o[i][half * 2], r.o[i][half * 2 + 1]);
-    if ((lane & 3) == 0) {
-      dst[HD] = half ? r.max_hi : r.max_lo;
-      dst[HD + 1] = half ? r.sum_hi : r.sum_lo;
-    }
+    if ((lane & 3) == 0) tile_stats[rec] = half ? make_float2(r.max_hi, r.sum_hi) : make_float2(r.max_lo, r.sum_lo);
   }
 }
 #endif  // BW_HEAD_DIM == 64 || BW_HEAD_DIM == 128
 
-// Second half of split mode: per (row, head) the tile results are merged in ascending tile
-// order with the same formula as in whole mode; thread d carries output element d. The records
-// of up to kMergeBatch tiles are brought into shared memory by all threads together (one
-// round trip to memory instead of one per tile), then each thread walks them in order.
-constexpr int kMergeBatch = (10 * 1024) / (HD + 2) > 64 ? 64 : (10 * 1024) / (HD + 2);  // at most 40 KB of records
-constexpr int kMergeThreads = HD < 64 ? 64 : HD;
+// Second half of split mode: per (row, head) the tile results are merged in ascending tile order with the same formula as in whole
+// mode, by a warp. The running maximum before and after each tile is a prefix maximum (exact in any order), so the lanes form
+// the weights of 32 tiles at a time, a tile each; then the lanes, each with its columns, walk the tiles with two multiply-adds a
+// column and tile. The outputs of a batch of tiles are asked for before the batch before them is used, the first ones before
+// the maxima have arrived. (Threads that each formed all weights for themselves along the walk took 17.2 us for 64 rows x 32 heads
+// of 128 over 900 to 4,090 keys and 4.2 for 8 rows x 32 heads of 64 over 2,048, beyond the kernel
+// before; now 12.4 and 3.8, and with keys and values that leave L2 first, tma_box_4d_once, about 8 and 2.5. A warp that merges when its result is a
+// row's last one, told by a counter, was slower: the fence and the counter hold every tile's block, 122 -> 168 us.)
+constexpr int kMergeWarps = 4;
+constexpr int kMergeVec = HD % 128 == 0 ? 4 : HD % 64 == 0 ? 2 : 1;  // columns of a lane that lie together
+constexpr int kMergeGroups = (HD + 32 * kMergeVec - 1) / (32 * kMergeVec);
+constexpr int kMergeCols = kMergeVec * kMergeGroups;
+constexpr int kMergeBatch = kMergeCols <= 4 ? 8 : 4;  // tiles
 
-__global__ void __launch_bounds__(kMergeThreads)
-merge_tiles_kernel(const float* __restrict__ tile_out, int max_tiles, const int* __restrict__ pos,
-                   __nv_bfloat16* __restrict__ out, int out_stride, int heads, int window) {
-  __shared__ float rec[kMergeBatch * (HD + 2)];
-  const int r = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
-  const int p = pos[r];  // copied before the step began
+__global__ void __launch_bounds__(kMergeWarps * 32)
+merge_tiles_kernel(const float* __restrict__ tile_out, const float2* __restrict__ tile_stats, int max_tiles, const int* __restrict__ pos,
+                   __nv_bfloat16* __restrict__ out, int out_stride, int n, int heads, int window) {
+  const int lane = threadIdx.x & 31;
+  const long long item = static_cast<long long>(blockIdx.x) * kMergeWarps + (threadIdx.x >> 5);
+  const int r = static_cast<int>(item / heads), h = static_cast<int>(item - static_cast<long long>(r) * heads);
+  const int p = r < n ? pos[r] : 0;  // copied before the step began
   const int t_first = (window > 0 && p - window + 1 > 0) ? (p - window + 1) / kTileKV : 0;
-  const int t_last = p / kTileKV;
-  const float* src = tile_out + (static_cast<size_t>(r) * heads + h) * max_tiles * (HD + 2);
+  const int t_end = p / kTileKV + 1;
   bw::pdl_enter();
-  float M = -INFINITY, L = 0.0f, O = 0.0f;
-  for (int t0 = t_first; t0 <= t_last; t0 += kMergeBatch) {
-    const int count = min(kMergeBatch, t_last + 1 - t0);
-    const int floats = count * (HD + 2);
-    const float* from = src + static_cast<size_t>(t0) * (HD + 2);
-    if (t0 > t_first) __syncthreads();  // the previous batch has been read
-    for (int i = d; i < floats; i += kMergeThreads) rec[i] = __ldcg(from + i);
-    __syncthreads();
-    if (d < HD) {
-      for (int t = 0; t < count; ++t) {
-        const float* s0 = rec + t * (HD + 2);
-        const MergeWeights w = merge_weights(M, s0[HD]);
-        M = w.mx, L = merge_value(L, s0[HD + 1], w), O = merge_value(O, s0[d], w);
+  if (r >= n) return;
+  const float* src = tile_out + static_cast<size_t>(item) * max_tiles * HD;
+  const float2* stats = tile_stats + static_cast<size_t>(item) * max_tiles;
+  auto fetch = [&](int t0, float (&v)[kMergeBatch][kMergeCols]) {
+#pragma unroll
+    for (int e = 0; e < kMergeBatch; ++e) {
+#pragma unroll
+      for (int gr = 0; gr < kMergeGroups; ++gr) {
+        const int col = (gr * 32 + lane) * kMergeVec;
+        float* to = &v[e][gr * kMergeVec];
+        const bool ok = t0 + e < t_end && col < HD;
+        const float* from = src + static_cast<size_t>(t0 + e) * HD + col;
+        if (kMergeVec == 4) {
+          const float4 x = ok ? __ldcg(reinterpret_cast<const float4*>(from)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          to[0] = x.x, to[kMergeVec > 1 ? 1 : 0] = x.y, to[kMergeVec > 2 ? 2 : 0] = x.z, to[kMergeVec > 2 ? 3 : 0] = x.w;
+        } else if (kMergeVec == 2) {
+          const float2 x = ok ? __ldcg(reinterpret_cast<const float2*>(from)) : make_float2(0.0f, 0.0f);
+          to[0] = x.x, to[kMergeVec > 1 ? 1 : 0] = x.y;
+        } else {
+          to[0] = ok ? __ldcg(from) : 0.0f;
+        }
       }
     }
+  };
+  float M = -INFINITY, L = 0.0f, O[kMergeCols];
+#pragma unroll
+  for (int i = 0; i < kMergeCols; ++i) O[i] = 0.0f;
+  float now[kMergeBatch][kMergeCols], next[kMergeBatch][kMergeCols];
+  fetch(t_first, now);
+  for (int t0 = t_first; t0 < t_end; t0 += 32) {
+    const int count = min(32, t_end - t0);
+    const float2 st = lane < count ? __ldcg(stats + t0 + lane) : make_float2(-INFINITY, 0.0f);
+    float upto = fmaxf(M, st.x);  // the maximum of everything up to this lane's tile
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const float other = __shfl_up_sync(0xffffffffu, upto, d);
+      if (lane >= d) upto = fmaxf(other, upto);
+    }
+    float before = __shfl_up_sync(0xffffffffu, upto, 1);
+    if (lane == 0) before = M;
+    const MergeWeights w = merge_weights(before, st.x);
+    M = __shfl_sync(0xffffffffu, upto, 31);
+    for (int u0 = 0; u0 < count; u0 += kMergeBatch) {
+      fetch(t0 + u0 + kMergeBatch, next);
+#pragma unroll
+      for (int e = 0; e < kMergeBatch; ++e) {
+        MergeWeights we;
+        we.a = __shfl_sync(0xffffffffu, w.a, u0 + e), we.b = __shfl_sync(0xffffffffu, w.b, u0 + e), we.mx = 0.0f;
+        const float sum = __shfl_sync(0xffffffffu, st.y, u0 + e);
+        if (u0 + e < count) {
+          L = merge_value(L, sum, we);
+#pragma unroll
+          for (int i = 0; i < kMergeCols; ++i) O[i] = merge_value(O[i], now[e][i], we);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < kMergeBatch; ++e)
+#pragma unroll
+        for (int i = 0; i < kMergeCols; ++i) now[e][i] = next[e][i];
+    }
   }
-  if (d < HD) out[static_cast<size_t>(r) * out_stride + h * HD + d] = __float2bfloat16_rn(__fmul_rn(O, __fdiv_rn(1.0f, L)));
+  const float inv = __fdiv_rn(1.0f, L);
+  __nv_bfloat16* dst = out + static_cast<size_t>(r) * out_stride + h * HD;
+  const bool wide = kMergeVec > 1 && (reinterpret_cast<uintptr_t>(dst) & (2 * kMergeVec - 1)) == 0;
+#pragma unroll
+  for (int gr = 0; gr < kMergeGroups; ++gr) {
+    const int col = (gr * 32 + lane) * kMergeVec;
+    if (col >= HD) continue;
+    __align__(8) __nv_bfloat16 v[kMergeVec];
+#pragma unroll
+    for (int i = 0; i < kMergeVec; ++i) v[i] = __float2bfloat16_rn(__fmul_rn(O[gr * kMergeVec + i], inv));
+    if (wide && kMergeVec == 4)
+      *reinterpret_cast<uint2*>(dst + col) = *reinterpret_cast<const uint2*>(v);
+    else if (wide && kMergeVec == 2)
+      *reinterpret_cast<uint32_t*>(dst + col) = *reinterpret_cast<const uint32_t*>(v);
+    else
+#pragma unroll
+      for (int i = 0; i < kMergeVec; ++i) dst[col + i] = v[i];
+  }
+}
+
+// Tile results of n rows in the caller's scratch (bw_bf16_attention_scratch_floats), and their merge.
+float2* stats_of(float* scratch, int n, int heads, int key_tiles) {
+  return reinterpret_cast<float2*>(scratch + static_cast<size_t>(n) * heads * key_tiles * HD);
+}
+void launch_merge(float* scratch, int key_tiles, const int* pos, __nv_bfloat16* out, int out_stride, int n, int heads, int window,
+                  cudaStream_t stream) {
+  const long long items = static_cast<long long>(n) * heads;
+  bw::launch_pdl(merge_tiles_kernel, dim3(static_cast<unsigned>((items + kMergeWarps - 1) / kMergeWarps)), dim3(kMergeWarps * 32), 0, stream,
+                 scratch, stats_of(scratch, n, heads, key_tiles), key_tiles, pos, out, out_stride, n, heads, window);
 }
 
 }  // namespace
@@ -854,8 +939,8 @@ BW_API int bw_bf16_attention(const __nv_bfloat16* qkv, int q_stride, const __nv_
       configured[1] = true;
     }
     bw::launch_pdl(attention_split_kernel, dim3(dim3(n, kv_heads, (key_tiles + kSplitWarps - 1) / kSplitWarps)), dim3(kSplitWarps * 32), split_smem, stream, qkv, q_stride, kcache, vcache, block_table, max_blocks, row_seq, pos, heads,
-                                       kv_heads, page, page_shift, window, scale_log2, scratch, key_tiles);
-    bw::launch_pdl(merge_tiles_kernel, dim3(dim3(n, heads)), dim3(kMergeThreads), 0, stream, scratch, key_tiles, pos, out, out_stride, heads, window);
+                                       kv_heads, page, page_shift, window, scale_log2, scratch, stats_of(scratch, n, heads, key_tiles), key_tiles);
+    launch_merge(scratch, key_tiles, pos, out, out_stride, n, heads, window, stream);
   } else {
     constexpr int smem = kQBytes + kStages * 2 * kKVBytes;
     if (!configured[0]) {
@@ -964,9 +1049,8 @@ BW_API int bw_bf16_attention_stream(const __nv_bfloat16* qkv, int q_stride, cons
     const int slices = (key_tiles + kTileGridZ - 1) / kTileGridZ;
     bw::launch_pdl(attention_tile_tma_kernel, dim3(n * slices, kv_heads, key_tiles < kTileGridZ ? key_tiles : kTileGridZ), dim3(32),
                    tile_smem, stream, map_k, map_v, qkv, q_stride, block_table, max_blocks, row_seq, pos, heads, kv_heads, page, window,
-                   scale_log2, scratch, key_tiles, n, word);
-    bw::launch_pdl(merge_tiles_kernel, dim3(dim3(n, heads)), dim3(kMergeThreads), 0, stream, scratch, key_tiles, pos, out,
-                   out_stride, heads, window);
+                   scale_log2, scratch, stats_of(scratch, n, heads, key_tiles), key_tiles, n, word);
+    launch_merge(scratch, key_tiles, pos, out, out_stride, n, heads, window, stream);
     return bw::launch_status();
   }
 #if BW_HEAD_DIM == 64
@@ -1001,10 +1085,9 @@ BW_API int bw_bf16_attention_stream(const __nv_bfloat16* qkv, int q_stride, cons
   const unsigned grid = static_cast<unsigned>(
       items < static_cast<long long>(sms) * kStreamWarps ? (items + kStreamWarps - 1) / kStreamWarps : sms);
   bw::launch_pdl(attention_stream_kernel, dim3(grid), dim3(kStreamWarps * 32), smem, stream, map_q, map_k, map_v,
-                 block_table, max_blocks, row_seq, pos, n, heads, kv_heads, page, window, scale_log2, scratch, key_tiles,
-                 word);
-  bw::launch_pdl(merge_tiles_kernel, dim3(dim3(n, heads)), dim3(kMergeThreads), 0, stream, scratch, key_tiles, pos, out,
-                 out_stride, heads, window);
+                 block_table, max_blocks, row_seq, pos, n, heads, kv_heads, page, window, scale_log2, scratch,
+                 stats_of(scratch, n, heads, key_tiles), key_tiles, word);
+  launch_merge(scratch, key_tiles, pos, out, out_stride, n, heads, window, stream);
   return bw::launch_status();
 #else
   return -1;

@@ -1280,3 +1280,25 @@ def test_a_bounded_wait_that_runs_out_raises_the_failure_word_once():
     ref = x.double() @ w.double().t()
     assert float((y.double() - ref).abs().max()) <= 1e-3 * float(ref.abs().max())
     assert not ops.device_failure()
+
+
+@pytest.mark.parametrize("hd,heads,kv_heads,page,window", [(64, 4, 2, 16, 0), (64, 4, 2, 8, 700), (128, 8, 2, 16, 0), (32, 3, 1, 16, 0), (80, 4, 4, 16, 90),
+                                                           (256, 2, 1, 16, 0), (48, 4, 1, 16, 0)])
+def test_bf16_attention_decode_merge_of_any_number_of_tiles(hd, heads, kv_heads, page, window):
+    """Rows of 1 to 70 key tiles (whole and partial groups of 32, batches that end early), every width a lane can hold: the bits of
+    the kernel that walks a row's tiles in one block; and an output that starts on two bytes only."""
+    rng = np.random.default_rng(hd)
+    ops = _ops("bfloat16")
+    lens = [1, 64, 65, 15 * 64 + 3, 16 * 64, 17 * 64 - 1, 31 * 64 + 1, 32 * 64, 33 * 64 + 5, 70 * 64 - 7]
+    k, v, table, _, _ = _paged(rng, lens, kv_heads, hd, page)
+    rows = [(n - 1, 1) for n in lens]
+    q = bf(rnd(rng, len(lens), heads, hd))
+    k, v = bf(k), bf(v)
+    split, _, _ = _run_bf16_attention(q, rows, k, v, table, heads, kv_heads, hd, window)
+    # the same rows as ends of portions of two are no decode step: they run whole
+    at = [(n - 2, 2) if n > 1 else (0, 1) for n in lens]
+    q2 = np.concatenate([np.concatenate([q[i:i + 1]] * c) for i, (_, c) in enumerate(at)])
+    whole, _, _ = _run_bf16_attention(q2, at, k, v, table, heads, kv_heads, hd, window)
+    last = np.cumsum([c for _, c in at]) - 1
+    assert_same_bits(split, whole[last], f"head size {hd}")
+    assert not ops.device_failure()
