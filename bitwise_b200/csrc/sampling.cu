@@ -204,17 +204,17 @@ sample_rows_kernel(const float* __restrict__ logits, int vocab, const float* __r
   if (tid == 0) out_token[row] = (s_pick != 0x7fffffff) ? s_pick : s_last;
 }
 
-// The same for larger vocabularies, a cluster of eight blocks per row. What bounds it is latency: a row is a stream of logits
-// and two serial sums in 64 bits (within a segment, and over the segments), of hundreds of dependent additions each. Each
-// block brings the logits of 64 of the 512 segments into shared memory with coalesced reads and forms the weights in place.
-// The sums are then taken as trees, by warps. They differ from the serial ones by rounding only, and the bound on that
+// The same for larger vocabularies, a cluster of eight blocks per row, each with 64 of the 512 segments. What bounds it is
+// latency: a row is a stream of logits and two serial sums in 64 bits (within a segment, and over the segments), of hundreds
+// of dependent additions each. The logits are read twice, for the maximum 16 bytes a lane and for the weights a segment a warp; the
+// head has just written them, so both come from L2. (Kept in shared memory in between, a block of 128,256 logits took 64 KB, and 64
+// rows did not run at once.) The sums are taken as trees, by warps. They differ from the serial ones by rounding only, and the bound on that
 // difference is known, so the token is the serial kernel's wherever the target lies further than the bound from the two
 // running sums it falls between. Where it does not (a uniform number of 0 or nearly 1, a logit that is no number, or a chance
 // of some 1e-9 a row) the row is done again with one thread per segment and every sum in the serial kernel's order.
-// Head and sampler together for 64 rows of 128,256 logits, half of them greedy: 550 us with a block per row and serial sums,
-// 258 us with serial sums here, 229 us with trees (the product alone takes 185 us). The sampler alone: 64 rows 71 -> 39 us, one
-// row of 49,152 23 -> 12 us.
-constexpr int kSampleBlocks = 8, kSampleBlockThreads = 256, kSegmentsPerBlock = kSampleThreads / kSampleBlocks;
+// The sampler alone, us, all rows greedy and all at a temperature: 64 rows of 128,256 logits 16.3 -> 8.5, 48.7 -> 30.8; one row 6.1 ->
+// 4.6, 19.4 -> 13; 64 rows of 32,000 7.2 -> 5.7, 17.9 -> 14.8; one row of 49,152 3.5 -> 3.8, 9.8 -> 9.1.
+constexpr int kSampleBlocks = 8, kSegmentsPerBlock = kSampleThreads / kSampleBlocks;
 
 __device__ __forceinline__ void sample_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -246,10 +246,12 @@ __device__ __forceinline__ bool sample_better(float v, int i, float best, int be
   return i >= 0 && (best_i < 0 || v > best || (v == best && i < best_i));
 }
 
-__global__ void __launch_bounds__(kSampleBlockThreads)
+// With 256 threads the 512 blocks of 64 rows run at once (64 registers); up to 8 rows take 512 threads (8 rows of 49,152 10.7 -> 9.4 us
+// at a temperature; 16 rows 10.5 -> 15.6: one such block fits an SM, and not every cluster finds eight).
+template <int kSampleBlockThreads>
+__global__ void __launch_bounds__(kSampleBlockThreads, kSampleBlockThreads == 256 ? 4 : 1)
 sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
                            const double* __restrict__ uniform, int* __restrict__ out_token) {
-  extern __shared__ float seg_values[];  // [kSegmentsPerBlock][seg]
   constexpr int kWarps = kSampleBlockThreads / 32;
   __shared__ float w_val[kWarps];
   __shared__ int w_idx[kWarps];
@@ -270,16 +272,42 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
   if (tid == 0) b_pick = 0x7fffffff;
   bw::pdl_enter();
 
-  // the logits of this block's segments, and their maximum
+  // the maximum of this block's segments and its first index: single logits up to 16 bytes' alignment, fours, and the rest
   float best = -INFINITY;
   int best_i = -1;
   const int first = min(vocab, seg0 * seg), count = min(vocab, (seg0 + kSegmentsPerBlock) * seg) - first;
-#pragma unroll 8
-  for (int j = tid; j < count; j += kSampleBlockThreads) {
-    const float v = l[first + j];
-    seg_values[j] = v;
-    if (v > best || (best_i < 0 && v == v)) best = v, best_i = first + j;  // a thread's indices come in increasing order
+  const float* mine = l + first;
+  auto see = [&](float v, int j) {  // a thread's indices come in increasing order
+    if (v > best || (best_i < 0 && v == v)) best = v, best_i = first + j;
+  };
+  const int lead = min(count, static_cast<int>((16u - (reinterpret_cast<uintptr_t>(mine) & 15u)) & 15u) / 4);
+  const int fours = (count - lead) / 4;
+  if (tid < lead) see(mine[tid], tid);
+  {
+    const float4* m4 = reinterpret_cast<const float4*>(mine + lead);
+    constexpr int kAhead = 8;
+    int q = tid;
+    for (; q + (kAhead - 1) * kSampleBlockThreads < fours; q += kAhead * kSampleBlockThreads) {
+      float4 v[kAhead];
+#pragma unroll
+      for (int e = 0; e < kAhead; ++e) v[e] = m4[q + e * kSampleBlockThreads];
+#pragma unroll
+      for (int e = 0; e < kAhead; ++e) {
+        const int j = lead + 4 * (q + e * kSampleBlockThreads);
+        see(v[e].x, j), see(v[e].y, j + 1), see(v[e].z, j + 2), see(v[e].w, j + 3);
+      }
+    }
+    float4 v[kAhead];
+#pragma unroll
+    for (int e = 0; e < kAhead; ++e)
+      v[e] = q + e * kSampleBlockThreads < fours ? m4[q + e * kSampleBlockThreads] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+#pragma unroll
+    for (int e = 0; e < kAhead; ++e) {
+      const int j = lead + 4 * (q + e * kSampleBlockThreads);
+      if (q + e * kSampleBlockThreads < fours) see(v[e].x, j), see(v[e].y, j + 1), see(v[e].z, j + 2), see(v[e].w, j + 3);
+    }
   }
+  if (tid < count - lead - 4 * fours) see(mine[lead + 4 * fours + tid], lead + 4 * fours + tid);
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, d);
@@ -291,8 +319,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
   if (tid == 0) {
     for (int w = 1; w < kWarps; ++w)
       if (sample_better(w_val[w], w_idx[w], best, best_i)) best = w_val[w], best_i = w_idx[w];
-    const float head = seg_values[0];  // (this thread's own store)
-    if (rank == 0 && head != head) best = head, best_i = 0;
+    if (rank == 0 && l[0] != l[0]) best = l[0], best_i = 0;
     b_val = best, b_idx = best_i;
   }
   sample_cluster_sync();
@@ -311,29 +338,46 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
     return;
   }
 
-  // the weights, in place, and the sum of every segment
-  for (int s = warp; s < kSegmentsPerBlock; s += kWarps) {
-    const int len = max(0, min(seg, count - s * seg));
-    float* v = seg_values + s * seg;
-    double local = 0.0;
-#pragma unroll 4
-    for (int j = lane; j < len; j += 32) {
-      const float w = sample_weight(v[j], mx, temp);
-      v[j] = w;
-      local += static_cast<double>(w);
+  // the sum of the weights of every segment, four segments of a warp at a time
+  constexpr int kTogether = 4, kAhead = 4;  // segments, and logits of each that a lane asks for together
+  static_assert(kSegmentsPerBlock % (kTogether * kWarps) == 0, "a warp's segments come in fours");
+  for (int s = kTogether * warp; s < kSegmentsPerBlock; s += kTogether * kWarps) {
+    double sum[kTogether];
+#pragma unroll
+    for (int k = 0; k < kTogether; ++k) sum[k] = 0.0;
+    for (int j0 = lane; j0 < seg; j0 += 32 * kAhead) {
+      float x[kTogether][kAhead];
+#pragma unroll
+      for (int k = 0; k < kTogether; ++k) {
+        const int len = min(seg, count - (s + k) * seg);  // (negative behind the vocabulary's end)
+#pragma unroll
+        for (int e = 0; e < kAhead; ++e) x[k][e] = j0 + 32 * e < len ? mine[(s + k) * seg + j0 + 32 * e] : -INFINITY;
+      }
+#pragma unroll
+      for (int k = 0; k < kTogether; ++k) {
+        const int len = min(seg, count - (s + k) * seg);
+#pragma unroll
+        for (int e = 0; e < kAhead; ++e)
+          if (j0 + 32 * e < len) sum[k] += static_cast<double>(sample_weight(x[k][e], mx, temp));
+      }
     }
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) local += __shfl_xor_sync(0xffffffffu, local, d);
-    if (lane == 0) b_sum[s] = local;
+    for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+      for (int k = 0; k < kTogether; ++k) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], d);
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < kTogether; ++k) b_sum[s + k] = sum[k];
   }
   sample_cluster_sync();
 
-  // what lies before every segment (two segments a thread)
-  static_assert(kSampleThreads == 2 * kSampleBlockThreads && kSegmentsPerBlock % 2 == 0, "a pair lies in one block");
+  // what lies before every segment
+  constexpr int kPerThread = kSampleThreads / kSampleBlockThreads;
+  static_assert((kPerThread == 1 || kPerThread == 2) && kSegmentsPerBlock % 2 == 0, "a thread's segments lie in one block");
   {
-    const int t = 2 * tid;
+    const int t = kPerThread * tid;
     const double v0 = sample_peer_double(&b_sum[t % kSegmentsPerBlock], t / kSegmentsPerBlock);
-    const double v1 = sample_peer_double(&b_sum[t % kSegmentsPerBlock + 1], t / kSegmentsPerBlock);
+    const double v1 = kPerThread == 2 ? sample_peer_double(&b_sum[t % kSegmentsPerBlock + 1], t / kSegmentsPerBlock) : 0.0;
     double run = v0 + v1;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -351,7 +395,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
       sum += w_sum[w];
     }
     all_sum[t] = base + before;
-    all_sum[t + 1] = base + before + v0;
+    if (kPerThread == 2) all_sum[t + 1] = base + before + v0;
     if (tid == 0) total = sum;
   }
   __syncthreads();
@@ -370,8 +414,8 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
       if (tid == 0) b_pick = -1;
     } else if (candidates == 1 && warp == 0) {
       const int s = b_last[0], len = max(0, min(seg, count - s * seg));
-      const float* v = seg_values + s * seg;
-      const int at = sample_scan(len, [&](int j) { return v[j]; }, all_sum[seg0 + s], target, near, lane);
+      const float* v = mine + s * seg;
+      const int at = sample_scan(len, [&](int j) { return sample_weight(v[j], mx, temp); }, all_sum[seg0 + s], target, near, lane);
       if (lane == 0) b_pick = at < 0 ? -1 : first + s * seg + at;
     }
   }
@@ -389,13 +433,12 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
 
   // near a running sum: one thread per segment, every sum in order
   const int my_lo = min(vocab, (seg0 + tid) * seg), my_len = tid < kSegmentsPerBlock ? min(vocab, my_lo + seg) - my_lo : 0;
-  const float* mine = seg_values + tid * seg;
+  const float* own = mine + (my_lo - first);
   if (tid < kSegmentsPerBlock) {
     double local = 0.0;
     int last_pos = -1;
-#pragma unroll 8
     for (int j = 0; j < my_len; ++j) {
-      const float w = mine[j];
+      const float w = sample_weight(own[j], mx, temp);
       if (w > 0.0f) last_pos = my_lo + j;
       local += static_cast<double>(w);
     }
@@ -425,7 +468,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, int vocab, const fl
     const double target = uniform[row] * total;
     double cum = all_sum[seg0 + tid];
     for (int j = 0; j < my_len; ++j) {
-      const float w = mine[j];
+      const float w = sample_weight(own[j], mx, temp);
       if (w <= 0.0f) continue;
       cum += static_cast<double>(w);
       if (cum > target) {
@@ -466,29 +509,19 @@ BW_API int bw_sample_rows(const float* logits, int rows, int vocab, const float*
     bw::set_error("sample_rows: vocabulary size %d", vocab);
     return -1;
   }
-  // A cluster per row where the blocks of all rows run at once or nearly so, the row is long enough for eight blocks to gain on
-  // one, and the segments fit into shared memory. Beyond that a block per row is as fast or faster. Cluster / block, us, all rows
-  // greedy and all rows at a temperature: 1 row of 8,192 logits 5.6 / 4.2, 10.3 / 8.3; 16,000: 6.2 / 6.2, 10.3 / 12.4;
-  // 128,256: 8.3 / 12.4, 21.2 / 58.9; 64 rows of 16,000: 8.3 / 6.2, 14.4 / 12.8; 49,152: 8.3 / 8.2, 18.5 / 26.7; 128,256: 24.1 /
-  // 26.7, 56.5 / 66.8; 128 rows of 49,152: 12.4 / 8.3, 29.1 / 26.9; 512 rows of 8,192: 28.8 / 6.3, 65.6 / 16.6.
-  constexpr int kClusterVocab = 12288, kLongVocab = 24576, kMaxSmem = 200 * 1024, kMaxDevices = 64;
-  const int seg = (vocab + kSampleThreads - 1) / kSampleThreads;
-  const long long smem = 4ll * kSegmentsPerBlock * seg;
-  const bool cluster = g_sample_kernel == 2 || (g_sample_kernel == 0 && vocab >= kClusterVocab && rows <= (vocab >= kLongVocab ? 64 : 32));
-  if (cluster && smem <= kMaxSmem && rows <= 0x7fffffff / kSampleBlocks) {
-    static bool configured[kMaxDevices] = {false};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = 0;
-    if (!configured[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(sample_rows_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-      if (e != cudaSuccess) {
-        bw::set_error("sample_rows: cannot raise shared memory: %s", cudaGetErrorString(e));
-        return static_cast<int>(e);
-      }
-      configured[dev] = true;
-    }
-    bw::launch_pdl_cluster(kSampleBlocks, sample_rows_cluster_kernel, dim3(static_cast<unsigned>(rows) * kSampleBlocks),
-                           dim3(kSampleBlockThreads), static_cast<size_t>(smem), stream, logits, vocab, temperature, uniform, out_token);
+  // A cluster per row where the blocks of all rows run at once or nearly so and the row is long enough for eight blocks to gain on
+  // one. Beyond that a block per row is as fast or faster. Cluster / block, us, all rows greedy
+  // and all rows at a temperature: 1 row of 16,000 logits 3.5 / 4.4, 7.2 / 11.0; 1 of 128,256 4.6 / 10.2, 13 / 57; 64 rows of 16,000 5.4 /
+  // 4.6, 12.6 / 11.4; of 32,000 5.7 / 5.9, 14.8 / 17.4; of 128,256 8.5 / 15.4, 30.8 / 63.7; 128 rows of 49,152 11.0 / 8.7, 31.3 / 31.5;
+  // of 128,256 15.4 / 18.4, 56 / 75; 512 rows of 32,000 35.5 / 11.2, 94 / 44; 1 row of 8,192 was 5.6 / 4.2, 10.3 / 8.3.
+  constexpr int kClusterVocab = 12288, kLongVocab = 24576, kLongestVocab = 98304, kFewRows = 8;
+  const int most = vocab >= kLongestVocab ? 128 : vocab >= kLongVocab ? 64 : 32;
+  const bool cluster = g_sample_kernel == 2 || (g_sample_kernel == 0 && vocab >= kClusterVocab && rows <= most);
+  if (cluster && rows <= 0x7fffffff / kSampleBlocks) {
+    const bool few = rows <= kFewRows;
+    bw::launch_pdl_cluster(kSampleBlocks, few ? sample_rows_cluster_kernel<512> : sample_rows_cluster_kernel<256>,
+                           dim3(static_cast<unsigned>(rows) * kSampleBlocks), dim3(few ? 512 : 256), 0, stream, logits, vocab, temperature,
+                           uniform, out_token);
     return bw::launch_status();
   }
   bw::launch_pdl(sample_rows_kernel, dim3(rows), dim3(kSampleThreads), 0, stream, logits, vocab, temperature, uniform, out_token);

@@ -1302,3 +1302,29 @@ def test_bf16_attention_decode_merge_of_any_number_of_tiles(hd, heads, kv_heads,
     last = np.cumsum([c for _, c in at]) - 1
     assert_same_bits(split, whole[last], f"head size {hd}")
     assert not ops.device_failure()
+
+
+@pytest.mark.parametrize("rows", [8, 9, 40])
+@pytest.mark.parametrize("vocab", [12289, 16386, 49152, 98307])
+def test_sample_rows_clusters_of_either_size_over_rows_of_any_start(rows, vocab):
+    """Up to eight rows and more take blocks of other sizes; rows of an odd vocabulary start anywhere.  The block kernel's tokens,
+    with ties of the maximum and logits that are no number at a segment's edges, greedy and at temperatures."""
+    ops = _ops("bfloat16")
+    gen = torch.Generator(device=DEV).manual_seed(rows * vocab)
+    logits = torch.randn(rows, vocab, generator=gen, device=DEV) * 3
+    seg = (vocab + 511) // 512
+    logits[1, 64 * seg - 1] = logits[1, 64 * seg] = logits[1, vocab - 1] = 40.0
+    logits[2, 0] = float("nan")
+    logits[3, 3 * seg:3 * seg + 5] = float("nan")
+    temperature = torch.tensor([(0.0, 0.7, 1.3)[i % 3] for i in range(rows)], device=DEV)
+    uniform = torch.rand(rows, generator=gen, dtype=torch.float64, device=DEV)
+    got = {}
+    for kernel in (1, 2):
+        before = ops.sampler_kernel(kernel)
+        try:
+            out = torch.full((rows,), -1, dtype=torch.int32, device=DEV)
+            ops.sample_rows(logits, temperature, uniform, out)
+        finally:
+            ops.sampler_kernel(before)
+        got[kernel] = out.tolist()
+    assert got[1] == got[2] and min(got[1]) >= 0
