@@ -35,7 +35,41 @@ def _p(t: Optional[torch.Tensor]):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
 
+def _a(t: Optional[torch.Tensor]) -> Optional[int]:
+    """A tensor's address, for a function whose argument types are declared (_SIGNATURES)."""
+    return None if t is None else t.data_ptr()
+
+
+# Argument types of the functions that a step calls for every layer: p an address, i int, q long long, f float. Plain numbers
+# go through declared types in half the time that building a ctypes object for each of them took (a decode step's attention layer
+# called part by part is five launches and twice as many microseconds in Python).
+_KINDS = {"p": ctypes.c_void_p, "i": ctypes.c_int, "q": ctypes.c_longlong, "f": ctypes.c_float}
+_SIGNATURES = {
+    "bw_bf16_linear": "ppp i p iii pp i p",
+    "bw_bf16_linear_tc_swiglu": "ppp iii p i p",
+    "bw_bf16_linear_rows_rope": "ppp iii ppppp i pp iiiii pp",
+    "bw_bf16_attention": "p i ppp i ppp i pppp p iiiiiii f i pp",
+    "bw_bf16_attention_tc": "p i pp i p i ppp i pp p iiiiiii f p",
+    "bw_bf16_attention_stream": "p i pp i p i pp p iiiiiii f i pp",
+    "bw_bf16_attention_stream_usable": "iiiiii",
+    "bw_f32_linear": "pppp iii p",
+    "bw_f32_attention": "p i ppp i pp ppp i pp p iiiiiiii f p q p",
+    "bw_sample_rows": "p ii ppp p",
+}
+for _k in ("f32", "bf16"):
+    _SIGNATURES.update({f"bw_{_k}_rmsnorm": "pppp ii f p", f"bw_{_k}_rope_cache": "p i ppppp i pp iiiiii p", f"bw_{_k}_swiglu": "pp ii p"})
+
+
+def _declare(lib, names) -> None:
+    for name in names:
+        if hasattr(lib, name):
+            fn = getattr(lib, name)
+            fn.restype, fn.argtypes = ctypes.c_int, [_KINDS[c] for c in _SIGNATURES[name] if c != " "]
+
+
 def _need(t: torch.Tensor, dtype, what: str, dims: Optional[int] = None) -> None:
+    if t.is_cuda and t.dtype is dtype and t.is_contiguous() and (dims is None or t.dim() == dims):
+        return
     if not t.is_cuda:
         raise KernelError(f"{what}: tensor is on {t.device}; the kernels run on a CUDA device only")
     if t.dtype != dtype:
@@ -120,6 +154,12 @@ class KernelOps:
             return ctypes.c_void_p(_raw_stream(self._device_index()))
         return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
+    def _stream_handle(self) -> int:
+        """The same as a number, for functions whose argument types are declared."""
+        if _raw_stream is not None and self._dev_index is not None:
+            return _raw_stream(self._dev_index)
+        return self._stream().value or 0
+
     def _device_index(self) -> int:
         if self._dev_index is None:
             self._dev_index = torch.cuda.current_device()
@@ -135,9 +175,13 @@ class KernelOps:
         if fn is None:
             fn = getattr(lib or self.lib, name)
             fn.restype = _c_int
+            if lib is None and name in _SIGNATURES:
+                _declare(self.lib, (name,))
             if lib is None:
                 self._fns[name] = fn
-        self._check(fn(*args), name)
+        rc = fn(*args)
+        if rc != 0:
+            self._check(rc, name)
         self.launches += launches
 
     # -- shared kernels ----------------------------------------------------------------
@@ -167,8 +211,7 @@ class KernelOps:
         _need(temperature, torch.float32, "sample_rows temperature")
         _need(uniform, torch.float64, "sample_rows uniform")
         _need(out_tokens, torch.int32, "sample_rows out")
-        self._call("bw_sample_rows", _p(logits), _c_int(rows), _c_int(vocab), _p(temperature), _p(uniform),
-                   _p(out_tokens), self._stream())
+        self._call("bw_sample_rows", _a(logits), rows, vocab, _a(temperature), _a(uniform), _a(out_tokens), self._stream_handle())
 
     def sampler_kernel(self, kernel: int = 0) -> int:
         """Tests and measurements: which kernel samples (0 chosen from the sizes, 1 a block per row, 2 a cluster per row where the
@@ -196,8 +239,8 @@ class KernelOps:
             raise KernelError("rmsnorm: widths differ")
         if rows is not None:
             _need(rows, torch.int32, "rmsnorm rows")
-        self._call(f"bw_{self.kind}_rmsnorm", _p(x), _p(weight), _p(out), _p(rows), _c_int(n), _c_int(width),
-                   _c_float(eps), self._stream())
+        self._call("bw_f32_rmsnorm" if self.kind == "f32" else "bw_bf16_rmsnorm", _a(x), _a(weight), _a(out), _a(rows), n, width, eps,
+                   self._stream_handle())
 
     def linear(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor,
                residual: Optional[torch.Tensor] = None, legacy: bool = False, activation: Optional[str] = None,
@@ -234,8 +277,7 @@ class KernelOps:
                 raise KernelError("linear: residual shape differs from the output's")
         if self.kind == "f32":
             _need(out, torch.float32, "linear out", 2)
-            self._call("bw_f32_linear", _p(x), _p(w), _p(out), _p(residual), _c_int(m), _c_int(n), _c_int(k),
-                       self._stream())
+            self._call("bw_f32_linear", _a(x), _a(w), _a(out), _a(residual), m, n, k, self._stream_handle())
             if act:
                 self.activate_rows(out, out, activation)
         else:
@@ -243,9 +285,8 @@ class KernelOps:
                 raise KernelError("linear: out must be float32 or bfloat16")
             _need(out, out.dtype, "linear out", 2)
             partials, counters = self._linear_scratch(x.device, n, k) if m <= self._split_rows else (self._cut_scratch(x.device), None)
-            self._call("bw_bf16_linear", _p(x), _p(w), _p(out), _c_int(2 * act + int(out.dtype == torch.float32)),
-                       _p(residual), _c_int(m), _c_int(n), _c_int(k), _p(partials), _p(counters),
-                       _c_int(int(legacy)), self._stream(),
+            self._call("bw_bf16_linear", _a(x), _a(w), _a(out), 2 * act + int(out.dtype == torch.float32), _a(residual), m, n, k,
+                       _a(partials), _a(counters), int(legacy), self._stream_handle(),
                        launches=1 if legacy else self._linear_kernels(m, n, k, False, counters is not None and partials is not None))
 
     def _linear_then(self, x, w, out, residual, then) -> bool:
@@ -298,8 +339,8 @@ class KernelOps:
             raise KernelError("linear_swiglu: unsupported shapes or precision")
         split = m <= self._split_rows
         partials = self._linear_scratch(x.device, n, k)[0] if split else self._cut_scratch(x.device)
-        self._call("bw_bf16_linear_tc_swiglu", _p(x), _p(w_interleaved), _p(out), _c_int(m), _c_int(n), _c_int(k),
-                   _p(partials), _c_int(self.FUSED_ACTIVATIONS.index(activation)), self._stream(),
+        self._call("bw_bf16_linear_tc_swiglu", _a(x), _a(w_interleaved), _a(out), m, n, k, _a(partials),
+                   self.FUSED_ACTIVATIONS.index(activation), self._stream_handle(),
                    launches=self._linear_kernels(m, n, k, True, split and partials is not None))
 
     def _linear_kernels(self, m: int, n: int, k: int, swiglu: bool, scratch: bool) -> int:
@@ -477,9 +518,8 @@ class KernelOps:
     def _attention_scratch(self, lib, device, n: int, heads: int, max_keys: int) -> torch.Tensor:
         """Scratch of the split attention: one (output, maximum, sum) record per row, head and
         tile of 64 keys.  Sized for contexts rounded up to 2048 keys so that it seldom grows."""
-        lib.bw_bf16_attention_scratch_floats.restype = ctypes.c_longlong
         keys = (max_keys + 2047) // 2048 * 2048
-        floats = int(lib.bw_bf16_attention_scratch_floats(_c_int(n), _c_int(heads), _c_int(keys)))
+        floats = lib.bw_bf16_attention_scratch_floats(n, heads, keys)
         if self._attn_scratch is None or self._attn_scratch.numel() < floats:
             self._retired.append(self._attn_scratch)  # a captured graph may still point at the old one
             self._attn_scratch = torch.empty(floats, dtype=torch.float32, device=device)
@@ -494,6 +534,8 @@ class KernelOps:
             except OSError as e:
                 raise KernelError(f"cannot load the attention library {path}: {e}") from None
             lib.bw_last_error.restype = ctypes.c_char_p
+            lib.bw_bf16_attention_scratch_floats.restype = ctypes.c_longlong
+            _declare(lib, ("bw_bf16_attention", "bw_bf16_attention_tc", "bw_bf16_attention_stream", "bw_bf16_attention_stream_usable"))
             if self._failure_word is not None:
                 lib.bw_set_failure_word(_p(self._failure_word))
             self._attn_libs[head_dim] = lib
@@ -521,10 +563,9 @@ class KernelOps:
             _need(sin, torch.float32, "rope_cache sin", 2)
             if cos.shape[1] != head_dim // 2 or cos.shape != sin.shape:
                 raise KernelError("rope_cache: table width is not head_dim / 2")
-        self._call(f"bw_{self.kind}_rope_cache", _p(qkv), _c_int(qkv.shape[1]), _p(pos), _p(row_seq), _p(cos),
-                   _p(sin), _p(block_table), _c_int(block_table.shape[1]), _p(kcache), _p(vcache), _c_int(n),
-                   _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(kcache.shape[2]),
-                   _c_int(int(write_kv)), self._stream())
+        self._call(f"bw_{self.kind}_rope_cache", _a(qkv), qkv.shape[1], _a(pos), _a(row_seq), _a(cos), _a(sin), _a(block_table),
+                   block_table.shape[1], _a(kcache), _a(vcache), n, heads, kv_heads, head_dim, kcache.shape[2], int(write_kv),
+                   self._stream_handle())
 
     def fuses_rope(self, m: int, width: int, heads: int, kv_heads: int, head_dim: int) -> bool:
         """Whether ``linear_rope_cache`` takes a step of m rows: then the fused q/k/v product
@@ -568,10 +609,9 @@ class KernelOps:
             _need(sin, torch.float32, "linear_rope_cache sin", 2)
             if cos.shape[1] != head_dim // 2 or cos.shape != sin.shape:
                 raise KernelError("linear_rope_cache: table width is not head_dim / 2")
-        self._call("bw_bf16_linear_rows_rope", _p(x), _p(w_qkv), _p(qkv), _c_int(m), _c_int(n), _c_int(k), _p(pos),
-                   _p(row_seq), _p(cos), _p(sin), _p(block_table), _c_int(block_table.shape[1]), _p(kcache), _p(vcache),
-                   _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(kcache.shape[2]), _c_int(int(write_kv)),
-                   _p(self._cut_scratch(x.device) if m > self._split_rows else None), self._stream())
+        self._call("bw_bf16_linear_rows_rope", _a(x), _a(w_qkv), _a(qkv), m, n, k, _a(pos), _a(row_seq), _a(cos), _a(sin),
+                   _a(block_table), block_table.shape[1], _a(kcache), _a(vcache), heads, kv_heads, head_dim, kcache.shape[2],
+                   int(write_kv), _a(self._cut_scratch(x.device) if m > self._split_rows else None), self._stream_handle())
 
     def attention(self, qkv: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor,
                   block_table: torch.Tensor, row_seq: torch.Tensor, pos: torch.Tensor, out: torch.Tensor,
@@ -606,12 +646,11 @@ class KernelOps:
                     self._attn_scratch = torch.empty(floats, dtype=torch.float32, device=qkv.device)
                 scratch, launches = self._attn_scratch, 2
             t_seq, t_row0, t_rows, t_count = tiles if tiles is not None else (None, None, None, 0)
-            self._call("bw_f32_attention", _p(qkv), _c_int(qkv.shape[1]), _p(kcache), _p(vcache), _p(block_table),
-                       _c_int(block_table.shape[1]), _p(row_seq), _p(pos), _p(t_seq), _p(t_row0), _p(t_rows),
-                       _c_int(t_count), _p(batch.seq_pos0) if tiles is not None else None,
-                       _p(batch.seq_row0) if tiles is not None else None, _p(out), _c_int(out.shape[1]), _c_int(n),
-                       _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(page), _c_int(window),
-                       _c_int(max_keys), _c_float(scale), _p(scratch), ctypes.c_longlong(floats), self._stream(),
+            self._call("bw_f32_attention", _a(qkv), qkv.shape[1], _a(kcache), _a(vcache), _a(block_table), block_table.shape[1],
+                       _a(row_seq), _a(pos), _a(t_seq), _a(t_row0), _a(t_rows), t_count,
+                       _a(batch.seq_pos0) if tiles is not None else None, _a(batch.seq_row0) if tiles is not None else None, _a(out),
+                       out.shape[1], n, heads, kv_heads, head_dim, page, window, max_keys, scale, _a(scratch), floats,
+                       self._stream_handle(),
                        launches=launches)
         else:
             if batch is None:
@@ -639,13 +678,10 @@ class KernelOps:
                     q_seq, q_row0, q_rows, q_count = batch.query_tiles(rows_tc)
                     for t_ in (q_seq, q_row0, q_rows):
                         _need(t_, torch.int32, "attention step arrays")
-                    fn = lib.bw_bf16_attention_tc
-                    fn.restype = _c_int
-                    rc = fn(_p(qkv), _c_int(qkv.shape[1]), _p(kcache), _p(vcache), _c_int(kcache.shape[0]),
-                            _p(block_table), _c_int(block_table.shape[1]), _p(q_seq), _p(q_row0), _p(q_rows),
-                            _c_int(q_count), _p(batch.seq_pos0), _p(batch.seq_row0), _p(out), _c_int(out.shape[1]),
-                            _c_int(n), _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(page), _c_int(window),
-                            _c_float(scale), self._stream())
+                    rc = lib.bw_bf16_attention_tc(
+                        _a(qkv), qkv.shape[1], _a(kcache), _a(vcache), kcache.shape[0], _a(block_table), block_table.shape[1], _a(q_seq),
+                        _a(q_row0), _a(q_rows), q_count, _a(batch.seq_pos0), _a(batch.seq_row0), _a(out), out.shape[1], n, heads,
+                        kv_heads, head_dim, page, window, scale, self._stream_handle())
                     if rc != 0:
                         raise KernelError(f"bw_bf16_attention_tc failed ({rc}): "
                                           + lib.bw_last_error().decode("utf-8", "replace"))
@@ -654,26 +690,20 @@ class KernelOps:
             if split:
                 scratch = self._attention_scratch(lib, qkv.device, n, heads, max_keys)
                 # head sizes 64 and 128: the cache arrives as TMA page boxes (same bits)
-                if lib.bw_bf16_attention_stream_usable(_c_int(n), _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(page),
-                                                       _c_int(qkv.shape[1])):
-                    fn = lib.bw_bf16_attention_stream
-                    fn.restype = _c_int
-                    rc = fn(_p(qkv), _c_int(qkv.shape[1]), _p(kcache), _p(vcache), _c_int(kcache.shape[0]),
-                            _p(block_table), _c_int(block_table.shape[1]), _p(row_seq), _p(pos), _p(out),
-                            _c_int(out.shape[1]), _c_int(n), _c_int(heads), _c_int(kv_heads), _c_int(head_dim),
-                            _c_int(page), _c_int(window), _c_float(scale), _c_int(max_keys), _p(scratch), self._stream())
+                if lib.bw_bf16_attention_stream_usable(n, heads, kv_heads, head_dim, page, qkv.shape[1]):
+                    rc = lib.bw_bf16_attention_stream(
+                        _a(qkv), qkv.shape[1], _a(kcache), _a(vcache), kcache.shape[0], _a(block_table), block_table.shape[1],
+                        _a(row_seq), _a(pos), _a(out), out.shape[1], n, heads, kv_heads, head_dim, page, window, scale, max_keys,
+                        _a(scratch), self._stream_handle())
                     if rc != 0:
                         raise KernelError(f"bw_bf16_attention_stream failed ({rc}): "
                                           + lib.bw_last_error().decode("utf-8", "replace"))
                     self.launches += 2
                     return
-            fn = lib.bw_bf16_attention
-            fn.restype = _c_int
-            rc = fn(_p(qkv), _c_int(qkv.shape[1]), _p(kcache), _p(vcache), _p(block_table),
-                    _c_int(block_table.shape[1]), _p(t_seq), _p(t_row0), _p(t_rows), _c_int(t_count),
-                    _p(batch.seq_pos0), _p(batch.seq_row0), _p(row_seq), _p(pos), _p(out), _c_int(out.shape[1]), _c_int(n),
-                    _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(page), _c_int(window), _c_float(scale),
-                    _c_int(max_keys), _p(scratch), self._stream())
+            rc = lib.bw_bf16_attention(
+                _a(qkv), qkv.shape[1], _a(kcache), _a(vcache), _a(block_table), block_table.shape[1], _a(t_seq), _a(t_row0), _a(t_rows),
+                t_count, _a(batch.seq_pos0), _a(batch.seq_row0), _a(row_seq), _a(pos), _a(out), out.shape[1], n, heads, kv_heads,
+                head_dim, page, window, scale, max_keys, _a(scratch), self._stream_handle())
             if rc != 0:
                 raise KernelError(f"bw_bf16_attention failed ({rc}): "
                                   + lib.bw_last_error().decode("utf-8", "replace"))
@@ -773,7 +803,7 @@ class KernelOps:
         _need(out, self.act_dtype, "swiglu out", 2)
         if gate_up.shape[1] != 2 * inter or gate_up.shape[0] != n:
             raise KernelError("swiglu: input is not [rows, 2 * intermediate]")
-        self._call(f"bw_{self.kind}_swiglu", _p(gate_up), _p(out), _c_int(n), _c_int(inter), self._stream())
+        self._call(f"bw_{self.kind}_swiglu", _a(gate_up), _a(out), n, inter, self._stream_handle())
 
     # -- parts that only some architectures have (their library is loaded at first use) ------
     def _parts_lib(self):

@@ -97,11 +97,15 @@ class Workspace:
         self.device = device
         self.max_rows = max_rows
         self._buffers: Dict[str, torch.Tensor] = {}
+        self._views: Dict[tuple, torch.Tensor] = {}  # rows() of fixed buffers as given out before
 
     def rows(self, name: str, n: int, width: int, dtype: torch.dtype, growable: bool = False) -> torch.Tensor:
         """A [n, width] view of the buffer ``name``.  Fixed buffers are allocated
         [max_rows, width] on first use and never move; a ``growable`` one starts small and
         is replaced by a larger one when a step needs more rows (logits of many positions)."""
+        view = self._views.get((name, n, width, dtype))
+        if view is not None and not growable:
+            return view
         key = f"{name}:{width}:{dtype}"
         buf = self._buffers.get(key)
         if n > self.max_rows:
@@ -115,7 +119,12 @@ class Workspace:
                 cap = min(cap, self.max_rows)
             buf = torch.empty((cap, width), dtype=dtype, device=self.device)
             self._buffers[key] = buf
-        return buf[:n]
+        view = buf[:n]
+        if not growable:
+            if len(self._views) >= 512:
+                self._views.clear()
+            self._views[(name, n, width, dtype)] = view
+        return view
 
     def nbytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._buffers.values())

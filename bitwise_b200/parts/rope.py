@@ -97,11 +97,10 @@ class RotaryEncoding(PositionEncoding):
         return self._cos.shape[0]
 
     def rotary_tables(self, device):
-        key = str(device)
-        if key not in self._device_tables:
-            self._device_tables[key] = (torch.from_numpy(self._cos).to(device),
-                                        torch.from_numpy(self._sin).to(device))
-        return self._device_tables[key]
+        got = self._device_tables.get(device)  # (a device or its name)
+        if got is None:
+            got = self._device_tables[device] = (torch.from_numpy(self._cos).to(device), torch.from_numpy(self._sin).to(device))
+        return got
 
 
 class RampScaling:
