@@ -9,13 +9,13 @@
 // before (the accumulator dependency), 3.2 us per chunk however narrow the tile, and the
 // chunk sums of a product that is split over the machine pass through scratch memory and a
 // second kernel. Here a block per SM stays for the whole product and walks output tiles of 8
-// or 16 columns. Four warps share the chunks of 8 columns (warp w takes chunks w, w + 4, ...);
+// or 16 columns. CW warps (2, 4 or 8, by the number of chunks) share the chunks of 8 columns (warp w takes chunks w, w + CW, ...);
 // a work item is (tile, chunk): 8 KB of W per 8 columns, fetched by ONE TMA copy (a box of
 // 8 rows x 8 k-tiles of 64, 128-byte swizzle) into the warp's own ring of buffers, two items
 // ahead of the arithmetic (the first ones before the wait for the kernel before this one:
 // weights do not depend on it). The step's rows of x are loaded once per block and stay in
 // shared memory. An item's 32 k-steps run on mma.sync (m16n8k16: a dependent step every 28
-// cycles, measured; a tile of 16 columns has a second set of four warps for its second half,
+// cycles, measured; a tile of 16 columns has a second set of warps for its second half,
 // so that every warp runs one chain). The chunk sums of a tile meet in shared memory, are
 // added in ascending order and leave as finished outputs. No scratch, no second kernel.
 //
@@ -33,7 +33,6 @@ constexpr int kChunk = 512;            // canonical summation chunk along k (as 
 constexpr int kTileK = 64;             // k-elements of a shared-memory line (128 bytes, swizzled)
 constexpr int kTilesPerChunk = kChunk / kTileK;
 constexpr int kGroupBytes = 8 * kChunk * 2;  // 8 rows x one chunk: [k-tile][row][128 bytes]
-constexpr int kWarps = 4;              // warps per group of 8 columns; chunk c belongs to warp c % kWarps of the group
 constexpr int kStages = 2;             // buffers in a warp's ring of W items
 constexpr int kSmemLimit = 227 * 1024;
 
@@ -83,10 +82,10 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 // q goes to y, k and v go straight into their page of the cache (what rope_cache_bf16_kernel
 // does to a stored product, with its arithmetic: same bits).
 // ROWS16: up to 16 rows (else up to 8: the upper half of the tensor core's 16 rows is zero).
-// NT: groups of 8 output columns per tile (1 or 2), each with kWarps warps of its own.
+// NT: groups of 8 output columns per tile (1 or 2), each with CW warps of its own.
 //
 // Shared memory (1024-byte aligned for the swizzle): the rows of x [chunk][k-tile][R][128 B],
-// the rings [warp][stage][k-tile][8][128 B], the barriers, and the chunk sums of two tiles in
+// the rings [warp that has chunks][stage][k-tile][8][128 B], the barriers, and the chunk sums of two tiles in
 // turn [2][chunk][NT][R][8].
 struct RopeCache {
   const int* pos;            // position of every row
@@ -108,37 +107,38 @@ struct TanhNormOut {
   __nv_bfloat16* out;  // [m][N], or null: no norm
 };
 
-template <int EPI, bool ROWS16, int NT>
-__global__ void __launch_bounds__(NT * kWarps * 32)
+template <int EPI, bool ROWS16, int NT, int CW>
+__global__ void __launch_bounds__(NT * CW * 32)
 linear_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, void* Y,
                    const float* residual, int M, int N, int K, int tiles, RopeCache rc, int* failure, int act, TanhNormOut tn) {
   static_assert(EPI != 3 || NT == 2, "a rotation needs both halves of a head in the tile");
   constexpr int R = ROWS16 ? 16 : 8;
   constexpr int kItemBytes = kGroupBytes;  // what a warp fetches per (tile, chunk): its group's 8 rows
-  constexpr int kThreads = NT * kWarps * 32;
+  constexpr int kThreads = NT * CW * 32;
   constexpr int kXChunkBytes = R * kChunk * 2;
   constexpr int kOutputs = R * NT * 8;                                // outputs of a tile, chunk sums of one chunk
   constexpr int kMine = (kOutputs + kThreads - 1) / kThreads;         // outputs per thread in the epilogue
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = bw::smem_align_1024(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp_all = tid >> 5;
-  const int grp = warp_all / kWarps, warp = warp_all % kWarps;  // group of 8 columns; which chunks of it
+  const int grp = warp_all / CW, warp = warp_all % CW;  // group of 8 columns; which chunks of it
   const int num_chunks = (K + kChunk - 1) / kChunk;
+  const int busy = min(CW, num_chunks);  // warps of a group that have chunks
   unsigned char* xs = smem;
-  unsigned char* ring = xs + num_chunks * kXChunkBytes + warp_all * (kStages * kItemBytes);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(xs + num_chunks * kXChunkBytes + NT * kWarps * kStages * kItemBytes);
-  uint64_t* wbar = bars + warp_all * kStages;            // one barrier per buffer of this warp's ring
-  uint64_t* xbar = bars + NT * kWarps * kStages + warp;  // the chunks of x that this warp works on
-  float* part = reinterpret_cast<float*>(bars + NT * kWarps * kStages + kWarps);
+  unsigned char* ring = xs + num_chunks * kXChunkBytes + (grp * busy + warp) * (kStages * kItemBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(xs + num_chunks * kXChunkBytes + NT * busy * kStages * kItemBytes);
+  uint64_t* wbar = bars + warp_all * kStages;   // one barrier per buffer of this warp's ring
+  uint64_t* xbar = bars + NT * CW * kStages;    // one per chunk of x: a warp begins when the first of its own is there
+  float* part = reinterpret_cast<float*>(xbar + num_chunks + (num_chunks & 1));
 
   if (tid == 0) {
-    for (int i = 0; i < NT * kWarps * kStages + kWarps; ++i) mbar_init(bars + i, 1);
+    for (int i = 0; i < NT * CW * kStages + num_chunks; ++i) mbar_init(bars + i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
 
-  // This warp's items: for tile = blockIdx.x, + gridDim.x, ...: chunks warp, warp + kWarps, ...
-  const int my_chunks = warp < num_chunks ? (num_chunks - warp + kWarps - 1) / kWarps : 0;
+  // This warp's items: for tile = blockIdx.x, + gridDim.x, ...: chunks warp, warp + CW, ...
+  const int my_chunks = warp < num_chunks ? (num_chunks - warp + CW - 1) / CW : 0;
   // Requests item (tile, chunk) into buffer `stage`: one box of this warp's group of 8 rows of W
   // (with interleaved gate/up weights the up rows of 8 outputs lie 64 rows after their gate rows).
   auto request = [&](int tile, int chunk, int stage) {
@@ -163,7 +163,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   int req_tile = blockIdx.x, req_cc = 0;  // next item to request: tile and index among this warp's chunks
   if (my_chunks > 0) {
     for (int s = 0; s < kStages && req_tile < tiles; ++s) {
-      request(req_tile, warp + req_cc * kWarps, s);
+      request(req_tile, warp + req_cc * CW, s);
       if (++req_cc == my_chunks) req_cc = 0, req_tile += gridDim.x;
     }
   }
@@ -171,16 +171,12 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   bw::pdl_wait();
   // x, once per block: the warps of the first group bring the chunks they work on, which are
   // those of their namesakes in the other group too (rows beyond the step's arrive as zeros)
-  if (my_chunks > 0) {
-    if (lane == 0 && grp == 0) {
-      mbar_expect_tx(xbar, static_cast<uint32_t>(my_chunks * kXChunkBytes));
-      for (int cc = 0; cc < my_chunks; ++cc) {
-        const int chunk = warp + cc * kWarps;
-        tma_load_box(xs + chunk * kXChunkBytes, &map_x, 0, chunk * kTilesPerChunk, xbar);
-      }
+  if (lane == 0 && grp == 0)
+    for (int cc = 0; cc < my_chunks; ++cc) {
+      const int chunk = warp + cc * CW;
+      mbar_expect_tx(xbar + chunk, kXChunkBytes);
+      tma_load_box(xs + chunk * kXChunkBytes, &map_x, 0, chunk * kTilesPerChunk, xbar + chunk);
     }
-    mbar_wait(xbar, 0, failure);
-  }
 
   // Shared-memory addresses of this lane's ldmatrix rows. A line of 128 bytes holds 64
   // k-elements of one row; its 16-byte pieces are swizzled with the row's low three bits.
@@ -212,10 +208,11 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
     float* sums = part + flip * num_chunks * kOutputs;
     for (int cc = 0; cc < my_chunks; ++cc, ++used) {
-      const int chunk = warp + cc * kWarps;
+      const int chunk = warp + cc * CW;
       const int stage = used % kStages;
       const uint32_t wb = smem_u32(ring + stage * kItemBytes) + b_off;
       const uint32_t xa = smem_u32(xs + chunk * kXChunkBytes) + a_off;
+      if (used < static_cast<uint32_t>(my_chunks)) mbar_wait(xbar + chunk, 0, failure);  // (the block's first tile)
       mbar_wait(wbar + stage, (used / kStages) & 1, failure);
       const int k_here = min(kChunk, K - chunk * kChunk);
       const int pairs = (k_here / kTileK) * 2;  // pairs of k-steps of 16 (k is a multiple of 64)
@@ -259,7 +256,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       // delivered (the MMAs that consumed them were issued), so the copy may overwrite it.
       __syncwarp();
       if (req_tile < tiles) {
-        request(req_tile, warp + req_cc * kWarps, stage);
+        request(req_tile, warp + req_cc * CW, stage);
         if (++req_cc == my_chunks) req_cc = 0, req_tile += gridDim.x;
       }
       // chunk sums: d[0..1] are columns 2 (lane % 4) + {0, 1} of row lane / 4 of this group,
@@ -372,7 +369,7 @@ bool rows_map(CUtensorMap* map, const void* base, int rows, int k, int box_rows)
 }
 
 struct RowsShape {
-  int nt, rows16, tiles;
+  int nt, cw, rows16, tiles;
   size_t smem;
   unsigned grid;
 };
@@ -388,36 +385,43 @@ int rows_sm_count() {
   return sms;
 }
 
+int g_rows_warps = 0;  // 0: chosen; else the warps that share the chunks, where they fit (tests, measurements)
+
 // How a product of m rows runs here, or false when it has to take another path (more than 16
 // rows, k no multiple of 64, or k so long that the step's rows of x do not fit into shared
-// memory beside the rings).
+// memory beside the rings). As many warps share the chunks as there are, up to eight where their rings fit: a chunk is a chain of
+// 900 cycles. With two chunks that makes blocks of half the size, two on an SM. In a chain of decode steps (one row, us, four warps
+// always and now): SwiGLU of 960 x 5,120 5.0 -> 3.9, 2,560 x 960 3.4 -> 2.9, 960 x 49,152 26 -> 15.8.
 bool rows_shape(int m, int n, int k, bool swiglu, RowsShape* s) {
   if (m < 1 || m > 16 || k < kTileK || k % kTileK || n < 1) return false;
   const long long chunks = (k + kChunk - 1) / kChunk;
   s->rows16 = m > 8;
   const int R = s->rows16 ? 16 : 8;
+  const int want = g_rows_warps ? g_rows_warps : chunks <= 2 ? 2 : chunks <= 4 ? 4 : 8;
   for (int nt = 2; nt >= 1; --nt) {
     if (swiglu && nt != 2) break;
-    const long long smem = 1024 + chunks * R * kChunk * 2 + static_cast<long long>(kWarps) * kStages * nt * kGroupBytes +
-                           (nt * kWarps * kStages + kWarps) * 8 + 2 * chunks * nt * R * 8 * 4;
-    if (smem > kSmemLimit) continue;
-    const long long tiles = swiglu ? n / 16 : (n + nt * 8 - 1) / (nt * 8);
-    if (tiles > 0x7fffffffLL) return false;
-    const long long resident = static_cast<long long>(rows_sm_count()) * (kSmemLimit / smem);
-    s->nt = nt;
-    s->tiles = static_cast<int>(tiles);
-    s->smem = static_cast<size_t>(smem);
-    s->grid = static_cast<unsigned>(tiles < resident ? tiles : resident);
-    return true;
+    for (int cw = want; cw >= 2; cw >>= 1) {
+      const long long busy = chunks < cw ? chunks : cw;
+      const long long smem = 1024 + chunks * R * kChunk * 2 + busy * kStages * nt * kGroupBytes +
+                             (nt * cw * kStages + chunks + 1) * 8 + 2 * chunks * nt * R * 8 * 4;
+      if (smem > kSmemLimit || (cw < 4 && cw < want)) continue;
+      const long long tiles = swiglu ? n / 16 : (n + nt * 8 - 1) / (nt * 8);
+      if (tiles > 0x7fffffffLL) return false;
+      const long long resident = static_cast<long long>(rows_sm_count()) * (kSmemLimit / smem);
+      s->nt = nt, s->cw = cw;
+      s->tiles = static_cast<int>(tiles);
+      s->smem = static_cast<size_t>(smem);
+      s->grid = static_cast<unsigned>(tiles < resident ? tiles : resident);
+      return true;
+    }
   }
   return false;
 }
 
-template <int EPI, bool ROWS16, int NT>
-int launch_rows(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, const float* residual, int m, int n, int k,
-                const RowsShape& s, cudaStream_t stream, const RopeCache& rc = RopeCache{}, int act = 0,
-                const TanhNormOut& tn = TanhNormOut{}) {
-  auto kernel = linear_rows_kernel<EPI, ROWS16, NT>;
+template <int EPI, bool ROWS16, int NT, int CW>
+int launch_rows_cw(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, const float* residual, int m, int n, int k,
+                   const RowsShape& s, cudaStream_t stream, const RopeCache& rc, int act, const TanhNormOut& tn) {
+  auto kernel = linear_rows_kernel<EPI, ROWS16, NT, CW>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
@@ -434,9 +438,17 @@ int launch_rows(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, const f
   }
   int* word = bw::failure_word();
   if (!word) return -1;
-  bw::launch_pdl(kernel, dim3(s.grid), dim3(NT * kWarps * 32), s.smem, stream, map_x, map_w, y, residual, m, n, k, s.tiles, rc,
+  bw::launch_pdl(kernel, dim3(s.grid), dim3(NT * CW * 32), s.smem, stream, map_x, map_w, y, residual, m, n, k, s.tiles, rc,
                  word, act, tn);
   return bw::launch_status();
+}
+
+template <int EPI, bool ROWS16, int NT>
+int launch_rows(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, const float* residual, int m, int n, int k, const RowsShape& s,
+                cudaStream_t stream, const RopeCache& rc = RopeCache{}, int act = 0, const TanhNormOut& tn = TanhNormOut{}) {
+  if (s.cw == 2) return launch_rows_cw<EPI, ROWS16, NT, 2>(x, w, y, residual, m, n, k, s, stream, rc, act, tn);
+  if (s.cw == 4) return launch_rows_cw<EPI, ROWS16, NT, 4>(x, w, y, residual, m, n, k, s, stream, rc, act, tn);
+  return launch_rows_cw<EPI, ROWS16, NT, 8>(x, w, y, residual, m, n, k, s, stream, rc, act, tn);
 }
 
 template <int EPI>
@@ -458,6 +470,12 @@ BW_API int bw_bf16_linear_rows_enable(int on) {
   const int before = g_rows_enabled;
   g_rows_enabled = on ? 1 : 0;
   return before;
+}
+
+// The warps that share the chunks of 8 columns: 0 chosen from the shape, else 2, 4 or 8 where their rings fit. Every choice gives
+// the same bits. For tests and measurements.
+BW_API void bw_bf16_linear_rows_force_warps(int warps) {
+  if (warps == 0 || warps == 2 || warps == 4 || warps == 8) g_rows_warps = warps;
 }
 
 // Whether a product of this shape runs on this path (rows that start on 16 bytes, at most 16

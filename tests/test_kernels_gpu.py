@@ -1328,3 +1328,35 @@ def test_sample_rows_clusters_of_either_size_over_rows_of_any_start(rows, vocab)
             ops.sampler_kernel(before)
         got[kernel] = out.tolist()
     assert got[1] == got[2] and min(got[1]) >= 0
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(960, 64), (168, 512), (1600, 960), (520, 2560), (264, 4160)])
+def test_bf16_products_of_few_rows_by_any_number_of_warps(m, n, k):
+    """Two, four or eight warps share the chunks of a tile (fewer chunks than warps, as many, and more): the bits of the tcgen05 path."""
+    ops = _ops("bfloat16")
+    gen = torch.Generator(device=DEV).manual_seed(m * n + k)
+    x, w = (torch.randn(*s, generator=gen, device=DEV).to(torch.bfloat16) for s in ((m, k), (n, k)))
+    res = torch.randn(m, n, generator=gen, device=DEV)
+    glu = torch.randn(2 * 320, k, generator=gen, device=DEV).to(torch.bfloat16)
+
+    def run():
+        y, z, h = torch.empty(m, n, device=DEV, dtype=torch.bfloat16), res.clone(), torch.empty(m, 320, device=DEV, dtype=torch.bfloat16)
+        ops.linear(x, w, y)
+        ops.linear(x, w, z, residual=z)
+        ops.linear_swiglu(x, glu, h)
+        return y.view(torch.int16), z.view(torch.int32), h.view(torch.int16)
+    before = ops.rows_path(False)
+    try:
+        want = run()
+    finally:
+        ops.rows_path(before)
+    for warps in (0, 2, 4, 8):
+        ops.lib.bw_bf16_linear_rows_force_warps(warps)
+        try:
+            got = run()
+        finally:
+            ops.lib.bw_bf16_linear_rows_force_warps(0)
+        for a, b in zip(got, want):
+            assert torch.equal(a, b), f"{warps} warps"
+    assert not ops.device_failure()
