@@ -336,6 +336,167 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   }
 }
 
+// The same product for an inner size whose rows of x leave no room for the rings (8 rows x 8,192 are 128 KB), EPI 0 and 2. x is not
+// resident: a warp's item (tile of 16 columns, chunk) brings its chunk of x beside its 16 KB of W, and the warp runs the two groups
+// of 8 columns as two chains side by side on the same fragments of x. x then comes from L2 once for every tile, half as many
+// bytes as W for 8 rows, but nothing waits for all of it, and 128 KB of W are in flight where there was room for 64.
+template <bool ROWS16>
+struct LongShape {
+  static constexpr int R = ROWS16 ? 16 : 8, kWarps = ROWS16 ? 3 : 4;
+  static constexpr int kWBytes = 2 * kGroupBytes, kXBytes = R * kChunk * 2, kItemBytes = kWBytes + kXBytes;
+  static constexpr int kRing = kWarps * kStages * kItemBytes, kOutputs = R * 16;
+  static constexpr long long smem(long long chunks) { return 1024 + kRing + kWarps * kStages * 8 + chunks * kOutputs * 4; }
+};
+
+template <int EPI, bool ROWS16>
+__global__ void __launch_bounds__(LongShape<ROWS16>::kWarps * 32)
+linear_long_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, void* Y, const float* residual,
+                   int M, int N, int K, int tiles, int* failure, int act, TanhNormOut tn) {
+  using S = LongShape<ROWS16>;
+  constexpr int R = S::R, kThreads = S::kWarps * 32, kMine = (S::kOutputs + kThreads - 1) / kThreads;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = bw::smem_align_1024(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int num_chunks = (K + kChunk - 1) / kChunk;
+  unsigned char* ring = smem + warp * (kStages * S::kItemBytes);  // a stage: W [k-tile][16][128 B], then x [k-tile][R][128 B]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kRing) + warp * kStages;
+  float* sums = reinterpret_cast<float*>(reinterpret_cast<uint64_t*>(smem + S::kRing) + S::kWarps * kStages);  // [chunk][2][R][8]
+  if (tid == 0) {
+    for (int i = 0; i < S::kWarps * kStages; ++i) mbar_init(reinterpret_cast<uint64_t*>(smem + S::kRing) + i, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const int my_chunks = warp < num_chunks ? (num_chunks - warp + S::kWarps - 1) / S::kWarps : 0;
+  int req_tile = blockIdx.x, req_cc = 0;  // next item to request
+  auto next_item = [&]() {
+    if (++req_cc == my_chunks) req_cc = 0, req_tile += gridDim.x;
+  };
+  auto load_w = [&](int stage) {
+    mbar_expect_tx(bars + stage, S::kItemBytes);
+    tma_load_box(ring + stage * S::kItemBytes, &map_w, req_tile * 16, (warp + req_cc * S::kWarps) * kTilesPerChunk, bars + stage);
+  };
+  auto load_x = [&](int cc, int stage) {
+    tma_load_box(ring + stage * S::kItemBytes + S::kWBytes, &map_x, 0, (warp + cc * S::kWarps) * kTilesPerChunk, bars + stage);
+  };
+  // the weights of the first items at once, their x behind the kernel that writes it
+  int early = 0, early_cc[kStages];
+  if (my_chunks > 0) {
+#pragma unroll
+    for (int s = 0; s < kStages; ++s) {
+      early_cc[s] = 0;
+      if (req_tile >= tiles) continue;
+      if (lane == 0) load_w(s);
+      early_cc[s] = req_cc, early = s + 1;
+      next_item();
+    }
+  }
+  bw::pdl_launch();
+  bw::pdl_wait();
+#pragma unroll
+  for (int s = 0; s < kStages; ++s)
+    if (s < early && lane == 0) load_x(early_cc[s], s);
+
+  // fragments as in linear_rows_kernel
+  const int lrow = lane & 7, lblk = lane >> 3;
+  const uint32_t b_off = lrow * 128;
+  const int arow = ROWS16 ? lrow + ((lane >> 3) & 1) * 8 : lrow;
+  const int ablk = ROWS16 ? (lane >> 4) : lblk;
+  const uint32_t a_off = S::kWBytes + arow * 128;
+  uint32_t used = 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    float res[kMine], nw[kMine], nb[kMine];
+#pragma unroll
+    for (int e = 0; e < kMine; ++e) {
+      res[e] = 0.0f, nw[e] = 0.0f, nb[e] = 0.0f;
+      if (EPI == 2) {
+        const int o = tid + e * kThreads;
+        const int r = o / 16, n = tile * 16 + o % 16;
+        if (o < S::kOutputs && r < M && n < N) {
+          if (residual) res[e] = residual[static_cast<size_t>(r) * N + n];
+          if (tn.out) nw[e] = tn.w[n], nb[e] = tn.b[n];
+        }
+      }
+    }
+    for (int cc = 0; cc < my_chunks; ++cc, ++used) {
+      const int chunk = warp + cc * S::kWarps, stage = used % kStages;
+      const uint32_t at = smem_u32(ring + stage * S::kItemBytes);
+      const uint32_t wb = at + b_off, xa = at + a_off;
+      mbar_wait(bars + stage, (used / kStages) & 1, failure);
+      const int pairs = (min(kChunk, K - chunk * kChunk) / kTileK) * 2;  // pairs of k-steps of 16 (k is a multiple of 64)
+      float d[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+      uint32_t a[2][ROWS16 ? 8 : 4], b[2][2][4];
+      auto fetch = [&](int p, int slot) {
+        const int kt = p >> 1, q0 = (p & 1) * 4;
+        if (ROWS16) {
+          uint32_t lo[4], hi[4];
+          ldmatrix_x4(lo, xa + kt * (R * 128) + (((q0 + ablk) ^ lrow) << 4));
+          ldmatrix_x4(hi, xa + kt * (R * 128) + (((q0 + 2 + ablk) ^ lrow) << 4));
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[slot][e] = lo[e], a[slot][4 + e] = hi[e];
+        } else {
+          uint32_t v[4];
+          ldmatrix_x4(v, xa + kt * (R * 128) + (((q0 + ablk) ^ lrow) << 4));
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[slot][e] = v[e];
+        }
+#pragma unroll
+        for (int g = 0; g < 2; ++g) ldmatrix_x4(b[slot][g], wb + kt * 2048 + g * 1024 + (((q0 + lblk) ^ lrow) << 4));
+      };
+      auto steps = [&](int slot) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            if (ROWS16)
+              mma_bf16(d[g], a[slot][4 * h], a[slot][4 * h + 1], a[slot][4 * h + 2], a[slot][4 * h + 3], b[slot][g][2 * h], b[slot][g][2 * h + 1]);
+            else
+              mma_bf16(d[g], a[slot][2 * h], 0u, a[slot][2 * h + 1], 0u, b[slot][g][2 * h], b[slot][g][2 * h + 1]);
+          }
+      };
+      fetch(0, 0);
+      for (int p = 0; p < pairs; p += 2) {  // pairs is even
+        fetch(p + 1, 1);
+        steps(0);
+        if (p + 2 < pairs) fetch(p + 2, 0);
+        steps(1);
+      }
+      __syncwarp();  // every ldmatrix of this item has delivered: the buffer may be filled again
+      if (req_tile < tiles) {
+        if (lane == 0) {
+          load_w(stage);
+          load_x(req_cc, stage);
+        }
+        next_item();
+      }
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        float* mine = sums + chunk * S::kOutputs + g * (R * 8) + (lane >> 2) * 8 + 2 * (lane & 3);
+        *reinterpret_cast<float2*>(mine) = make_float2(d[g][0], d[g][1]);
+        if (ROWS16) *reinterpret_cast<float2*>(mine + 64) = make_float2(d[g][2], d[g][3]);
+      }
+    }
+    __syncthreads();  // the chunk sums of this tile are complete
+#pragma unroll
+    for (int e = 0; e < kMine; ++e) {
+      const int o = tid + e * kThreads;
+      const int r = o / 16, cj = o % 16, n = tile * 16 + cj;
+      if (o >= S::kOutputs || r >= M || n >= N) continue;
+      const float* p = sums + (cj >> 3) * (R * 8) + r * 8 + (cj & 7);
+      float v = p[0];
+      for (int c = 1; c < num_chunks; ++c) v = v + p[c * S::kOutputs];
+      const size_t to = static_cast<size_t>(r) * N + n;
+      if (EPI == 2) {
+        if (residual) v = res[e] + v;
+        static_cast<float*>(Y)[to] = v;
+        if (tn.out) tn.out[to] = __float2bfloat16_rn(bw::tanh_norm_one(v, tn.alpha[0], nw[e], nb[e]));
+      } else {
+        static_cast<__nv_bfloat16*>(Y)[to] = __float2bfloat16_rn(bw::out_act(v, act));
+      }
+    }
+    __syncthreads();  // and read: the next tile's go over them
+  }
+}
+
 int g_rows_enabled = 1;
 
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -370,6 +531,7 @@ bool rows_map(CUtensorMap* map, const void* base, int rows, int k, int box_rows)
 
 struct RowsShape {
   int nt, cw, rows16, tiles;
+  bool by_chunks;  // x is not resident (linear_long_kernel)
   size_t smem;
   unsigned grid;
 };
@@ -385,11 +547,12 @@ int rows_sm_count() {
   return sms;
 }
 
+int g_rows_long = 0;   // x by chunks: 0 where it is chosen, 1 never, 2 wherever it can (tests, measurements)
 int g_rows_warps = 0;  // 0: chosen; else the warps that share the chunks, where they fit (tests, measurements)
 
 // How a product of m rows runs here, or false when it has to take another path (more than 16
 // rows, k no multiple of 64, or k so long that the step's rows of x do not fit into shared
-// memory beside the rings). As many warps share the chunks as there are, up to eight where their rings fit: a chunk is a chain of
+// memory beside the rings, nor its chunk sums beside those of linear_long_kernel). As many warps share the chunks as there are, up to eight where their rings fit: a chunk is a chain of
 // 900 cycles. With two chunks that makes blocks of half the size, two on an SM. In a chain of decode steps (one row, us, four warps
 // always and now): SwiGLU of 960 x 5,120 5.0 -> 3.9, 2,560 x 960 3.4 -> 2.9, 960 x 49,152 26 -> 15.8.
 bool rows_shape(int m, int n, int k, bool swiglu, RowsShape* s) {
@@ -397,6 +560,21 @@ bool rows_shape(int m, int n, int k, bool swiglu, RowsShape* s) {
   const long long chunks = (k + kChunk - 1) / kChunk;
   s->rows16 = m > 8;
   const int R = s->rows16 ? 16 : 8;
+  s->by_chunks = false;
+  // x by chunks above k 4,096, where the rows of x leave the rings little room or none. Resident (or, where it does not fit, the
+  // tcgen05 path) / by chunks, us: 8 rows x 8,192 x 2,048 10.3 / 8.4; x 5,632 x 2,048 7.1 / 6.5; x 14,336 x 4,096 30.0 / 21.5; 16 rows x
+  // 8,192 x 2,048 12.6 / 9.6; but 8 rows x 4,096 x 4,096 7.6 / 7.6, 16 rows 9.6 / 10.5, one row x 2,560 x 960 3.2 / 3.4, 16 rows x 2,048 x
+  // 49,152 39.8 / 61.0.
+  constexpr int kLongChunks = 9;
+  if (!swiglu && g_rows_long != 1 && (g_rows_long == 2 || chunks >= kLongChunks)) {
+    const long long smem = s->rows16 ? LongShape<true>::smem(chunks) : LongShape<false>::smem(chunks);
+    const long long tiles = (n + 15) / 16;
+    if (smem <= kSmemLimit && tiles <= 0x7fffffffLL) {
+      s->by_chunks = true, s->nt = 2, s->cw = 0, s->tiles = static_cast<int>(tiles), s->smem = static_cast<size_t>(smem);
+      s->grid = static_cast<unsigned>(tiles < rows_sm_count() ? tiles : rows_sm_count());
+      return true;
+    }
+  }
   const int want = g_rows_warps ? g_rows_warps : chunks <= 2 ? 2 : chunks <= 4 ? 4 : 8;
   for (int nt = 2; nt >= 1; --nt) {
     if (swiglu && nt != 2) break;
@@ -451,9 +629,40 @@ int launch_rows(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, const f
   return launch_rows_cw<EPI, ROWS16, NT, 8>(x, w, y, residual, m, n, k, s, stream, rc, act, tn);
 }
 
+template <int EPI, bool ROWS16>
+int launch_long(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, const float* residual, int m, int n, int k, const RowsShape& s,
+                cudaStream_t stream, int act, const TanhNormOut& tn) {
+  static bool configured[64] = {false};  // by device
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  auto kernel = linear_long_kernel<EPI, ROWS16>;
+  if (!configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    if (e != cudaSuccess) {
+      bw::set_error("linear (few rows): cannot raise shared memory: %s", cudaGetErrorString(e));
+      return static_cast<int>(e);
+    }
+    configured[dev] = true;
+  }
+  CUtensorMap map_x, map_w;
+  if (!rows_map(&map_x, x, m, k, LongShape<ROWS16>::R) || !rows_map(&map_w, w, n, k, 16)) {
+    bw::set_error("linear (few rows): cuTensorMapEncodeTiled refused [%d x %d] / [%d x %d]", m, k, n, k);
+    return -1;
+  }
+  int* word = bw::failure_word();
+  if (!word) return -1;
+  bw::launch_pdl(kernel, dim3(s.grid), dim3(LongShape<ROWS16>::kWarps * 32), s.smem, stream, map_x, map_w, y, residual, m, n, k, s.tiles, word,
+                 act, tn);
+  return bw::launch_status();
+}
+
 template <int EPI>
 int launch_rows_epi(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, const float* residual, int m, int n, int k,
                     const RowsShape& s, cudaStream_t stream, int act = 0, const TanhNormOut& tn = TanhNormOut{}) {
+  if constexpr (EPI != 1)
+    if (s.by_chunks)
+      return s.rows16 ? launch_long<EPI, true>(x, w, y, residual, m, n, k, s, stream, act, tn)
+                      : launch_long<EPI, false>(x, w, y, residual, m, n, k, s, stream, act, tn);
   if (s.nt == 2)
     return s.rows16 ? launch_rows<EPI, true, 2>(x, w, y, residual, m, n, k, s, stream, RopeCache{}, act, tn)
                     : launch_rows<EPI, false, 2>(x, w, y, residual, m, n, k, s, stream, RopeCache{}, act, tn);
@@ -478,8 +687,14 @@ BW_API void bw_bf16_linear_rows_force_warps(int warps) {
   if (warps == 0 || warps == 2 || warps == 4 || warps == 8) g_rows_warps = warps;
 }
 
+// x resident or by chunks: 0 chosen from the shape, 1 always resident, 2 by chunks wherever it can. Same bits. For tests and
+// measurements.
+BW_API void bw_bf16_linear_rows_force_long(int how) {
+  if (how >= 0 && how <= 2) g_rows_long = how;
+}
+
 // Whether a product of this shape runs on this path (rows that start on 16 bytes, at most 16
-// rows, k a multiple of 64 and short enough for the step's rows of x to stay in shared memory).
+// rows, k a multiple of 64; gate/up products only with k short enough for the step's rows of x to stay in shared memory).
 BW_API int bw_bf16_linear_rows_usable(const void* x, const void* w, int m, int n, int k, int swiglu) {
   RowsShape s;
   return g_rows_enabled && (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (reinterpret_cast<uintptr_t>(w) % 16 == 0) &&

@@ -1360,3 +1360,38 @@ def test_bf16_products_of_few_rows_by_any_number_of_warps(m, n, k):
         for a, b in zip(got, want):
             assert torch.equal(a, b), f"{warps} warps"
     assert not ops.device_failure()
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(168, 64), (1, 576), (520, 4160), (2400, 8192), (24, 16896)])
+def test_bf16_products_of_few_rows_with_x_by_chunks(m, n, k):
+    """Long inner sizes bring x chunk by chunk (here all sizes, down to one chunk and up to the last that fits): the bits of the tcgen05
+    path, with a residual, an activation, and the norm that follows."""
+    ops = _ops("bfloat16")
+    gen = torch.Generator(device=DEV).manual_seed(m * n + k)
+    x, w = (torch.randn(*s, generator=gen, device=DEV).to(torch.bfloat16) for s in ((m, k), (n, k)))
+    w *= 0.05
+    res, nw, nb = (torch.randn(*s, generator=gen, device=DEV) for s in ((m, n), (n,), (n,)))
+    alpha = torch.full((1,), 0.5, device=DEV)
+
+    def run():
+        y, z, u = torch.empty(m, n, device=DEV, dtype=torch.bfloat16), res.clone(), res.clone()
+        rows = torch.empty(m, n, device=DEV, dtype=torch.bfloat16)
+        ops.linear(x, w, y, activation="relu2")
+        ops.linear(x, w, z, residual=z)
+        ops.linear(x, w, u, residual=u, then=(alpha, nw, nb, rows))
+        return y.view(torch.int16), z.view(torch.int32), u.view(torch.int32), rows.view(torch.int16)
+    before = ops.rows_path(False)
+    try:
+        want = run()
+    finally:
+        ops.rows_path(before)
+    for how in (2, 0):
+        ops.lib.bw_bf16_linear_rows_force_long(how)
+        try:
+            got = run()
+        finally:
+            ops.lib.bw_bf16_linear_rows_force_long(0)
+        for a, b in zip(got, want):
+            assert torch.equal(a, b), f"mode {how}"
+    assert not ops.device_failure()
