@@ -107,10 +107,23 @@ struct TanhNormOut {
   __nv_bfloat16* out;  // [m][N], or null: no norm
 };
 
-template <int EPI, bool ROWS16, int NT, int CW>
+// NORM (up to 8 rows of up to 1,024): x is the float32 stream, and every block forms the normed rows itself, with the arithmetic and
+// the order of rmsnorm_bf16_kernel, whose 256 threads its 128 stand for two by two (same bits). A norm of its own is a
+// kernel whose launch and hand-over take 1.4 us of a chain of decode steps for a row that comes from L2 in the same time
+// as the normed one. Only where a block leaves room for another on its SM: a product's first weights are asked for while the kernel before
+// it still runs, and with blocks that fill an SM and no small kernel between them that ends (tried at width 2,048, a step went
+// from 1.74 to 2.54 ms). A one-row step of the SmolLM2-360M shape: 671 -> 633 us.
+struct NormIn {
+  const float* x;  // [m][K]
+  const float* w;  // [K]
+  float eps;
+};
+constexpr int kNormRows = 8, kNormWidth = 1024, kNormSmem = 100 * 1024;  // (beside a kilobyte of its own)
+
+template <int EPI, bool ROWS16, int NT, int CW, bool NORM = false>
 __global__ void __launch_bounds__(NT * CW * 32)
 linear_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, void* Y,
-                   const float* residual, int M, int N, int K, int tiles, RopeCache rc, int* failure, int act, TanhNormOut tn) {
+                   const float* residual, int M, int N, int K, int tiles, RopeCache rc, int* failure, int act, TanhNormOut tn, NormIn ni) {
   static_assert(EPI != 3 || NT == 2, "a rotation needs both halves of a head in the tile");
   constexpr int R = ROWS16 ? 16 : 8;
   constexpr int kItemBytes = kGroupBytes;  // what a warp fetches per (tile, chunk): its group's 8 rows
@@ -168,10 +181,60 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
   }
   bw::pdl_launch();
-  bw::pdl_wait();
+  if constexpr (NORM) {
+    static_assert(kThreads == 128 && !ROWS16, "a thread stands for two of the norm's 256");
+    constexpr int kEach = kNormWidth / kThreads, kBatch = 4;  // entries of a row per thread, rows at a time
+    __shared__ float red[kBatch][8];
+    float g[kEach];
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) g[q] = tid + q * kThreads < K ? ni.w[tid + q * kThreads] : 0.0f;
+    for (int i = tid; i < num_chunks * kTilesPerChunk * R * 8; i += kThreads)  // 16-byte pieces of rows that the step does not have
+      if ((i >> 3) % R >= M) *reinterpret_cast<uint4*>(xs + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+    bw::pdl_wait();
+    for (int r0 = 0; r0 < M; r0 += kBatch) {
+      float v[kBatch][kEach], acc[kBatch][2];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+        for (int q = 0; q < kEach; ++q)
+          v[b][q] = r0 + b < M && tid + q * kThreads < K ? ni.x[static_cast<size_t>(r0 + b) * K + tid + q * kThreads] : 0.0f;
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        acc[b][0] = acc[b][1] = 0.0f;
+#pragma unroll
+        for (int q = 0; q < kEach; ++q)
+          if (tid + q * kThreads < K) acc[b][q & 1] = __fmaf_rn(v[b][q], v[b][q], acc[b][q & 1]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          acc[b][0] = __fadd_rn(acc[b][0], __shfl_xor_sync(0xffffffffu, acc[b][0], o));
+          acc[b][1] = __fadd_rn(acc[b][1], __shfl_xor_sync(0xffffffffu, acc[b][1], o));
+        }
+        if (lane == 0) red[b][warp_all] = acc[b][0], red[b][warp_all + 4] = acc[b][1];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        if (r0 + b >= M) continue;
+        float ss = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss = __fadd_rn(ss, red[b][i]);
+        const float inv = bw::rms_scale(ss, K, ni.eps);
+#pragma unroll
+        for (int q = 0; q < kEach; ++q) {
+          const int i = tid + q * kThreads, r = r0 + b;
+          if (i < K)
+            *reinterpret_cast<__nv_bfloat16*>(xs + (i >> 6) * (R * 128) + r * 128 + ((((i & 63) >> 3) ^ (r & 7)) << 4) + (i & 7) * 2) =
+                __float2bfloat16_rn(bw::rms_apply(v[b][q], inv, g[q]));
+        }
+      }
+      __syncthreads();  // before the next rows' sums, and before the products read
+    }
+  } else {
+    bw::pdl_wait();
+  }
   // x, once per block: the warps of the first group bring the chunks they work on, which are
   // those of their namesakes in the other group too (rows beyond the step's arrive as zeros)
-  if (lane == 0 && grp == 0)
+  if (!NORM && lane == 0 && grp == 0)
     for (int cc = 0; cc < my_chunks; ++cc) {
       const int chunk = warp + cc * CW;
       mbar_expect_tx(xbar + chunk, kXChunkBytes);
@@ -212,7 +275,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       const int stage = used % kStages;
       const uint32_t wb = smem_u32(ring + stage * kItemBytes) + b_off;
       const uint32_t xa = smem_u32(xs + chunk * kXChunkBytes) + a_off;
-      if (used < static_cast<uint32_t>(my_chunks)) mbar_wait(xbar + chunk, 0, failure);  // (the block's first tile)
+      if (!NORM && used < static_cast<uint32_t>(my_chunks)) mbar_wait(xbar + chunk, 0, failure);  // (the block's first tile)
       mbar_wait(wbar + stage, (used / kStages) & 1, failure);
       const int k_here = min(kChunk, K - chunk * kChunk);
       const int pairs = (k_here / kTileK) * 2;  // pairs of k-steps of 16 (k is a multiple of 64)
@@ -596,13 +659,13 @@ bool rows_shape(int m, int n, int k, bool swiglu, RowsShape* s) {
   return false;
 }
 
-template <int EPI, bool ROWS16, int NT, int CW>
+template <int EPI, bool ROWS16, int NT, int CW, bool NORM = false>
 int launch_rows_cw(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, const float* residual, int m, int n, int k,
-                   const RowsShape& s, cudaStream_t stream, const RopeCache& rc, int act, const TanhNormOut& tn) {
-  auto kernel = linear_rows_kernel<EPI, ROWS16, NT, CW>;
+                   const RowsShape& s, cudaStream_t stream, const RopeCache& rc, int act, const TanhNormOut& tn, const NormIn& ni = NormIn{}) {
+  auto kernel = linear_rows_kernel<EPI, ROWS16, NT, CW, NORM>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NORM ? kNormSmem : kSmemLimit);
     if (e != cudaSuccess) {
       bw::set_error("linear (few rows): cannot raise shared memory: %s", cudaGetErrorString(e));
       return static_cast<int>(e);
@@ -610,14 +673,15 @@ int launch_rows_cw(const __nv_bfloat16* x, const __nv_bfloat16* w, void* y, cons
     configured = true;
   }
   CUtensorMap map_x, map_w;
-  if (!rows_map(&map_x, x, m, k, ROWS16 ? 16 : 8) || !rows_map(&map_w, w, n, k, 8)) {
+  if (!rows_map(&map_w, w, n, k, 8) || !(NORM || rows_map(&map_x, x, m, k, ROWS16 ? 16 : 8))) {
     bw::set_error("linear (few rows): cuTensorMapEncodeTiled refused [%d x %d] / [%d x %d]", m, k, n, k);
     return -1;
   }
+  if (NORM) map_x = map_w;  // (not used)
   int* word = bw::failure_word();
   if (!word) return -1;
   bw::launch_pdl(kernel, dim3(s.grid), dim3(NT * CW * 32), s.smem, stream, map_x, map_w, y, residual, m, n, k, s.tiles, rc,
-                 word, act, tn);
+                 word, act, tn, ni);
   return bw::launch_status();
 }
 
@@ -747,6 +811,40 @@ BW_API int bw_bf16_linear_rows_rope_usable(const void* x, const void* w, int m, 
   return g_rows_enabled && hd >= 16 && hd % 16 == 0 && heads > 0 && kv_heads > 0 && n == (heads + 2 * kv_heads) * hd &&
          (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (reinterpret_cast<uintptr_t>(w) % 16 == 0) &&
          rows_shape(m, n, k, true, &s) && rows_encoder() != nullptr;
+}
+
+// Whether a product with weights that take this path's TMA copies (w null: any) and n outputs of `width` forms the RMSNorm of the
+// stream's m rows itself (bw_bf16_linear_rows_norm_rope, where bw_bf16_linear_rows_rope_usable holds too, and
+// bw_bf16_linear_rows_norm_swiglu).
+BW_API int bw_bf16_linear_rows_norm_usable(const void* w, int m, int n, int width) {
+  RowsShape s;
+  return g_rows_enabled && m > 0 && m <= kNormRows && width <= kNormWidth && n % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
+         rows_shape(m, n, width, true, &s) && s.cw == 2 && s.smem <= kNormSmem && rows_encoder() != nullptr;
+}
+BW_API int bw_bf16_linear_rows_norm_rope(const float* x, const float* norm, float eps, const __nv_bfloat16* w, __nv_bfloat16* qkv, int m, int n,
+                                         int k, const int* pos, const int* row_seq, const float* cos_t, const float* sin_t,
+                                         const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache, int heads,
+                                         int kv_heads, int hd, int page, int write_kv, cudaStream_t stream) {
+  if (m <= 0 || n <= 0) return 0;
+  RowsShape s;
+  if (!bw_bf16_linear_rows_norm_usable(w, m, n, k) || !bw_bf16_linear_rows_rope_usable(nullptr, w, m, n, k, heads, kv_heads, hd) ||
+      !rows_shape(m, n, k, true, &s) || page <= 0) {
+    bw::set_error("linear with norm and rotation (few rows): shape [%d x %d] x [%d x %d], %d/%d heads of %d is not for this path", m, k, n,
+                  k, heads, kv_heads, hd);
+    return -1;
+  }
+  const RopeCache rc{pos, row_seq, cos_t, sin_t, block_table, max_blocks, kcache, vcache, heads, kv_heads, hd, page, write_kv};
+  return launch_rows_cw<3, false, 2, 2, true>(nullptr, w, qkv, nullptr, m, n, k, s, stream, rc, 0, TanhNormOut{}, NormIn{x, norm, eps});
+}
+BW_API int bw_bf16_linear_rows_norm_swiglu(const float* x, const float* norm, float eps, const __nv_bfloat16* w, __nv_bfloat16* h, int m, int n,
+                                           int k, int act, cudaStream_t stream) {
+  if (m <= 0 || n <= 0) return 0;
+  RowsShape s;
+  if (n % 128 || !bw_bf16_linear_rows_norm_usable(w, m, n, k) || !rows_shape(m, n, k, true, &s) || (act != bw::kGluSilu && act != bw::kGluGeluTanh)) {
+    bw::set_error("linear with norm and SwiGLU (few rows): shape [%d x %d] x [%d x %d] is not for this path", m, k, n, k);
+    return -1;
+  }
+  return launch_rows_cw<1, false, 2, 2, true>(nullptr, w, h, nullptr, m, n, k, s, stream, RopeCache{}, act, TanhNormOut{}, NormIn{x, norm, eps});
 }
 
 // qkv = x W^T for the fused q/k/v weights, then what bw_bf16_rope_cache does to it, in the same

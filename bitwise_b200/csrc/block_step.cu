@@ -24,6 +24,13 @@ BW_API int bw_bf16_linear_rows_rope(const __nv_bfloat16* x, const __nv_bfloat16*
                                     const int* pos, const int* row_seq, const float* cos_t, const float* sin_t,
                                     const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache, int heads,
                                     int kv_heads, int hd, int page, int write_kv, float* partials, cudaStream_t stream);
+BW_API int bw_bf16_linear_rows_norm_usable(const void* w, int m, int n, int width);
+BW_API int bw_bf16_linear_rows_norm_rope(const float* x, const float* norm, float eps, const __nv_bfloat16* w, __nv_bfloat16* qkv, int m, int n,
+                                         int k, const int* pos, const int* row_seq, const float* cos_t, const float* sin_t,
+                                         const int* block_table, int max_blocks, __nv_bfloat16* kcache, __nv_bfloat16* vcache, int heads,
+                                         int kv_heads, int hd, int page, int write_kv, cudaStream_t stream);
+BW_API int bw_bf16_linear_rows_norm_swiglu(const float* x, const float* norm, float eps, const __nv_bfloat16* w, __nv_bfloat16* h, int m, int n,
+                                           int k, int act, cudaStream_t stream);
 
 namespace {
 
@@ -89,8 +96,15 @@ BW_API int bw_bf16_block(void* call, float eps1, float eps2, float scale, cudaSt
   c.launches += (KERNELS_)
   auto kernels = [&](int m, int out, int in, int swiglu) { return bw_bf16_linear_tc_kernels(m, out, in, swiglu, scratch && partials != nullptr); };
 
-  BW_DO(1, bw_bf16_rmsnorm(c.x, c.norm1, c.normed, nullptr, n, width, eps1, stream));
-  if (bw_bf16_linear_rows_rope_usable(nullptr, nullptr, n, qkv_dim, width, heads, kv_heads, hd)) {
+  const bool rotates = bw_bf16_linear_rows_rope_usable(nullptr, nullptr, n, qkv_dim, width, heads, kv_heads, hd) != 0;
+  const bool norm1_rides = rotates && bw_bf16_linear_rows_norm_usable(c.w_qkv, n, qkv_dim, width);
+  if (!norm1_rides) {
+    BW_DO(1, bw_bf16_rmsnorm(c.x, c.norm1, c.normed, nullptr, n, width, eps1, stream));
+  }
+  if (norm1_rides) {
+    BW_DO(1, bw_bf16_linear_rows_norm_rope(c.x, c.norm1, eps1, c.w_qkv, c.qkv, n, qkv_dim, width, c.pos, c.row_seq, c.cos_t, c.sin_t,
+                                           c.block_table, max_blocks, c.k, c.v, heads, kv_heads, hd, page, writable, stream));
+  } else if (rotates) {
     BW_DO(1, bw_bf16_linear_rows_rope(c.normed, c.w_qkv, c.qkv, n, qkv_dim, width, c.pos, c.row_seq, c.cos_t, c.sin_t, c.block_table,
                                       max_blocks, c.k, c.v, heads, kv_heads, hd, page, writable, partials, stream));
   } else {
@@ -119,8 +133,13 @@ BW_API int bw_bf16_block(void* call, float eps1, float eps2, float scale, cudaSt
   c.attention_failed = 0;
 
   BW_DO(kernels(n, width, q_dim, 0), bw_bf16_linear(c.attn, c.w_o, c.x, 1, c.x, n, width, q_dim, partials, counters, 0, stream));
-  BW_DO(1, bw_bf16_rmsnorm(c.x, c.norm2, c.normed, nullptr, n, width, eps2, stream));
-  if (c.fused_glu) {
+  const bool norm2_rides = c.fused_glu && bw_bf16_linear_rows_norm_usable(c.w_gate_up, n, 2 * inter, width);
+  if (!norm2_rides) {
+    BW_DO(1, bw_bf16_rmsnorm(c.x, c.norm2, c.normed, nullptr, n, width, eps2, stream));
+  }
+  if (norm2_rides) {
+    BW_DO(1, bw_bf16_linear_rows_norm_swiglu(c.x, c.norm2, eps2, c.w_gate_up, c.h, n, 2 * inter, width, bw::kGluSilu, stream));
+  } else if (c.fused_glu) {
     BW_DO(kernels(n, 2 * inter, width, 1),
           bw_bf16_linear_tc_swiglu(c.normed, c.w_gate_up, c.h, n, 2 * inter, width, partials, bw::kGluSilu, stream));
   } else {

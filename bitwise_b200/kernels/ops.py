@@ -52,6 +52,8 @@ _SIGNATURES = {
     "bw_bf16_attention_tc": "p i pp i p i ppp i pp p iiiiiii f p",
     "bw_bf16_attention_stream": "p i pp i p i pp p iiiiiii f i pp",
     "bw_bf16_attention_stream_usable": "iiiiii",
+    "bw_bf16_linear_rows_norm_rope": "pp f pp iii ppppp i pp iiiii p",
+    "bw_bf16_linear_rows_norm_swiglu": "pp f pp iii i p",
     "bw_f32_linear": "pppp iii p",
     "bw_f32_attention": "p i ppp i pp ppp i pp p iiiiiiii f p q p",
     "bw_sample_rows": "p ii ppp p",
@@ -582,6 +584,37 @@ class KernelOps:
             self._kernel_counts[key] = c
         return bool(c)
 
+    def fuses_norm(self, m: int, width: int, w: torch.Tensor) -> bool:
+        """Whether the product of an RMSNorm's m rows with ``w`` ([outputs, width]) forms the norm itself: few rows of a
+        small width on the serving precision (``norm_linear_rope_cache`` where ``fuses_rope`` says so too, ``norm_linear_swiglu``)."""
+        return self.kind == "bf16" and bool(self.lib.bw_bf16_linear_rows_norm_usable(_p(w), _c_int(m), _c_int(w.shape[0]), _c_int(width)))
+
+    def _need_norm(self, x: torch.Tensor, weight: torch.Tensor, k: int, what: str) -> None:
+        _need(x, torch.float32, f"{what} x", 2)
+        _need(weight, torch.float32, f"{what} norm weight", 1)
+        if x.shape[1] != k or weight.shape[0] != k:
+            raise KernelError(f"{what}: widths differ")
+
+    def norm_linear_swiglu(self, x: torch.Tensor, norm_weight: torch.Tensor, eps: float, w_interleaved: torch.Tensor,
+                           out: torch.Tensor) -> None:
+        """``rmsnorm(x, norm_weight, eps)`` followed by ``linear_swiglu``, in one kernel; only where ``fuses_norm`` says so."""
+        n, k = w_interleaved.shape
+        m = x.shape[0]
+        self._need_norm(x, norm_weight, k, "norm_linear_swiglu")
+        _need(w_interleaved, self.act_dtype, "norm_linear_swiglu w", 2)
+        _need(out, self.act_dtype, "norm_linear_swiglu out", 2)
+        if self.kind != "bf16" or n % 128 or tuple(out.shape) != (m, n // 2):
+            raise KernelError("norm_linear_swiglu: unsupported shapes or precision")
+        self._call("bw_bf16_linear_rows_norm_swiglu", _a(x), _a(norm_weight), eps, _a(w_interleaved), _a(out), m, n, k, 0,
+                   self._stream_handle())
+
+    def norm_linear_rope_cache(self, x: torch.Tensor, norm_weight: torch.Tensor, eps: float, w_qkv: torch.Tensor, qkv: torch.Tensor,
+                               *args, write_kv: bool = True) -> None:
+        """``rmsnorm(x, norm_weight, eps)`` followed by ``linear_rope_cache`` (whose arguments follow), in one kernel; only where
+        ``fuses_rope`` and ``fuses_norm`` say so."""
+        self._need_norm(x, norm_weight, w_qkv.shape[1], "norm_linear_rope_cache")
+        self._rope_product((x, norm_weight, eps), w_qkv, qkv, *args, write_kv)
+
     def linear_rope_cache(self, x: torch.Tensor, w_qkv: torch.Tensor, qkv: torch.Tensor, pos: torch.Tensor,
                           row_seq: torch.Tensor, cos: Optional[torch.Tensor], sin: Optional[torch.Tensor],
                           block_table: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, heads: int,
@@ -590,9 +623,14 @@ class KernelOps:
         rotated q lands in qkv's first heads * head_dim columns, the rotated k and v in their
         pages; the k and v columns of qkv are NOT written.  Same bits as the two calls.  Only
         where ``fuses_rope`` says so."""
+        _need(x, self.act_dtype, "linear_rope_cache x", 2)
+        self._rope_product((x,), w_qkv, qkv, pos, row_seq, cos, sin, block_table, kcache, vcache, heads, kv_heads, head_dim, write_kv)
+
+    def _rope_product(self, rows: tuple, w_qkv, qkv, pos, row_seq, cos, sin, block_table, kcache, vcache, heads, kv_heads, head_dim,
+                      write_kv) -> None:
+        x = rows[0]
         m, k = x.shape
         n = w_qkv.shape[0]
-        _need(x, self.act_dtype, "linear_rope_cache x", 2)
         _need(w_qkv, self.act_dtype, "linear_rope_cache w", 2)
         _need(qkv, self.act_dtype, "linear_rope_cache qkv", 2)
         _need(pos, torch.int32, "linear_rope_cache pos")
@@ -609,9 +647,12 @@ class KernelOps:
             _need(sin, torch.float32, "linear_rope_cache sin", 2)
             if cos.shape[1] != head_dim // 2 or cos.shape != sin.shape:
                 raise KernelError("linear_rope_cache: table width is not head_dim / 2")
-        self._call("bw_bf16_linear_rows_rope", _a(x), _a(w_qkv), _a(qkv), m, n, k, _a(pos), _a(row_seq), _a(cos), _a(sin),
-                   _a(block_table), block_table.shape[1], _a(kcache), _a(vcache), heads, kv_heads, head_dim, kcache.shape[2],
-                   int(write_kv), _a(self._cut_scratch(x.device) if m > self._split_rows else None), self._stream_handle())
+        rest = (_a(w_qkv), _a(qkv), m, n, k, _a(pos), _a(row_seq), _a(cos), _a(sin), _a(block_table), block_table.shape[1], _a(kcache),
+                _a(vcache), heads, kv_heads, head_dim, kcache.shape[2], int(write_kv))
+        if len(rows) == 3:
+            self._call("bw_bf16_linear_rows_norm_rope", _a(x), _a(rows[1]), rows[2], *rest, self._stream_handle())
+            return
+        self._call("bw_bf16_linear_rows_rope", _a(x), *rest, _a(self._cut_scratch(x.device) if m > self._split_rows else None), self._stream_handle())
 
     def attention(self, qkv: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor,
                   block_table: torch.Tensor, row_seq: torch.Tensor, pos: torch.Tensor, out: torch.Tensor,

@@ -67,13 +67,24 @@ class GQAAttention(Mixer):
     def param_bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in (self.w_qkv, self.w_o))
 
-    def forward(self, ctx: StepContext, xn: torch.Tensor, x: torch.Tensor, cache: PagedKVView) -> None:
+    def takes_norm(self, ctx: StepContext) -> bool:
+        """Whether this step's q/k/v product forms the RMSNorm before it itself (then ``forward`` is given that norm)."""
+        ops = ctx.ops
+        fuses = getattr(ops, "fuses_norm", None)
+        return bool(fuses and ops.fuses_rope(ctx.n, self.width, self.heads, self.kv_heads, self.head_dim)
+                    and fuses(ctx.n, self.width, self.w_qkv))
+
+    def forward(self, ctx: StepContext, xn: torch.Tensor, x: torch.Tensor, cache: PagedKVView, norm=None) -> None:
+        """``norm``: an RMSNorm of ``x`` to be formed here (where ``takes_norm`` says so); ``xn`` is not read then."""
         ops, n = ctx.ops, ctx.n
         qkv = ctx.workspace.rows("qkv", n, self.q_dim + 2 * self.kv_dim, ctx.act_dtype)
         tables = self.position.rotary_tables(x.device) if self.position is not None else None
         cos, sin = tables if tables is not None else (None, None)
         fuses = getattr(ops, "fuses_rope", None)
-        if fuses and fuses(n, self.width, self.heads, self.kv_heads, self.head_dim):
+        if norm is not None:
+            ops.norm_linear_rope_cache(x, norm.weight, norm.eps, self.w_qkv, qkv, ctx.pos, ctx.row_seq, cos, sin, cache.block_table, cache.k,
+                                       cache.v, self.heads, self.kv_heads, self.head_dim, write_kv=cache.writable)
+        elif fuses and fuses(n, self.width, self.heads, self.kv_heads, self.head_dim):
             # the projection rotates and stores its outputs itself
             ops.linear_rope_cache(xn, self.w_qkv, qkv, ctx.pos, ctx.row_seq, cos, sin, cache.block_table, cache.k,
                                   cache.v, self.heads, self.kv_heads, self.head_dim, write_kv=cache.writable)

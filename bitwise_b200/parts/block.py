@@ -69,6 +69,15 @@ class PreNormBlock(Part):
         if self._in_one_call(ctx, x, cache):
             return
         xn = ctx.workspace.rows("normed", ctx.n, self.width, ctx.act_dtype)
+        if self._plain() and not self.opened and self.next_norm is None:
+            # a product of few rows of a small width forms the norm before it itself
+            for norm, part, rest in ((self.mixer_norm, self.mixer, (cache,)), (self.ffn_norm, self.feed_forward, ())):
+                if part.takes_norm(ctx):
+                    part.forward(ctx, xn, x, *rest, norm=norm)
+                else:
+                    norm.forward(ctx, x, xn)
+                    part.forward(ctx, xn, x, *rest)
+            return
         if not self.opened:
             self.mixer_norm.forward(ctx, x, xn)
         last = {"then": self.next_norm.after(xn)} if self.next_norm is not None else {}
@@ -83,15 +92,17 @@ class PreNormBlock(Part):
         self.feed_forward.forward(ctx, xn, x, **last)
 
 
+    def _plain(self) -> bool:
+        return (_is_plain(self.mixer, GQAAttention) and _is_plain(self.feed_forward, SwiGLU) and _is_plain(self.mixer_norm, RMSNorm)
+                and _is_plain(self.ffn_norm, RMSNorm))
+
     def _in_one_call(self, ctx: StepContext, x: torch.Tensor, cache) -> bool:
         """The plain arrangement of exactly these parts goes to the kernel library as one call, where the library offers it
         and takes the sizes: the launches are those that the parts make below."""
         call = getattr(ctx.ops, "prenorm_block", None)
         if call is None or self.opened or self.next_norm is not None or type(cache) is not PagedKVView:
             return False
-        if not (_is_plain(self.mixer, GQAAttention) and _is_plain(self.feed_forward, SwiGLU) and self.feed_forward.activation == "silu"):
-            return False
-        if not (_is_plain(self.mixer_norm, RMSNorm) and _is_plain(self.ffn_norm, RMSNorm)):
+        if not (self._plain() and self.feed_forward.activation == "silu"):
             return False
         return call(ctx, x, cache, (self.mixer_norm, self.mixer, self.ffn_norm, self.feed_forward))
 

@@ -62,13 +62,20 @@ class SwiGLU(FeedForward):
         # (only an activation other than SiLU is named to the kernels' bindings)
         return {} if self.activation == "silu" else {"activation": self.activation}
 
+    def takes_norm(self, ctx: StepContext) -> bool:
+        """Whether this step's gate/up product forms the RMSNorm before it itself (then ``forward`` is given that norm)."""
+        fuses = getattr(ctx.ops, "fuses_norm", None)
+        return bool(fuses and self.fused and self.activation == "silu" and fuses(ctx.n, self.width, self.w_gate_up))
+
     def forward(self, ctx: StepContext, xn: torch.Tensor, x: torch.Tensor, accumulate: bool = True,
-                then: Optional[tuple] = None) -> None:
-        """``accumulate`` False: the output is written to ``x`` (float32) instead of added to it.  ``then``: the norm that
+                then: Optional[tuple] = None, norm=None) -> None:
+        """``norm``: an RMSNorm of ``x`` to be formed here (where ``takes_norm`` says so); ``xn`` is not read then.  ``accumulate`` False: the output is written to ``x`` (float32) instead of added to it.  ``then``: the norm that
         follows on the finished rows (``TanhNorm.after``)."""
         ops, n = ctx.ops, ctx.n
         h = ctx.workspace.rows("ffn_h", n, self.intermediate, ctx.act_dtype)
-        if self.fused:
+        if norm is not None:
+            ops.norm_linear_swiglu(x, norm.weight, norm.eps, self.w_gate_up, h)
+        elif self.fused:
             ops.linear_swiglu(xn, self.w_gate_up, h, **self._act)
         else:
             gate_up = ctx.workspace.rows("gate_up", n, 2 * self.intermediate, ctx.act_dtype)

@@ -1395,3 +1395,38 @@ def test_bf16_products_of_few_rows_with_x_by_chunks(m, n, k):
         for a, b in zip(got, want):
             assert torch.equal(a, b), f"mode {how}"
     assert not ops.device_failure()
+
+
+@pytest.mark.parametrize("m", [1, 3, 4, 5, 8])
+@pytest.mark.parametrize("width,heads,kv_heads,hd,inter", [(64, 2, 1, 64, 64), (576, 9, 3, 64, 1536), (960, 15, 5, 64, 2560), (1024, 8, 2, 128, 448)])
+def test_bf16_products_of_few_rows_that_form_the_norm_before_them(m, width, heads, kv_heads, hd, inter):
+    """The q/k/v product with rotation and the gate/up product with SwiGLU from the float32 stream: the bits of the norm and the
+    product one after the other."""
+    ops = _ops("bfloat16")
+    from bitwise_b200.parts.rope import RotaryEncoding
+    gen = torch.Generator(device=DEV).manual_seed(m * width)
+    b16, n, page = torch.bfloat16, (heads + 2 * kv_heads) * hd, 16
+    draw = lambda *shape, dtype=torch.float32: torch.randn(*shape, generator=gen, device=DEV).to(dtype)
+    x, nw = draw(m, width) * 3, draw(width)
+    w, gu = draw(n, width, dtype=b16), draw(2 * inter, width, dtype=b16)
+    assert ops.fuses_norm(m, width, w) and ops.fuses_norm(m, width, gu) and ops.fuses_rope(m, width, heads, kv_heads, hd)
+    assert not ops.fuses_norm(9, width, w)
+    cos, sin = RotaryEncoding(hd, 10000.0, None, positions=64).rotary_tables(torch.device(DEV))
+    pos = torch.arange(5, 5 + 3 * m, 3, dtype=torch.int32, device=DEV)
+    seq, table = torch.zeros(m, dtype=torch.int32, device=DEV), torch.arange(4, dtype=torch.int32, device=DEV).view(1, -1)
+    outs = []
+    for rides in (False, True):
+        k, v = (torch.zeros(4, kv_heads, page, hd, device=DEV, dtype=b16) for _ in range(2))
+        qkv, h, xn = torch.zeros(m, n, device=DEV, dtype=b16), torch.zeros(m, inter, device=DEV, dtype=b16), torch.empty(m, width, device=DEV, dtype=b16)
+        args = (qkv, pos, seq, cos, sin, table, k, v, heads, kv_heads, hd)
+        if rides:
+            ops.norm_linear_rope_cache(x, nw, 1e-5, w, *args)
+            ops.norm_linear_swiglu(x, nw, 1e-5, gu, h)
+        else:
+            ops.rmsnorm(x, nw, 1e-5, xn)
+            ops.linear_rope_cache(xn, w, *args)
+            ops.linear_swiglu(xn, gu, h)
+        outs.append((qkv, k, v, h))
+    for a, b in zip(*outs):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    assert not ops.device_failure()
